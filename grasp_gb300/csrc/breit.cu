@@ -9,10 +9,12 @@
 // stride-4 Newton-Cotes chain), the frequency-dependent terms weighted by
 // spherical Bessel factors (bessel.f90). On the device:
 //
-//  0. k_plan_table / k_plan_items: the integrals and their terms. A table
-//     row (k, a, b) holds the (c, d) whose TRIANGBREIT pair masks share a
-//     bit, in the reference's order; one pass counts each row's integrals
-//     and terms, the host scans the counts, a second pass writes them.
+//  The tables are dot products of pair densities with one vector per (pair,
+//  k): run_table and the k_br_* kernels. A list (gg_brintf), and the entries
+//  of a table that the contraction cannot take, go term by term:
+//
+//  0. k_plan_items: the integrals' terms; one pass counts them, the host scans
+//     the counts, a second pass writes them.
 //  1. k_bessel: every Bessel function the integrals need, (pair, order) with
 //     W = WFACT |E(a) - E(b)| / C, one block each: the series where it
 //     converges in four terms, the asymptotic form from the first point where
@@ -229,16 +231,21 @@ __device__ __forceinline__ double prod(const double *PF, const double *QF, int l
   return v;
 }
 
-__global__ void __launch_bounds__(128) k_breit_jobs(const BrJob *__restrict__ jobs, int64_t njobs,
-                                                    const double *__restrict__ PF, const double *__restrict__ QF,
-                                                    int ld, const int *__restrict__ MF, const double *__restrict__ R,
-                                                    const double *__restrict__ RP, const double *__restrict__ RPOR,
-                                                    const double *__restrict__ Pow, int np, QuadConst q,
-                                                    const double *__restrict__ BJt, const double *__restrict__ BNt,
-                                                    double *__restrict__ out) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= njobs) return;
-  const BrJob jb = jobs[t];
+// the grid, orbitals and Bessel tables a term reads
+struct TermTabs {
+  const double *PF, *QF;
+  int ld;
+  const int *MF;
+  const double *R, *RP, *RPOR, *Pow;
+  int np;
+  const double *BJ, *BN;
+};
+
+__device__ double breit_term(const BrJob &jb, const TermTabs &tt, const QuadConst &q) {
+  const double *PF = tt.PF, *QF = tt.QF, *R = tt.R, *RP = tt.RP, *RPOR = tt.RPOR, *Pow = tt.Pow;
+  const double *BJt = tt.BJ, *BNt = tt.BN;
+  const int *MF = tt.MF;
+  const int ld = tt.ld, np = tt.np;
   const int form = jb.form, K = jb.k;
   const bool saug = jb.flags & 1, paug = jb.flags & 2;
   const int mtpz = min(MF[jb.sx], MF[jb.sy]);
@@ -345,7 +352,15 @@ __global__ void __launch_bounds__(128) k_breit_jobs(const BrJob *__restrict__ jo
       ta = part * (1.0 + bn) * ZA * R[i] * RP[i];
     Q.push(i, ta, R, RP, q);
   }
-  out[t] = Q.finish(q);
+  return Q.finish(q);
+}
+
+__global__ void __launch_bounds__(128) k_breit_jobs(const BrJob *__restrict__ jobs, int64_t njobs, TermTabs tt,
+                                                    QuadConst q, double *__restrict__ out) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= njobs) return;
+  const BrJob jb = jobs[t];
+  out[t] = breit_term(jb, tt, q);
 }
 
 // One integral: its first term, the combination (code) and SKINT's data.
@@ -518,42 +533,6 @@ __device__ int plan_one(int type, int a, int b, int c, int d, int K, const PlanT
   return n;
 }
 
-// a table row: the (c, d) that TRIANGBREIT admits with (k, a, b) (pair
-// masks share a bit), in the reference's order; pass 0 counts integrals and
-// terms, pass 1 writes them from the scanned offsets
-__global__ void k_plan_table(int type, int nw, int kmax, const unsigned char *__restrict__ mask, PlanTabs T,
-                             int pass, int *__restrict__ cnt_i, int *__restrict__ cnt_j,
-                             const int64_t *__restrict__ off_i, const int64_t *__restrict__ off_j,
-                             int32_t *__restrict__ ind, BrInt *__restrict__ ints, BrJob *__restrict__ jobs) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (kmax + 1) * nw * nw) return;
-  const int K = t / (nw * nw), a = (t / nw) % nw + 1, b = t % nw + 1;
-  const int KEY = nw + 1;
-  const unsigned char *mk = mask + (size_t)K * (nw + 1) * (nw + 1);
-  const unsigned char mab = mk[a * (nw + 1) + b];
-  int ni = 0, nj = 0;
-  if (mab) {
-    int64_t pi = pass ? off_i[t] : 0, pj = pass ? off_j[t] : 0;
-    for (int c = 1; c <= nw; ++c)
-      for (int d = 1; d <= nw; ++d)
-        if (mab & mk[c * (nw + 1) + d]) {
-          if (pass) {
-            ind[pi] = ((a * KEY + b) * KEY + c) * KEY + d;
-            const int q = plan_one(type, a, b, c, d, K, T, (int)pj, ints + pi, jobs + pj);
-            ++pi;
-            pj += q;
-          } else {
-            ++ni;
-            nj += plan_one(type, a, b, c, d, K, T, 0, nullptr, nullptr);
-          }
-        }
-  }
-  if (!pass) {
-    cnt_i[t] = ni;
-    cnt_j[t] = nj;
-  }
-}
-
 // a list of integrals (items[6 t ..] = type, a, b, c, d, k)
 __global__ void k_plan_items(const int32_t *__restrict__ items, int n, PlanTabs T, int pass, int *__restrict__ cnt_j,
                              const int64_t *__restrict__ off_j, BrInt *__restrict__ ints, BrJob *__restrict__ jobs) {
@@ -564,6 +543,607 @@ __global__ void k_plan_items(const int32_t *__restrict__ items, int n, PlanTabs 
     plan_one(it[0], it[1], it[2], it[3], it[4], it[5], T, (int)off_j[t], ints + t, jobs + off_j[t]);
   else
     cnt_j[t] = plan_one(it[0], it[1], it[2], it[3], it[4], it[5], T, 0, nullptr, nullptr);
+}
+
+// ---------------------------------------------------------------------------
+// The tables by contraction. For one k, a term is linear in its source pair's
+// density and in its partner pair's: with pair s the source and pair p the
+// part, TA(i) = rho_p(i) q(i) Z(i), Z the stride-4 chain of e(j) rho_s(j),
+//   sum_i w_i TA(i) = rho_p . F_s   (the frequency is s's: F_s = q Z[e rho_s])
+//                   = rho_s . U_p   (the frequency is p's: U_p = e A[w q rho_p],
+//                                    A the transposed chain, run backwards),
+// so every integral of a table is a dot product of a pair density with one
+// vector per (pair, k), where the term list ran a chain per term: 131 ms of
+// FP64 pipe for the 1.16 M type-1 integrals of 34 subshells, against 1.8 ms
+// for all the kernels below (same table), 5.1 ms against 0.40 ms for the 26 K
+// type-2 integrals of 16. Bound: the FP64 pipe in k_br_gemm (1.34 ms).
+//
+// QUAD's weights w depend on the head index h (its first point with a
+// positive ratio TA(h+1)/TA(h)) and on the last point mtpq = min(MTP_s,
+// MTP_p). h is a property of the source (its chain's signs at points 2..5),
+// found once per (pair, k) by k_br_heads; mtpq depends on the column's MTP.
+// The columns (the pairs whose density is dotted) of one k are therefore
+// grouped by (MTP, h) into buckets, a warp takes 32 rows of one bucket's
+// columns (up to BR_NC), and U is U^(M0) plus a term per residue class:
+//   U^(m)(j) = e(j) (c^(M0)(j) + K(j mod 4)),  j <= J0,
+// with M0 the smallest MTP of all pairs, J0 <= M0 - 4, and K the class sums
+// of w q rho over (M0, mtpq] (added, so nothing cancels); the points J0 < j
+// <= m have their vectors per bucket (k_br_tail). An entry whose terms do not
+// have the head index assumed for their bucket is evaluated term by term
+// (breit_term), as are the lists of gg_brintf.
+// The sums are FMA chains over the points and the 1/r^k factors multiply by
+// the power table's reciprocals; the values agree with the term by term form
+// to a few ulps of the largest partial sum.
+// ---------------------------------------------------------------------------
+constexpr int BR_NC = 8;      // columns of one warp's tile
+constexpr int BR_MIN_MF = 16; // shortest orbital the contraction takes
+
+struct BrRow {  // one (k, pair) row, padded rows have a = 0
+  short a, b, K;
+  int mtp;
+  int fa, fb;        // Bessel functions: type 1 order k; type 2 orders k - 1, k + 1
+  double w;          // the pair's frequency
+  long long off;     // position of the row's first integral
+  int lo, P, pad;    // the k's first row, pairs and padded rows
+  unsigned char mask, h[3];  // TRIANGBREIT mask; heads by operator (k_br_heads)
+};
+
+struct BrEnt {  // up to BR_NC columns of one bucket
+  int lo, P, pad, m, h, set, nc, col[BR_NC];
+  long long xt, kv, g;  // offsets: tail vectors, class terms, output block
+};
+
+struct BrBucket {
+  int lo, P, pad, m, h, set;
+  long long xt, kv;
+};
+
+// the arrays [point][pitch] over all rows: densities, operators (e, q) of the
+// chains (0, 1: the terms with RPOR weights, 2: SKINT's second form), forward
+// vectors F, class sums S of q rho up to M0 and the base vectors by set and head
+struct BrArr {
+  double *rho, *e[3], *q[3], *F[2], *S[3], *base[2][3];
+  int pitch, maxm, m0, j0, type;
+};
+
+__device__ __forceinline__ double br_pat(const QuadConst &q, int ph) {
+  ph &= 3;
+  return (ph & 1) ? q.C2 : (ph == 2) ? q.C3 : q.C4;
+}
+
+// QUAD's weight of point i for head h and last point mq
+__device__ __forceinline__ double br_w(const QuadConst &q, int i, int h, int mq) {
+  if (i < h) return 0.0;
+  if (i == h) return q.C1;
+  const double w = br_pat(q, i - h);
+  return (i == mq && ((mq - h) & 3) == 0) ? w - q.C1 : w;
+}
+
+// densities by pair [nw * nw][np] (P_a Q_b on 2..MTP) for the columns
+__global__ void k_br_rho(int nw, const double *__restrict__ PF, const double *__restrict__ QF, int ld,
+                         const int *__restrict__ MF, int np, double *__restrict__ rho) {
+  const int a = blockIdx.y + 1, b = blockIdx.x + 1;
+  const int m = min(MF[a], MF[b]);
+  double *r = rho + ((size_t)(a - 1) * nw + (b - 1)) * np;
+  for (int i = threadIdx.x; i < np; i += blockDim.x)
+    r[i] = (i >= 2 && i <= m) ? pfv(PF, ld, i, a) * pfv(QF, ld, i, b) : 0.0;
+}
+
+// the head index each pair's chain gives as a source, from the signs of its
+// first values: operator 0 (type 1: Z_k; type 2 at a frequency: the leading
+// r^2 order of SKINT's first term), 1 (SKINT at zero frequency), 2 (SKINT's
+// second term, Z_{k+1}); 2 where none of 2..4 qualifies (the entry's own
+// check then sends it to the term by term form)
+__global__ void k_br_heads(BrRow *__restrict__ rows, int nrows, int type, const double *__restrict__ rho, int nw,
+                           int np, const double *__restrict__ R, const double *__restrict__ RP,
+                           const double *__restrict__ Pow, QuadConst q, unsigned char *__restrict__ out) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= nrows) return;
+  const BrRow b = rows[r];
+  unsigned char h[3] = {2, 2, 2};
+  if (b.a) {
+    const double *p = rho + ((size_t)(b.a - 1) * nw + (b.b - 1)) * np;
+    auto pw = [&](int k, int i) { return k > 0 ? Pow[(size_t)k * np + i] : k < 0 ? Pow[i] : 1.0; };
+    // Z(2..5) of order k over src(i)
+    auto chain = [&](int k, int extra, double *z) {
+      double t[4];
+      for (int i = 2; i <= 5; ++i) {
+        t[i - 2] = RP[i] * pw(k, i) * p[i];
+        if (extra) t[i - 2] = t[i - 2] * (R[i] * R[i]);
+      }
+      for (int s = 0; s < 3; ++s) {
+        z[s] = 0.0;
+        for (int c = 0; c < 4; ++c) z[s] = z[s] + q.CNC5C[c][s] * t[c];
+      }
+      z[3] = q.C1 * t[3] + q.C2 * (t[0] + t[2]) + q.C3 * t[1];
+    };
+    auto head = [&](const double *z) {
+      for (int i = 0; i < 3; ++i)
+        if (z[i] != 0.0 && ((z[i] > 0.0 && z[i + 1] > 0.0) || (z[i] < 0.0 && z[i + 1] < 0.0)))
+          return (unsigned char)(i + 2);
+      return (unsigned char)2;
+    };
+    double za[4], zb[4], d[4];
+    if (type == 1) {
+      chain(b.K, 0, za);
+      h[0] = head(za);
+    } else {
+      chain(b.K - 1, 0, za);
+      chain(b.K - 1, 1, zb);
+      for (int i = 0; i < 4; ++i) d[i] = zb[i] - (R[i + 2] * R[i + 2]) * za[i];
+      h[0] = head(d);
+      chain(b.K + 1, 0, zb);
+      h[2] = head(zb);
+      for (int i = 0; i < 4; ++i) d[i] = zb[i] / pw(b.K + 1, i + 2) - za[i] / pw(b.K - 1, i + 2);
+      h[1] = head(d);
+    }
+  }
+  for (int t = 0; t < 3; ++t) {
+    rows[r].h[t] = h[t];
+    out[(size_t)3 * r + t] = h[t];
+  }
+}
+
+// densities and operators per (row, point)
+__global__ void k_br_elem(const BrRow *__restrict__ rows, BrArr A, const double *__restrict__ rhop, int nw, int np,
+                          const double *__restrict__ R, const double *__restrict__ RP,
+                          const double *__restrict__ RPOR, const double *__restrict__ Pow,
+                          const double *__restrict__ BJ, const double *__restrict__ BN) {
+  const int r = blockIdx.x * 32 + threadIdx.x;
+  const BrRow b = rows[r];
+  for (int i = blockIdx.y * blockDim.y + threadIdx.y; i <= A.maxm; i += gridDim.y * blockDim.y) {
+    const size_t at = (size_t)i * A.pitch + r;
+    double rho = 0.0, e0 = 0.0, e1 = 0.0, e2 = 0.0, q0 = 0.0, q1 = 0.0, q2 = 0.0;
+    if (b.a && i >= 2) {
+      rho = rhop[((size_t)(b.a - 1) * nw + (b.b - 1)) * np + i];
+      const int K = b.K;
+      // r^k and 1 / r^k, k = -1 .. KLIM
+      auto up = [&](int k) { return k > 0 ? Pow[(size_t)k * np + i] : k < 0 ? Pow[i] : 1.0; };
+      auto dn = [&](int k) { return k > 0 ? Pow[(size_t)(KLIM + 1 + k) * np + i] : k < 0 ? R[i] : 1.0; };
+      if (A.type == 1) {
+        const double bj = b.fa >= 0 ? BJ[(size_t)b.fa * np + i] : 0.0, bn = b.fa >= 0 ? BN[(size_t)b.fa * np + i] : 0.0;
+        e0 = RP[i] * up(K) * (1.0 + bj);
+        q0 = (1.0 + bn) * RPOR[i] * dn(K);
+      } else {
+        const double ra = RP[i] * up(K - 1), rb = RP[i] * up(K + 1), da = dn(K - 1), db = dn(K + 1);
+        const double WK = (double)(K + K + 1);
+        if (fabs(b.w) < 1.0e-10) {
+          // WK / 2 part RPOR (Z_{k+1} - Z_{k-1})
+          e0 = rb;
+          q0 = 0.5 * WK * RPOR[i] * db;
+          e1 = ra;
+          q1 = -0.5 * WK * RPOR[i] * da;
+        } else {
+          const double j1 = b.fa >= 0 ? BJ[(size_t)b.fa * np + i] : 0.0, n1 = b.fa >= 0 ? BN[(size_t)b.fa * np + i] : 0.0;
+          const double j2 = b.fb >= 0 ? BJ[(size_t)b.fb * np + i] : 0.0, n2 = b.fb >= 0 ? BN[(size_t)b.fb * np + i] : 0.0;
+          const double wr = WK / b.w, al = wr * wr * RPOR[i] / (R[i] * R[i]) * da;
+          e0 = -ra * j1;
+          q0 = al * (1.0 + n2);
+          e1 = ra;
+          q1 = -al * n2;
+          e2 = rb * (1.0 + j2);
+          q2 = -(b.w * b.w / (double)((2 * K + 3) * (2 * K - 1))) * (1.0 + n1) * R[i] * RP[i] * db;
+        }
+      }
+    }
+    A.rho[at] = rho;
+    A.e[0][at] = e0;
+    A.q[0][at] = q0;
+    if (A.type == 2) {
+      A.e[1][at] = e1;
+      A.q[1][at] = q1;
+      A.e[2][at] = e2;
+      A.q[2][at] = q2;
+    }
+  }
+}
+
+// the forward vectors F = sum_chains q Z[e rho] (task 0: operator 0 (+ 1),
+// task 1: operator 2) and the backward class sums S(i) = sum q rho over i, i +
+// 4, .. <= M0 (tasks 2..: chain t - 2). A block takes 32 rows; a warp one
+// residue class and one of BR_SEG runs of its points: it adds its run, the
+// runs' sums are added through shared memory, and the second pass shifts it.
+// One thread per (row, class) walking all points took 257 us for 16 subshells
+// (three dependent loads and an addition per step, few warps), this 24 us.
+constexpr int BR_SEG = 8;
+__global__ void __launch_bounds__(32 * BR_SEG) k_br_chains(const BrRow *__restrict__ rows, BrArr A, QuadConst q) {
+  __shared__ double tot[BR_SEG][32];
+  const int lane = threadIdx.x, cls = blockIdx.z, seg = threadIdx.y;
+  const int r = blockIdx.x * 32 + lane;
+  const int nfwd = A.type == 1 ? 1 : 2;
+  const int task = blockIdx.y, s = cls + 2;
+  const size_t p = A.pitch;
+  const double *rho = A.rho + r;
+  const bool fwd = task < nfwd;
+  const int end = fwd ? A.maxm : A.m0;
+  const int steps = (end - s) / 4 + 1, run = (steps + BR_SEG - 1) / BR_SEG;
+  const int c0 = fwd ? (task == 0 ? 0 : 2) : task - nfwd, nch = (task == 0 && A.type == 2) ? 2 : 1;
+  const int mt = fwd ? rows[r].mtp : A.m0;
+  for (int c = c0; c < c0 + nch; ++c) {
+    const double *e = A.e[c] + r, *qq = A.q[c] + r;
+    double *out = fwd ? A.F[task] + r : A.S[c] + r;
+    // the second chain's own sums wait in a base plane, written later
+    double *part = c > c0 ? A.base[0][0] + r : out;
+    double v = 0.0;
+    if (fwd) {
+      auto t = [&](int j) { return __ldg(e + j * p) * __ldg(rho + j * p); };
+      for (int u = seg * run; u < min(steps, (seg + 1) * run); ++u) {
+        const int i = s + 4 * u;
+        if (i <= mt) {
+          if (i <= 4) {
+            for (int k = 2; k <= 5; ++k) v = fma(q.CNC5C[k - 2][i - 2], t(k), v);
+          } else {
+            v = v + fma(q.C1, t(i - 4) + t(i), fma(q.C2, t(i - 3) + t(i - 1), q.C3 * t(i - 2)));
+          }
+        }
+        part[i * p] = v;
+      }
+    } else {
+      for (int u = min(steps, (seg + 1) * run) - 1; u >= seg * run; --u) {
+        const int i = s + 4 * u;
+        v = fma(__ldg(qq + i * p), __ldg(rho + i * p), v);
+        part[i * p] = v;
+      }
+    }
+    tot[seg][lane] = v;
+    __syncthreads();
+    double off = 0.0;
+    if (fwd)
+      for (int g = 0; g < seg; ++g) off = off + tot[g][lane];
+    else
+      for (int g = BR_SEG - 1; g > seg; --g) off = off + tot[g][lane];
+    for (int u = seg * run; u < min(steps, (seg + 1) * run); ++u) {
+      const int i = s + 4 * u;
+      const double z = part[i * p] + off;
+      if (!fwd)
+        out[i * p] = z;
+      else
+        out[i * p] = i <= mt ? fma(__ldg(qq + i * p), z, c > c0 ? out[i * p] : 0.0) : 0.0;
+    }
+    __syncthreads();
+  }
+}
+
+// adjoint chains of a set: type 1: 0; type 2 set 0 (source's frequency first
+// pair): 2; set 1: 0 and 1
+__device__ __forceinline__ int br_adj(int type, int set, int &first) {
+  first = (type == 2 && set == 0) ? 2 : 0;
+  return (type == 2 && set == 1) ? 2 : 1;
+}
+// operator whose head a row's forward vector has, -1: no forward vector
+__device__ __forceinline__ int br_fwd(int type, int set, const BrRow &b) {
+  const bool zero = type == 2 && fabs(b.w) < 1.0e-10;
+  if (type == 1) return 0;
+  if (set == 0) return zero ? 1 : 0;
+  return zero ? -1 : 2;
+}
+
+// the transposed chain's weights times QUAD's: a point j >= 6 takes
+// sum_t w[(j - h) & 3][t] S(j + t)
+struct BrFold {
+  double w[4][5];
+};
+
+// base vectors: the transposed chains cut at M0, by assumed head of the
+// column, plus the weighted forward vector; points 2..J0
+__global__ void k_br_base(const BrRow *__restrict__ rows, BrArr A, QuadConst q, BrFold fold) {
+  const int r = blockIdx.x * 32 + threadIdx.x, set = blockIdx.z;
+  const BrRow b = rows[r];
+  const size_t p = A.pitch;
+  int c0;
+  const int nch = br_adj(A.type, set, c0);
+  const int fo = b.a ? br_fwd(A.type, set, b) : -1;
+  for (int j = 2 + blockIdx.y * blockDim.y + threadIdx.y; j <= A.j0; j += gridDim.y * blockDim.y) {
+    const double f = fo < 0 ? 0.0 : br_w(q, j, b.h[fo], 0) * __ldg(A.F[set] + j * p + r);
+    double x[3] = {f, f, f};
+    for (int c = c0; c < c0 + nch; ++c) {
+      const double *S = A.S[c] + r;
+      const double e = __ldg(A.e[c] + j * p + r);
+      if (j >= 6) {
+        double sv[5];
+#pragma unroll
+        for (int t = 0; t < 5; ++t) sv[t] = __ldg(S + (j + t) * p);
+#pragma unroll
+        for (int h = 2; h <= 4; ++h) {
+          const double *w = fold.w[(j - h) & 3];
+          double v = w[0] * sv[0];
+#pragma unroll
+          for (int t = 1; t < 5; ++t) v = fma(w[t], sv[t], v);
+          x[h - 2] = fma(e, v, x[h - 2]);
+        }
+      } else {
+        for (int h = 2; h <= 4; ++h) {
+          auto sw = [&](int i) {  // suffix sum of the class of i with QUAD's weights
+            if (i > h) return br_pat(q, i - h) * S[i * p];
+            if (i == h) return q.C4 * S[i * p] - q.C1 * (A.q[c][i * p + r] * A.rho[i * p + r]);
+            return br_pat(q, i + 4 - h) * S[(i + 4) * p];
+          };
+          double v = 0.0;
+          for (int i = 2; i <= 4; ++i) v = fma(q.CNC5C[j - 2][i - 2], sw(i), v);
+          for (int i = 5; i <= j + 4; ++i) {
+            const int dlt = i - j;
+            v = fma((dlt == 0 || dlt == 4) ? q.C1 : dlt == 2 ? q.C3 : q.C2, sw(i), v);
+          }
+          x[h - 2] = fma(e, v, x[h - 2]);
+        }
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 3; ++h) A.base[set][h][j * p + r] = x[h];
+  }
+}
+
+// a bucket's own part: the vectors of the points J0 < j <= m and the class
+// terms K of the points up to J0 (8 per chain: j = 2..5, then j mod 4). One
+// thread per (row, bucket), the transposed chain run backwards in registers
+__global__ void k_br_tail(const BrBucket *__restrict__ bk, const BrRow *__restrict__ rows, BrArr A, QuadConst q,
+                          double *__restrict__ xt, double *__restrict__ kv) {
+  const BrBucket B = bk[blockIdx.x];
+  const int l = blockIdx.y * blockDim.x + threadIdx.x;
+  if (l >= B.pad) return;
+  const int r = B.lo + l;
+  const BrRow b = rows[r];
+  const size_t p = A.pitch;
+  const int m = B.m, h = B.h, mq = b.a ? min(m, (int)b.mtp) : 0;
+  int c0;
+  const int nch = br_adj(A.type, B.set, c0);
+  const int fo = b.a ? br_fwd(A.type, B.set, b) : -1;
+  const int tl = (m - A.j0 + 1) & ~1;
+  double *X = xt + B.xt + l;
+  double *Kv = kv + B.kv + l;
+  if (tl > m - A.j0) X[(size_t)(tl - 1) * B.pad] = 0.0;
+  // S(j), S(j+1), S(j+2), S(j+3) of each chain
+  double s0[2] = {0.0, 0.0}, s1[2] = {0.0, 0.0}, s2[2] = {0.0, 0.0}, s3[2] = {0.0, 0.0};
+#pragma unroll 4
+  for (int j = m; j > A.j0; --j) {
+    double x = 0.0;
+    if (j <= mq) {
+      const double rho = __ldg(A.rho + j * p + r), w = br_w(q, j, h, mq) * rho;
+      for (int c = 0; c < nch; ++c) {
+        const double o = s3[c], n = fma(w, __ldg(A.q[c0 + c] + j * p + r), o);
+        const double v = fma(q.C1, n + o, fma(q.C2, s0[c] + s2[c], q.C3 * s1[c]));
+        s3[c] = s2[c];
+        s2[c] = s1[c];
+        s1[c] = s0[c];
+        s0[c] = n;
+        x = fma(__ldg(A.e[c0 + c] + j * p + r), v, x);
+      }
+      if (fo >= 0) x = fma(br_w(q, j, b.h[fo], mq), __ldg(A.F[B.set] + j * p + r), x);
+    }
+    X[(size_t)(j - A.j0 - 1) * B.pad] = x;
+    if (j == A.m0 + 1 || (m == A.m0 && j == m)) {
+      // class sums of the points beyond M0: D[i & 3]
+      for (int c = 0; c < nch; ++c) {
+        double D[4] = {0.0, 0.0, 0.0, 0.0};
+        if (m > A.m0) {
+          D[j & 3] = s0[c];
+          D[(j + 1) & 3] = s1[c];
+          D[(j + 2) & 3] = s2[c];
+          D[(j + 3) & 3] = s3[c];
+        }
+        // QUAD's last point is M0 itself, which the base weights as an inner one
+        if (mq == A.m0 && ((mq - h) & 3) == 0) D[mq & 3] = -q.C1 * (A.q[c0 + c][mq * p + r] * A.rho[mq * p + r]);
+        for (int t = 2; t <= 5; ++t) {
+          double v = 0.0;
+          for (int i = 2; i <= 4; ++i) v = fma(q.CNC5C[t - 2][i - 2], D[i & 3], v);
+          for (int i = 5; i <= t + 4; ++i) {
+            const int dlt = i - t;
+            v = fma((dlt == 0 || dlt == 4) ? q.C1 : dlt == 2 ? q.C3 : q.C2, D[i & 3], v);
+          }
+          Kv[(size_t)(8 * c + t - 2) * B.pad] = v;
+        }
+        for (int t = 0; t < 4; ++t)
+          Kv[(size_t)(8 * c + 4 + t) * B.pad] =
+              2.0 * q.C1 * D[t] + q.C2 * (D[(t + 1) & 3] + D[(t + 3) & 3]) + q.C3 * D[(t + 2) & 3];
+      }
+    }
+  }
+}
+
+// QUAD's head term from TA(h), TA(h+1); *ok is cleared where h is not QUAD's
+// head index (the test at h fails, or one before it passes)
+__device__ __forceinline__ double br_head(const double *ta, int h, const double *HD, int np, bool *ok) {
+  bool good = true;
+  double res = 0.0;
+#pragma unroll
+  for (int i = 2; i <= 4; ++i) {
+    const double t0 = ta[i - 2], t1 = ta[i - 1];
+    if (i < h) {
+      if ((t0 > 0.0 && t1 > 0.0) || (t0 < 0.0 && t1 < 0.0) || t0 != t0 || t1 != t1) good = false;
+    } else if (i == h) {
+      const double t = t1 / t0;
+      if (fabs(t0) > 0.0 && t > 0.0) {
+        const double sigma = log(t * HD[np + h]) * HD[h];
+        res = (t0 * HD[2 * np + h]) / (sigma + 1.0);
+      } else {
+        good = false;
+      }
+    }
+  }
+  if (!good) *ok = false;
+  return res;
+}
+
+// One block: 32 rows x NC columns of one bucket, the points shared out among
+// its four warps (a set of few pairs has too few warps otherwise: 239 us with
+// a warp per tile, 76 us so, 16 subshells). Per point the row's vector value
+// is formed (base + e K, or the tail's) and multiplied into NC accumulators:
+// 1 + NC (2 + NC with two chains) FP64 instructions, the columns' densities
+// read uniformly. The warps' sums meet in shared memory; each warp then adds
+// the head contributions of its columns.
+template <int NC, int NCH>
+__device__ __forceinline__ void br_gemm(const BrEnt &E, int lane, int warp, double (*red)[BR_NC][32],
+                                        const BrRow *__restrict__ rows, const BrArr &A, int c0,
+                                        const double *__restrict__ rhop, int nw, int np,
+                                        const double *__restrict__ xt, const double *__restrict__ kv,
+                                        const double *__restrict__ HD, const QuadConst &q, double *__restrict__ G) {
+  const int l = blockIdx.y * 32 + lane, r = E.lo + l;
+  const size_t p = A.pitch;
+  const double *e0 = A.e[c0] + r, *e1 = A.e[c0 + NCH - 1] + r;
+  const double *rc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const BrRow cr = rows[E.lo + E.col[c]];
+    rc[c] = rhop + ((size_t)(cr.a - 1) * nw + (cr.b - 1)) * np;
+  }
+  {
+    const double *B = A.base[E.set][E.h - 2] + r;
+    const double *Kv = kv + E.kv + l;
+    double K[NCH][4], acc[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+    auto add2 = [&](int j, double xa, double xb) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const double2 v = __ldg(reinterpret_cast<const double2 *>(rc[c] + j));
+        acc[c] = fma(xa, v.x, acc[c]);
+        acc[c] = fma(xb, v.y, acc[c]);
+      }
+    };
+    auto step = [&](int j) {  // points j .. j + 3 with the class terms K[..][0..3]
+      double x[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const size_t o = (size_t)(j + t) * p;
+        x[t] = fma(__ldg(e0 + o), K[0][t], __ldg(B + o));
+        if (NCH == 2) x[t] = fma(__ldg(e1 + o), K[NCH - 1][t], x[t]);
+      }
+      add2(j, x[0], x[1]);
+      add2(j + 2, x[2], x[3]);
+    };
+    if (warp == 0) {
+#pragma unroll
+      for (int c = 0; c < NCH; ++c)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) K[c][t] = Kv[(size_t)(8 * c + t) * E.pad];
+      step(2);
+    }
+#pragma unroll
+    for (int c = 0; c < NCH; ++c)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) K[c][t] = Kv[(size_t)(8 * c + 4 + ((6 + t) & 3)) * E.pad];
+#pragma unroll 4
+    for (int j = 6 + 4 * warp; j < A.j0; j += 16) step(j);
+    const double *X = xt + E.xt + l;
+    const int tl = (E.m - A.j0 + 1) & ~1;
+#pragma unroll 4
+    for (int t = 2 * warp; t < tl; t += 8)
+      add2(A.j0 + 1 + t, __ldg(X + (size_t)t * E.pad), __ldg(X + (size_t)(t + 1) * E.pad));
+#pragma unroll
+    for (int c = 0; c < NC; ++c) red[warp][c][lane] = acc[c];
+  }
+  __syncthreads();
+  if (l >= E.P) return;
+  const BrRow b = rows[r];
+  const int fo = br_fwd(A.type, E.set, b);
+  const bool adj = A.type == 1 || E.set == 1 || fo == 0;  // set 0 at zero frequency has no second term
+  for (int c = warp; c < NC; c += 4) {
+    double v = (red[0][c][lane] + red[1][c][lane]) + (red[2][c][lane] + red[3][c][lane]), s[4], ta[4];
+    bool ok = true;
+    const BrRow cr = rows[E.lo + E.col[c]];
+    const double *rs = rhop + ((size_t)(cr.a - 1) * nw + (cr.b - 1)) * np;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[i] = rs[i + 2];
+    if (fo >= 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ta[i] = __ldg(A.F[E.set] + (i + 2) * p + r) * s[i];
+      v += br_head(ta, b.h[fo], HD, np, &ok);
+    }
+    if (adj) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ta[i] = 0.0;
+#pragma unroll
+      for (int u = 0; u < NCH; ++u) {
+        const double *ee = u ? e1 : e0;
+        double t[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) t[i] = __ldg(ee + (i + 2) * p) * s[i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (i > E.h - 1) continue;  // TA(h + 1) is the last one read
+          double z;
+          if (i < 3)
+            z = fma(q.CNC5C[3][i], t[3], fma(q.CNC5C[2][i], t[2], fma(q.CNC5C[1][i], t[1], q.CNC5C[0][i] * t[0])));
+          else
+            z = fma(q.C3, t[1], fma(q.C2, t[0] + t[2], q.C1 * t[3]));
+          ta[i] = fma(__ldg(A.q[c0 + u] + (i + 2) * p + r) * __ldg(A.rho + (i + 2) * p + r), z, ta[i]);
+        }
+      }
+      v += br_head(ta, E.h, HD, np, &ok);
+    }
+    G[E.g + (size_t)E.col[c] * E.pad + l] = ok ? v : __longlong_as_double(0x7ff8000000000000ll);
+  }
+}
+
+template <int NCH>
+__global__ void __launch_bounds__(128) k_br_gemm(const BrEnt *__restrict__ ents, const BrRow *__restrict__ rows,
+                                                 BrArr A, int c0, const double *__restrict__ rhop, int nw, int np,
+                                                 const double *__restrict__ xt, const double *__restrict__ kv,
+                                                 const double *__restrict__ HD, QuadConst q, double *__restrict__ G) {
+  __shared__ double red[4][BR_NC][32];
+  __shared__ BrEnt E;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) E = ents[blockIdx.x];
+  __syncthreads();
+  if ((int)blockIdx.y * 32 >= E.pad) return;
+  switch (E.nc) {
+#define BR_CASE(N) \
+  case N: br_gemm<N, NCH>(E, lane, warp, red, rows, A, c0, rhop, nw, np, xt, kv, HD, q, G); break;
+    BR_CASE(1) BR_CASE(2) BR_CASE(3) BR_CASE(4) BR_CASE(5) BR_CASE(6) BR_CASE(7) BR_CASE(8)
+#undef BR_CASE
+  }
+}
+
+// the integrals: row (k, a, b) x column (c, d), half the sum of the two
+// orders, at the row's position plus the column's rank among those the row's
+// mask admits; a value that is not a number (an entry marked by k_br_gemm, or
+// inputs that are not finite) goes to the term by term list
+struct BrRedo {
+  long long pos;
+  int row, col;
+};
+__global__ void k_br_table(const BrRow *__restrict__ rows, const int *__restrict__ rank, const double *__restrict__ G1,
+                           const double *__restrict__ G2, const long long *__restrict__ g0, int KEY,
+                           int32_t *__restrict__ ind, double *__restrict__ val, BrRedo *__restrict__ redo,
+                           int *__restrict__ nredo) {
+  const int r = blockIdx.x;
+  const BrRow b = rows[r];
+  if (!b.a) return;
+  const int l = r - b.lo;
+  const long long g = g0[b.K];
+  const int *rk = rank + (size_t)8 * b.lo + (size_t)b.mask * b.pad;
+  for (int s = threadIdx.x; s < b.P; s += blockDim.x) {
+    const BrRow c = rows[b.lo + s];
+    if (!(b.mask & c.mask)) continue;
+    const double v = G1 ? 0.5 * (G1[g + (size_t)s * b.pad + l] + G2[g + (size_t)l * b.pad + s])
+                        : __longlong_as_double(0x7ff8000000000000ll);
+    const long long pos = b.off + rk[s];
+    ind[pos] = ((b.a * KEY + b.b) * KEY + c.a) * KEY + c.b;
+    val[pos] = v;
+    if (v != v) redo[atomicAdd(nredo, 1)] = BrRedo{pos, r, b.lo + s};
+  }
+}
+
+// an entry of the table term by term: one thread per (entry, term), then the
+// combination
+__global__ void __launch_bounds__(128) k_br_redo(int type, const BrRedo *__restrict__ redo, int n,
+                                                 const BrRow *__restrict__ rows, PlanTabs T, TermTabs tt, QuadConst q,
+                                                 double *__restrict__ v, BrInt *__restrict__ ints) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 4 * n) return;
+  const BrRedo e = redo[t >> 2];
+  const BrRow a = rows[e.row], c = rows[e.col];
+  BrJob jb[4];
+  BrInt bi;
+  const int k = plan_one(type, a.a, a.b, c.a, c.b, a.K, T, (t >> 2) * 4, &bi, jb);
+  if ((t & 3) == 0) ints[t >> 2] = bi;
+  if ((t & 3) < k) v[t] = breit_term(jb[t & 3], tt, q);
+}
+
+__global__ void k_br_redo_store(const BrRedo *__restrict__ redo, int n, const double *__restrict__ v,
+                                double *__restrict__ val) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) val[redo[t].pos] = v[t];
 }
 
 template <class T> int upload_vec(DBuf<T> &b, const std::vector<T> &h, cudaStream_t s) {
@@ -605,6 +1185,10 @@ struct Plan {
     GG_TRY(upload_vec(dW, W, s));
     GG_TRY(upload_vec(dbid, bid, s));
     return GG_OK;
+  }
+  int id(int x, int y, int nn) const {
+    const int lo = std::min(x, y), hi = std::max(x, y);
+    return bid[((size_t)(nn + 1) * nw + (lo - 1)) * nw + (hi - 1)];
   }
   PlanTabs tabs() const { return PlanTabs{dW.p, dbid.p, nw}; }
 };
@@ -653,9 +1237,8 @@ int run_terms(gg_ctx *ctx, const Plan &P, const BrJob *djobs, int64_t nj, const 
     ::gg::note_launch();
   }
   if (nj > 0) {
-    k_breit_jobs<<<(unsigned)((nj + 127) / 128), 128, 0, s>>>(djobs, nj, o.dPF.p, o.dQF.p, o.ld, o.dMF.p, g.dR.p,
-                                                               g.dRP.p, g.dRPOR.p, g.dPow.p, g.np, g.q, dBJ.p,
-                                                               dBN.p, dv.p);
+    const TermTabs tt{o.dPF.p, o.dQF.p, o.ld, o.dMF.p, g.dR.p, g.dRP.p, g.dRPOR.p, g.dPow.p, g.np, dBJ.p, dBN.p};
+    k_breit_jobs<<<(unsigned)((nj + 127) / 128), 128, 0, s>>>(djobs, nj, tt, g.q, dv.p);
     ::gg::note_launch();
   }
   if (ni > 0) {
@@ -673,6 +1256,285 @@ int run_terms(gg_ctx *ctx, const Plan &P, const BrJob *djobs, int64_t nj, const 
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
   }
+  return GG_OK;
+}
+
+// the tables' contraction: rows, operators, buckets and the dense products
+int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector<unsigned char> &mask, BreitTable &T,
+              double *plan_ms, double *kernel_ms) {
+  const Grid &g = ctx->grid;
+  const Orbitals &o = ctx->orb;
+  cudaStream_t s = ctx->stream;
+  const int nw = o.nw, KEY = nw + 1, np = g.np;
+  const size_t msz = (size_t)(nw + 1) * (nw + 1);
+  const auto th0 = std::chrono::steady_clock::now();
+  // rows: the admitted pairs of each k in (a, b) order, padded to whole warps
+  std::vector<BrRow> rows;
+  std::vector<int> lo(j2max + 2, 0), cnt(j2max + 1, 0);
+  std::vector<long long> g0(j2max + 1, 0);
+  std::vector<int> rank;
+  long long ni = 0, nj = 0, gsz = 0;
+  T.kstart.assign(j2max + 2, 1);
+  int maxm = 0, m0 = INT32_MAX;
+  for (int x = 1; x <= nw; ++x) {
+    maxm = std::max(maxm, o.mf[x]);
+    m0 = std::min(m0, o.mf[x]);
+  }
+  for (int K = 0; K <= j2max; ++K) {
+    const unsigned char *mk = mask.data() + (size_t)K * msz;
+    lo[K] = (int)rows.size();
+    for (int a = 1; a <= nw; ++a)
+      for (int b = 1; b <= nw; ++b)
+        if (mk[a * (nw + 1) + b]) {
+          BrRow r{};
+          r.a = (short)a;
+          r.b = (short)b;
+          r.K = (short)K;
+          r.mtp = std::min(o.mf[a], o.mf[b]);
+          r.fa = P.id(a, b, type == 1 ? K : K - 1);
+          r.fb = type == 1 ? -1 : P.id(a, b, K + 1);
+          r.w = P.W[(size_t)(a - 1) * nw + (b - 1)];
+          r.mask = mk[a * (nw + 1) + b];
+          rows.push_back(r);
+        }
+    const int np_ = cnt[K] = (int)rows.size() - lo[K];
+    while (rows.size() % 32) rows.push_back(BrRow{});
+    const int pad = (int)rows.size() - lo[K];
+    g0[K] = gsz;
+    gsz += (long long)pad * pad;
+    // positions: rank of a column among those a row's mask admits
+    rank.resize((size_t)8 * rows.size(), 0);
+    int n[8] = {}, nz[8] = {};  // admitted columns by row mask; those at a frequency
+    for (int c = 0; c < np_; ++c) {
+      const BrRow &r = rows[lo[K] + c];
+      for (int m = 1; m < 8; ++m) {
+        rank[(size_t)8 * lo[K] + (size_t)m * pad + c] = n[m];
+        if (m & r.mask) {
+          ++n[m];
+          nz[m] += std::fabs(r.w) >= 1.0e-10;
+        }
+      }
+    }
+    for (int c = lo[K]; c < (int)rows.size(); ++c) {
+      BrRow &r = rows[c];
+      r.lo = lo[K];
+      r.P = np_;
+      r.pad = pad;
+      r.off = ni;
+      if (!r.a) continue;
+      ni += n[r.mask];
+      // the terms of the row's integrals (plan_one), which bound the table
+      const int own = type == 1 ? 2 : std::fabs(r.w) >= 1.0e-10 ? 2 : 1;
+      nj += type == 1 ? 4LL * n[r.mask] : (long long)own * n[r.mask] + n[r.mask] + nz[r.mask];
+      nj -= type == 1 ? (r.a == r.b ? 3 : 5) : (r.a == r.b ? own : 2 * own);
+    }
+    T.kstart[K + 1] = (int32_t)(ni + 1);
+  }
+  if (ni > INT32_MAX || nj > INT32_MAX) return fail(GG_ERR_RANGE, "gg_genintbreit: table too large");
+  T.n = ni;
+  T.hInd.resize(ni);
+  T.hVal.resize(ni);
+  const int R = (int)rows.size();
+  if (ni == 0) return GG_OK;
+  // the contraction takes orbitals that reach past the chains' start and end
+  // on the grid; any other set is evaluated term by term
+  const bool plain = m0 >= BR_MIN_MF && maxm <= g.n;
+
+  // the operators, forward vectors and class sums need no buckets: they run
+  // while the host waits for the heads and builds them
+  const int nch = type == 1 ? 1 : 3, nset = type == 1 ? 1 : 2;
+  const size_t plane = plain ? (size_t)(maxm + 1) * R : 0;
+  const int j0 = 5 + 4 * ((m0 - 9) / 4);
+  DBuf<BrRow> drows;
+  DBuf<double> drho, darr, dBJ, dBN, dG, dval;
+  DBuf<BessDesc> dbd;
+  DBuf<unsigned char> dheads;
+  DBuf<int> drank, dnredo;
+  DBuf<long long> dg0;
+  DBuf<int32_t> dind;
+  GG_TRY(upload_vec(drows, rows, s));
+  GG_TRY(upload_vec(drank, rank, s));
+  GG_TRY(upload_vec(dg0, g0, s));
+  GG_TRY(upload_vec(dbd, P.bess, s));
+  const int nb = (int)P.bess.size();
+  GG_TRY(drho.alloc((size_t)nw * nw * np));
+  GG_TRY(darr.alloc(plane * (size_t)(1 + 3 * nch + nset * 4)));
+  GG_TRY(dBJ.alloc((size_t)std::max(1, nb) * np));
+  GG_TRY(dBN.alloc((size_t)std::max(1, nb) * np));
+  GG_TRY(dheads.alloc((size_t)3 * R));
+  GG_TRY(dG.alloc(plain ? (size_t)gsz * nset : 0));
+  GG_TRY(dind.alloc(ni));
+  GG_TRY(dval.alloc(ni));
+  GG_TRY(dnredo.alloc(1));
+  BrArr A{};
+  {
+    double *p = darr.p;
+    auto take = [&] {
+      double *r = p;
+      p += plane;
+      return r;
+    };
+    A.rho = take();
+    for (int c = 0; c < nch; ++c) {
+      A.e[c] = take();
+      A.q[c] = take();
+      A.S[c] = take();
+    }
+    for (int t = 0; t < nset; ++t) {
+      A.F[t] = take();
+      for (int h = 0; h < 3; ++h) A.base[t][h] = take();
+    }
+    A.pitch = R;
+    A.maxm = maxm;
+    A.m0 = m0;
+    A.j0 = j0;
+    A.type = type;
+  }
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  GG_CUDA(cudaEventCreate(&e0));
+  GG_CUDA(cudaEventCreate(&e1));
+  struct Ev {
+    cudaEvent_t a, b, c;
+    ~Ev() {
+      cudaEventDestroy(a);
+      cudaEventDestroy(b);
+      if (c) cudaEventDestroy(c);
+    }
+  } ev{e0, e1, nullptr};
+  GG_CUDA(cudaEventRecord(e0, s));
+  GG_CUDA(cudaMemsetAsync(dnredo.p, 0, sizeof(int), s));
+  k_br_rho<<<dim3(nw, nw), 128, 0, s>>>(nw, o.dPF.p, o.dQF.p, o.ld, o.dMF.p, np, drho.p);
+  ::gg::note_launch();
+  k_br_heads<<<(R + 127) / 128, 128, 0, s>>>(drows.p, R, type, drho.p, nw, np, g.dR.p, g.dRP.p, g.dPow.p, g.q,
+                                            dheads.p);
+  ::gg::note_launch();
+  std::vector<unsigned char> heads((size_t)3 * R);
+  GG_CUDA(cudaMemcpyAsync(heads.data(), dheads.p, heads.size(), cudaMemcpyDeviceToHost, s));
+  cudaEvent_t eh = nullptr;
+  GG_CUDA(cudaEventCreateWithFlags(&eh, cudaEventDisableTiming));
+  ev.c = eh;
+  GG_CUDA(cudaEventRecord(eh, s));
+  if (nb > 0) {
+    k_bessel<<<nb, 128, 0, s>>>(dbd.p, g.dR.p, std::min(maxm, g.n), np, P.epsi, dBJ.p, dBN.p);
+    ::gg::note_launch();
+  }
+  DBuf<BrBucket> dbk;
+  DBuf<BrEnt> dents;
+  DBuf<double> dxt, dkv;
+  if (plain) {
+    k_br_elem<<<dim3(R / 32, (maxm + 32) / 32), dim3(32, 8), 0, s>>>(drows.p, A, drho.p, nw, np, g.dR.p, g.dRP.p,
+                                                                    g.dRPOR.p, g.dPow.p, dBJ.p, dBN.p);
+    ::gg::note_launch();
+    k_br_chains<<<dim3(R / 32, nset + nch, 4), dim3(32, BR_SEG), 0, s>>>(drows.p, A, g.q);
+    ::gg::note_launch();
+    BrFold fold;
+    for (int f = 0; f < 4; ++f) {
+      const double pat[4] = {g.q.C4, g.q.C2, g.q.C3, g.q.C2}, inc[5] = {g.q.C1, g.q.C2, g.q.C3, g.q.C2, g.q.C1};
+      for (int t = 0; t < 5; ++t) fold.w[f][t] = inc[t] * pat[(f + t) & 3];
+    }
+    k_br_base<<<dim3(R / 32, (j0 + 31) / 32, nset), dim3(32, 8), 0, s>>>(drows.p, A, g.q, fold);
+    ::gg::note_launch();
+    GG_CUDA(cudaEventSynchronize(eh));
+
+    // buckets: the columns of each (set, k) by (MTP, head as a source)
+    bool moving = false;
+    for (const BrRow &r : rows) moving |= r.a && std::fabs(r.w) >= 1.0e-10;
+    std::vector<BrBucket> bk;
+    std::vector<BrEnt> ents;
+    std::vector<int> cols;
+    long long xt = 0, kv = 0;
+    int maxpad = 0, split = 0;  // ents[0, split): set 0
+    for (int set = 0; set < nset; ++set) {
+      const int op = type == 1 ? 0 : set == 0 ? 2 : moving ? 0 : 1;
+      const int ac = (type == 2 && set == 1) ? 2 : 1;
+      for (int K = 0; K <= j2max; ++K) {
+        const int n = cnt[K], pad = (K < j2max ? lo[K + 1] : R) - lo[K];
+        if (n == 0) continue;
+        maxpad = std::max(maxpad, pad);
+        cols.resize(n);
+        for (int c = 0; c < n; ++c) cols[c] = c;
+        auto key = [&](int c) { return (int)rows[lo[K] + c].mtp * 8 + heads[(size_t)3 * (lo[K] + c) + op]; };
+        std::stable_sort(cols.begin(), cols.end(), [&](int x, int y) { return key(x) > key(y); });
+        for (int c = 0; c < n;) {
+          int e = c;
+          while (e < n && key(cols[e]) == key(cols[c])) ++e;
+          const int m = rows[lo[K] + cols[c]].mtp, h = heads[(size_t)3 * (lo[K] + cols[c]) + op];
+          bk.push_back(BrBucket{lo[K], n, pad, m, h, set, xt, kv});
+          const int tiles = (e - c + BR_NC - 1) / BR_NC;
+          for (int t = 0; t < tiles; ++t) {  // columns shared out evenly
+            BrEnt E{};
+            E.lo = lo[K];
+            E.P = n;
+            E.pad = pad;
+            E.m = m;
+            E.h = h;
+            E.set = set;
+            const int b0 = c + (e - c) * t / tiles, b1 = c + (e - c) * (t + 1) / tiles;
+            E.nc = b1 - b0;
+            for (int u = 0; u < E.nc; ++u) E.col[u] = cols[b0 + u];
+            E.xt = xt;
+            E.kv = kv;
+            E.g = g0[K] + (long long)set * gsz;
+            ents.push_back(E);
+          }
+          xt += (long long)((m - j0 + 1) & ~1) * pad;
+          kv += 8LL * ac * pad;
+          c = e;
+        }
+      }
+      if (set == 0) split = (int)ents.size();
+    }
+    GG_TRY(upload_vec(dbk, bk, s));
+    GG_TRY(upload_vec(dents, ents, s));
+    GG_TRY(dxt.alloc((size_t)xt));
+    GG_TRY(dkv.alloc((size_t)kv));
+    const int yt = (maxpad + 127) / 128;
+    k_br_tail<<<dim3((unsigned)bk.size(), yt), 128, 0, s>>>(dbk.p, drows.p, A, g.q, dxt.p, dkv.p);
+    ::gg::note_launch();
+    k_br_gemm<1><<<dim3((unsigned)split, maxpad / 32), 128, 0, s>>>(dents.p, drows.p, A, type == 1 ? 0 : 2, drho.p, nw, np, dxt.p,
+                                                          dkv.p, g.dHead.p, g.q, dG.p);
+    ::gg::note_launch();
+    if (nset == 2) {
+      k_br_gemm<2><<<dim3((unsigned)(ents.size() - split), maxpad / 32), 128, 0, s>>>(dents.p + split, drows.p, A, 0, drho.p, nw,
+                                                                            np, dxt.p, dkv.p, g.dHead.p, g.q, dG.p);
+      ::gg::note_launch();
+    }
+  }
+  DBuf<BrRedo> dredo;
+  GG_TRY(dredo.alloc(ni));
+  k_br_table<<<R, 128, 0, s>>>(drows.p, drank.p, plain ? dG.p : nullptr, dG.p + (nset == 2 ? gsz : 0), dg0.p, KEY, dind.p, dval.p,
+                               dredo.p, dnredo.p);
+  ::gg::note_launch();
+  GG_CUDA(cudaGetLastError());
+  int nredo = 0;
+  GG_CUDA(cudaMemcpyAsync(&nredo, dnredo.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaMemcpyAsync(T.hInd.data(), dind.p, ni * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  *plan_ms = 1e3 * std::chrono::duration<double>(std::chrono::steady_clock::now() - th0).count();
+  GG_CUDA(cudaStreamSynchronize(s));
+  if (nredo > 0) {
+    // k_bessel ran to the longest orbital, which covers every term
+    DBuf<double> dv, dout;
+    DBuf<BrInt> dints;
+    GG_TRY(dv.alloc((size_t)4 * nredo));
+    GG_TRY(dout.alloc(nredo));
+    GG_TRY(dints.alloc(nredo));
+    const TermTabs tt{o.dPF.p, o.dQF.p, o.ld, o.dMF.p, g.dR.p, g.dRP.p, g.dRPOR.p, g.dPow.p, np, dBJ.p, dBN.p};
+    k_br_redo<<<(unsigned)((4LL * nredo + 127) / 128), 128, 0, s>>>(type, dredo.p, nredo, drows.p, P.tabs(), tt, g.q,
+                                                                   dv.p, dints.p);
+    ::gg::note_launch();
+    k_breit_combine<<<(nredo + 255) / 256, 256, 0, s>>>(dints.p, nredo, dv.p, dout.p);
+    ::gg::note_launch();
+    k_br_redo_store<<<(nredo + 255) / 256, 256, 0, s>>>(dredo.p, nredo, dout.p, dval.p);
+    ::gg::note_launch();
+    GG_CUDA(cudaGetLastError());
+  }
+  ctx->stats[34] = nredo;
+  GG_CUDA(cudaEventRecord(e1, s));
+  GG_CUDA(cudaMemcpyAsync(T.hVal.data(), dval.p, ni * sizeof(double), cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaStreamSynchronize(s));
+  float ms = 0.f;
+  cudaEventElapsedTime(&ms, e0, e1);
+  *kernel_ms = ms;
   return GG_OK;
 }
 
@@ -701,7 +1563,6 @@ int gg_genintbreit(gg_ctx *ctx, int type, double wfact, const double *e, double 
   Plan P;
   GG_TRY(make_plan(ctx, wfact, e, accy, P));
   GG_TRY(timer_start(ctx));
-  const auto th0 = std::chrono::steady_clock::now();
   const Orbitals &o = ctx->orb;
   const int nw = o.nw;
   int j2max = o.nkj[1];
@@ -738,45 +1599,7 @@ int gg_genintbreit(gg_ctx *ctx, int type, double wfact, const double *e, double 
         mask[(size_t)K * msz + (size_t)a * (nw + 1) + b] = m;
       }
   GG_TRY(P.upload(s));
-  DBuf<unsigned char> dmask;
-  GG_TRY(upload_vec(dmask, mask, s));
-  const int rows = (j2max + 1) * nw * nw;
-  DBuf<int> dci, dcj;
-  GG_TRY(dci.alloc(rows));
-  GG_TRY(dcj.alloc(rows));
-  k_plan_table<<<(rows + 127) / 128, 128, 0, s>>>(type, nw, j2max, dmask.p, P.tabs(), 0, dci.p, dcj.p, nullptr,
-                                                  nullptr, nullptr, nullptr, nullptr);
-  ::gg::note_launch();
-  GG_CUDA(cudaGetLastError());
-  std::vector<int> ci(rows), cj(rows);
-  GG_CUDA(cudaMemcpyAsync(ci.data(), dci.p, rows * sizeof(int), cudaMemcpyDeviceToHost, s));
-  GG_CUDA(cudaMemcpyAsync(cj.data(), dcj.p, rows * sizeof(int), cudaMemcpyDeviceToHost, s));
-  GG_CUDA(cudaStreamSynchronize(s));
-  std::vector<int64_t> oi, oj;
-  const int64_t ni = scan(ci, oi), nj = scan(cj, oj);
-  if (ni > INT32_MAX || nj > INT32_MAX) return fail(GG_ERR_RANGE, "gg_genintbreit: table too large");
-  T.kstart.assign(j2max + 2, 1);
-  for (int K = 0; K <= j2max; ++K) T.kstart[K + 1] = (int32_t)((K + 1 <= j2max ? oi[(size_t)(K + 1) * nw * nw] : ni) + 1);
-  DBuf<int64_t> doi, doj;
-  DBuf<int32_t> dind;
-  DBuf<BrInt> dints;
-  DBuf<BrJob> djobs;
-  GG_TRY(upload_vec(doi, oi, s));
-  GG_TRY(upload_vec(doj, oj, s));
-  GG_TRY(dind.alloc(std::max<int64_t>(1, ni)));
-  GG_TRY(dints.alloc(std::max<int64_t>(1, ni)));
-  GG_TRY(djobs.alloc(std::max<int64_t>(1, nj)));
-  k_plan_table<<<(rows + 127) / 128, 128, 0, s>>>(type, nw, j2max, dmask.p, P.tabs(), 1, nullptr, nullptr, doi.p,
-                                                  doj.p, dind.p, dints.p, djobs.p);
-  ::gg::note_launch();
-  GG_CUDA(cudaGetLastError());
-  T.n = ni;
-  T.hInd.resize(ni);
-  if (ni > 0) GG_CUDA(cudaMemcpyAsync(T.hInd.data(), dind.p, ni * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  ctx->stats[32] = 1e3 * std::chrono::duration<double>(std::chrono::steady_clock::now() - th0).count();
-  T.hVal.assign(std::max<int64_t>(1, ni), 0.0);
-  GG_TRY(run_terms(ctx, P, djobs.p, nj, dints.p, ni, T.hVal.data(), &ctx->stats[33]));
-  T.hVal.resize(ni);
+  GG_TRY(run_table(ctx, type, P, j2max, mask, T, &ctx->stats[32], &ctx->stats[33]));
   T.valid = true;
   double ms = 0;
   GG_TRY(timer_stop(ctx, &ms));
