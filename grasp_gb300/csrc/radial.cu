@@ -877,166 +877,75 @@ __global__ void k_quad_table(const QuadItem *__restrict__ items, const int *__re
   }
 }
 
-// YPOT / XPOT (rmcdhf90/ypot.f90:35-49, xpot.f90:31-54): one thread per grid
-// point combines the list's Y functions in the list's order (the reference's
-// per-point operations: YP = YP - COEFF*TB; CTB = COEFF*TB, XP += CTB*QF,
-// XQ -= CTB*PF, with COEFF = XA/C). One launch takes the lists of several
-// jobs (blockIdx.y); each thread loads the next group of terms (index,
-// coefficient, Y value, orbital values; 16 for YPOT, 8 for XPOT) before it
-// combines the current ones, so the loads do not wait on the chain.
-struct PotSeg {
-  const int *fidx, *iorb;
+// YPOT / XPOT (rmcdhf90/ypot.f90:35-49, xpot.f90:31-54): sum_t COEFF TB (YPOT),
+// sum_t CTB QF and sum_t CTB PF with CTB = COEFF TB (XPOT), cut into chunks of
+// terms. A block takes 64 grid points of one chunk, its four rows of threads
+// every fourth term; the rows' sums meet in shared memory and the chunk's are
+// stored for k_pot_final, which adds them in list order. Bound: the FP64 pipe
+// (three operations per XPOT term and point; 34 subshells' lists of 6,600 terms
+// 35 us per orbital). One thread per point adding the terms in list order
+// left the pipe to one dependent addition per term: 233 us for the same list.
+constexpr int POT_CHUNK = 128;  // terms staged in shared memory at a time
+struct PotChunk {
+  const int *key, *iorb;  // iorb null: YPOT
   const double *coef;
-  double *out0, *out1;
-  int ncof;
-};
-template <int MODE>
-__global__ void k_potential(const PotSeg *__restrict__ segs, const double *__restrict__ Y, int np,
-                            const double *__restrict__ ZZ, const double *__restrict__ PF,
-                            const double *__restrict__ QF, int ld, int n) {
-  constexpr int A = MODE == 0 ? 16 : 8;  // terms loaded ahead
-  const PotSeg g = segs[blockIdx.y];
-  const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > n) return;
-  const int nc = g.ncof;
-  double cy[A], cc[A], cq[A], cp[A];
-  double ny[A], nc_[A], nq[A], npf[A];
-  // terms t0 .. t0 + A - 1 (those below nc when `guard`)
-  auto load = [&](int t0, bool guard, double *y, double *c, double *qv, double *pv) {
-#pragma unroll
-    for (int u = 0; u < A; ++u) {
-      const int t = t0 + u;
-      y[u] = c[u] = qv[u] = pv[u] = 0.0;
-      if (!guard || t < nc) {
-        c[u] = g.coef[t];
-        y[u] = Y[(size_t)g.fidx[t] * np + i];
-        if (MODE == 1) {
-          const int io = g.iorb[t];
-          qv[u] = pf(QF, ld, i, io);
-          pv[u] = pf(PF, ld, i, io);
-        }
-      }
-    }
-  };
-  double a0 = (MODE == 0) ? ZZ[i] : 0.0, a1 = 0.0;
-  auto combine = [&](int t0, const double *y, const double *c, const double *qv, const double *pv) {
-#pragma unroll
-    for (int u = 0; u < A; ++u)
-      if (t0 + u < nc) {
-        if (MODE == 0) {
-          a0 = a0 - c[u] * y[u];
-        } else {
-          const double ctb = c[u] * y[u];
-          a0 = a0 + ctb * qv[u];
-          a1 = a1 - ctb * pv[u];
-        }
-      }
-  };
-  load(0, true, cy, cc, cq, cp);
-  int t = 0;
-  // while the next group is complete its loads need no bounds test
-  for (; t + 2 * A <= nc; t += A) {
-    load(t + A, false, ny, nc_, nq, npf);
-    combine(t, cy, cc, cq, cp);
-#pragma unroll
-    for (int u = 0; u < A; ++u) {
-      cy[u] = ny[u];
-      cc[u] = nc_[u];
-      cq[u] = nq[u];
-      cp[u] = npf[u];
-    }
-  }
-  if (t + A <= nc) {  // cur is complete; fewer than A terms follow it
-    load(t + A, true, ny, nc_, nq, npf);
-    combine(t, cy, cc, cq, cp);
-    combine(t + A, ny, nc_, nq, npf);
-  } else {
-    combine(t, cy, cc, cq, cp);
-  }
-  g.out0[i - 1] = a0;
-  if (MODE == 1) g.out1[i - 1] = a1;
-}
-
-// XPOT in two passes for long lists: the products of a segment of terms at
-// every grid point (CTB = COEFF TB, CTB QF and CTB PF) by all SMs, then per
-// grid point the sums XP = XP + CTB QF, XQ = XQ - CTB PF in list order (the
-// same operations as k_potential; only the additions stay sequential). A
-// segment is terms t0 .. t0+nt of one job's list; one launch takes the
-// segments of several jobs (blockIdx.y / blockIdx.z).
-struct XSeg {
-  const int *fidx, *iorb;
-  const double *coef;
-  double *P1, *P2;  // nt * n products each
-  double *xp, *xq;
+  size_t out;             // where its n sums (YPOT) or 2 n (XPOT) go
   int nt;
 };
-__global__ void k_xprod(const XSeg *__restrict__ segs, const double *__restrict__ Y, int np,
-                        const double *__restrict__ PF, const double *__restrict__ QF, int ld, int n) {
-  const XSeg g = segs[blockIdx.y];
-  const int tot = g.nt * n;  // the caller keeps nt * n below 2^26
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += gridDim.x * blockDim.x) {
-    const int t = e / n, i = e % n + 1;
-    const double ctb = g.coef[t] * Y[(size_t)g.fidx[t] * np + i];
-    g.P1[e] = ctb * pf(QF, ld, i, g.iorb[t]);
-    g.P2[e] = ctb * pf(PF, ld, i, g.iorb[t]);
+__global__ void __launch_bounds__(256) k_pot_part(const PotChunk *__restrict__ ch, const int *__restrict__ tab,
+                                                  const double *__restrict__ Y, int np,
+                                                  const double *__restrict__ PF, const double *__restrict__ QF,
+                                                  int ld, int n, double *__restrict__ part) {
+  __shared__ int sf[POT_CHUNK], so[POT_CHUNK];
+  __shared__ double sc[POT_CHUNK], red[2][4][64];
+  const PotChunk g = ch[blockIdx.y];
+  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+  const int i = 1 + blockIdx.x * 64 + tx;
+  const bool x = g.iorb != nullptr, in = i <= n;
+  double a0 = 0.0, a1 = 0.0;
+  for (int t0 = 0; t0 < g.nt; t0 += POT_CHUNK) {
+    const int nt = min(POT_CHUNK, g.nt - t0);
+    __syncthreads();
+    if ((int)threadIdx.x < nt) {
+      sf[threadIdx.x] = tab[g.key[t0 + threadIdx.x]] - 1;
+      so[threadIdx.x] = x ? g.iorb[t0 + threadIdx.x] : 1;
+      sc[threadIdx.x] = g.coef[t0 + threadIdx.x];
+    }
+    __syncthreads();
+    if (!in) continue;
+    if (x) {
+#pragma unroll 8
+      for (int t = ty; t < nt; t += 4) {
+        const double ctb = sc[t] * __ldg(Y + (size_t)sf[t] * np + i);
+        a0 = fma(ctb, pf(QF, ld, i, so[t]), a0);
+        a1 = fma(ctb, pf(PF, ld, i, so[t]), a1);
+      }
+    } else {
+#pragma unroll 8
+      for (int t = ty; t < nt; t += 4) a0 = fma(sc[t], __ldg(Y + (size_t)sf[t] * np + i), a0);
+    }
   }
-}
-// k_xsum: 32 grid points of segment blockIdx.z per block; blockIdx.y = 0
-// sums XP = XP + P1, blockIdx.y = 1 sums XQ = XQ - P2. The loads run XSUM_AHEAD terms ahead of
-// the additions (register double buffer) so that the chain of dependent
-// FP64 additions, not the load latency, sets the time.
-constexpr int XSUM_AHEAD = 48;
-template <bool SUB>
-__device__ __forceinline__ double xsum_chain(double acc, const double *__restrict__ P, int nt, int n) {
-  constexpr int A = XSUM_AHEAD;
-  double cur[A], nxt[A];
-#pragma unroll
-  for (int u = 0; u < A; ++u) cur[u] = (u < nt) ? P[(size_t)u * n] : 0.0;
-  int t = 0;
-  // while the next group is complete its loads need no bounds test
-  for (; t + 2 * A <= nt; t += A) {
-    const double *q = P + (size_t)(t + A) * n;
-#pragma unroll
-    for (int u = 0; u < A; ++u) nxt[u] = q[(size_t)u * n];
-#pragma unroll
-    for (int u = 0; u < A; ++u) acc = SUB ? acc - cur[u] : acc + cur[u];
-#pragma unroll
-    for (int u = 0; u < A; ++u) cur[u] = nxt[u];
-  }
-  if (t + A <= nt) {  // cur is a complete group; fewer than A terms follow it
-    const int t1 = t + A;
-#pragma unroll
-    for (int u = 0; u < A; ++u) nxt[u] = (t1 + u < nt) ? P[(size_t)(t1 + u) * n] : 0.0;
-#pragma unroll
-    for (int u = 0; u < A; ++u) acc = SUB ? acc - cur[u] : acc + cur[u];
-#pragma unroll
-    for (int u = 0; u < A; ++u)
-      if (t1 + u < nt) acc = SUB ? acc - nxt[u] : acc + nxt[u];
-  } else {  // fewer than A terms in all
-#pragma unroll
-    for (int u = 0; u < A; ++u)
-      if (t + u < nt) acc = SUB ? acc - cur[u] : acc + cur[u];
-  }
-  return acc;
-}
-__global__ void k_xsum(const XSeg *__restrict__ segs, int n) {
-  const XSeg g = segs[blockIdx.z];
-  const int i = blockIdx.x * 32 + threadIdx.x;
-  if (i >= n) return;
-  if (blockIdx.y == 0)
-    g.xp[i] = xsum_chain<false>(g.xp[i], g.P1 + i, g.nt, n);
-  else
-    g.xq[i] = xsum_chain<true>(g.xq[i], g.P2 + i, g.nt, n);
+  red[0][ty][tx] = a0;
+  red[1][ty][tx] = a1;
+  __syncthreads();
+  if (ty < (x ? 2 : 1) && in)
+    part[g.out + (size_t)ty * n + i - 1] = (red[ty][0][tx] + red[ty][1][tx]) + (red[ty][2][tx] + red[ty][3][tx]);
 }
 
 // The lists' labels decoded on the device, one thread per term (mode 0:
 // YPOT labels, 1: XPOT labels): the term's (K, a, b) key into a dense table
-// over K <= KLIMIT and the orbital pairs, marked present; the orbital it
-// multiplies (XPOT) and COEFF (XPOT: XA/C, as the reference forms it). A
-// label outside the orbital set or with K above KLIMIT sets *err.
+// over K <= KLIMIT and the orbital pairs; the orbital it multiplies (XPOT) and
+// COEFF (XPOT: XA/C, as the reference forms it). The first term of a key
+// takes the next function number (info[0]), writes its YZK descriptor and
+// leaves the number + 1 in the table. The numbers depend on the order in
+// which the threads run, no value does: every term finds its function by its
+// key. (Marking the keys and numbering them by one block in table order took
+// 16 us of a 34-subshell COFPOT call.) A label outside the orbital set or
+// with K above KLIMIT sets info[1].
 __global__ void k_parse_terms(int mode, int64_t nt, const int32_t *__restrict__ lab, const double *__restrict__ co,
-                              int nw, double c, int *__restrict__ tab, int *__restrict__ key,
-                              int *__restrict__ iorb, double *__restrict__ coef, int *__restrict__ err) {
+                              int nw, double c, const int *__restrict__ MF, int n, int *__restrict__ tab,
+                              YDesc *__restrict__ yd, int *__restrict__ key, int *__restrict__ iorb,
+                              double *__restrict__ coef, int *__restrict__ info) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nt; e += (int64_t)gridDim.x * blockDim.x) {
     const int32_t l0 = lab[e];
     int64_t l = l0;
@@ -1047,52 +956,22 @@ __global__ void k_parse_terms(int mode, int64_t nt, const int32_t *__restrict__ 
     const int64_t b = mode == 0 ? l : l % KEYORB;
     const int64_t io = mode == 0 ? 1 : l / KEYORB;
     if (l0 < 0 || k > KLIMIT || a < 1 || a > nw || b < 1 || b > nw || io < 1 || io > nw) {
-      atomicOr(err, 1);
+      atomicOr(info + 1, 1);
       key[e] = 0;
       iorb[e] = 1;
       coef[e] = 0.0;
       continue;
     }
     const int kk = (k * nw + (a - 1)) * nw + (int)(b - 1);
-    tab[kk] = 1;
+    if (atomicCAS(tab + kk, 0, -1) == 0) {
+      const int f = atomicAdd(info, 1);
+      yd[f] = YDesc{k, a, (int)b, min(MF[a], MF[b]), n, 0, 1};
+      tab[kk] = f + 1;
+    }
     key[e] = kk;
     iorb[e] = (int)io;
     coef[e] = mode == 0 ? co[e] : co[e] / c;
   }
-}
-
-// numbers the table's present (K, a, b) in table order (one block): the
-// entry becomes its function index + 1, the function's YZK descriptor is
-// written there, info[0] = the number of functions
-__global__ void __launch_bounds__(1024) k_number_functions(int *__restrict__ tab, int size, int nw,
-                                                            const int *__restrict__ MF, int n,
-                                                            YDesc *__restrict__ yd, int *__restrict__ info) {
-  __shared__ int part[1024];
-  const int per = (size + 1023) / 1024, lo = threadIdx.x * per, hi = min(size, lo + per);
-  int cnt = 0;
-  for (int e = lo; e < hi; ++e) cnt += tab[e] != 0;
-  part[threadIdx.x] = cnt;
-  __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {  // inclusive scan of the counts
-    const int v = threadIdx.x >= (unsigned)off ? part[threadIdx.x - off] : 0;
-    __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
-  }
-  int f = part[threadIdx.x] - cnt;
-  for (int e = lo; e < hi; ++e)
-    if (tab[e]) {
-      const int k = e / (nw * nw), a = (e / nw) % nw + 1, b = e % nw + 1;
-      yd[f] = YDesc{k, a, b, min(MF[a], MF[b]), n, 0, 1};
-      tab[e] = ++f;
-    }
-  if (threadIdx.x == 1023) info[0] = part[1023];
-}
-
-__global__ void k_term_functions(int64_t nt, const int *__restrict__ key, const int *__restrict__ tab,
-                                 int *__restrict__ fidx) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nt; e += (int64_t)gridDim.x * blockDim.x)
-    fidx[e] = tab[key[e]] - 1;
 }
 
 // DPBDT (lib9290/dpbdt.f90:39-99): 13-point derivative of orbital J at grid
@@ -1134,69 +1013,79 @@ __device__ void dpbdt_warp(const double *PF, const double *QF, int ld, int J, co
   }
 }
 
+// One orbital's potentials at each grid point from its lists' chunk sums:
+//   YP = ZZ - sum, XP = sum CTB QF, XQ = -sum CTB PF (the chunks in list order);
 // LAGCON (rmcdhf90/lagcon.f90:46-55): per multiplier in list order,
-// XP(I) = XP(I) + WARI QF(I,M), XQ(I) = XQ(I) - WARI PF(I,M), WARI = WA R(I),
-// I = 1..MF(M); mo[t] = M and wa[t] = ECV WB of the multipliers the host kept
-// (those of pairs with this orbital, |WA| >= EPS). xp, xq 0-based.
-// One job's LAGCON or DACON list (blockIdx.y selects the job): the entries'
-// orbitals and weights, and the job's XP, XQ.
-struct TermSeg {
-  const int *idx;
-  const double *w;
-  double *xp, *xq;
-  int nt;
-};
-__global__ void k_lagcon(const TermSeg *__restrict__ segs, int n, const int *__restrict__ MF,
-                         const double *__restrict__ R, const double *__restrict__ PF, const double *__restrict__ QF,
-                         int ld) {
-  const TermSeg g = segs[blockIdx.y];
-  const int nt = g.nt, *mo = g.idx;
-  const double *wa = g.w;
-  double *xp = g.xp, *xq = g.xq;
-  for (int i = 1 + blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
-    double p = xp[i - 1], qv = xq[i - 1];
-    for (int t = 0; t < nt; ++t) {
-      const int M = mo[t];
-      if (i > MF[M]) continue;
-      const double wari = wa[t] * R[i];
-      p = p + wari * pf(QF, ld, i, M);
-      qv = qv - wari * pf(PF, ld, i, M);
-    }
-    xp[i - 1] = p;
-    xq[i - 1] = qv;
-  }
-}
-
+//   XP = XP + WARI QF(I,M), XQ = XQ - WARI PF(I,M), WARI = WA R(I), I <= MF(M);
+//   lag[t] = M and lag_w[t] = ECV WB of the multipliers the host kept (those of
+//   pairs with this orbital, |WA| >= EPS);
 // DACON (rmcdhf90/dacon.f90:25-46): per entry of the list in order, with TA,
-// TB = DPBDT(IORB) at the point, for I = 2..MF(IORB):
+//   TB = DPBDT(IORB) at the point, for I = 2..MF(IORB):
 //   XP(I) += COEFF (TA RPORII + FK PFI - (2C R(I) + ZBCI) QFI),
 //   XQ(I) += COEFF (TB RPORII - FK QFI + ZBCI PFI),
-// RPORII = 1/(H RPOR(I)), ZBCI = ZZ(I)/C, FK = kappa(IORB). xp, xq 0-based.
-__global__ void k_dacon(const TermSeg *__restrict__ segs, int n, const int *__restrict__ NAK,
-                        const int *__restrict__ MF, const double *__restrict__ R, const double *__restrict__ RPOR,
-                        const double *__restrict__ ZZ, const double *__restrict__ PF, const double *__restrict__ QF,
-                        int ld, QuadConst q) {
-  const TermSeg g = segs[blockIdx.y];
-  const int nd = g.nt, *nda = g.idx;
-  const double *da = g.w;
-  double *xp = g.xp, *xq = g.xq;
-  const double twoc = q.c + q.c;
-  for (int i = 2 + blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
-    double p = xp[i - 1], qv = xq[i - 1];
-    for (int t = 0; t < nd; ++t) {
-      const int io = nda[t];
-      if (i > MF[io]) continue;
-      double ta, tb;
-      dpbdt_point(PF, QF, ld, io, q, i, ta, tb);
-      const double coeff = da[t], fk = (double)NAK[io];
-      const double rporii = 1.0 / (q.h * RPOR[i]);
-      const double pfi = pf(PF, ld, i, io), qfi = pf(QF, ld, i, io);
-      const double zbci = ZZ[i] / q.c;
-      p = p + coeff * (ta * rporii + fk * pfi - (twoc * R[i] + zbci) * qfi);
-      qv = qv + coeff * (tb * rporii - fk * qfi + zbci * pfi);
+//   RPORII = 1/(H RPOR(I)), ZBCI = ZZ(I)/C, FK = kappa(IORB).
+struct PotFinal {
+  double *out;  // YP, XP, XQ: n each
+  size_t yc, xc;  // the lists' chunk sums
+  int nyc, nxc;
+  const int *lag, *da;
+  const double *lag_w, *da_w;
+  int nlag, nda;
+};
+// A block takes 32 points, its PF_ROWS rows of threads every PF_ROWS-th chunk,
+// multiplier and DACON entry; the rows' sums are added in row order.
+constexpr int PF_ROWS = 8;
+__global__ void __launch_bounds__(32 * PF_ROWS) k_pot_final(const PotFinal *__restrict__ jobs,
+                                                            const double *__restrict__ part, int n,
+                                                            const int *__restrict__ NAK, const int *__restrict__ MF,
+                                                            const double *__restrict__ R,
+                                                            const double *__restrict__ RPOR,
+                                                            const double *__restrict__ ZZ,
+                                                            const double *__restrict__ PF,
+                                                            const double *__restrict__ QF, int ld, QuadConst q) {
+  __shared__ double red[3][PF_ROWS][32];
+  const PotFinal g = jobs[blockIdx.y];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int i = 1 + blockIdx.x * 32 + tx;
+  double y = 0.0, p = 0.0, m = 0.0;
+  if (i <= n) {
+    const double *yc = part + g.yc + i - 1, *xc = part + g.xc + i - 1;
+    for (int c = ty; c < g.nyc; c += PF_ROWS) y += __ldg(yc + (size_t)c * n);
+#pragma unroll 4
+    for (int c = ty; c < g.nxc; c += PF_ROWS) {
+      p += __ldg(xc + (size_t)2 * c * n);
+      m -= __ldg(xc + (size_t)(2 * c + 1) * n);
     }
-    xp[i - 1] = p;
-    xq[i - 1] = qv;
+    for (int t = ty; t < g.nlag; t += PF_ROWS) {
+      const int M = g.lag[t];
+      if (i > MF[M]) continue;
+      const double wari = g.lag_w[t] * R[i];
+      p = p + wari * pf(QF, ld, i, M);
+      m = m - wari * pf(PF, ld, i, M);
+    }
+    if (ty < g.nda && i >= 2) {
+      const double twoc = q.c + q.c, rporii = 1.0 / (q.h * RPOR[i]), zbci = ZZ[i] / q.c;
+      for (int t = ty; t < g.nda; t += PF_ROWS) {
+        const int io = g.da[t];
+        if (i > MF[io]) continue;
+        double ta, tb;
+        dpbdt_point(PF, QF, ld, io, q, i, ta, tb);
+        const double coeff = g.da_w[t], fk = (double)NAK[io];
+        const double pfi = pf(PF, ld, i, io), qfi = pf(QF, ld, i, io);
+        p = p + coeff * (ta * rporii + fk * pfi - (twoc * R[i] + zbci) * qfi);
+        m = m + coeff * (tb * rporii - fk * qfi + zbci * pfi);
+      }
+    }
+  }
+  red[0][ty][tx] = y;
+  red[1][ty][tx] = p;
+  red[2][ty][tx] = m;
+  __syncthreads();
+  if (ty < 3 && i <= n) {
+    double v = red[ty][0][tx];
+#pragma unroll
+    for (int r = 1; r < PF_ROWS; ++r) v += red[ty][r][tx];
+    g.out[(size_t)ty * n + i - 1] = ty == 0 ? ZZ[i] - v : v;
   }
 }
 
@@ -1971,10 +1860,6 @@ static int raw_list(int ncof, const int32_t *lab, const double *co, RawList &r) 
   return GG_OK;
 }
 
-// XPOT lists at least this long take the two-pass form (products by all
-// SMs, then the per-point sums, all such lists of one call together)
-constexpr int XPOT_SPLIT = 512;
-
 // One orbital's potentials on the device: YP, XP, XQ (N each, 0-based) at
 // out, out + n, out + 2 n.
 struct PotJob {
@@ -2021,16 +1906,16 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, DBuf<dou
   }
   const size_t tsize = (size_t)(KLIMIT + 1) * nw * nw;
   DBuf<char> draw;
-  DBuf<int> dterm, dtab, dinfo;  // dterm: key, orbital, function index per term
+  DBuf<int> dterm, dtab, dinfo;  // dterm: key, orbital per term
   DBuf<double> dcoef;
   DBuf<YDesc> dy;
   GG_TRY(draw.alloc(std::max<size_t>(need, 16)));
-  GG_TRY(dterm.alloc(3 * std::max<size_t>(T, 1)));
+  GG_TRY(dterm.alloc(2 * std::max<size_t>(T, 1)));
   GG_TRY(dcoef.alloc(std::max<size_t>(T, 1)));
   GG_TRY(dtab.alloc(tsize));
   GG_TRY(dinfo.alloc(2));
   GG_TRY(dy.alloc(std::max<size_t>(1, std::min(T, tsize))));
-  int *dkey = dterm.p, *diorb = dkey + std::max<size_t>(T, 1), *dfidx = diorb + std::max<size_t>(T, 1);
+  int *dkey = dterm.p, *diorb = dkey + std::max<size_t>(T, 1);
   const int32_t *dlab = reinterpret_cast<const int32_t *>(draw.p);
   const double *dco = reinterpret_cast<const double *>(draw.p + lab_bytes);
   if (T > 0) GG_CUDA(cudaMemcpyAsync(draw.p, stage, need, cudaMemcpyHostToDevice, s));
@@ -2040,20 +1925,14 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, DBuf<dou
   for (int m = 0; m < 2; ++m) {
     const size_t a = m == 0 ? 0 : TY, cnt = m == 0 ? TY : T - TY;
     if (cnt == 0) continue;
-    k_parse_terms<<<pgrid, 256, 0, s>>>(m, (int64_t)cnt, dlab + a, dco + a, nw, g.c, dtab.p, dkey + a, diorb + a,
-                                        dcoef.p + a, dinfo.p + 1);
+    k_parse_terms<<<pgrid, 256, 0, s>>>(m, (int64_t)cnt, dlab + a, dco + a, nw, g.c, o.dMF.p, n, dtab.p, dy.p,
+                                        dkey + a, diorb + a, dcoef.p + a, dinfo.p);
     ::gg::note_launch();
   }
-  k_number_functions<<<1, 1024, 0, s>>>(dtab.p, (int)tsize, nw, o.dMF.p, n, dy.p, dinfo.p);
-  ::gg::note_launch();
   int info[2] = {0, 0};
   GG_CUDA(cudaMemcpyAsync(info, dinfo.p, sizeof(info), cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaStreamSynchronize(s));
   if (info[1]) return fail(GG_ERR_ARG, "potential: label outside the orbital set or K above 20");
-  if (T > 0) {
-    k_term_functions<<<pgrid, 256, 0, s>>>((int64_t)T, dkey, dtab.p, dfidx);
-    ::gg::note_launch();
-  }
   const int nf = std::max(1, info[0]);
   DBuf<double> dY, scratch;
   GG_TRY(dY.alloc((size_t)nf * g.np));
@@ -2071,119 +1950,50 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, DBuf<dou
     off[j] = Off{pi(J.nda), pd(J.da), pi(J.lag_m), pd(J.lag_wa)};
   }
   DBuf<int> di;
-  DBuf<double> dd, prod;
+  DBuf<double> dd, dpart;
   GG_TRY(upload(di, ih, s));
   GG_TRY(upload(dd, dh, s));
-  const unsigned blocks = (unsigned)((n + 127) / 128);
-  GG_CUDA(cudaMemsetAsync(dPot.p, 0, (size_t)3 * n * jobs.size() * sizeof(double), s));
-  // YPOT of every job and the short XPOT lists: one launch each
-  std::vector<int> longj;  // jobs whose XPOT takes the two-pass form
-  std::vector<PotSeg> hp;
+  // every list cut into chunks (a few thousand at most), one launch for all
+  // of them, then one for every job's point values
+  const int len = (int)(POT_CHUNK * (T / ((size_t)POT_CHUNK * 16384) + 1));
+  std::vector<PotChunk> hc;
+  std::vector<PotFinal> hf(jobs.size());
+  size_t po = 0;  // partial sums, in doubles
+  auto cut = [&](size_t at, int nt, bool x) {
+    const size_t start = po;
+    for (int t0 = 0; t0 < nt; t0 += len) {
+      hc.push_back(PotChunk{dkey + at + t0, x ? diorb + at + t0 : nullptr, dcoef.p + at + t0,
+                            po, std::min(len, nt - t0)});
+      po += (size_t)(x ? 2 : 1) * n;
+    }
+    return start;
+  };
+  std::vector<size_t> py(jobs.size()), px(jobs.size());
   for (size_t j = 0; j < jobs.size(); ++j) {
-    double *yp = dPot.p + (size_t)3 * n * j;
-    hp.push_back(PotSeg{dfidx + oy[j], nullptr, dcoef.p + oy[j], yp, nullptr, jobs[j].y.n});
+    py[j] = cut(oy[j], jobs[j].y.n, false);
+    px[j] = cut(ox[j], jobs[j].x.n, true);
   }
-  const size_t nyseg = hp.size();
+  GG_TRY(dpart.alloc(po));
   for (size_t j = 0; j < jobs.size(); ++j) {
-    const int nx = jobs[j].x.n;
-    double *xp = dPot.p + (size_t)3 * n * j + n;
-    if (nx >= XPOT_SPLIT)
-      longj.push_back((int)j);
-    else
-      hp.push_back(PotSeg{dfidx + ox[j], diorb + ox[j], dcoef.p + ox[j], xp, xp + n, nx});
+    const PotJob &J = jobs[j];
+    hf[j] = PotFinal{dPot.p + (size_t)3 * n * j, py[j], px[j], (J.y.n + len - 1) / len,
+                     (J.x.n + len - 1) / len, di.p + off[j].lm, di.p + off[j].dn, dd.p + off[j].lw, dd.p + off[j].dd,
+                     (int)J.lag_m.size(), (int)J.nda.size()};
   }
-  DBuf<PotSeg> dpseg;
-  if (!hp.empty()) {
-    GG_TRY(upload(dpseg, hp, s));
-    for (size_t a = 0; a < hp.size(); a += 65535) {  // gridDim.y limit
-      const size_t b = std::min(hp.size(), a + 65535);
-      if (a < nyseg) {
-        const size_t e = std::min(b, nyseg);
-        k_potential<0><<<dim3(blocks, (unsigned)(e - a)), 128, 0, s>>>(dpseg.p + a, dY.p, g.np, g.dZZ.p, o.dPF.p,
-                                                                        o.dQF.p, o.ld, n);
-        ::gg::note_launch();
-      }
-      if (b > nyseg) {
-        const size_t a1 = std::max(a, nyseg);
-        k_potential<1><<<dim3(blocks, (unsigned)(b - a1)), 128, 0, s>>>(dpseg.p + a1, dY.p, g.np, g.dZZ.p, o.dPF.p,
-                                                                         o.dQF.p, o.ld, n);
-        ::gg::note_launch();
-      }
-    }
+  DBuf<PotChunk> dchunk;
+  DBuf<PotFinal> dfin;
+  GG_TRY(upload(dchunk, hc, s));
+  GG_TRY(upload(dfin, hf, s));
+  if (!hc.empty()) {
+    k_pot_part<<<dim3((n + 63) / 64, (unsigned)hc.size()), 256, 0, s>>>(dchunk.p, dtab.p, dY.p, g.np, o.dPF.p, o.dQF.p,
+                                                                       o.ld, n, dpart.p);
+    ::gg::note_launch();
   }
-  // the long lists of all jobs together, in rounds of at most `per` terms of
-  // each job (a job's rounds run in its list's order), each round one
-  // product launch and one sum launch over its segments
-  DBuf<XSeg> dseg;
-  std::vector<size_t> rstart;
-  if (!longj.empty()) {
-    const int64_t round_terms = std::max<int64_t>(1, (512ll << 20) / (16ll * n));
-    const int per = (int)std::max<int64_t>(1, std::min<int64_t>(round_terms / (int64_t)longj.size(), (1 << 26) / n));
-    std::vector<XSeg> hs;
-    std::vector<size_t> poff;
-    size_t maxprod = 0;
-    for (int t0 = 0;; t0 += per) {
-      const size_t r0 = hs.size();
-      size_t po = 0;
-      for (int j : longj) {
-        const int nx = jobs[j].x.n;
-        if (t0 >= nx) continue;
-        const int nt = std::min(per, nx - t0);
-        double *yp = dPot.p + (size_t)3 * n * j;
-        hs.push_back(XSeg{dfidx + ox[j] + t0, diorb + ox[j] + t0, dcoef.p + ox[j] + t0, nullptr, nullptr, yp + n,
-                          yp + 2 * n, nt});
-        poff.push_back(po);
-        po += (size_t)2 * nt * n;
-      }
-      if (hs.size() == r0) break;
-      rstart.push_back(r0);
-      maxprod = std::max(maxprod, po);
-    }
-    rstart.push_back(hs.size());
-    GG_TRY(prod.alloc(maxprod));
-    for (size_t e = 0; e < hs.size(); ++e) {
-      hs[e].P1 = prod.p + poff[e];
-      hs[e].P2 = hs[e].P1 + (size_t)hs[e].nt * n;
-    }
-    GG_TRY(upload(dseg, hs, s));
-    for (size_t r = 0; r + 1 < rstart.size(); ++r) {
-      const unsigned nseg = (unsigned)(rstart[r + 1] - rstart[r]);
-      const unsigned bx = std::max(1u, (unsigned)(4 * ctx->sms) / nseg);
-      k_xprod<<<dim3(bx, nseg), 256, 0, s>>>(dseg.p + rstart[r], dY.p, g.np, o.dPF.p, o.dQF.p, o.ld, n);
-      k_xsum<<<dim3((n + 31) / 32, 2, nseg), 32, 0, s>>>(dseg.p + rstart[r], n);
-      ::gg::note_launch();
-      ::gg::note_launch();
-    }
-  }
-  // then every job's LAGCON terms (one launch) and DACON terms (one launch),
-  // in that order per job as in COFPOT
-  std::vector<TermSeg> ht;
-  size_t nlag = 0;
-  for (int pass = 0; pass < 2; ++pass) {
-    for (size_t j = 0; j < jobs.size(); ++j) {
-      const PotJob &J = jobs[j];
-      double *xp = dPot.p + (size_t)3 * n * j + n;
-      if (pass == 0 && !J.lag_m.empty())
-        ht.push_back(TermSeg{di.p + off[j].lm, dd.p + off[j].lw, xp, xp + n, (int)J.lag_m.size()});
-      if (pass == 1 && !J.nda.empty())
-        ht.push_back(TermSeg{di.p + off[j].dn, dd.p + off[j].dd, xp, xp + n, (int)J.nda.size()});
-    }
-    if (pass == 0) nlag = ht.size();
-  }
-  DBuf<TermSeg> dtseg;
-  if (!ht.empty()) {
-    GG_TRY(upload(dtseg, ht, s));
-    for (size_t a = 0; a < nlag; a += 65535) {  // gridDim.y limit
-      const unsigned c = (unsigned)std::min<size_t>(65535, nlag - a);
-      k_lagcon<<<dim3(blocks, c), 128, 0, s>>>(dtseg.p + a, n, o.dMF.p, g.dR.p, o.dPF.p, o.dQF.p, o.ld);
-      ::gg::note_launch();
-    }
-    for (size_t a = nlag; a < ht.size(); a += 65535) {
-      const unsigned c = (unsigned)std::min<size_t>(65535, ht.size() - a);
-      k_dacon<<<dim3(blocks, c), 128, 0, s>>>(dtseg.p + a, n, o.dNAK.p, o.dMF.p, g.dR.p, g.dRPOR.p, g.dZZ.p, o.dPF.p,
-                                              o.dQF.p, o.ld, g.q);
-      ::gg::note_launch();
-    }
+  if (!hf.empty()) {
+    k_pot_final<<<dim3((n + 31) / 32, (unsigned)hf.size()), 32 * PF_ROWS, 0, s>>>(dfin.p, dpart.p, n, o.dNAK.p, o.dMF.p, g.dR.p,
+                                                                       g.dRPOR.p, g.dZZ.p, o.dPF.p, o.dQF.p, o.ld,
+                                                                       g.q);
+    ::gg::note_launch();
   }
   GG_CUDA(cudaGetLastError());
   GG_CUDA(cudaStreamSynchronize(s));  // the uploads and scratch are freed on return
