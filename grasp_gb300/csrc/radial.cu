@@ -90,6 +90,51 @@ __device__ double quad_seq(double *TA, int mtp, const double *R, const double *R
   return 0.0;
 }
 
+// quad_seq by the lanes of a warp, the same value to the bit: the head index
+// by ballot, the four-point panels (quad.f90:94-99) one per lane into `panel`,
+// then lane 0 adds them in order, the only serial part. TA is zero beyond
+// MTP; the result is lane 0's. (Sequential QUADs on one lane of each warp were
+// most of RINTI: four of 148 panels of seven operations each, 168 us per I(ab)
+// table whatever its size; this form 22 us.)
+__device__ double quad_warp(const double *TA, double *panel, int mtp, const double *R, const double *RP,
+                            const QuadConst &q, int lane) {
+  int h = 0;
+  for (int i0 = 2; i0 <= mtp - 1 && h == 0; i0 += 32) {
+    const int i = i0 + lane;
+    bool hit = false;
+    if (i <= mtp - 1) {
+      const double tai = TA[i];
+      if (!(fabs(tai) <= 0.0)) hit = !(TA[i + 1] / tai <= 0.0);
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, hit);
+    if (bal) h = i0 + __ffs(bal) - 1;
+  }
+  if (h == 0) return 0.0;
+  const int np = (mtp - h + 3) / 4;
+  for (int t = lane; t < np; t += 32) {
+    const int j = h + 1 + 4 * t;
+    panel[t] = q.C2 * (TA[j] + TA[j + 2]) + q.C3 * TA[j + 1] + q.C4 * TA[j + 3];
+  }
+  __syncwarp();
+  double result = 0.0;
+  if (lane == 0) {
+    const double tai = TA[h], frip1 = TA[h + 1] / RP[h + 1];
+    double fri = tai / RP[h];
+    const double ratio = frip1 / fri;
+    const double sigma = log(ratio) / log(R[h + 1] / R[h]);
+    fri = R[h] * fri;
+    result = fri / (sigma + 1.0);
+    result = result + q.C1 * tai;
+    double s = 0.0;
+#pragma unroll 8
+    for (int t = 0; t < np; ++t) s = s + panel[t];
+    result = result + s;
+    if ((mtp - h) % 4 == 0) result = result - q.C1 * TA[mtp];
+  }
+  __syncwarp();
+  return result;
+}
+
 // ---------------------------------------------------------------------------
 // YZK part 1 (yzk.f90:105-126, 190-201): RHOP and the two TEMP arrays.
 //   TZ(i) = r^k RHOP(i), TW(i) = RHOP(i) / r^(k+1) on 2 <= i <= MTP, else 0.
@@ -1001,18 +1046,6 @@ __device__ __forceinline__ void dpbdt_point(const double *PF, const double *QF, 
   }
 }
 
-// DPBDT of orbital J at every grid index into dP, dQ (1-based), by the lanes
-// of a warp
-__device__ void dpbdt_warp(const double *PF, const double *QF, int ld, int J, const QuadConst &q, double *dP,
-                           double *dQ, int lane) {
-  for (int i = 1 + lane; i <= q.n; i += 32) {
-    double hp, hq;
-    dpbdt_point(PF, QF, ld, J, q, i, hp, hq);
-    dP[i] = hp;
-    dQ[i] = hq;
-  }
-}
-
 // One orbital's potentials at each grid point from its lists' chunk sums:
 //   YP = ZZ - sum, XP = sum CTB QF, XQ = -sum CTB PF (the chunks in list order);
 // LAGCON (rmcdhf90/lagcon.f90:46-55): per multiplier in list order,
@@ -1091,13 +1124,14 @@ __global__ void __launch_bounds__(32 * PF_ROWS) k_pot_final(const PotFinal *__re
 
 // SETLAG's quadrature (rmcdhf90/setlag.f90:177-219), one block per pair
 // {J, M, case, MTP}: TA(I), I = 2..MTP, from the two orbitals' potentials
-// (pot + 3 n slot: YP, XP, XQ, 0-based), then QUAD by thread 0. case 0: M
+// (pot + 3 n slot: YP, XP, XQ, 0-based), then QUAD by one warp. case 0: M
 // fixed; 1: J fixed; 2: occupations more than 10 % apart; 3: otherwise.
 __global__ void k_setlag_quad(const int4 *__restrict__ pj, const int2 *__restrict__ slots,
                               const double *__restrict__ pot, int n, const double *__restrict__ PF,
                               const double *__restrict__ QF, int ld, const double *__restrict__ R,
                               const double *__restrict__ RP, const double *__restrict__ RPOR, QuadConst q, int np,
                               double *__restrict__ TAall, double *__restrict__ result) {
+  extern __shared__ double sm[];
   const int4 w = pj[blockIdx.x];
   const int J = w.x, M = w.y, cs = w.z, mtp = w.w;
   const double *ypj = pot + (size_t)3 * n * slots[blockIdx.x].x, *xpj = ypj + n, *xqj = xpj + n;
@@ -1122,7 +1156,10 @@ __global__ void k_setlag_quad(const int4 *__restrict__ pj, const int2 *__restric
     TA[i] = v;
   }
   __syncthreads();
-  if (threadIdx.x == 0) result[blockIdx.x] = quad_seq(TA, mtp, R, RP, q);
+  if (threadIdx.x < 32) {
+    const double v = quad_warp(TA, sm, mtp, R, RP, q, threadIdx.x);
+    if (threadIdx.x == 0) result[blockIdx.x] = v;
+  }
 }
 
 // ECV from the pair's quadrature and RINTI (setlag.f90:184, 194, 205, 218)
@@ -1140,64 +1177,55 @@ __global__ void k_setlag_final(int np_, const int4 *__restrict__ pj, const doubl
   }
 }
 
-// RINTI (lib9290/rinti.f90:53-100) for a list of (J, K) pairs: one warp each.
-__global__ void k_rinti(const int2 *__restrict__ jk, int npairs, int mode, const double *__restrict__ PF,
-                        const double *__restrict__ QF, int ld, const int *__restrict__ MF,
-                        const int *__restrict__ NAK, const double *__restrict__ R, const double *__restrict__ RP,
-                        const double *__restrict__ RPOR, const double *__restrict__ ZZ, int np, QuadConst q,
-                        double *__restrict__ out, const int *__restrict__ outidx) {
+// RINTI (lib9290/rinti.f90:53-100) for a list of (J, K) pairs: one block of
+// four warps each, the four integrands formed by all threads, one QUAD per warp.
+constexpr int RINTI_WARPS = 4;
+__host__ __device__ constexpr size_t rinti_smem(int np) { return (size_t)RINTI_WARPS * (np + np / 4 + 4); }  // doubles
+__global__ void __launch_bounds__(32 * RINTI_WARPS) k_rinti(const int2 *__restrict__ jk, int npairs, int mode,
+                                                           const double *__restrict__ PF,
+                                                           const double *__restrict__ QF, int ld,
+                                                           const int *__restrict__ MF, const int *__restrict__ NAK,
+                                                           const double *__restrict__ R,
+                                                           const double *__restrict__ RP,
+                                                           const double *__restrict__ RPOR,
+                                                           const double *__restrict__ ZZ, int np, QuadConst q,
+                                                           double *__restrict__ out, const int *__restrict__ outidx) {
   extern __shared__ double sm[];
+  __shared__ double piece[RINTI_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wpb = blockDim.x >> 5;
-  double *dP = sm + (size_t)warp * 3 * np;
-  double *dQ = dP + np;
-  double *TA = dQ + np;
-  for (int it = blockIdx.x * wpb + warp; it < npairs; it += gridDim.x * wpb) {
+  double *TA = sm, *panel = sm + (size_t)RINTI_WARPS * np + (size_t)warp * (np / 4 + 4);
+  for (int it = blockIdx.x; it < npairs; it += gridDim.x) {
     const int J = jk[it].x, K = jk[it].y;
     const int mtp = max(MF[J], MF[K]);
     const double C = q.c;
-    dpbdt_warp(PF, QF, ld, K, q, dP, dQ, lane);
-    __syncwarp();
-    for (int i = lane; i < np; i += 32) TA[i] = (i >= 2 && i <= mtp) ? pf(QF, ld, i, J) * dP[i] - pf(PF, ld, i, J) * dQ[i] : 0.0;
-    __syncwarp();
-    double piece1 = 0.0, piece2 = 0.0, piece3 = 0.0, piece4 = 0.0;
-    if (lane == 0) {
-      piece1 = quad_seq(TA, mtp, R, RP, q);
-      piece1 = C * piece1 / q.h;
-    }
-    __syncwarp();
-    for (int i = lane; i < np; i += 32)
-      TA[i] = (i >= 2 && i <= mtp) ? RP[i] * pf(QF, ld, i, J) * pf(QF, ld, i, K) : 0.0;
-    __syncwarp();
-    if (lane == 0) {
-      piece2 = quad_seq(TA, mtp, R, RP, q);
-      piece2 = -2.0 * C * C * piece2;
-    }
-    __syncwarp();
-    for (int i = lane; i < np; i += 32)
-      TA[i] = (i >= 2 && i <= mtp)
-                  ? RPOR[i] * (pf(PF, ld, i, J) * pf(QF, ld, i, K) + pf(QF, ld, i, J) * pf(PF, ld, i, K))
-                  : 0.0;
-    __syncwarp();
-    if (lane == 0) {
-      piece3 = quad_seq(TA, mtp, R, RP, q);
-      piece3 = piece3 * C * (double)NAK[K];
-    }
-    __syncwarp();
-    if (mode == 0) {
-      for (int i = lane; i < np; i += 32)
-        TA[i] = (i >= 2 && i <= mtp)
-                    ? RPOR[i] * ZZ[i] * (pf(PF, ld, i, J) * pf(PF, ld, i, K) + pf(QF, ld, i, J) * pf(QF, ld, i, K))
-                    : 0.0;
-      __syncwarp();
-      if (lane == 0) {
-        piece4 = quad_seq(TA, mtp, R, RP, q);
-        piece4 = -piece4;
+    for (int i = threadIdx.x; i < np; i += blockDim.x) {
+      double t1 = 0.0, t2 = 0.0, t3 = 0.0, t4 = 0.0;
+      if (i >= 2 && i <= mtp) {
+        const double pj = pf(PF, ld, i, J), qj = pf(QF, ld, i, J), pk = pf(PF, ld, i, K), qk = pf(QF, ld, i, K);
+        double dp = 0.0, dq = 0.0;
+        if (i <= q.n) dpbdt_point(PF, QF, ld, K, q, i, dp, dq);
+        t1 = qj * dp - pj * dq;
+        t2 = RP[i] * qj * qk;
+        t3 = RPOR[i] * (pj * qk + qj * pk);
+        if (mode == 0) t4 = RPOR[i] * ZZ[i] * (pj * pk + qj * qk);
       }
-      __syncwarp();
+      TA[i] = t1;
+      TA[np + i] = t2;
+      TA[2 * np + i] = t3;
+      TA[3 * np + i] = t4;
     }
-    if (lane == 0) out[outidx ? outidx[it] : it] = piece1 + piece2 + piece3 + piece4;
-    __syncwarp();
+    __syncthreads();
+    double v = 0.0;
+    if (warp < 3 || mode == 0) v = quad_warp(TA + (size_t)warp * np, panel, mtp, R, RP, q, lane);
+    if (lane == 0) {
+      if (warp == 0) v = C * v / q.h;
+      if (warp == 1) v = -2.0 * C * C * v;
+      if (warp == 2) v = v * C * (double)NAK[K];
+      if (warp == 3 && mode == 0) v = -v;
+      piece[warp] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) out[outidx ? outidx[it] : it] = piece[0] + piece[1] + piece[2] + piece[3];
   }
 }
 
@@ -2147,7 +2175,7 @@ int gg_setlag(gg_ctx *ctx, int nec, const int32_t *iecc, const double *ucf, cons
   GG_TRY(drij.alloc(nec));
   GG_TRY(decv.alloc(nec));
   GG_CUDA(cudaMemsetAsync(drij.p, 0, nec * sizeof(double), s));
-  k_setlag_quad<<<nec, 128, 0, s>>>(dpj.p, dps.p, pot.p, g.n, o.dPF.p, o.dQF.p, o.ld, g.dR.p, g.dRP.p, g.dRPOR.p,
+  k_setlag_quad<<<nec, 128, (g.np / 4 + 4) * sizeof(double), s>>>(dpj.p, dps.p, pot.p, g.n, o.dPF.p, o.dQF.p, o.ld, g.dR.p, g.dRP.p, g.dRPOR.p,
                                     g.q, g.np, dTA.p, dres.p);
   ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
@@ -2272,10 +2300,9 @@ static int run_rinti(gg_ctx *ctx, const std::vector<int2> &jk, int mode, double 
   DBuf<int> didx;
   GG_TRY(upload(djk, jk, ctx->stream));
   if (outidx) GG_TRY(upload(didx, *outidx, ctx->stream));
-  const int wpb = 2;
-  const size_t smem = (size_t)wpb * 3 * g.np * sizeof(double);
-  const int blocks = std::max(1, std::min(((int)jk.size() + wpb - 1) / wpb, 2048));
-  k_rinti<<<blocks, 32 * wpb, smem, ctx->stream>>>(djk.p, (int)jk.size(), mode, o.dPF.p, o.dQF.p, o.ld, o.dMF.p,
+  const size_t smem = rinti_smem(g.np) * sizeof(double);
+  const int blocks = std::max(1, std::min((int)jk.size(), 2048));
+  k_rinti<<<blocks, 32 * RINTI_WARPS, smem, ctx->stream>>>(djk.p, (int)jk.size(), mode, o.dPF.p, o.dQF.p, o.ld, o.dMF.p,
                                                    o.dNAK.p, g.dR.p, g.dRP.p, g.dRPOR.p, g.dZZ.p, g.np, g.q, dOut,
                                                    outidx ? didx.p : nullptr); ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
