@@ -133,7 +133,8 @@ int gg_set_grid(gg_ctx *ctx, int n, double rnt, double h, double c, const double
   g.rnt = rnt;
   g.h = h;
   g.c = c;
-  const size_t sz = (size_t)n + GPAD + 10;
+  // an even pitch: rows of arrays [..][np] start on 16 bytes (double2 loads)
+  const size_t sz = ((size_t)n + GPAD + 11) / 2 * 2;
   g.R.assign(sz, 0.0);
   g.RP.assign(sz, 0.0);
   g.RPOR.assign(sz, 0.0);

@@ -10,7 +10,8 @@ additions, a few 1e-16 of the largest partial sum)."""
 import numpy as np
 import pytest
 
-from tests.common import hydrogenic_case, oracle_for
+from inputs import synth as S
+from tests.common import oracle_for
 
 pytestmark = pytest.mark.gpu
 
@@ -32,12 +33,20 @@ SETS = {
 }
 
 
+def _case(n, z=10.0):
+    orbs = S.orbital_set(3, 2)
+    rnt, r = S.grid(n, z)
+    ob = S.hydrogenic_orbitals(orbs, z, S.screenpar([k for _, k in orbs], 1), r, n=n)
+    return dict(n=n, rnt=rnt, h=0.05, c=S.CVAC, zz=np.full(n, z), orb=ob)
+
+
+@pytest.mark.parametrize("n", [590, 513])
 @pytest.mark.parametrize("wfact", [1.0, 0.0])
 @pytest.mark.parametrize("itype", [1, 2])
 @pytest.mark.parametrize("which", sorted(SETS))
-def test_contraction_matches_oracle(gpu_ready, oracle_mod, which, itype, wfact):
+def test_contraction_matches_oracle(gpu_ready, oracle_mod, which, itype, wfact, n):
     from grasp_gb300 import Context
-    case = hydrogenic_case(nmax=3, lmax=2, z=10.0)
+    case = _case(n)
     ob = case["orb"]
     nw = len(ob.nak)
     e = -np.linspace(50.0, 1.0, nw)
