@@ -29,8 +29,7 @@ namespace gg {
 
 namespace {
 
-constexpr int KC_TILE = 16;  // contraction depth per shared-memory stage
-constexpr int BM = 32, BN = 64;
+constexpr int KC_TILE = 16;  // the pair arrays' row length is a multiple of this
 
 struct YDesc {
   int k, b, d;  // Y^k_{bd}
@@ -41,17 +40,12 @@ struct YDesc {
 };
 
 struct RkTile {
-  int k, a;
-  int ncA;        // |C(a,k)|: rows of the (k,a) problem
-  int r0;         // first row of this tile
-  int rowpair0;   // offset into the row-pair list of the (k,a) problem
-  int cs_a;       // first column (Y function) of the (k,a) problem
-  int c0, c1;     // column range [c0, c1) of this tile
-  long long base; // 0-based VALTEIRK position of the (k,a) problem
+  int r0, rn;  // first row ((a, c) pair of the k) and how many
+  int f0, fn;  // first Y function and how many
 };
 
 struct QuadItem {  // one integral evaluated with the general QUAD
-  int a, c, f, mtp;
+  int a, c, p, f, mtp;  // p: the pair's row of the pair arrays
   long long pos;
 };
 
@@ -95,7 +89,7 @@ __device__ double quad_seq(double *TA, int mtp, const double *R, const double *R
 // then lane 0 adds them in order, the only serial part. TA is zero beyond
 // MTP; the result is lane 0's. (Sequential QUADs on one lane of each warp were
 // most of RINTI: four of 148 panels of seven operations each, 168 us per I(ab)
-// table whatever its size; this form 22 us.)
+// table whatever its size; this form RNT us.)
 __device__ double quad_warp(const double *TA, double *panel, int mtp, const double *R, const double *RP,
                             const QuadConst &q, int lane) {
   int h = 0;
@@ -244,170 +238,143 @@ __global__ void k_ychain(const YDesc *__restrict__ yd, int nf, const double *__r
   }
 }
 
-// A rows: w(i) (P_a P_c + Q_a Q_c) RPOR on 2 <= i <= min(MF(a), MF(c)).
-// w is the closed Newton-Cotes weight pattern of QUAD started at i = 2:
+// Pair arrays on 2 <= i <= min(MF(a), MF(c)): D = (P_a P_c + Q_a Q_c) RPOR and
+// A = w D, w the closed Newton-Cotes weight pattern of QUAD started at i = 2:
 // C1 at 2, then C2, C3, C2, C4 repeating.
 __global__ void k_apairs(const int2 *__restrict__ pairs, int npairs, const double *__restrict__ PF,
                          const double *__restrict__ QF, int ld, const int *__restrict__ MF,
-                         const double *__restrict__ RPOR, int KC, QuadConst q, double *__restrict__ A) {
+                         const double *__restrict__ RPOR, int KC, QuadConst q, double *__restrict__ A,
+                         double *__restrict__ D) {
   const int p = blockIdx.y;
   if (p >= npairs) return;
   const int a = pairs[p].x, c = pairs[p].y;
   const int m = min(MF[a], MF[c]);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < KC; i += gridDim.x * blockDim.x) {
-    double v = 0.0;
+  // the last row is followed by zeros: k_rk_dot reads up to three points past
+  // a row's last one
+  const int end = p + 1 < npairs ? KC : KC + KC_TILE;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
+    double v = 0.0, rho = 0.0;
     if (i >= 2 && i <= m) {
-      const double rho = (pf(PF, ld, i, a) * pf(PF, ld, i, c) + pf(QF, ld, i, a) * pf(QF, ld, i, c)) * RPOR[i];
+      rho = (pf(PF, ld, i, a) * pf(PF, ld, i, c) + pf(QF, ld, i, a) * pf(QF, ld, i, c)) * RPOR[i];
       const int ph = (i - 2) & 3;
       const double w = (i == 2) ? q.C1 : (ph == 1 || ph == 3) ? q.C2 : (ph == 2) ? q.C3 : q.C4;
       v = w * rho;
     }
     A[(size_t)p * KC + i] = v;
+    D[(size_t)p * KC + i] = rho;
   }
 }
 
-// Completes one R^k(ab;cd) from its contraction sum: QUAD's power-law head
-// term at i = 2 and the end-panel correction at MTP (quad.f90), written at
-// its GENINTRK position; entries whose QUAD head index is not 2 go to the
-// general per-integral QUAD instead.
 // QUAD's power-law head term and end-panel correction (quad.f90:52-103) for
-// integral (a, c; f) of order k whose GEMM part (grid points 3.., the
-// Newton-Cotes weights folded into A) is `sum`, stored at VALTEIRK position
-// pos; an integral whose head index is not 2 goes to the general QUAD list.
-__device__ __forceinline__ void rk_head_store(int k, int a, int c, int f, long long pos, double sum,
-                                              const YDesc *__restrict__ yd, const double *__restrict__ Y, int np,
-                                              const double *__restrict__ PF, const double *__restrict__ QF, int ld,
-                                              const int *__restrict__ MF, const double *__restrict__ R,
-                                              const double *__restrict__ RP, const double *__restrict__ RPOR,
-                                              const double *__restrict__ HD, const QuadConst &q,
-                                              double *__restrict__ val, QuadItem *__restrict__ fb,
-                                              int *__restrict__ nfb) {
-  const YDesc y = yd[f];
-  int mtp;
-  if (k == 0 && y.b == y.d)
-    mtp = min(MF[a], MF[c]);
-  else
-    mtp = min(min(y.mtp, MF[a]), MF[c]);
-  const double *Yf = Y + (size_t)f * np;
-  auto ta = [&](int i) {
-    return ((pf(PF, ld, i, a) * pf(PF, ld, i, c) + pf(QF, ld, i, a) * pf(QF, ld, i, c)) * RPOR[i]) * Yf[i];
-  };
+// integral (a, c; f) whose GEMM part (grid points 3.., the Newton-Cotes weights
+// folded into A) is `sum`, stored at VALTEIRK position pos; an integral whose
+// head index is not 2 goes to the general QUAD list. TA(i) = D(i) Y(i).
+struct RkTabs {
+  const double *D, *Y;
+  const YDesc *yd;
+  const int *MF;
+  const double *HD;
+  int KC, np;
+};
+__device__ __forceinline__ void rk_head_store(int a, int c, int p, int f, long long pos, double sum, const RkTabs &t,
+                                              const QuadConst &q, double *__restrict__ val,
+                                              QuadItem *__restrict__ fb, int *__restrict__ nfb) {
+  const YDesc y = t.yd[f];
+  int mtp = min(t.MF[a], t.MF[c]);
+  if (!(y.k == 0 && y.b == y.d)) mtp = min(mtp, y.mtp);
+  const double *D = t.D + (size_t)p * t.KC, *Y = t.Y + (size_t)f * t.np, *HD = t.HD;
   bool ok = mtp >= 3;
   double res = 0.0;
   if (ok) {
-    const double tai = ta(2), taip1 = ta(3);
-    const double t = taip1 / tai;
-    ok = !(fabs(tai) <= 0.0) && (t > 0.0);
+    const double tai = D[2] * Y[2], taip1 = D[3] * Y[3];
+    const double r = taip1 / tai;
+    ok = !(fabs(tai) <= 0.0) && (r > 0.0);
     if (ok) {
       // QUAD's head term with the grid's factors per point (HD): the ratio
       // (TA(3)/RP(3)) / (TA(2)/RP(2)), sigma = log(ratio) / log(R(3)/R(2)),
       // R(2) TA(2)/RP(2) / (sigma + 1); equal to quad.f90's to rounding
-      const double sigma = log(t * HD[np + 2]) * HD[2];
-      const double fri = tai * HD[2 * np + 2];
+      const double sigma = log(r * HD[t.np + 2]) * HD[2];
+      const double fri = tai * HD[2 * t.np + 2];
       res = fri / (sigma + 1.0) + sum;
-      if ((mtp - 2) % 4 == 0) res = res - q.C1 * ta(mtp);
+      if ((mtp - 2) % 4 == 0) res = res - q.C1 * (D[mtp] * Y[mtp]);
     }
   }
   if (ok) {
     val[pos] = res;
   } else {
     const int slot = atomicAdd(nfb, 1);
-    fb[slot] = QuadItem{a, c, f, mtp, pos};
+    fb[slot] = QuadItem{a, c, p, f, mtp, pos};
   }
 }
 
-// the GEMM part `sum` of canonical entry (p = (a, c), f) of tile T: its
-// GENINTRK position, then the head term
-__device__ __forceinline__ void rk_finish(const RkTile &T, int p, int idx_c, int f, double sum,
-                                          const int2 *__restrict__ pairs, const YDesc *__restrict__ yd,
-                                          const double *__restrict__ Y, int np, const double *__restrict__ PF,
-                                          const double *__restrict__ QF, int ld, const int *__restrict__ MF,
-                                          const double *__restrict__ R, const double *__restrict__ RP,
-                                          const double *__restrict__ RPOR, const double *__restrict__ HD,
-                                          const QuadConst &q, double *__restrict__ val, long long nval,
-                                          QuadItem *__restrict__ fb, int *__restrict__ nfb) {
-  const YDesc y = yd[f];
-  const long long pos = T.base + (long long)T.ncA * (y.cs - T.cs_a) + (long long)idx_c * y.nd + (long long)(f - y.cs);
-  if (pos < 0 || pos >= nval) {  // position outside the table: report, never write
-    atomicExch(nfb + 1, 1);
-    return;
-  }
-  rk_head_store(T.k, T.a, pairs[p].y, f, pos, sum, yd, Y, np, PF, QF, ld, MF, R, RP, RPOR, HD, q, val, fb, nfb);
-}
-
 // ---------------------------------------------------------------------------
-// R^k contraction: for each (k, a) the GEMM  O[c, f] = sum_i A[(a,c), i] Y[f, i]
-// over the rows c in C(a,k) and the Y functions f = (b,d) with b >= a, then
-// QUAD's power-law head term and end-panel correction per entry. Output
-// positions follow GENINTRK's loop order (k, a, b, c, d).
+// R^k contraction in FP64: for each k, O[p, f] = sum_i A[p, i] Y[f, i] over its
+// pairs p = (a, c) and the Y functions f = (b, d) with b >= a, then QUAD's head
+// term and end-panel correction per entry, written at the GENINTRK position
+// (k, a, b, c, d). A warp takes 32 functions, one per lane, x NR pairs, whose
+// rows are read uniformly; each entry is one FMA chain over the points in
+// order, up to the pairs' last point. Bound: the FP64 pipe on large sets, the
+// chain's latency on small ones; NR is the largest of 8, 4, 2, 1 that still
+// gives every SM four warps (fewer rows per warp read Y more often, more leave
+// SMs idle). A block of 32 x 64 entries in shared memory left most rows of a
+// tile empty (a (k, a) problem has 2 to 12 pairs) and most SMs idle: 371 us
+// for 16 subshells, now 52 us; the chains are the same, so are the bits.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_rk_gemm(const RkTile *__restrict__ tiles, const int *__restrict__ rowpair,
-                                                 const int2 *__restrict__ pairs, const double *__restrict__ A,
-                                                 const double *__restrict__ Y, const YDesc *__restrict__ yd, int KC,
-                                                 int np, const double *__restrict__ PF, const double *__restrict__ QF,
-                                                 int ld, const int *__restrict__ MF, const double *__restrict__ R,
-                                                 const double *__restrict__ RP, const double *__restrict__ RPOR,
-                                                 const double *__restrict__ HD, QuadConst q,
-                                                 double *__restrict__ val, long long nval,
-                                                 QuadItem *__restrict__ fb, int *__restrict__ nfb) {
-  __shared__ double As[2][KC_TILE][BM];
-  __shared__ double Bs[2][KC_TILE][BN + 1];
-  __shared__ int rowp[BM];
-  const RkTile T = tiles[blockIdx.x];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int nrow = min(BM, T.ncA - T.r0);
-  const int ncol = T.c1 - T.c0;
-  if (tid < BM) rowp[tid] = (tid < nrow) ? rowpair[T.rowpair0 + T.r0 + tid] : -1;
-  __syncthreads();
-  double acc[2][4];
+struct TcRow {  // one row of a k: its pair, problem and position data
+  int p, a, c, ic, ncA, cs_a;
+  long long base;
+};
+template <int NR>
+__global__ void __launch_bounds__(128) k_rk_dot(const RkTile *__restrict__ tiles, int ntiles,
+                                                const TcRow *__restrict__ rows, const double *__restrict__ A,
+                                                RkTabs t, QuadConst q, double *__restrict__ val, long long nval,
+                                                QuadItem *__restrict__ fb, int *__restrict__ nfb) {
+  const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (w >= ntiles) return;
+  const RkTile T = tiles[w];
+  const double *ar[NR];
+  int m = 0;
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
-
-  auto load = [&](int buf, int k0) {
-    // A: BM rows x KC_TILE ; 256 threads -> 2 elements each
-    for (int e = tid; e < BM * KC_TILE; e += 256) {
-      const int r = e / KC_TILE, kk = e % KC_TILE;
-      const int p = rowp[r];
-      As[buf][kk][r] = (p >= 0) ? A[(size_t)p * KC + k0 + kk] : 0.0;
-    }
-    for (int e = tid; e < BN * KC_TILE; e += 256) {
-      const int j = e / KC_TILE, kk = e % KC_TILE;
-      Bs[buf][kk][j] = (j < ncol) ? Y[(size_t)(T.c0 + j) * np + k0 + kk] : 0.0;
-    }
-  };
-  const int nk = KC / KC_TILE;
-  load(0, 0);
-  __syncthreads();
-  for (int s = 0; s < nk; ++s) {
-    const int buf = s & 1;
-    if (s + 1 < nk) load(buf ^ 1, (s + 1) * KC_TILE);
-#pragma unroll
-    for (int kk = 0; kk < KC_TILE; ++kk) {
-      const double a0 = As[buf][kk][ty * 2 + 0], a1 = As[buf][kk][ty * 2 + 1];
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const double b = Bs[buf][kk][tx * 4 + v];
-        acc[0][v] = fma(a0, b, acc[0][v]);
-        acc[1][v] = fma(a1, b, acc[1][v]);
-      }
-    }
-    __syncthreads();
+  for (int r = 0; r < NR; ++r) {  // rows past the tile repeat its last one
+    const TcRow rw = rows[T.r0 + min(r, T.rn - 1)];
+    ar[r] = A + (size_t)rw.p * t.KC;
+    m = max(m, min(t.MF[rw.a], t.MF[rw.c]));
   }
-  // epilogue
+  const int f = T.f0 + min(lane, T.fn - 1);
+  const double *y = t.Y + (size_t)f * t.np;
+  double acc[NR];
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int r = ty * 2 + u;
-    if (r >= nrow) continue;
+  for (int r = 0; r < NR; ++r) acc[r] = 0.0;
+  // points 2 .. m in groups of four; A is zero from m + 1 on (the row's end,
+  // then points 0 and 1 of the next row)
+#pragma unroll 2
+  for (int i = 2; i <= m; i += 4) {
+    const double2 y0 = __ldg(reinterpret_cast<const double2 *>(y + i));
+    const double2 y1 = __ldg(reinterpret_cast<const double2 *>(y + i + 2));
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int j = tx * 4 + v;
-      if (j >= ncol) continue;
-      rk_finish(T, rowp[r], T.r0 + r, T.c0 + j, acc[u][v], pairs, yd, Y, np, PF, QF, ld, MF, R, RP, RPOR, HD, q,
-                val, nval, fb, nfb);
+    for (int r = 0; r < NR; ++r) {
+      const double2 a0 = __ldg(reinterpret_cast<const double2 *>(ar[r] + i));
+      const double2 a1 = __ldg(reinterpret_cast<const double2 *>(ar[r] + i + 2));
+      acc[r] = fma(a0.x, y0.x, acc[r]);
+      acc[r] = fma(a0.y, y0.y, acc[r]);
+      acc[r] = fma(a1.x, y1.x, acc[r]);
+      acc[r] = fma(a1.y, y1.y, acc[r]);
     }
+  }
+  if (lane >= T.fn) return;
+  const YDesc yd = t.yd[f];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    if (r >= T.rn) continue;
+    const TcRow rw = rows[T.r0 + r];
+    if (f < rw.cs_a) continue;  // b < a: not a GENINTRK entry
+    const long long pos =
+        rw.base + (long long)rw.ncA * (yd.cs - rw.cs_a) + (long long)rw.ic * yd.nd + (long long)(f - yd.cs);
+    if (pos < 0 || pos >= nval) {  // position outside the table: report, never write
+      atomicExch(nfb + 1, 1);
+      continue;
+    }
+    rk_head_store(rw.a, rw.c, rw.p, f, pos, acc[r], t, q, val, fb, nfb);
   }
 }
 
@@ -462,10 +429,6 @@ constexpr uint32_t TC_TMEM_COLS = 512;  // >= OZ_S * TC_N, a power of two
 constexpr int TC_SPIN = 1 << 24;
 constexpr int TC_THREADS = 160;  // warps 0-3: accumulators; warp 4: copies and MMAs
 
-struct TcRow {  // one row of a k: its pair, problem and position data
-  int p, a, ic, ncA, cs_a;
-  long long base;
-};
 struct TcTile {
   int k, fg, pg;  // k; global indices of the Y block column and the A block column
   int f0, fn;     // first Y function and how many are valid
@@ -481,8 +444,9 @@ struct TcTile {
 struct RkCache {
   std::vector<int> key;
   int nf = 0, npairs = 0;
+  int nr = 8;  // rows of a tile of the FP64 contraction
   std::vector<YDesc> yd;
-  std::vector<int> kend, rowpair, yslot, aslot, fidx;
+  std::vector<int> kend, yslot, aslot, fidx, pidx;
   std::vector<int2> pairs;
   std::vector<RkTile> tiles;
   std::vector<TcRow> tcrows;
@@ -490,7 +454,7 @@ struct RkCache {
   DBuf<YDesc> dYd;
   DBuf<int2> dPairs;
   DBuf<RkTile> dTiles;
-  DBuf<int> dRowpair, dYslot, dAslot, dFidx, dNfb, dEA, dEY;
+  DBuf<int> dYslot, dAslot, dFidx, dPidx, dNfb, dEA, dEY;
   DBuf<int32_t> dKst;
   DBuf<TcTile> dTct;
   // split-K form of tct (each tile's grid chunks over nsplit CTAs) for the
@@ -500,7 +464,7 @@ struct RkCache {
   DBuf<TcTile> dTcs;
   DBuf<double> dParts;
   DBuf<TcRow> dTcr;
-  DBuf<double> dY, dA, scratch;
+  DBuf<double> dY, dA, dD, scratch;
   DBuf<QuadItem> dFb;
   DBuf<__half> dYt, dAt;
 };
@@ -792,17 +756,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_rk_tc(const TcTile *__restric
 }
 
 // QUAD head term for every table entry, one thread per entry: (a, b, c, d)
-// from INDTEIRK, k from KSTART, the Y function from fidx[(k KEY + b) KEY + d];
-// the entry's GEMM part is the sum, in split order, of parts[s n + i] for
-// s < nsplit (parts == val when the contraction was not split).
+// from INDTEIRK, k from KSTART, the pair from pidx[a KEY + c] and the Y
+// function from fidx[(k KEY + b) KEY + d]; the entry's GEMM part is the sum, in
+// split order, of parts[s n + i] for s < nsplit (parts == val when the
+// contraction was not split).
 __global__ void k_rk_finish_all(const int32_t *__restrict__ ind, long long n, const int32_t *__restrict__ kstart,
-                                int kloop, int KEY, const int *__restrict__ fidx, const YDesc *__restrict__ yd,
-                                const double *__restrict__ Y, int np, const double *__restrict__ PF,
-                                const double *__restrict__ QF, int ld, const int *__restrict__ MF,
-                                const double *__restrict__ R, const double *__restrict__ RP,
-                                const double *__restrict__ RPOR, const double *__restrict__ HD, QuadConst q,
-                                double *__restrict__ val, QuadItem *__restrict__ fb, int *__restrict__ nfb,
-                                const double *__restrict__ parts, int nsplit) {
+                                int kloop, int KEY, const int *__restrict__ fidx, const int *__restrict__ pidx,
+                                RkTabs tb, QuadConst q, double *__restrict__ val, QuadItem *__restrict__ fb,
+                                int *__restrict__ nfb, const double *__restrict__ parts, int nsplit) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     int p = ind[i];
     const int d = p % KEY;
@@ -812,14 +773,14 @@ __global__ void k_rk_finish_all(const int32_t *__restrict__ ind, long long n, co
     const int b = p % KEY, a = p / KEY;
     int k = 0;
     while (k < kloop && (long long)kstart[k + 1] - 1 <= i) ++k;
-    const int f = fidx[((size_t)k * KEY + b) * KEY + d];
-    if (f < 0) {
+    const int f = fidx[((size_t)k * KEY + b) * KEY + d], pr = pidx[(size_t)a * KEY + c];
+    if (f < 0 || pr < 0) {
       atomicExch(nfb + 1, 1);
       continue;
     }
     double gemm = parts[i];
     for (int t = 1; t < nsplit; ++t) gemm += parts[(long long)t * n + i];
-    rk_head_store(k, a, c, f, i, gemm, yd, Y, np, PF, QF, ld, MF, R, RP, RPOR, HD, q, val, fb, nfb);
+    rk_head_store(a, c, pr, f, i, gemm, tb, q, val, fb, nfb);
   }
 }
 
@@ -853,48 +814,43 @@ __global__ void k_quad_items(const QuadItem *__restrict__ items, const int *__re
 // TA(i) != 0 and TA(i+1)/TA(i) > 0) by ballot, the 4-point panel sums
 // (quad.f90:94-99) split over the lanes and combined by a fixed butterfly,
 // so the result is deterministic. Only the order of the panel sum differs
-// from quad_seq (a few ulps of the sum of |terms|). TA values are formed
-// where they are used, so no grid size limit comes from shared memory.
+// from quad_seq (a few ulps of the sum of |terms|). TA(i) = D(i) Y(i) from the
+// pair array; formed from the orbitals at every use the 43-orbital table's
+// items took 103 us, so 55 us.
 __global__ void k_quad_table(const QuadItem *__restrict__ items, const int *__restrict__ nitems_p, int nitems_max,
-                             const double *__restrict__ Y, int np, const double *__restrict__ PF,
-                             const double *__restrict__ QF, int ld, const double *__restrict__ R,
-                             const double *__restrict__ RP, const double *__restrict__ RPOR,
-                             const double *__restrict__ HD, QuadConst q, double *__restrict__ out) {
+                             RkTabs tb, QuadConst q, double *__restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   const int nitems = min(*nitems_p, nitems_max);
-  // TA(i) of quad.f90 for item w, zero outside [2, MTP] (the pads TA(MTP+1..MTP+3))
-  auto ta = [&](const QuadItem &w, int i) -> double {
-    if (i < 2 || i > w.mtp) return 0.0;
-    const double *Pa = PF + (size_t)(w.a - 1) * ld, *Pc = PF + (size_t)(w.c - 1) * ld;
-    const double *Qa = QF + (size_t)(w.a - 1) * ld, *Qc = QF + (size_t)(w.c - 1) * ld;
-    return ((Pa[i - 1] * Pc[i - 1] + Qa[i - 1] * Qc[i - 1]) * RPOR[i]) * Y[(size_t)w.f * np + i];
-  };
-  // One item per warp for the head index and the panel sum; the block's
-  // items then get their head terms (a logarithm and divisions: serial FP64
-  // work that would otherwise occupy a warp per item) from the lanes of
-  // warp 0, one item each
+  const double *HD = tb.HD;
+  const int np = tb.np;
+  // One item per warp for the head index and the sum; the block's items then
+  // get their head terms (a logarithm and divisions: serial FP64 work that
+  // would otherwise occupy a warp per item) from the lanes of warp 0, one
+  // item each
   __shared__ int sh_head[32];
   __shared__ double sh_s[32];
   for (int base = blockIdx.x * wpb; base < nitems; base += gridDim.x * wpb) {
     const int it = base + (threadIdx.x >> 5);
     if (it < nitems) {
       const QuadItem w = items[it];
+      const double *D = tb.D + (size_t)w.p * tb.KC, *Y = tb.Y + (size_t)w.f * np;
       int head = -1;
       for (int i0 = 2; i0 <= w.mtp - 1 && head < 0; i0 += 32) {
         const int i = i0 + lane;
         bool hit = false;
         if (i <= w.mtp - 1) {
-          const double tai = ta(w, i);
-          hit = !(fabs(tai) <= 0.0) && (ta(w, i + 1) / tai > 0.0);
+          const double t0 = D[i] * Y[i], t1 = D[i + 1] * Y[i + 1];
+          hit = (t0 > 0.0 && t1 > 0.0) || (t0 < 0.0 && t1 < 0.0);
         }
         const unsigned bal = __ballot_sync(0xffffffffu, hit);
         if (bal) head = i0 + __ffs(bal) - 1;
       }
       double sp = 0.0;
+      auto ta = [&](int j) { return j <= w.mtp ? D[j] * Y[j] : 0.0; };
       if (head >= 0)
         for (int j = head + 1 + 4 * lane; j <= w.mtp; j += 128)
-          sp += q.C2 * (ta(w, j) + ta(w, j + 2)) + q.C3 * ta(w, j + 1) + q.C4 * ta(w, j + 3);
+          sp += q.C2 * (ta(j) + ta(j + 2)) + q.C3 * ta(j + 1) + q.C4 * ta(j + 3);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) sp += __shfl_xor_sync(0xffffffffu, sp, o);
       if (lane == 0) {
@@ -905,16 +861,17 @@ __global__ void k_quad_table(const QuadItem *__restrict__ items, const int *__re
     __syncthreads();
     if (threadIdx.x < wpb && base + (int)threadIdx.x < nitems) {
       const QuadItem w = items[base + threadIdx.x];
+      const double *D = tb.D + (size_t)w.p * tb.KC, *Y = tb.Y + (size_t)w.f * np;
       const int i = sh_head[threadIdx.x];
       double result = 0.0;
       if (i >= 0) {
         // quad.f90:61-103 with the grid's factors per point (HD)
-        const double tai = ta(w, i), taip1 = ta(w, i + 1);
+        const double tai = D[i] * Y[i], taip1 = D[i + 1] * Y[i + 1];
         const double sigma = log((taip1 / tai) * HD[np + i]) * HD[i];
         result = (tai * HD[2 * np + i]) / (sigma + 1.0);
         result = result + q.C1 * tai;
         result = result + sh_s[threadIdx.x];
-        if ((w.mtp - i) % 4 == 0) result = result - q.C1 * ta(w, w.mtp);
+        if ((w.mtp - i) % 4 == 0) result = result - q.C1 * (D[w.mtp] * Y[w.mtp]);
       }
       out[w.pos] = result;
     }
@@ -928,7 +885,7 @@ __global__ void k_quad_table(const QuadItem *__restrict__ items, const int *__re
 // every fourth term; the rows' sums meet in shared memory and the chunk's are
 // stored for k_pot_final, which adds them in list order. Bound: the FP64 pipe
 // (three operations per XPOT term and point; 34 subshells' lists of 6,600 terms
-// 35 us per orbital). One thread per point adding the terms in list order
+// 24 us per orbital). One thread per point adding the terms in list order
 // left the pipe to one dependent addition per term: 233 us for the same list.
 constexpr int POT_CHUNK = 128;  // terms staged in shared memory at a time
 struct PotChunk {
@@ -1498,10 +1455,8 @@ static int rk_build_structure(gg_ctx *ctx, int kloop, RkCache &C) {
   rk.kstart.assign(kloop + 2, 0);
   rk.hInd.clear();
   std::vector<RkTile> &tiles = C.tiles;
-  std::vector<int> &rowpair = C.rowpair;
   std::vector<TcRow> &tcrows = C.tcrows;
   tiles.clear();
-  rowpair.clear();
   tcrows.clear();
   std::vector<int> tcr0(kloop + 2, 0);  // first tcrows entry of each k
   int64_t N = 0;
@@ -1511,7 +1466,7 @@ static int rk_build_structure(gg_ctx *ctx, int kloop, RkCache &C) {
     for (int a = 1; a <= NW; ++a) {
       const int ncA = nd[k][a];
       if (ncA == 0) continue;
-      const int c0 = cs[k][a], c1 = kend[k];
+      const int c0 = cs[k][a];
       const long long base = N;
       // integer index list in reference order
       for (int b = a; b <= NW; ++b)
@@ -1523,28 +1478,25 @@ static int rk_build_structure(gg_ctx *ctx, int kloop, RkCache &C) {
           }
         }
       N = (int64_t)rk.hInd.size();
-      const int rp0 = (int)rowpair.size();
-      for (int ic = 0; ic < ncA; ++ic) rowpair.push_back(pidx[(size_t)a * (NW + 1) + yd[cs[k][a] + ic].d]);
-      for (int r0 = 0; r0 < ncA; r0 += BM)
-        for (int cc = c0; cc < c1; cc += BN) {
-          RkTile t;
-          t.k = k;
-          t.a = a;
-          t.ncA = ncA;
-          t.r0 = r0;
-          t.rowpair0 = rp0;
-          t.cs_a = c0;
-          t.c0 = cc;
-          t.c1 = std::min(c1, cc + BN);
-          t.base = base;
-          tiles.push_back(t);
-        }
-      // rows of the tcgen05 form (all problems of one k, in order)
-      for (int ic = 0; ic < ncA; ++ic) tcrows.push_back(TcRow{rowpair[rp0 + ic], a, ic, ncA, c0, base});
+      // the contraction's rows (all problems of one k, in order)
+      for (int ic = 0; ic < ncA; ++ic) {
+        const int c = yd[cs[k][a] + ic].d;
+        tcrows.push_back(TcRow{pidx[(size_t)a * (NW + 1) + c], a, c, ic, ncA, c0, base});
+      }
     }
     rk.kstart[k + 1] = (int32_t)(N + 1);
   }
   tcr0[kloop + 1] = (int)tcrows.size();
+  // the FP64 form's tiles; the rows are ordered by a, so a tile's first row
+  // has its smallest cs_a
+  for (C.nr = 8;; C.nr /= 2) {
+    tiles.clear();
+    for (int k = 0; k <= kloop; ++k)
+      for (int r = tcr0[k]; r < tcr0[k + 1]; r += C.nr)
+        for (int f = tcrows[r].cs_a; f < kend[k]; f += 32)
+          tiles.push_back(RkTile{r, std::min(C.nr, tcr0[k + 1] - r), f, std::min(32, kend[k] - f)});
+    if (C.nr == 1 || (int)tiles.size() >= 4 * ctx->sms) break;
+  }
   if (N > INT32_MAX) return fail(GG_ERR_RANGE, "genintrk: table too large");
   rk.n = N;
   C.nf = (int)yd.size();
@@ -1596,12 +1548,12 @@ static int rk_build_structure(gg_ctx *ctx, int kloop, RkCache &C) {
   }
   GG_TRY(upload(C.dPairs, pairs, ctx->stream));
   GG_TRY(upload(C.dTiles, tiles, ctx->stream));
-  GG_TRY(upload(C.dRowpair, rowpair, ctx->stream));
   GG_TRY(upload(C.dTct, C.tct, ctx->stream));
   GG_TRY(upload(C.dTcr, tcrows, ctx->stream));
   GG_TRY(upload(C.dYslot, C.yslot, ctx->stream));
   GG_TRY(upload(C.dAslot, C.aslot, ctx->stream));
   GG_TRY(upload(C.dFidx, C.fidx, ctx->stream));
+  GG_TRY(upload(C.dPidx, pidx, ctx->stream));
   GG_TRY(upload(C.dKst, rk.kstart, ctx->stream));
   GG_TRY(rk.dInd.alloc(std::max<int64_t>(N, 1)));
   if (N > 0)
@@ -1656,14 +1608,16 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
   GG_TRY(rk.dVal.alloc(std::max<int64_t>(N, 1)));
   GG_TRY(C.dY.alloc((size_t)std::max(nf, 1) * np));
   if (nf > 0) GG_TRY(build_y(ctx, C.dYd.p, nf, C.dY.p, C.scratch));
-  GG_TRY(C.dA.alloc((size_t)std::max(npairs, 1) * KC));
+  GG_TRY(C.dA.alloc((size_t)std::max(npairs, 1) * KC + KC_TILE));
+  GG_TRY(C.dD.alloc((size_t)std::max(npairs, 1) * KC + KC_TILE));
   if (npairs > 0) {
     dim3 gr((KC + 127) / 128, npairs);
     k_apairs<<<gr, 128, 0, ctx->stream>>>(C.dPairs.p, npairs, o.dPF.p, o.dQF.p, o.ld, o.dMF.p, g.dRPOR.p, KC, g.q,
-                                          C.dA.p);
+                                          C.dA.p, C.dD.p);
     ::gg::note_launch();
     GG_CUDA(cudaGetLastError());
   }
+  const RkTabs tabs{C.dD.p, C.dY.p, C.dYd.p, o.dMF.p, g.dHead.p, KC, np};
   GG_TRY(C.dFb.alloc(std::max<int64_t>(N, 1)));
   GG_TRY(C.dNfb.alloc(3));  // [0] fallback count, [1] position error flag, [2] tensor-core wait timed out
   GG_CUDA(cudaMemsetAsync(C.dNfb.p, 0, 3 * sizeof(int), ctx->stream));
@@ -1732,16 +1686,16 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
       GG_CUDA(cudaGetLastError());
       const unsigned fb_blocks = (unsigned)std::min<long long>((N + 255) / 256, 8LL * ctx->sms);
       k_rk_finish_all<<<std::max(1u, fb_blocks), 256, 0, ctx->stream>>>(
-          rk.dInd.p, (long long)N, C.dKst.p, kloop, KEY, C.dFidx.p, C.dYd.p, C.dY.p, np, o.dPF.p, o.dQF.p, o.ld,
-          o.dMF.p, g.dR.p, g.dRP.p, g.dRPOR.p, g.dHead.p, g.q, rk.dVal.p, C.dFb.p, C.dNfb.p, parts, nsplit);
+          rk.dInd.p, (long long)N, C.dKst.p, kloop, KEY, C.dFidx.p, C.dPidx.p, tabs, g.q, rk.dVal.p, C.dFb.p, C.dNfb.p,
+          parts, nsplit);
       ::gg::note_launch();
     }
     GG_CUDA(cudaGetLastError());
   } else if (!tiles.empty()) {
-    k_rk_gemm<<<(unsigned)tiles.size(), 256, 0, ctx->stream>>>(C.dTiles.p, C.dRowpair.p, C.dPairs.p, C.dA.p, C.dY.p,
-                                                              C.dYd.p, KC, np, o.dPF.p, o.dQF.p, o.ld, o.dMF.p,
-                                                              g.dR.p, g.dRP.p, g.dRPOR.p, g.dHead.p, g.q, rk.dVal.p,
-                                                              (long long)N, C.dFb.p, C.dNfb.p);
+    auto dot = C.nr == 8 ? k_rk_dot<8> : C.nr == 4 ? k_rk_dot<4> : C.nr == 2 ? k_rk_dot<2> : k_rk_dot<1>;
+    dot<<<(unsigned)((tiles.size() + 3) / 4), 128, 0, ctx->stream>>>(C.dTiles.p, (int)tiles.size(), C.dTcr.p, C.dA.p,
+                                                                    tabs, g.q, rk.dVal.p, (long long)N, C.dFb.p,
+                                                                    C.dNfb.p);
     ::gg::note_launch();
     GG_CUDA(cudaGetLastError());
   }
@@ -1759,8 +1713,7 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
   if (nfb > 0) {
     const int wpb = 16;  // warps per block: an item each, their head terms by warp 0
     const int blocks = std::min((nfb + wpb - 1) / wpb, 4 * ctx->sms);
-    k_quad_table<<<blocks, 32 * wpb, 0, ctx->stream>>>(C.dFb.p, C.dNfb.p, nfb, C.dY.p, np, o.dPF.p, o.dQF.p, o.ld,
-                                                       g.dR.p, g.dRP.p, g.dRPOR.p, g.dHead.p, g.q, rk.dVal.p);
+    k_quad_table<<<blocks, 32 * wpb, 0, ctx->stream>>>(C.dFb.p, C.dNfb.p, nfb, tabs, g.q, rk.dVal.p);
     ::gg::note_launch();
     GG_CUDA(cudaGetLastError());
   }
@@ -1841,7 +1794,7 @@ int gg_slater(gg_ctx *ctx, int ia, int ib, int ic, int id, int k, double *out) {
   y.cs = 0;
   y.nd = 1;
   // SLATER's integration limit (slater.f90:56-60)
-  QuadItem it;
+  QuadItem it{};
   it.a = ia;
   it.c = ic;
   it.f = 0;
@@ -2267,7 +2220,7 @@ extern "C" int gg_slater_noalloc(gg_ctx *ctx, int ia, int ib, int ic, int id, in
   y.mtpb = (k == 0 && ib == id) ? g.n : y.mtp;
   y.cs = 0;
   y.nd = 1;
-  QuadItem it;
+  QuadItem it{};
   it.a = ia;
   it.c = ic;
   it.f = 0;
