@@ -8,9 +8,9 @@
 // contributions' DSUBRS(IR, IC) COEFF (dsubrs.f90: the generalized weight of
 // the CSF pair). Those label sums do not depend on the orbital except
 // through the final 1/UCF(J), so here one pass computes them for every label
-// of every block (one thread per label, contributions added in list order,
-// as the reference does), together with the diagonal FCO/GCO sums of every
-// (J, IB, K) (one thread each, CSFs in block and row order). A call for
+// of every block, together with the diagonal FCO/GCO sums of every pair of
+// orbitals. DSUBRS depends on the position only, so it is formed once per EMT
+// position (k_dsubrs_pos) and a contribution costs one FMA. A call for
 // orbital J then only filters and merges the labels on the host, in the
 // reference's order (FCO, GCO, the T list by block, the V^k lists by k and
 // block), so its lists are the reference's entry for entry.
@@ -45,20 +45,6 @@ struct SetcofState {
 
 namespace {
 
-// DSUBRS (rmcdhf90/dsubrs.f90:20-33): EOL, sum over the block's levels of
-// EVEC(I) EVEC(J) WT(level); otherwise WT(I) on the diagonal, 0 elsewhere.
-// ev holds the levels' coefficients by CSF ([ncf][nev]: one CSF's nev
-// values contiguous), the same products in the same order.
-__device__ __forceinline__ double dsubrs(int eol, int i, int j, int nev, const double *ev, const double *wt) {
-  if (eol) {
-    const double *a = ev + (size_t)(i - 1) * nev, *b = ev + (size_t)(j - 1) * nev;
-    double d = 0.0;
-    for (int k = 0; k < nev; ++k) d = d + a[k] * b[k] * wt[k];
-    return d;
-  }
-  return i == j ? wt[i - 1] : 0.0;
-}
-
 // the levels' coefficients by CSF: evr[r][k] = evec[k][r]
 __global__ void k_by_csf(const double *__restrict__ evec, int ncf, int nev, double *__restrict__ evr) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)ncf * nev;
@@ -68,58 +54,74 @@ __global__ void k_by_csf(const double *__restrict__ evec, int ncf, int nev, doub
   }
 }
 
-// DSUBRS(IR, IR) of every CSF
-__global__ void k_dsubrs_diag(int eol, int ncf, int nev, const double *__restrict__ ev, const double *__restrict__ wt,
-                              double *__restrict__ d) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < ncf) d[r] = dsubrs(eol, r + 1, r + 1, nev, ev, wt);
-}
-
-// the column owning each EMT position (ICLMN of the mcp records, 1-based)
-__global__ void k_owner(const int64_t *__restrict__ iendc, int ncf, int32_t *__restrict__ owner) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= ncf) return;
-  for (int64_t p = iendc[w] + lane; p < iendc[w + 1]; p += 32) owner[p] = w + 1;
-}
-
-// SUM over a label's contributions (setcof.f90:242-251 for the T list,
-// :302-311 for the V lists): CONTR = DSUBRS(IR, IC) COEFF, doubled when
-// IR != IC, added in list order; IR = IROW(INDX), IC = ICLMN. One warp per
-// label: the lanes form 32 consecutive CONTR at a time (their gathers in
-// flight together) into shared memory, lane 0 adds them in order.
+// DSUBRS (rmcdhf90/dsubrs.f90:20-33) of every EMT position, doubled off the
+// diagonal (setcof.f90:242-251): EOL, sum over the block's levels of EVEC(IR)
+// EVEC(IC) WT(level); otherwise WT(IR) on the diagonal, 0 elsewhere. ev holds
+// the levels' coefficients by CSF ([ncf][nev]). One warp per row IC, whose
+// EVEC(IC) WT it holds in shared memory, 32 levels at a time; the diagonal's
+// value also goes to diag. Bound: the FP64 pipe, one FMA per position and
+// level. (Formed per contribution, three operations per level and about 2.4
+// contributions per position, the label sums took 9.2 ms for 20,011 CSFs and
+// 10 levels; now 98 us, and 100 us for the sums.)
 constexpr int LS_WARPS = 4;
-__global__ void __launch_bounds__(LS_WARPS * 32) k_label_sums(int64_t nlab, const int64_t *__restrict__ start,
-                                                              const int32_t *__restrict__ loc,
-                                                              const double *__restrict__ coeff,
-                                                              const int32_t *__restrict__ irow,
-                                                              const int32_t *__restrict__ owner, int eol, int nev,
-                                                              const double *__restrict__ ev,
-                                                              const double *__restrict__ wt,
-                                                              double *__restrict__ out) {
-  __shared__ double cs[LS_WARPS][32];
+__global__ void __launch_bounds__(LS_WARPS * 32) k_dsubrs_pos(const int64_t *__restrict__ iendc,
+                                                              const int32_t *__restrict__ irow, int ncf, int eol,
+                                                              int nev, const double *__restrict__ ev,
+                                                              const double *__restrict__ wt, double *__restrict__ d,
+                                                              double *__restrict__ diag) {
+  __shared__ double sb[LS_WARPS][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t l = blockIdx.x * (int64_t)LS_WARPS + w;
-  if (l >= nlab) return;
-  double sum = 0.0;
-  const int64_t i0 = start[l], i1 = start[l + 1];
-  for (int64_t c = i0; c < i1; c += 32) {
-    const int64_t i = c + lane;
-    double contr = 0.0;
-    if (i < i1) {
-      const int p = loc[i] - 1;
-      const int ir = irow[p], ic = owner[p];
-      contr = dsubrs(eol, ir, ic, nev, ev, wt) * coeff[i];
-      if (ir != ic) contr = contr + contr;
+  const int r = blockIdx.x * LS_WARPS + w;
+  if (r >= ncf) return;
+  const int64_t p0 = iendc[r], p1 = iendc[r + 1];
+  for (int k0 = 0; k0 < (eol ? nev : 1); k0 += 32) {
+    const int nk = min(32, nev - k0);
+    if (eol) {
+      __syncwarp();
+      if (lane < nk) sb[w][lane] = ev[(size_t)r * nev + k0 + lane] * wt[k0 + lane];
+      __syncwarp();
     }
-    cs[w][lane] = contr;
-    __syncwarp();
-    if (lane == 0) {
-      const int n = (int)min((int64_t)32, i1 - c);
-      for (int t = 0; t < n; ++t) sum = sum + cs[w][t];
+    for (int64_t p = p0 + lane; p < p1; p += 32) {
+      const int c = irow[p] - 1;
+      double v = 0.0;
+      if (eol) {
+        const double *a = ev + (size_t)c * nev + k0;
+#pragma unroll 4
+        for (int k = 0; k < nk; ++k) v = fma(__ldg(a + k), sb[w][k], v);
+      } else if (c == r) {
+        v = wt[r];
+      }
+      if (k0 > 0) v += c == r ? diag[r] : 0.5 * d[p];
+      if (c == r) diag[r] = v;
+      d[p] = c == r ? v : v + v;
     }
-    __syncwarp();
   }
-  if (lane == 0) out[l] = sum;
+}
+
+// each label's sum of DSUBRS COEFF (setcof.f90:242-251 for the T list,
+// :302-311 for the V lists), one block per label: its threads take every
+// 256th contribution, eight gathers in flight, and a fixed tree adds them. Lists
+// are uneven (a few labels hold tens of thousands of contributions), so the
+// longest label sets the time: 193 us with 128 threads and four gathers.
+constexpr int LAB_THREADS = 256;
+__global__ void __launch_bounds__(LAB_THREADS) k_label_sums(const int64_t *__restrict__ start,
+                                                            const int32_t *__restrict__ loc,
+                                                            const double *__restrict__ coeff,
+                                                            const double *__restrict__ d, double *__restrict__ out) {
+  __shared__ double ws[LAB_THREADS / 32];
+  const int64_t l = blockIdx.x, i0 = start[l], i1 = start[l + 1];
+  double sum = 0.0;
+#pragma unroll 8
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += LAB_THREADS) sum = fma(__ldg(d + loc[i] - 1), coeff[i], sum);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double v = ws[0];
+    for (int w = 1; w < LAB_THREADS / 32; ++w) v += ws[w];
+    out[l] = v;
+  }
 }
 
 // one block's CSFs for the diagonal sums
@@ -130,61 +132,48 @@ struct DiagBlock {
   const int32_t *conf;    // [ncf]
 };
 
-// one diagonal sum: kind 0 FCO(K, IR, J, IB) (fco.f90), 1 GCO(K, IR, J, IB)
-// (gco.f90); c = CLRX of the item
-struct DiagItem {
-  int kind, j, ib, k;
-  int fullj, fullb;  // 2j + 1 of J and IB (a full subshell)
-  double c;
-};
-
-// SUMR = sum over blocks and CSFs of DSUBRS(IR, IR) FCO/GCO (setcof.f90:82-90,
-// 121-129), CSFs in block and row order. One warp per sum: the lanes form
-// 32 consecutive terms, lane 0 adds them in order.
-__global__ void __launch_bounds__(LS_WARPS * 32) k_diag_sums(const DiagItem *__restrict__ items, int nitems,
+// The diagonal sums over blocks and CSFs of DSUBRS(IR, IR) times the
+// occupation factors FCO (fco.f90) and GCO (gco.f90) are made of. They depend
+// on K through a factor CLRX^2 only, so one block per pair a <= b of orbitals
+// forms them all: a < b, sum d qa qb over all CSFs and over those where a or b
+// is full; a = b, sum d qa (qa - 1) / 2 and sum d qa^2 over those where a is
+// full. (One warp per (J, IB, K), adding 32 terms at a time on one lane, took
+// 5.0 ms for 34 subshells and 20,011 CSFs; now 117 us.)
+constexpr int DIAG_THREADS = 256;
+__global__ void __launch_bounds__(DIAG_THREADS) k_diag_pairs(const int *__restrict__ full,
                                                              const DiagBlock *__restrict__ blocks, int nblocks,
                                                              int nw, double *__restrict__ out) {
-  __shared__ double cs[LS_WARPS][32];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * LS_WARPS + w;
-  if (t >= nitems) return;
-  const DiagItem it = items[t];
-  double sumr = 0.0;
-  for (int b = 0; b < nblocks; ++b) {
-    const DiagBlock B = blocks[b];
-    for (int r0 = 1; r0 <= B.ncf; r0 += 32) {
-      const int ir = r0 + lane;
-      double term = 0.0;
-      if (ir <= B.ncf) {
-      const uint8_t *q = B.iq + (size_t)B.conf[ir - 1] * nw;
-      const int qa = q[it.j - 1], qb = q[it.ib - 1];
-      double f = 0.0;
-      if (it.kind == 0) {
-        if (it.j == it.ib) {
-          if (it.k == 0) {
-            f = (double)((qa * (qa - 1)) / 2);
-          } else if (qa == it.fullj) {
-            const double fac = it.c * (double)qa;
-            f = -0.5 * fac * fac;
-          }
-        } else if (it.k == 0) {
-          f = (double)(qa * qb);
-        }
-      } else if (qa == it.fullj || qb == it.fullb) {
-        f = -(double)(qa * qb) * it.c * it.c;
-      }
-      term = B.d[ir - 1] * f;
-      }
-      cs[w][lane] = term;
-      __syncwarp();
-      if (lane == 0) {
-        const int n = min(32, B.ncf - r0 + 1);
-        for (int u = 0; u < n; ++u) sumr = sumr + cs[w][u];
-      }
-      __syncwarp();
+  __shared__ double ws[2][DIAG_THREADS / 32];
+  const int a = blockIdx.y, b = blockIdx.x;
+  if (a > b) return;
+  const int fa = full[a], fb = full[b];
+  double s0 = 0.0, s1 = 0.0;
+  for (int t = 0; t < nblocks; ++t) {
+    const DiagBlock B = blocks[t];
+#pragma unroll 4
+    for (int r = threadIdx.x; r < B.ncf; r += DIAG_THREADS) {
+      const uint8_t *q = B.iq + (size_t)B.conf[r] * nw;
+      const int qa = q[a], qb = q[b];
+      const double d = B.d[r];
+      s0 = fma(d, (double)(a == b ? qa * (qa - 1) / 2 : qa * qb), s0);
+      if (qa == fa || qb == fb) s1 = fma(d, (double)(qa * qb), s1);
     }
   }
-  if (lane == 0) out[t] = sumr;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    ws[0][threadIdx.x >> 5] = s0;
+    ws[1][threadIdx.x >> 5] = s1;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double v = ws[threadIdx.x][0];
+    for (int i = 1; i < DIAG_THREADS / 32; ++i) v += ws[threadIdx.x][i];
+    out[2 * ((size_t)a * nw + b) + threadIdx.x] = v;
+  }
 }
 
 template <class T> int upv(DBuf<T> &b, const std::vector<T> &h, cudaStream_t s) {
@@ -253,18 +242,16 @@ int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *ne
       GG_TRY(dwt[b].alloc(ncf));
       GG_CUDA(cudaMemcpyAsync(dwt[b].p, wt[b], ncf * sizeof(double), cudaMemcpyHostToDevice, s));
     }
-    // every label's sum
-    DBuf<int32_t> owner;
-    DBuf<double> dsum;
-    GG_TRY(owner.alloc(std::max<int64_t>(1, m->nnz)));
-    k_owner<<<(unsigned)(((int64_t)ncf * 32 + 255) / 256), 256, 0, s>>>(m->dIendc.p, ncf, owner.p);
+    // DSUBRS by position, then every label's sum
+    DBuf<double> dpos, dsum;
+    GG_TRY(dpos.alloc(std::max<int64_t>(1, m->nnz)));
+    GG_TRY(ddiag[b].alloc(ncf));
+    k_dsubrs_pos<<<(ncf + LS_WARPS - 1) / LS_WARPS, LS_WARPS * 32, 0, s>>>(m->dIendc.p, m->dIrow.p, ncf, st->eol, ne,
+                                                                          devec[b].p, dwt[b].p, dpos.p, ddiag[b].p);
     ::gg::note_launch();
     GG_TRY(dsum.alloc(std::max<int64_t>(1, L.nlab)));
     if (L.nlab > 0) {
-      k_label_sums<<<(unsigned)((L.nlab + LS_WARPS - 1) / LS_WARPS), LS_WARPS * 32, 0, s>>>(
-          L.nlab, L.dStart.p, L.dLoc.p, L.dCoeff.p,
-                                                                   m->dIrow.p, owner.p, st->eol, ne, devec[b].p,
-                                                                   dwt[b].p, dsum.p);
+      k_label_sums<<<(unsigned)L.nlab, LAB_THREADS, 0, s>>>(L.dStart.p, L.dLoc.p, L.dCoeff.p, dpos.p, dsum.p);
       ::gg::note_launch();
     }
     GG_CUDA(cudaGetLastError());
@@ -274,54 +261,50 @@ int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *ne
       GG_CUDA(cudaMemcpyAsync(st->labs.back().data(), L.dLab.p, L.nlab * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
       GG_CUDA(cudaMemcpyAsync(st->sums.back().data(), dsum.p, L.nlab * sizeof(double), cudaMemcpyDeviceToHost, s));
     }
-    GG_CUDA(cudaStreamSynchronize(s));  // owner and dsum are freed here
+    GG_CUDA(cudaStreamSynchronize(s));  // dpos and dsum are freed here
     st->lab0.push_back(L.list_lab0);
     st->bkmaxf.push_back(L.kmaxf);
     st->kmaxf = std::max(st->kmaxf, L.kmaxf);
-    GG_TRY(ddiag[b].alloc(ncf));
-    k_dsubrs_diag<<<(ncf + 255) / 256, 256, 0, s>>>(st->eol, ncf, ne, devec[b].p, dwt[b].p, ddiag[b].p);
-    ::gg::note_launch();
     hb[b] = DiagBlock{ncf, ddiag[b].p, L.dIq.p, L.dConf.p};
   }
-  // the diagonal sums of every (J, IB, K) SETCOF asks for
+  // the diagonal sums of every (J, IB, K) SETCOF asks for, from the pairs' sums
   int jmax = 0;
   for (int a = 1; a <= nw; ++a) jmax = std::max(jmax, o.nkj[a]);
   st->kdim = jmax + 2;
-  std::vector<DiagItem> items;
-  std::vector<size_t> where;
-  for (int j = 1; j <= nw; ++j)
-    for (int ib = 1; ib <= nw; ++ib) {
-      const int kmax = (ib == j) ? o.nkj[j] - 1 : 0;
-      for (int k = 0; k <= kmax; k += 2) {
-        items.push_back(DiagItem{0, j, ib, k, o.nkj[j] + 1, o.nkj[ib] + 1, k > 0 ? clrx_host(o.nak[j], k, o.nak[j]) : 0.0});
-        where.push_back(st->idx(j, ib, k) * 2);
-      }
-      if (ib == j) continue;
-      const int kmin = (o.nak[j] * o.nak[ib] > 0) ? std::abs((o.nkj[j] - o.nkj[ib]) / 2)
-                                                   : std::abs((o.nkj[j] - o.nkj[ib]) / 2) + 1;
-      for (int k = kmin; k <= (o.nkj[j] + o.nkj[ib]) / 2; k += 2) {
-        items.push_back(DiagItem{1, j, ib, k, o.nkj[j] + 1, o.nkj[ib] + 1, clrx_host(o.nak[j], k, o.nak[ib])});
-        where.push_back(st->idx(j, ib, k) * 2 + 1);
-      }
-    }
-  DBuf<DiagItem> ditems;
+  std::vector<int> full(nw);
+  for (int a = 0; a < nw; ++a) full[a] = o.nkj[a + 1] + 1;
+  DBuf<int> dfull;
   DBuf<DiagBlock> dblocks;
   DBuf<double> dout;
-  GG_TRY(upv(ditems, items, s));
+  GG_TRY(upv(dfull, full, s));
   GG_TRY(upv(dblocks, hb, s));
-  GG_TRY(dout.alloc(std::max<size_t>(1, items.size())));
-  if (!items.empty()) {
-    k_diag_sums<<<(unsigned)((items.size() + LS_WARPS - 1) / LS_WARPS), LS_WARPS * 32, 0, s>>>(
-        ditems.p, (int)items.size(), dblocks.p, nblocks, nw, dout.p);
-    ::gg::note_launch();
-  }
+  GG_TRY(dout.alloc((size_t)2 * nw * nw));
+  k_diag_pairs<<<dim3(nw, nw), DIAG_THREADS, 0, s>>>(dfull.p, dblocks.p, nblocks, nw, dout.p);
+  ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
-  std::vector<double> hv(items.size());
-  if (!items.empty()) GG_CUDA(cudaMemcpyAsync(hv.data(), dout.p, hv.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+  std::vector<double> hv((size_t)2 * nw * nw);
+  GG_CUDA(cudaMemcpyAsync(hv.data(), dout.p, hv.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaStreamSynchronize(s));
   st->fco.assign((size_t)nw * nw * st->kdim, 0.0);
   st->gco.assign((size_t)nw * nw * st->kdim, 0.0);
-  for (size_t t = 0; t < items.size(); ++t) (where[t] % 2 ? st->gco : st->fco)[where[t] / 2] = hv[t];
+  for (int j = 1; j <= nw; ++j)
+    for (int ib = 1; ib <= nw; ++ib) {
+      const double *v = &hv[2 * ((size_t)(std::min(j, ib) - 1) * nw + (std::max(j, ib) - 1))];
+      st->fco[st->idx(j, ib, 0)] = v[0];
+      if (ib == j) {
+        for (int k = 2; k <= o.nkj[j] - 1; k += 2) {
+          const double c = clrx_host(o.nak[j], k, o.nak[j]);
+          st->fco[st->idx(j, ib, k)] = -0.5 * c * c * v[1];
+        }
+        continue;
+      }
+      const int kmin = (o.nak[j] * o.nak[ib] > 0) ? std::abs((o.nkj[j] - o.nkj[ib]) / 2)
+                                                   : std::abs((o.nkj[j] - o.nkj[ib]) / 2) + 1;
+      for (int k = kmin; k <= (o.nkj[j] + o.nkj[ib]) / 2; k += 2) {
+        const double c = clrx_host(o.nak[j], k, o.nak[ib]);
+        st->gco[st->idx(j, ib, k)] = -(c * c * v[1]);
+      }
+    }
   // the labels of each orbital, in visiting order
   st->tref.assign(nw + 1, {});
   st->vref.assign(nw + 1, {});
