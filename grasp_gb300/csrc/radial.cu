@@ -133,30 +133,35 @@ __device__ double quad_warp(const double *TA, double *panel, int mtp, const doub
 // YZK part 1 (yzk.f90:105-126, 190-201): RHOP and the two TEMP arrays.
 //   TZ(i) = r^k RHOP(i), TW(i) = RHOP(i) / r^(k+1) on 2 <= i <= MTP, else 0.
 // ---------------------------------------------------------------------------
-__global__ void k_ytemp(const YDesc *__restrict__ yd, int nf, const double *__restrict__ PF,
-                        const double *__restrict__ QF, int ld, const double *__restrict__ RP,
-                        const double *__restrict__ pw, int np, double *__restrict__ TZ, double *__restrict__ TW) {
-  const int f = blockIdx.y;
-  if (f >= nf) return;
-  const YDesc y = yd[f];
-  const double *RTTK = pw + (size_t)(0 * (KLIMIT + 1) + y.k) * np;
-  const double *RTTKM1 = pw + (size_t)(3 * (KLIMIT + 1) + y.k) * np;
-  const double *RM = pw;  // row k = 0 of table 0
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    double tz = 0.0, tw = 0.0;
-    if (i >= 2 && i <= y.mtp) {
-      const double rhop =
-          RP[i] * (pf(PF, ld, i, y.b) * pf(PF, ld, i, y.d) + pf(QF, ld, i, y.b) * pf(QF, ld, i, y.d));
-      if (y.k == 0) {
-        tz = rhop;
-        tw = rhop * RM[i];
-      } else {
-        tz = RTTK[i] * rhop;
-        tw = rhop * RTTKM1[i];
+// In all kernels over functions, nfp (may be null) points to a number of
+// functions on the device that replaces nf, the bound the launch was sized by.
+__device__ __forceinline__ int nfuncs(int nf, const int *nfp) { return nfp ? min(nf, *nfp) : nf; }
+__global__ void k_ytemp(const YDesc *__restrict__ yd, int nf, const int *__restrict__ nfp,
+                        const double *__restrict__ PF, const double *__restrict__ QF, int ld,
+                        const double *__restrict__ RP, const double *__restrict__ pw, int np,
+                        double *__restrict__ TZ, double *__restrict__ TW) {
+  nf = nfuncs(nf, nfp);
+  for (int f = blockIdx.y; f < nf; f += gridDim.y) {
+    const YDesc y = yd[f];
+    const double *RTTK = pw + (size_t)(0 * (KLIMIT + 1) + y.k) * np;
+    const double *RTTKM1 = pw + (size_t)(3 * (KLIMIT + 1) + y.k) * np;
+    const double *RM = pw;  // row k = 0 of table 0
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
+      double tz = 0.0, tw = 0.0;
+      if (i >= 2 && i <= y.mtp) {
+        const double rhop =
+            RP[i] * (pf(PF, ld, i, y.b) * pf(PF, ld, i, y.d) + pf(QF, ld, i, y.b) * pf(QF, ld, i, y.d));
+        if (y.k == 0) {
+          tz = rhop;
+          tw = rhop * RM[i];
+        } else {
+          tz = RTTK[i] * rhop;
+          tw = rhop * RTTKM1[i];
+        }
       }
+      TZ[(size_t)f * np + i] = tz;
+      TW[(size_t)f * np + i] = tw;
     }
-    TZ[(size_t)f * np + i] = tz;
-    TW[(size_t)f * np + i] = tw;
   }
 }
 
@@ -165,9 +170,11 @@ __global__ void k_ytemp(const YDesc *__restrict__ yd, int nf, const double *__re
 // recurrences for Z (forward) and W (backward). One thread per (function,
 // residue class mod 4); the four threads of a function are adjacent lanes.
 // ---------------------------------------------------------------------------
-__global__ void k_ychain(const YDesc *__restrict__ yd, int nf, const double *__restrict__ TZ,
+__global__ void k_ychain(const YDesc *__restrict__ yd, int nf, const int *__restrict__ nfp,
+                         const double *__restrict__ TZ,
                          const double *__restrict__ TW, const double *__restrict__ R,
                          const double *__restrict__ pw, int np, QuadConst q, double *__restrict__ Y) {
+  nf = nfuncs(nf, nfp);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int f = t >> 2, c = t & 3;
   const bool active = f < nf;
@@ -909,7 +916,7 @@ __global__ void __launch_bounds__(256) k_pot_part(const PotChunk *__restrict__ c
     const int nt = min(POT_CHUNK, g.nt - t0);
     __syncthreads();
     if ((int)threadIdx.x < nt) {
-      sf[threadIdx.x] = tab[g.key[t0 + threadIdx.x]] - 1;
+      sf[threadIdx.x] = max(tab[g.key[t0 + threadIdx.x]] - 1, 0);  // 0: a label the parser refused
       so[threadIdx.x] = x ? g.iorb[t0 + threadIdx.x] : 1;
       sc[threadIdx.x] = g.coef[t0 + threadIdx.x];
     }
@@ -1208,26 +1215,28 @@ bool triangrk(int la, int k, int lb) {  // rci90/triangrk.f90:27-37
 //   RW(i) = the three terms C1 (TW(i) + TW(i+4)), C2 (TW(i+1) + TW(i+3)),
 //     C3 TW(i+2), 2 <= i <= MTP, added to W one after the other
 //     (WK = ((WK + t1) + t2) + t3, k_ychain's left-to-right sum).
-__global__ void k_yincr(const YDesc *__restrict__ yd, int nf, const double *__restrict__ TZ,
-                        const double *__restrict__ TW, int np, QuadConst q, double *__restrict__ RZ,
-                        double *__restrict__ RW) {
-  const int f = blockIdx.y;
-  if (f >= nf) return;
-  const int MTP = yd[f].mtp;
-  const double *T = TZ + (size_t)f * np, *Tw = TW + (size_t)f * np;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    double rz = 0.0, w1 = 0.0, w2 = 0.0, w3 = 0.0;
-    if (i >= 5) rz = q.C1 * (T[i - 4] + T[i]) + q.C2 * (T[i - 3] + T[i - 1]) + q.C3 * T[i - 2];
-    if (i >= 2 && i <= MTP) {
-      w1 = q.C1 * (Tw[i] + Tw[i + 4]);
-      w2 = q.C2 * (Tw[i + 1] + Tw[i + 3]);
-      w3 = q.C3 * Tw[i + 2];
+// The chains read RZ up to MTP + 3 and RW up to MTP only.
+__global__ void k_yincr(const YDesc *__restrict__ yd, int nf, const int *__restrict__ nfp,
+                        const double *__restrict__ TZ, const double *__restrict__ TW, int np, QuadConst q,
+                        double *__restrict__ RZ, double *__restrict__ RW) {
+  nf = nfuncs(nf, nfp);
+  for (int f = blockIdx.y; f < nf; f += gridDim.y) {
+    const int MTP = yd[f].mtp;
+    const double *T = TZ + (size_t)f * np, *Tw = TW + (size_t)f * np;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= MTP + 3; i += gridDim.x * blockDim.x) {
+      double rz = 0.0, w1 = 0.0, w2 = 0.0, w3 = 0.0;
+      if (i >= 5) rz = q.C1 * (T[i - 4] + T[i]) + q.C2 * (T[i - 3] + T[i - 1]) + q.C3 * T[i - 2];
+      if (i >= 2 && i <= MTP) {
+        w1 = q.C1 * (Tw[i] + Tw[i + 4]);
+        w2 = q.C2 * (Tw[i + 1] + Tw[i + 3]);
+        w3 = q.C3 * Tw[i + 2];
+      }
+      RZ[(size_t)f * np + i] = rz;
+      double *rw = RW + ((size_t)f * np + i) * 3;
+      rw[0] = w1;
+      rw[1] = w2;
+      rw[2] = w3;
     }
-    RZ[(size_t)f * np + i] = rz;
-    double *rw = RW + ((size_t)f * np + i) * 3;
-    rw[0] = w1;
-    rw[1] = w2;
-    rw[2] = w3;
   }
 }
 
@@ -1272,10 +1281,12 @@ __device__ __forceinline__ double ychain_run(double acc, const double *__restric
 // the chains' additions (Z: 16 points loaded ahead, W: 8); writes Z into Y,
 // W into W, each chain's K = 0 correction DIF and the function's asymptotic
 // value ZKLIM
-__global__ void k_ychain_sum(const YDesc *__restrict__ yd, int nf, const double *__restrict__ TZ,
+__global__ void k_ychain_sum(const YDesc *__restrict__ yd, int nf, const int *__restrict__ nfp,
+                             const double *__restrict__ TZ,
                              const double *__restrict__ RZ, const double *__restrict__ RW, int np, QuadConst q,
                              double *__restrict__ Y, double *__restrict__ W, double *__restrict__ dif_out,
                              double *__restrict__ zk_out) {
+  nf = nfuncs(nf, nfp);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int f = t >> 2, c = t & 3;
   const bool active = f < nf;
@@ -1319,41 +1330,43 @@ __global__ void k_ychain_sum(const YDesc *__restrict__ yd, int nf, const double 
   ychain_run<3, 8>(0.0, Rw, Wf, s + 4 * (cnt - 1), -4, cnt);
 }
 
-__global__ void k_yassemble(const YDesc *__restrict__ yd, int nf, const double *__restrict__ R,
-                            const double *__restrict__ pw, int np, QuadConst q, const double *__restrict__ dif,
-                            const double *__restrict__ zk, const double *__restrict__ W, double *__restrict__ Y) {
-  const int f = blockIdx.y;
-  if (f >= nf) return;
-  const YDesc y = yd[f];
-  const int K = y.k, MTP = y.mtp, MTPP3 = MTP + 3, N = q.n;
-  const double zklim = zk[f];
-  const double *RTTKM = pw + (size_t)(1 * (KLIMIT + 1) + K) * np;
-  const double *RTTK1 = pw + (size_t)(2 * (KLIMIT + 1) + K) * np;
-  const double *Wf = W + (size_t)f * np;
-  double *Yf = Y + (size_t)f * np;
-  for (int i = 2 + blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    double yv = 0.0;
-    if (i <= N) {
-      double zf;
-      if (K == 0) {
-        if (i <= MTPP3) {
-          const double d = dif[(size_t)f * 4 + ((i - 2) & 3)];
-          zf = (d != 0.0) ? Yf[i] - d : Yf[i];
+__global__ void k_yassemble(const YDesc *__restrict__ yd, int nf, const int *__restrict__ nfp,
+                            const double *__restrict__ R, const double *__restrict__ pw, int np, QuadConst q,
+                            const double *__restrict__ dif, const double *__restrict__ zk,
+                            const double *__restrict__ W, double *__restrict__ Y) {
+  nf = nfuncs(nf, nfp);
+  for (int f = blockIdx.y; f < nf; f += gridDim.y) {
+    const YDesc y = yd[f];
+    const int K = y.k, MTP = y.mtp, MTPP3 = MTP + 3, N = q.n;
+    const double zklim = zk[f];
+    const double *RTTKM = pw + (size_t)(1 * (KLIMIT + 1) + K) * np;
+    const double *RTTK1 = pw + (size_t)(2 * (KLIMIT + 1) + K) * np;
+    const double *Wf = W + (size_t)f * np;
+    double *Yf = Y + (size_t)f * np;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
+      double yv = 0.0;
+      if (i >= 2 && i <= N) {
+        double zf;
+        if (K == 0) {
+          if (i <= MTPP3) {
+            const double d = dif[(size_t)f * 4 + ((i - 2) & 3)];
+            zf = (d != 0.0) ? Yf[i] - d : Yf[i];
+          } else {
+            zf = zklim;
+          }
         } else {
-          zf = zklim;
+          zf = (i <= MTPP3) ? Yf[i] * RTTKM[i] : zklim * RTTKM[i];
         }
-      } else {
-        zf = (i <= MTPP3) ? Yf[i] * RTTKM[i] : zklim * RTTKM[i];
+        double wkf = 0.0;
+        if (i <= MTP) {
+          const double wk = Wf[i];
+          wkf = (K == 0) ? wk * R[i] : wk * RTTK1[i];
+        }
+        yv = zf + wkf;
+        if (i > y.mtpb) yv = 0.0;
       }
-      double wkf = 0.0;
-      if (i <= MTP) {
-        const double wk = Wf[i];
-        wkf = (K == 0) ? wk * R[i] : wk * RTTK1[i];
-      }
-      yv = zf + wkf;
-      if (i > y.mtpb) yv = 0.0;
+      Yf[i] = yv;
     }
-    Yf[i] = yv;
   }
 }
 
@@ -1361,30 +1374,32 @@ __global__ void k_yassemble(const YDesc *__restrict__ yd, int nf, const double *
 constexpr int YSPLIT_MIN = 32;
 
 // Builds Y functions for the descriptor list on the device: TZ/TW scratch
-// then the chains. Y must hold nf * np doubles.
-int build_y(gg_ctx *ctx, const YDesc *d_yd, int nf, double *dY, DBuf<double> &scratch) {
+// then the chains. Y must hold nf * np doubles. nfp (may be null): the number
+// of functions on the device, at most nf.
+int build_y(gg_ctx *ctx, const YDesc *d_yd, int nf, double *dY, DBuf<double> &scratch, const int *nfp = nullptr) {
   Grid &g = ctx->grid;
   Orbitals &o = ctx->orb;
   const int np = g.np;
   const bool split = nf >= YSPLIT_MIN;
   GG_TRY(scratch.alloc(split ? (size_t)6 * nf * np + (size_t)5 * nf : (size_t)2 * nf * np));
   double *TZ = scratch.p, *TW = scratch.p + (size_t)nf * np;
-  dim3 grid1((np + 127) / 128, nf);
-  k_ytemp<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, o.dPF.p, o.dQF.p, o.ld, g.dRP.p, g.dPow.p, np, TZ, TW); ::gg::note_launch();
+  dim3 grid1((np + 127) / 128, std::min(nf, nfp ? 4 * ctx->sms : 65535));
+  k_ytemp<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, nfp, o.dPF.p, o.dQF.p, o.ld, g.dRP.p, g.dPow.p, np, TZ, TW);
+  ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
-  GG_CUDA(cudaMemsetAsync(dY, 0, (size_t)nf * np * sizeof(double), ctx->stream));
   const int nthr = nf * 4;
   if (!split) {
-    k_ychain<<<(nthr + 127) / 128, 128, 0, ctx->stream>>>(d_yd, nf, TZ, TW, g.dR.p, g.dPow.p, np, g.q, dY);
+    GG_CUDA(cudaMemsetAsync(dY, 0, (size_t)nf * np * sizeof(double), ctx->stream));
+    k_ychain<<<(nthr + 127) / 128, 128, 0, ctx->stream>>>(d_yd, nf, nfp, TZ, TW, g.dR.p, g.dPow.p, np, g.q, dY);
     ::gg::note_launch();
   } else {
     // RZ: one term per point; RW: three terms per point; DIF per chain; ZKLIM
     double *RZ = TW + (size_t)nf * np, *RW = RZ + (size_t)nf * np, *dif = RW + (size_t)3 * nf * np;
     double *zk = dif + 4 * nf;
-    k_yincr<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, TZ, TW, np, g.q, RZ, RW);
+    k_yincr<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, nfp, TZ, TW, np, g.q, RZ, RW);
     // W goes where TW was: k_yincr was its last reader
-    k_ychain_sum<<<(nthr + 127) / 128, 128, 0, ctx->stream>>>(d_yd, nf, TZ, RZ, RW, np, g.q, dY, TW, dif, zk);
-    k_yassemble<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, g.dR.p, g.dPow.p, np, g.q, dif, zk, TW, dY);
+    k_ychain_sum<<<(nthr + 127) / 128, 128, 0, ctx->stream>>>(d_yd, nf, nfp, TZ, RZ, RW, np, g.q, dY, TW, dif, zk);
+    k_yassemble<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, nfp, g.dR.p, g.dPow.p, np, g.q, dif, zk, TW, dY);
     ::gg::note_launch();
     ::gg::note_launch();
     ::gg::note_launch();
@@ -1851,133 +1866,163 @@ struct PotJob {
   std::vector<double> lag_wa;  // and their weights ECV WB
 };
 
-// the jobs' YPOT, XPOT, then LAGCON and DACON, into dPot (3 n per job): all
-// Y functions of all lists built once
-static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, DBuf<double> &dPot) {
+// What run_potentials keeps on the context between calls: a pinned staging
+// buffer and the device buffers, as far as a call's fit in POT_KEEP bytes (a
+// COFPOT call for each orbital of an SCF cycle then allocates nothing)
+struct PotWork {
+  void *stage = nullptr;
+  size_t stage_bytes = 0;
+  DBuf<char> up;  // the staged block on the device
+  DBuf<int> term, tab, info;
+  DBuf<double> coef, Y, scratch, pot, part;
+  DBuf<YDesc> yd;
+  ~PotWork() { cudaFreeHost(stage); }
+};
+constexpr size_t POT_KEEP = (size_t)512 << 20, POT_BOUND = (size_t)256 << 20;
+
+// the jobs' YPOT, XPOT, then LAGCON and DACON, into W.pot (3 n per job): all
+// Y functions of all lists built once. Everything the host prepares (lists,
+// chunk and job records) travels in one copy and the call waits once, at the
+// end; the launches over functions are sized by a bound and read the number
+// of functions on the device. out (may be null): where the potentials go on
+// the host.
+static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, double *out = nullptr) {
   Orbitals &o = ctx->orb;
   Grid &g = ctx->grid;
   cudaStream_t s = ctx->stream;
   const int n = g.n, nw = o.nw;
+  if (!ctx->pot_work) ctx->pot_work = std::make_shared<PotWork>();
+  PotWork &W = *std::static_pointer_cast<PotWork>(ctx->pot_work);
   // every job's YPOT list, then every job's XPOT list, as the caller passed
-  // them, staged in pinned memory and copied to the device in one transfer
+  // them; the chunks of every list; the DACON and LAGCON lists; the job records
   std::vector<size_t> oy(jobs.size()), ox(jobs.size());
-  size_t T = 0;
+  size_t T = 0, nd = 0, nl = 0;
   for (size_t j = 0; j < jobs.size(); ++j) oy[j] = T, T += (size_t)jobs[j].y.n;
   const size_t TY = T;
   for (size_t j = 0; j < jobs.size(); ++j) ox[j] = T, T += (size_t)jobs[j].x.n;
-  const size_t lab_bytes = (T * sizeof(int32_t) + 15) / 16 * 16, need = lab_bytes + T * sizeof(double);
-  if (need > ctx->pot_stage_bytes) {
-    void *hp = nullptr;
-    GG_CUDA(cudaHostAlloc(&hp, need + need / 4, cudaHostAllocDefault));
-    note_alloc();
-    ctx->pot_stage = std::shared_ptr<void>(hp, [](void *q) { cudaFreeHost(q); });
-    ctx->pot_stage_bytes = need + need / 4;
+  const int len = (int)(POT_CHUNK * (T / ((size_t)POT_CHUNK * 16384) + 1));
+  size_t nch = 0;
+  for (const PotJob &J : jobs) {
+    nch += (size_t)(J.y.n + len - 1) / len + (size_t)(J.x.n + len - 1) / len;
+    nd += J.nda.size();
+    nl += J.lag_m.size();
   }
-  char *stage = static_cast<char *>(ctx->pot_stage.get());
-  int32_t *hlab = reinterpret_cast<int32_t *>(stage);
-  double *hco = reinterpret_cast<double *>(stage + lab_bytes);
+  size_t need = 0;
+  auto place = [&](size_t bytes) {
+    const size_t at = need;
+    need += (bytes + 15) / 16 * 16;
+    return at;
+  };
+  const size_t alab = place(T * sizeof(int32_t)), aco = place(T * sizeof(double)), ach = place(nch * sizeof(PotChunk)),
+               afin = place(jobs.size() * sizeof(PotFinal)), aint = place((nd + nl) * sizeof(int)),
+               adbl = place((nd + nl) * sizeof(double));
+  const size_t ares = place(2 * sizeof(int) + (out ? (size_t)3 * n * jobs.size() * sizeof(double) : 0) + 16);
+  if (need > W.stage_bytes) {
+    cudaFreeHost(W.stage);
+    W.stage = nullptr;
+    W.stage_bytes = 0;
+    GG_CUDA(cudaHostAlloc(&W.stage, need + need / 4, cudaHostAllocDefault));
+    note_alloc();
+    W.stage_bytes = need + need / 4;
+  }
+  char *stage = static_cast<char *>(W.stage);
+  const size_t tsize = (size_t)(KLIMIT + 1) * nw * nw, T1 = std::max<size_t>(T, 1);
+  int nfb = (int)std::max<size_t>(1, std::min(T, tsize));  // at least as many as there are functions
+  GG_TRY(W.up.alloc(ares));
+  GG_TRY(W.term.alloc(2 * T1));
+  GG_TRY(W.coef.alloc(T1));
+  GG_TRY(W.tab.alloc(tsize));
+  GG_TRY(W.info.alloc(2));
+  GG_TRY(W.yd.alloc(nfb));
+  GG_TRY(W.pot.alloc((size_t)3 * n * std::max<size_t>(1, jobs.size())));
+  int *dkey = W.term.p, *diorb = dkey + T1;
+  int32_t *hlab = reinterpret_cast<int32_t *>(stage + alab);
+  double *hco = reinterpret_cast<double *>(stage + aco);
+  PotChunk *hc = reinterpret_cast<PotChunk *>(stage + ach);
+  PotFinal *hf = reinterpret_cast<PotFinal *>(stage + afin);
+  int *hi = reinterpret_cast<int *>(stage + aint);
+  double *hd = reinterpret_cast<double *>(stage + adbl);
+  const int *di = reinterpret_cast<const int *>(W.up.p + aint);
+  const double *dd = reinterpret_cast<const double *>(W.up.p + adbl);
+  size_t po = 0, ic = 0, il = 0;  // partial sums (in doubles), chunks, one-body and multiplier entries
   for (size_t j = 0; j < jobs.size(); ++j) {
-    const RawList *L[2] = {&jobs[j].y, &jobs[j].x};
+    const PotJob &J = jobs[j];
+    const RawList *L[2] = {&J.y, &J.x};
     const size_t at[2] = {oy[j], ox[j]};
-    for (int m = 0; m < 2; ++m)
+    size_t start[2];
+    for (int m = 0; m < 2; ++m) {
+      start[m] = po;
       if (L[m]->n > 0) {
         std::memcpy(hlab + at[m], L[m]->lab, (size_t)L[m]->n * sizeof(int32_t));
         std::memcpy(hco + at[m], L[m]->co, (size_t)L[m]->n * sizeof(double));
       }
+      for (int t0 = 0; t0 < L[m]->n; t0 += len) {
+        hc[ic++] = PotChunk{dkey + at[m] + t0, m ? diorb + at[m] + t0 : nullptr, W.coef.p + at[m] + t0, po,
+                            std::min(len, L[m]->n - t0)};
+        po += (size_t)(m ? 2 : 1) * n;
+      }
+    }
+    const size_t i0 = il;
+    for (size_t t = 0; t < J.lag_m.size(); ++t) hi[il] = J.lag_m[t], hd[il++] = J.lag_wa[t];
+    const size_t i1 = il;
+    for (size_t t = 0; t < J.nda.size(); ++t) hi[il] = J.nda[t], hd[il++] = J.da[t];
+    hf[j] = PotFinal{W.pot.p + (size_t)3 * n * j, start[0], start[1], (J.y.n + len - 1) / len, (J.x.n + len - 1) / len,
+                     di + i0, di + i1, dd + i0, dd + i1, (int)J.lag_m.size(), (int)J.nda.size()};
   }
-  const size_t tsize = (size_t)(KLIMIT + 1) * nw * nw;
-  DBuf<char> draw;
-  DBuf<int> dterm, dtab, dinfo;  // dterm: key, orbital per term
-  DBuf<double> dcoef;
-  DBuf<YDesc> dy;
-  GG_TRY(draw.alloc(std::max<size_t>(need, 16)));
-  GG_TRY(dterm.alloc(2 * std::max<size_t>(T, 1)));
-  GG_TRY(dcoef.alloc(std::max<size_t>(T, 1)));
-  GG_TRY(dtab.alloc(tsize));
-  GG_TRY(dinfo.alloc(2));
-  GG_TRY(dy.alloc(std::max<size_t>(1, std::min(T, tsize))));
-  int *dkey = dterm.p, *diorb = dkey + std::max<size_t>(T, 1);
-  const int32_t *dlab = reinterpret_cast<const int32_t *>(draw.p);
-  const double *dco = reinterpret_cast<const double *>(draw.p + lab_bytes);
-  if (T > 0) GG_CUDA(cudaMemcpyAsync(draw.p, stage, need, cudaMemcpyHostToDevice, s));
-  GG_CUDA(cudaMemsetAsync(dtab.p, 0, tsize * sizeof(int), s));
-  GG_CUDA(cudaMemsetAsync(dinfo.p, 0, 2 * sizeof(int), s));
+  GG_TRY(W.part.alloc(std::max<size_t>(1, po)));
+  if (ares > 0) GG_CUDA(cudaMemcpyAsync(W.up.p, stage, ares, cudaMemcpyHostToDevice, s));
+  GG_CUDA(cudaMemsetAsync(W.tab.p, 0, tsize * sizeof(int), s));
+  GG_CUDA(cudaMemsetAsync(W.info.p, 0, 2 * sizeof(int), s));
+  const int32_t *dlab = reinterpret_cast<const int32_t *>(W.up.p + alab);
+  const double *dco = reinterpret_cast<const double *>(W.up.p + aco);
   const unsigned pgrid = (unsigned)std::max<size_t>(1, std::min<size_t>((T + 255) / 256, (size_t)8 * ctx->sms));
   for (int m = 0; m < 2; ++m) {
     const size_t a = m == 0 ? 0 : TY, cnt = m == 0 ? TY : T - TY;
     if (cnt == 0) continue;
-    k_parse_terms<<<pgrid, 256, 0, s>>>(m, (int64_t)cnt, dlab + a, dco + a, nw, g.c, o.dMF.p, n, dtab.p, dy.p,
-                                        dkey + a, diorb + a, dcoef.p + a, dinfo.p);
+    k_parse_terms<<<pgrid, 256, 0, s>>>(m, (int64_t)cnt, dlab + a, dco + a, nw, g.c, o.dMF.p, n, W.tab.p, W.yd.p,
+                                        dkey + a, diorb + a, W.coef.p + a, W.info.p);
     ::gg::note_launch();
   }
-  int info[2] = {0, 0};
-  GG_CUDA(cudaMemcpyAsync(info, dinfo.p, sizeof(info), cudaMemcpyDeviceToHost, s));
-  GG_CUDA(cudaStreamSynchronize(s));
-  if (info[1]) return fail(GG_ERR_ARG, "potential: label outside the orbital set or K above 20");
-  const int nf = std::max(1, info[0]);
-  DBuf<double> dY, scratch;
-  GG_TRY(dY.alloc((size_t)nf * g.np));
-  if (info[0] > 0) GG_TRY(build_y(ctx, dy.p, nf, dY.p, scratch));  // no terms: no function is read
-  GG_TRY(dPot.alloc((size_t)3 * n * std::max<size_t>(1, jobs.size())));
-  // the DACON and LAGCON lists (a few entries per job) in one upload each
-  std::vector<int> ih;
-  std::vector<double> dh;
-  struct Off { size_t dn, dd, lm, lw; };
-  std::vector<Off> off(jobs.size());
-  for (size_t j = 0; j < jobs.size(); ++j) {
-    const PotJob &J = jobs[j];
-    auto pi = [&](const std::vector<int> &v) { size_t at = ih.size(); ih.insert(ih.end(), v.begin(), v.end()); ih.push_back(0); return at; };
-    auto pd = [&](const std::vector<double> &v) { size_t at = dh.size(); dh.insert(dh.end(), v.begin(), v.end()); dh.push_back(0.0); return at; };
-    off[j] = Off{pi(J.nda), pd(J.da), pi(J.lag_m), pd(J.lag_wa)};
+  if ((size_t)7 * nfb * g.np * sizeof(double) > POT_BOUND) {  // too much to reserve for a bound: wait for the number
+    int cnt = 0;
+    GG_CUDA(cudaMemcpyAsync(&cnt, W.info.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    GG_CUDA(cudaStreamSynchronize(s));
+    nfb = std::max(1, cnt);
   }
-  DBuf<int> di;
-  DBuf<double> dd, dpart;
-  GG_TRY(upload(di, ih, s));
-  GG_TRY(upload(dd, dh, s));
-  // every list cut into chunks (a few thousand at most), one launch for all
-  // of them, then one for every job's point values
-  const int len = (int)(POT_CHUNK * (T / ((size_t)POT_CHUNK * 16384) + 1));
-  std::vector<PotChunk> hc;
-  std::vector<PotFinal> hf(jobs.size());
-  size_t po = 0;  // partial sums, in doubles
-  auto cut = [&](size_t at, int nt, bool x) {
-    const size_t start = po;
-    for (int t0 = 0; t0 < nt; t0 += len) {
-      hc.push_back(PotChunk{dkey + at + t0, x ? diorb + at + t0 : nullptr, dcoef.p + at + t0,
-                            po, std::min(len, nt - t0)});
-      po += (size_t)(x ? 2 : 1) * n;
-    }
-    return start;
-  };
-  std::vector<size_t> py(jobs.size()), px(jobs.size());
-  for (size_t j = 0; j < jobs.size(); ++j) {
-    py[j] = cut(oy[j], jobs[j].y.n, false);
-    px[j] = cut(ox[j], jobs[j].x.n, true);
-  }
-  GG_TRY(dpart.alloc(po));
-  for (size_t j = 0; j < jobs.size(); ++j) {
-    const PotJob &J = jobs[j];
-    hf[j] = PotFinal{dPot.p + (size_t)3 * n * j, py[j], px[j], (J.y.n + len - 1) / len,
-                     (J.x.n + len - 1) / len, di.p + off[j].lm, di.p + off[j].dn, dd.p + off[j].lw, dd.p + off[j].dd,
-                     (int)J.lag_m.size(), (int)J.nda.size()};
-  }
-  DBuf<PotChunk> dchunk;
-  DBuf<PotFinal> dfin;
-  GG_TRY(upload(dchunk, hc, s));
-  GG_TRY(upload(dfin, hf, s));
-  if (!hc.empty()) {
-    k_pot_part<<<dim3((n + 63) / 64, (unsigned)hc.size()), 256, 0, s>>>(dchunk.p, dtab.p, dY.p, g.np, o.dPF.p, o.dQF.p,
-                                                                       o.ld, n, dpart.p);
+  GG_TRY(W.Y.alloc((size_t)nfb * g.np));
+  if (T > 0) GG_TRY(build_y(ctx, W.yd.p, nfb, W.Y.p, W.scratch, W.info.p));
+  // one launch for all chunks, one for every job's point values
+  if (nch > 0) {
+    k_pot_part<<<dim3((n + 63) / 64, (unsigned)nch), 256, 0, s>>>(reinterpret_cast<const PotChunk *>(W.up.p + ach),
+                                                                 W.tab.p, W.Y.p, g.np, o.dPF.p, o.dQF.p, o.ld, n,
+                                                                 W.part.p);
     ::gg::note_launch();
   }
-  if (!hf.empty()) {
-    k_pot_final<<<dim3((n + 31) / 32, (unsigned)hf.size()), 32 * PF_ROWS, 0, s>>>(dfin.p, dpart.p, n, o.dNAK.p, o.dMF.p, g.dR.p,
-                                                                       g.dRPOR.p, g.dZZ.p, o.dPF.p, o.dQF.p, o.ld,
-                                                                       g.q);
+  if (!jobs.empty()) {
+    k_pot_final<<<dim3((n + 31) / 32, (unsigned)jobs.size()), 32 * PF_ROWS, 0, s>>>(
+        reinterpret_cast<const PotFinal *>(W.up.p + afin), W.part.p, n, o.dNAK.p, o.dMF.p, g.dR.p, g.dRPOR.p,
+        g.dZZ.p, o.dPF.p, o.dQF.p, o.ld, g.q);
     ::gg::note_launch();
   }
   GG_CUDA(cudaGetLastError());
-  GG_CUDA(cudaStreamSynchronize(s));  // the uploads and scratch are freed on return
+  int *hinfo = reinterpret_cast<int *>(stage + ares);
+  double *hres = reinterpret_cast<double *>(stage + ares + 16);
+  GG_CUDA(cudaMemcpyAsync(hinfo, W.info.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  const size_t nres = (size_t)3 * n * jobs.size();
+  if (out) GG_CUDA(cudaMemcpyAsync(hres, W.pot.p, nres * sizeof(double), cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaStreamSynchronize(s));
+  const bool bad = hinfo[1] != 0;
+  if (out && !bad) std::memcpy(out, hres, nres * sizeof(double));
+  auto bytes = [](const DBuf<double> &b) { return b.n * sizeof(double); };
+  if (bytes(W.Y) + bytes(W.scratch) + bytes(W.part) + bytes(W.coef) * 2 + W.up.n > POT_KEEP) {
+    W.Y.release();
+    W.scratch.release();
+    W.part.release();
+    W.coef.release();
+    W.term.release();
+    W.up.release();
+  }
+  if (bad) return fail(GG_ERR_ARG, "potential: label outside the orbital set or K above 20");
   return GG_OK;
 }
 
@@ -1988,14 +2033,14 @@ static int potential(gg_ctx *ctx, int mode, int ncof, const int32_t *lab, const 
   GG_CUDA(cudaSetDevice(ctx->device));
   std::vector<PotJob> jobs(1);
   GG_TRY(raw_list(ncof, lab, co, mode == 0 ? jobs[0].y : jobs[0].x));
-  DBuf<double> pot;
-  GG_TRY(run_potentials(ctx, jobs, pot));
   const int n = ctx->grid.n;
+  std::vector<double> h((size_t)3 * n);
+  GG_TRY(run_potentials(ctx, jobs, h.data()));
   if (mode == 0) {
-    GG_CUDA(cudaMemcpy(out0, pot.p, n * sizeof(double), cudaMemcpyDeviceToHost));
+    std::copy(h.begin(), h.begin() + n, out0);
   } else {
-    GG_CUDA(cudaMemcpy(out0, pot.p + n, n * sizeof(double), cudaMemcpyDeviceToHost));
-    GG_CUDA(cudaMemcpy(out1, pot.p + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost));
+    std::copy(h.begin() + n, h.begin() + 2 * n, out0);
+    std::copy(h.begin() + 2 * n, h.end(), out1);
   }
   return GG_OK;
 }
@@ -2055,11 +2100,9 @@ int gg_cofpot(gg_ctx *ctx, int j, double ucfj, const gg_cof *cof, int nec, const
       jobs[0].lag_wa.push_back(wa);
     }
   }
-  DBuf<double> pot;
-  GG_TRY(run_potentials(ctx, jobs, pot));
   const int n = ctx->grid.n;
   std::vector<double> h((size_t)3 * n);  // one read-back of YP, XP, XQ
-  GG_CUDA(cudaMemcpy(h.data(), pot.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost));
+  GG_TRY(run_potentials(ctx, jobs, h.data()));
   std::copy(h.begin(), h.begin() + n, yp);
   std::copy(h.begin() + n, h.begin() + 2 * n, xp);
   std::copy(h.begin() + 2 * n, h.end(), xq);
@@ -2113,8 +2156,8 @@ int gg_setlag(gg_ctx *ctx, int nec, const int32_t *iecc, const double *ucf, cons
   }
   std::vector<PotJob> jobs(orbs.size());
   for (size_t i = 0; i < orbs.size(); ++i) GG_TRY(cof_job(ctx, &cof[orbs[i] - 1], jobs[i]));
-  DBuf<double> pot;
-  GG_TRY(run_potentials(ctx, jobs, pot));
+  GG_TRY(run_potentials(ctx, jobs));
+  const DBuf<double> &pot = std::static_pointer_cast<PotWork>(ctx->pot_work)->pot;
   cudaStream_t s = ctx->stream;
   DBuf<int4> dpj;
   DBuf<int2> dps;
@@ -2230,10 +2273,10 @@ extern "C" int gg_slater_noalloc(gg_ctx *ctx, int ia, int ib, int ic, int id, in
   GG_CUDA(cudaMemcpyAsync(dyd, &y, sizeof(YDesc), cudaMemcpyHostToDevice, ctx->stream));
   GG_CUDA(cudaMemcpyAsync(ditem, &it, sizeof(QuadItem), cudaMemcpyHostToDevice, ctx->stream));
   dim3 grid1((np + 127) / 128, 1);
-  k_ytemp<<<grid1, 128, 0, ctx->stream>>>(dyd, 1, o.dPF.p, o.dQF.p, o.ld, g.dRP.p, g.dPow.p, np, TZ, TW);
+  k_ytemp<<<grid1, 128, 0, ctx->stream>>>(dyd, 1, nullptr, o.dPF.p, o.dQF.p, o.ld, g.dRP.p, g.dPow.p, np, TZ, TW);
   ::gg::note_launch();
   GG_CUDA(cudaMemsetAsync(Y, 0, (size_t)np * sizeof(double), ctx->stream));
-  k_ychain<<<1, 128, 0, ctx->stream>>>(dyd, 1, TZ, TW, g.dR.p, g.dPow.p, np, g.q, Y);
+  k_ychain<<<1, 128, 0, ctx->stream>>>(dyd, 1, nullptr, TZ, TW, g.dR.p, g.dPow.p, np, g.q, Y);
   ::gg::note_launch();
   k_quad_items<<<1, 32, np * sizeof(double), ctx->stream>>>(ditem, nullptr, 1, Y, np, o.dPF.p, o.dQF.p, o.ld, g.dR.p,
                                                             g.dRP.p, g.dRPOR.p, g.q, dout);
