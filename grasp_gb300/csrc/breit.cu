@@ -1332,8 +1332,7 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   }
   if (ni > INT32_MAX || nj > INT32_MAX) return fail(GG_ERR_RANGE, "gg_genintbreit: table too large");
   T.n = ni;
-  T.hInd.resize(ni);
-  T.hVal.resize(ni);
+  T.hInd.clear();
   const int R = (int)rows.size();
   if (ni == 0) return GG_OK;
   // the contraction takes orbitals that reach past the chains' start and end
@@ -1346,12 +1345,11 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   const size_t plane = plain ? (size_t)(maxm + 1) * R : 0;
   const int j0 = 5 + 4 * ((m0 - 9) / 4);
   DBuf<BrRow> drows;
-  DBuf<double> drho, darr, dBJ, dBN, dG, dval;
+  DBuf<double> drho, darr, dBJ, dBN, dG;
   DBuf<BessDesc> dbd;
   DBuf<unsigned char> dheads;
   DBuf<int> drank, dnredo;
   DBuf<long long> dg0;
-  DBuf<int32_t> dind;
   GG_TRY(upload_vec(drows, rows, s));
   GG_TRY(upload_vec(drank, rank, s));
   GG_TRY(upload_vec(dg0, g0, s));
@@ -1363,8 +1361,8 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   GG_TRY(dBN.alloc((size_t)std::max(1, nb) * np));
   GG_TRY(dheads.alloc((size_t)3 * R));
   GG_TRY(dG.alloc(plain ? (size_t)gsz * nset : 0));
-  GG_TRY(dind.alloc(ni));
-  GG_TRY(dval.alloc(ni));
+  GG_TRY(T.dInd.alloc(ni));
+  GG_TRY(T.dVal.alloc(ni));
   GG_TRY(dnredo.alloc(1));
   BrArr A{};
   {
@@ -1502,13 +1500,12 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   }
   DBuf<BrRedo> dredo;
   GG_TRY(dredo.alloc(ni));
-  k_br_table<<<R, 128, 0, s>>>(drows.p, drank.p, plain ? dG.p : nullptr, dG.p + (nset == 2 ? gsz : 0), dg0.p, KEY, dind.p, dval.p,
-                               dredo.p, dnredo.p);
+  k_br_table<<<R, 128, 0, s>>>(drows.p, drank.p, plain ? dG.p : nullptr, dG.p + (nset == 2 ? gsz : 0), dg0.p, KEY, T.dInd.p,
+                               T.dVal.p, dredo.p, dnredo.p);
   ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
   int nredo = 0;
   GG_CUDA(cudaMemcpyAsync(&nredo, dnredo.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  GG_CUDA(cudaMemcpyAsync(T.hInd.data(), dind.p, ni * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   *plan_ms = 1e3 * std::chrono::duration<double>(std::chrono::steady_clock::now() - th0).count();
   GG_CUDA(cudaStreamSynchronize(s));
   if (nredo > 0) {
@@ -1524,13 +1521,12 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
     ::gg::note_launch();
     k_breit_combine<<<(nredo + 255) / 256, 256, 0, s>>>(dints.p, nredo, dv.p, dout.p);
     ::gg::note_launch();
-    k_br_redo_store<<<(nredo + 255) / 256, 256, 0, s>>>(dredo.p, nredo, dout.p, dval.p);
+    k_br_redo_store<<<(nredo + 255) / 256, 256, 0, s>>>(dredo.p, nredo, dout.p, T.dVal.p);
     ::gg::note_launch();
     GG_CUDA(cudaGetLastError());
   }
   ctx->stats[34] = nredo;
   GG_CUDA(cudaEventRecord(e1, s));
-  GG_CUDA(cudaMemcpyAsync(T.hVal.data(), dval.p, ni * sizeof(double), cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaStreamSynchronize(s));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, e0, e1);
@@ -1613,8 +1609,12 @@ int gg_get_breit_table(gg_ctx *ctx, int type, int32_t *indtp, double *valtp, int
   if (!ctx || (type != 1 && type != 2)) return fail(GG_ERR_ARG, "gg_get_breit_table: type 1 or 2");
   const BreitTable &T = ctx->breit[type - 1];
   if (!T.valid) return fail(GG_ERR_STATE, "gg_get_breit_table: no table of this type (call gg_genintbreit)");
-  if (indtp) std::copy(T.hInd.begin(), T.hInd.end(), indtp);
-  if (valtp) std::copy(T.hVal.begin(), T.hVal.end(), valtp);
+  // straight into the caller's arrays (a host copy of the table in between
+  // cost a quarter of the 34-subshell table's time)
+  GG_CUDA(cudaSetDevice(ctx->device));
+  if (indtp && T.n) GG_CUDA(cudaMemcpyAsync(indtp, T.dInd.p, T.n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+  if (valtp && T.n) GG_CUDA(cudaMemcpyAsync(valtp, T.dVal.p, T.n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  GG_CUDA(cudaStreamSynchronize(ctx->stream));
   if (kstart) std::copy(T.kstart.begin(), T.kstart.end(), kstart);
   return GG_OK;
 }
@@ -1622,11 +1622,20 @@ int gg_get_breit_table(gg_ctx *ctx, int type, int32_t *indtp, double *valtp, int
 // BRINT1 / BRINT2 (rci90/brint1.f90:30-66): binary search in the k range
 int gg_brint(gg_ctx *ctx, int type, int ia, int ib, int ic, int id, int k, double *tegral) {
   if (!ctx || (type != 1 && type != 2) || !tegral) return fail(GG_ERR_ARG, "gg_brint: bad arguments");
-  const BreitTable &T = ctx->breit[type - 1];
+  BreitTable &T = ctx->breit[type - 1];
   if (!T.valid) return fail(GG_ERR_STATE, "gg_brint: no table of this type (call gg_genintbreit)");
   const int nw = ctx->orb.nw, KEY = nw + 1;
   if (k < 0 || k > T.j2max || ia < 1 || ib < 1 || ic < 1 || id < 1 || ia > nw || ib > nw || ic > nw || id > nw)
     return fail(GG_ERR_NOTFOUND, "gg_brint: integral not in the table");
+  GG_CUDA(cudaSetDevice(ctx->device));
+  if (T.hInd.empty() && T.n) {
+    std::vector<int32_t> ind(T.n);
+    T.hVal.resize(T.n);
+    GG_CUDA(cudaMemcpyAsync(ind.data(), T.dInd.p, T.n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    GG_CUDA(cudaMemcpyAsync(T.hVal.data(), T.dVal.p, T.n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    GG_CUDA(cudaStreamSynchronize(ctx->stream));
+    T.hInd.swap(ind);
+  }
   const int32_t index = ((ia * KEY + ib) * KEY + ic) * KEY + id;
   const int32_t *b = T.hInd.data() + (T.kstart[k] - 1), *e = T.hInd.data() + (T.kstart[k + 1] - 1);
   const int32_t *p = std::lower_bound(b, e, index);

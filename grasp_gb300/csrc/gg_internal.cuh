@@ -145,8 +145,10 @@ struct BreitTable {
   int j2max = 0;
   int64_t n = 0;
   std::vector<int32_t> kstart;          // KSTARTBREIT(0:j2max+1), 1-based positions
-  std::vector<int32_t> hInd;            // INDTP
-  std::vector<double> hVal;             // VALTP
+  DBuf<int32_t> dInd;                   // INDTP
+  DBuf<double> dVal;                    // VALTP
+  std::vector<int32_t> hInd;            // both on the host, from the first gg_brint on the table
+  std::vector<double> hVal;
 };
 
 struct RkCache;  // radial.cu: GENINTRK's orbital-set structure, reused between calls
