@@ -165,7 +165,7 @@ class Context:
     def setcof(self, j, ucfj):
         """SETCOF(EOL, J)'s lists (gg_setcof) from the prepared sums: a dict
         nya/ya, nxa/xa, nda/da (gg_cofpot's and cofpot's input)."""
-        cap = 1024
+        cap = getattr(self, "_setcof_cap", 1024)
         while True:
             ny, nx, nd = C.c_int(), C.c_int(), C.c_int()
             nya = np.zeros(cap, np.int32); ya = np.zeros(cap); nxa = np.zeros(cap, np.int32); xa = np.zeros(cap)
@@ -174,7 +174,7 @@ class Context:
                                       C.byref(nx), ptr(nxa, _i32), ptr(xa, _d), C.byref(nd), ptr(nda, _i32),
                                       ptr(da, _d))
             if st == _lib_status("GG_ERR_RANGE"):
-                cap = max(ny.value, nx.value, nd.value)
+                cap = self._setcof_cap = max(ny.value, nx.value, nd.value)
                 continue
             check(st)
             return dict(nya=nya[:ny.value].copy(), ya=ya[:ny.value].copy(), nxa=nxa[:nx.value].copy(),

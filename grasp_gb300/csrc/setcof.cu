@@ -10,37 +10,63 @@
 // through the final 1/UCF(J), so here one pass computes them for every label
 // of every block, together with the diagonal FCO/GCO sums of every pair of
 // orbitals. DSUBRS depends on the position only, so it is formed once per EMT
-// position (k_dsubrs_pos) and a contribution costs one FMA. A call for
-// orbital J then only filters and merges the labels on the host, in the
-// reference's order (FCO, GCO, the T list by block, the V^k lists by k and
-// block), so its lists are the reference's entry for entry.
+// position (k_dsubrs_pos) and a contribution costs one FMA. The same pass
+// decodes every label once on the host and leaves each orbital's lists up to
+// the division by UCF(J), in the reference's order (FCO, GCO, the T list by
+// block, the V^k lists by k and block), so they are the reference's entry for
+// entry and a call for orbital J only divides. (Decoding the labels per
+// orbital took 3.4 of a 3.85 ms SETCOF over 34 subshells.)
 #include <algorithm>
 #include <cstring>
 #include <memory>
-#include <tuple>
-#include <utility>
+#include <unordered_map>
 #include <vector>
 
 #include "gg_internal.cuh"
 
 namespace gg {
 
-// the prepared sums of the last gg_setcof_prepare
+// One list of one orbital: its labels, and the values added to them in order,
+// each before the division by UCF(J). A value's entry is `at`; the first value
+// of an entry sets it (the labels of a later block that repeat one join it).
+struct SetcofList {
+  struct Add {
+    int at;
+    double v;
+  };
+  std::vector<int32_t> lab;
+  std::vector<Add> add;
+  std::unordered_map<int32_t, int> first;  // first entry of each label, filled when merging
+  size_t merged = 0;                       // labels entered into `first` so far
+  void put(int32_t l, double v, bool merge) {
+    if (merge) {
+      for (; merged < lab.size(); ++merged) first.emplace(lab[merged], (int)merged);
+      const auto f = first.find(l);
+      if (f != first.end()) {
+        add.push_back(Add{f->second, v});
+        return;
+      }
+    }
+    add.push_back(Add{(int)lab.size(), v});
+    lab.push_back(l);
+  }
+  void write(double ucf, int32_t *label, double *val) const {
+    std::copy(lab.begin(), lab.end(), label);
+    int n = 0;
+    for (const Add &a : add) {
+      const double v = a.v / ucf;
+      if (a.at == n)
+        val[n++] = v;
+      else
+        val[a.at] = val[a.at] + v;
+    }
+  }
+};
+
+// the lists of the last gg_setcof_prepare, [orbital] YPOT, XPOT, DACON
 struct SetcofState {
-  int nblocks = 0, eol = 0;
-  int kmaxf = -1;                             // largest over the blocks
-  std::vector<int> bkmaxf;                    // per block
-  std::vector<std::vector<int64_t>> lab0;     // per block: first label of each list (T, V0..)
-  std::vector<std::vector<int32_t>> labs;     // per block: the labels of all its lists
-  std::vector<std::vector<double>> sums;      // per block: each label's sum of DSUBRS COEFF (x2 off the diagonal)
-  std::vector<double> fco, gco;               // [J][IB][K] diagonal sums (index below)
-  int kdim = 0;
-  size_t idx(int j, int ib, int k) const { return ((size_t)(j - 1) * nw + (ib - 1)) * kdim + k; }
   int nw = 0;
-  // per orbital, the labels that name it: T labels as (block, label), V
-  // labels as (k, block, label), each in the order SETCOF visits them
-  std::vector<std::vector<std::pair<int, int64_t>>> tref;
-  std::vector<std::vector<std::tuple<int, int, int64_t>>> vref;
+  std::vector<SetcofList> y, x, d;
 };
 
 namespace {
@@ -182,20 +208,6 @@ template <class T> int upv(DBuf<T> &b, const std::vector<T> &h, cudaStream_t s) 
   return GG_OK;
 }
 
-// appends (label, value) or, when merge and the label is already listed,
-// adds to its value (the reference's "check it against the previously
-// recorded" search: the first entry with that label)
-void put(std::vector<int32_t> &lab, std::vector<double> &val, int32_t l, double v, bool merge) {
-  if (merge)
-    for (size_t i = 0; i < lab.size(); ++i)
-      if (lab[i] == l) {
-        val[i] = val[i] + v;
-        return;
-      }
-  lab.push_back(l);
-  val.push_back(v);
-}
-
 }  // namespace
 }  // namespace gg
 
@@ -213,9 +225,9 @@ int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *ne
   const int nw = o.nw;
   cudaStream_t s = ctx->stream;
   auto st = std::make_shared<SetcofState>();
-  st->nblocks = nblocks;
-  st->eol = eol ? 1 : 0;
   st->nw = nw;
+  std::vector<std::vector<int32_t>> labs;  // per block: the labels of all its lists
+  std::vector<std::vector<double>> sums;   // per block: each label's sum of DSUBRS COEFF (x2 off the diagonal)
   std::vector<DBuf<double>> devec(nblocks), dwt(nblocks), ddiag(nblocks);
   std::vector<DiagBlock> hb(nblocks);
   for (int b = 0; b < nblocks; ++b) {
@@ -246,7 +258,7 @@ int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *ne
     DBuf<double> dpos, dsum;
     GG_TRY(dpos.alloc(std::max<int64_t>(1, m->nnz)));
     GG_TRY(ddiag[b].alloc(ncf));
-    k_dsubrs_pos<<<(ncf + LS_WARPS - 1) / LS_WARPS, LS_WARPS * 32, 0, s>>>(m->dIendc.p, m->dIrow.p, ncf, st->eol, ne,
+    k_dsubrs_pos<<<(ncf + LS_WARPS - 1) / LS_WARPS, LS_WARPS * 32, 0, s>>>(m->dIendc.p, m->dIrow.p, ncf, eol ? 1 : 0, ne,
                                                                           devec[b].p, dwt[b].p, dpos.p, ddiag[b].p);
     ::gg::note_launch();
     GG_TRY(dsum.alloc(std::max<int64_t>(1, L.nlab)));
@@ -255,22 +267,16 @@ int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *ne
       ::gg::note_launch();
     }
     GG_CUDA(cudaGetLastError());
-    st->labs.emplace_back(L.nlab);
-    st->sums.emplace_back(L.nlab);
+    labs.emplace_back(L.nlab);
+    sums.emplace_back(L.nlab);
     if (L.nlab > 0) {
-      GG_CUDA(cudaMemcpyAsync(st->labs.back().data(), L.dLab.p, L.nlab * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-      GG_CUDA(cudaMemcpyAsync(st->sums.back().data(), dsum.p, L.nlab * sizeof(double), cudaMemcpyDeviceToHost, s));
+      GG_CUDA(cudaMemcpyAsync(labs.back().data(), L.dLab.p, L.nlab * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+      GG_CUDA(cudaMemcpyAsync(sums.back().data(), dsum.p, L.nlab * sizeof(double), cudaMemcpyDeviceToHost, s));
     }
     GG_CUDA(cudaStreamSynchronize(s));  // dpos and dsum are freed here
-    st->lab0.push_back(L.list_lab0);
-    st->bkmaxf.push_back(L.kmaxf);
-    st->kmaxf = std::max(st->kmaxf, L.kmaxf);
     hb[b] = DiagBlock{ncf, ddiag[b].p, L.dIq.p, L.dConf.p};
   }
-  // the diagonal sums of every (J, IB, K) SETCOF asks for, from the pairs' sums
-  int jmax = 0;
-  for (int a = 1; a <= nw; ++a) jmax = std::max(jmax, o.nkj[a]);
-  st->kdim = jmax + 2;
+  // the diagonal sums, by orbital pair
   std::vector<int> full(nw);
   for (int a = 0; a < nw; ++a) full[a] = o.nkj[a + 1] + 1;
   DBuf<int> dfull;
@@ -285,50 +291,93 @@ int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *ne
   std::vector<double> hv((size_t)2 * nw * nw);
   GG_CUDA(cudaMemcpyAsync(hv.data(), dout.p, hv.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaStreamSynchronize(s));
-  st->fco.assign((size_t)nw * nw * st->kdim, 0.0);
-  st->gco.assign((size_t)nw * nw * st->kdim, 0.0);
+  st->y.resize(nw + 1);
+  st->x.resize(nw + 1);
+  st->d.resize(nw + 1);
+  const int KEY = KEYORB;
   for (int j = 1; j <= nw; ++j)
     for (int ib = 1; ib <= nw; ++ib) {
       const double *v = &hv[2 * ((size_t)(std::min(j, ib) - 1) * nw + (std::max(j, ib) - 1))];
-      st->fco[st->idx(j, ib, 0)] = v[0];
+      // Y from FCO (setcof.f90:73-105): NYA = K + IB KEY (KEY + 1)
+      const int64_t ly = (int64_t)ib * KEY * (KEY + 1);
       if (ib == j) {
+        st->y[j].put((int32_t)ly, 2.0 * v[0], false);
         for (int k = 2; k <= o.nkj[j] - 1; k += 2) {
           const double c = clrx_host(o.nak[j], k, o.nak[j]);
-          st->fco[st->idx(j, ib, k)] = -0.5 * c * c * v[1];
+          st->y[j].put((int32_t)(k + ly), -(c * c * v[1]), false);
         }
         continue;
       }
+      st->y[j].put((int32_t)ly, v[0], false);
+      // X from GCO (:107-147): NXA = K + KEY J + IB KEY^2 (KEY + 1)
+      const int64_t lx = (int64_t)KEY * j + (int64_t)ib * KEY * KEY * (KEY + 1);
       const int kmin = (o.nak[j] * o.nak[ib] > 0) ? std::abs((o.nkj[j] - o.nkj[ib]) / 2)
                                                    : std::abs((o.nkj[j] - o.nkj[ib]) / 2) + 1;
       for (int k = kmin; k <= (o.nkj[j] + o.nkj[ib]) / 2; k += 2) {
         const double c = clrx_host(o.nak[j], k, o.nak[ib]);
-        st->gco[st->idx(j, ib, k)] = -(c * c * v[1]);
+        st->x[j].put((int32_t)(k + lx), -(c * c * v[1]), false);
       }
     }
-  // the labels of each orbital, in visiting order
-  st->tref.assign(nw + 1, {});
-  st->vref.assign(nw + 1, {});
-  for (int b = 0; b < nblocks; ++b)
-    for (int64_t l = st->lab0[b][0]; l < st->lab0[b][1]; ++l) {
-      const int32_t lab = st->labs[b][l];
-      const int ia = lab % KEYORB, ib = lab / KEYORB;
-      if (ia >= 1 && ia <= nw) st->tref[ia].push_back({b, l});
-      if (ib != ia && ib >= 1 && ib <= nw) st->tref[ib].push_back({b, l});
+  // DA from the T lists, block by block (:188-285)
+  int kmaxf = -1;
+  for (int b = 0; b < nblocks; ++b) {
+    const Lists &L = *h[b]->lists;
+    kmaxf = std::max(kmaxf, L.kmaxf);
+    for (int64_t l = L.list_lab0[0]; l < L.list_lab0[1]; ++l) {
+      const int32_t lab = labs[b][l];
+      const int ia = lab % KEY, ib = lab / KEY;
+      const double v = 0.5 * sums[b][l];
+      if (ia >= 1 && ia <= nw) st->d[ia].put(ib, v, b > 0);
+      if (ib != ia && ib >= 1 && ib <= nw) st->d[ib].put(ia, v, b > 0);
     }
-  for (int k = 0; k <= st->kmaxf; ++k)
+  }
+  // the V^k lists, k by k and block by block (:287-515): INDEXS = (a, b, c, d)
+  // of R^k(ab;cd), each orbital named in it
+  for (int k = 0; k <= kmaxf; ++k)
     for (int b = 0; b < nblocks; ++b) {
-      if (k > st->bkmaxf[b]) continue;
-      for (int64_t l = st->lab0[b][k + 1]; l < st->lab0[b][k + 2]; ++l) {
-        int32_t lab = st->labs[b][l];
+      const Lists &L = *h[b]->lists;
+      if (k > L.kmaxf) continue;
+      const bool merge = b > 0;
+      for (int64_t l = L.list_lab0[k + 1]; l < L.list_lab0[k + 2]; ++l) {
+        if (labs[b][l] < 0) continue;
+        uint32_t lab = (uint32_t)labs[b][l];  // unsigned: the divisions by KEY are multiplications
         int ix[4];
-        for (int t = 0; t < 4; ++t) {
-          ix[t] = lab % KEYORB;
-          lab /= KEYORB;
-        }
-        for (int t = 0; t < 4; ++t) {
+        ix[3] = lab % KEYORB;
+        lab /= KEYORB;
+        ix[1] = lab % KEYORB;
+        lab /= KEYORB;
+        ix[2] = lab % KEYORB;
+        ix[0] = lab / KEYORB;
+        const double v = 0.5 * sums[b][l];
+        for (int f = 0; f < 4; ++f) {
+          const int j = ix[f];
+          if (j < 1 || j > nw) continue;
+          int irank = 0, second = f, other = j;
           bool seen = false;
-          for (int u = 0; u < t; ++u) seen = seen || ix[u] == ix[t];
-          if (!seen && ix[t] >= 1 && ix[t] <= nw) st->vref[ix[t]].push_back(std::make_tuple(k, b, l));
+          for (int u = 0; u < 4; ++u) {
+            if (ix[u] != j) {
+              other = ix[u];
+              continue;
+            }
+            seen = seen || u < f;
+            if (++irank == 2) second = u;
+          }
+          if (seen) continue;  // done at its first place
+          const int o1 = ix[(f + 1) & 3], o2 = ix[(f + 2) & 3], o3 = ix[(f + 3) & 3];
+          const int32_t lx = ((o2 * KEY + o3) * KEY + o1) * KEY + k;
+          if (irank == 1) {
+            st->x[j].put(lx, v, merge);
+          } else if (irank == 2) {
+            if (second - f == 2)
+              st->y[j].put((o3 * KEY + o1) * KEY + k, v + v, merge);
+            else
+              st->x[j].put(lx, v + v, merge);
+          } else if (irank == 3) {
+            st->y[j].put((other * KEY + j) * KEY + k, v + v, merge);
+            st->x[j].put(((other * KEY + j) * KEY + j) * KEY + k, v, merge);
+          } else {
+            st->y[j].put((j * KEY + j) * KEY + k, 4.0 * v, merge);
+          }
         }
       }
     }
@@ -342,122 +391,16 @@ int gg_setcof(gg_ctx *ctx, int j, double ucfj, int cap, int *ny, int32_t *nya, d
     return fail(GG_ERR_ARG, "gg_setcof: bad arguments");
   const auto st = std::static_pointer_cast<SetcofState>(ctx->setcof);
   if (!st) return fail(GG_ERR_STATE, "gg_setcof: call gg_setcof_prepare first");
-  const Orbitals &o = ctx->orb;
-  const int nw = st->nw, KEY = KEYORB;
-  if (j < 1 || j > nw || o.nw != nw) return fail(GG_ERR_ARG, "gg_setcof: orbital outside the orbital set");
-  std::vector<int32_t> ly, lx, ld;
-  std::vector<double> vy, vx, vd;
-  // Y from FCO (setcof.f90:73-105): NYA = K + IB KEY (KEY + 1)
-  {
-    int64_t ilabel = 0;
-    const int64_t nwterm = (int64_t)KEY * (KEY + 1);
-    for (int ib = 1; ib <= nw; ++ib) {
-      ilabel += nwterm;
-      const int kmax = (ib == j) ? o.nkj[j] - 1 : 0;
-      for (int k = 0; k <= kmax; k += 2) {
-        const double sumr = st->fco[st->idx(j, ib, k)];
-        const double ykab = (ib == j) ? 2.0 * sumr / ucfj : sumr / ucfj;
-        ly.push_back((int32_t)(k + ilabel));
-        vy.push_back(ykab);
-      }
-    }
-  }
-  // X from GCO (:107-147): NXA = K + KEY J + IB KEY^2 (KEY + 1)
-  {
-    int64_t ilabel = (int64_t)KEY * j;
-    const int64_t nwterm = (int64_t)KEY * KEY * (KEY + 1);
-    for (int ib = 1; ib <= nw; ++ib) {
-      ilabel += nwterm;
-      if (ib == j) continue;
-      const int kmin = (o.nak[j] * o.nak[ib] > 0) ? std::abs((o.nkj[j] - o.nkj[ib]) / 2)
-                                                   : std::abs((o.nkj[j] - o.nkj[ib]) / 2) + 1;
-      for (int k = kmin; k <= (o.nkj[j] + o.nkj[ib]) / 2; k += 2) {
-        lx.push_back((int32_t)(k + ilabel));
-        vx.push_back(st->gco[st->idx(j, ib, k)] / ucfj);
-      }
-    }
-  }
-  // DA from the T lists, block by block (:188-285)
-  for (const auto &r : st->tref[j]) {
-    const int b = r.first;
-    const int64_t l = r.second;
-    const int32_t lab = st->labs[b][l];
-    const int ia = lab % KEY, ibb = lab / KEY;
-    const double sum = 0.5 * st->sums[b][l] / ucfj;
-    put(ld, vd, ia == j ? ibb : ia, sum, b > 0);
-  }
-  // the V^k lists, k by k and block by block (:287-515)
-  for (const auto &r : st->vref[j]) {
-      const int k = std::get<0>(r), b = std::get<1>(r);
-      const bool merge = b > 0;
-      {
-        const int64_t l = std::get<2>(r);
-        int32_t lab = st->labs[b][l];
-        int ix[4];
-        ix[3] = lab % KEY;
-        lab /= KEY;
-        ix[1] = lab % KEY;
-        lab /= KEY;
-        ix[2] = lab % KEY;
-        ix[0] = lab / KEY;
-        int irank = 0;
-        for (int t = 0; t < 4; ++t) irank += (ix[t] == j);
-        if (irank == 0) continue;
-        const double sum = 0.5 * st->sums[b][l] / ucfj;
-        auto at = [&](int p) { return ix[(p - 1) % 4]; };  // INDEXS(IL), IL wrapped into 1..4
-        if (irank == 1) {
-          int ithis = 0;
-          for (int iind = 1; iind <= 4; ++iind) {
-            if (ix[iind - 1] != j) continue;
-            ithis = ((at(iind + 2) * KEY + at(iind + 3)) * KEY + at(iind + 1)) * KEY + k;
-            break;
-          }
-          put(lx, vx, ithis, sum, merge);
-        } else if (irank == 2) {
-          int loc1 = 0, loc2 = 0, found = 0;
-          for (int iind = 1; iind <= 4; ++iind) {
-            if (ix[iind - 1] != j) continue;
-            if (found == 0) {
-              loc1 = iind;
-              found = 1;
-            } else {
-              loc2 = iind;
-              break;
-            }
-          }
-          if (loc2 - loc1 == 2) {
-            const int ithis = (at(loc1 + 3) * KEY + at(loc1 + 1)) * KEY + k;
-            put(ly, vy, ithis, sum + sum, merge);
-          } else {
-            const int ithis = ((at(loc1 + 2) * KEY + at(loc1 + 3)) * KEY + at(loc1 + 1)) * KEY + k;
-            put(lx, vx, ithis, sum + sum, merge);
-          }
-        } else if (irank == 3) {
-          int ithis = 0, ithis2 = 0;
-          for (int iind = 1; iind <= 4; ++iind) {
-            if (ix[iind - 1] == j) continue;
-            const int other = ix[iind - 1];
-            ithis = (other * KEY + j) * KEY + k;
-            ithis2 = ((other * KEY + j) * KEY + j) * KEY + k;
-          }
-          put(ly, vy, ithis, sum + sum, merge);
-          put(lx, vx, ithis2, sum, merge);
-        } else {
-          put(ly, vy, (j * KEY + j) * KEY + k, 4.0 * sum, merge);
-        }
-      }
-    }
-  *ny = (int)ly.size();
-  *nx = (int)lx.size();
-  *nd = (int)ld.size();
-  if ((int)ly.size() > cap || (int)lx.size() > cap || (int)ld.size() > cap)
+  if (j < 1 || j > st->nw || ctx->orb.nw != st->nw) return fail(GG_ERR_ARG, "gg_setcof: orbital outside the orbital set");
+  const SetcofList &ly = st->y[j], &lx = st->x[j], &ld = st->d[j];
+  *ny = (int)ly.lab.size();
+  *nx = (int)lx.lab.size();
+  *nd = (int)ld.lab.size();
+  if (*ny > cap || *nx > cap || *nd > cap)
     return fail(GG_ERR_RANGE, "gg_setcof: a list is longer than cap (the counts are set)");
-  std::copy(ly.begin(), ly.end(), nya);
-  std::copy(vy.begin(), vy.end(), ya);
-  std::copy(lx.begin(), lx.end(), nxa);
-  std::copy(vx.begin(), vx.end(), xa);
-  std::copy(ld.begin(), ld.end(), nda);
-  std::copy(vd.begin(), vd.end(), da);
+  ly.write(ucfj, nya, ya);
+  lx.write(ucfj, nxa, xa);
+  ld.write(ucfj, nda, da);
   return GG_OK;
 }
 
