@@ -325,7 +325,7 @@ __device__ __forceinline__ void rk_head_store(int a, int c, int p, int f, long l
 // gives every SM four warps (fewer rows per warp read Y more often, more leave
 // SMs idle). A block of 32 x 64 entries in shared memory left most rows of a
 // tile empty (a (k, a) problem has 2 to 12 pairs) and most SMs idle: 371 us
-// for 16 subshells, now 52 us; the chains are the same, so are the bits.
+// for 16 subshells, now 22 us; the chains are the same, so are the bits.
 // ---------------------------------------------------------------------------
 struct TcRow {  // one row of a k: its pair, problem and position data
   int p, a, c, ic, ncA, cs_a;
@@ -352,22 +352,44 @@ __global__ void __launch_bounds__(128) k_rk_dot(const RkTile *__restrict__ tiles
   double acc[NR];
 #pragma unroll
   for (int r = 0; r < NR; ++r) acc[r] = 0.0;
-  // points 2 .. m in groups of four; A is zero from m + 1 on (the row's end,
-  // then points 0 and 1 of the next row)
-#pragma unroll 2
-  for (int i = 2; i <= m; i += 4) {
-    const double2 y0 = __ldg(reinterpret_cast<const double2 *>(y + i));
-    const double2 y1 = __ldg(reinterpret_cast<const double2 *>(y + i + 2));
+  // points 2 .. m in groups of G, the next group loaded before the current one
+  // is added (a chain of loads and FMAs waits on L2 at every group otherwise).
+  // A(m + 1) is zero (the row's end or point 0 of the next row); the last
+  // group's loads reach up to G - 1 points past m, its sums stop at m
+  constexpr int G = NR >= 8 ? 4 : NR == 4 ? 8 : 16;
+  double2 cy[G / 2], ca[NR][G / 2];
+  auto load = [&](int i, double2 *yv, double2(*av)[G / 2]) {
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      const double2 a0 = __ldg(reinterpret_cast<const double2 *>(ar[r] + i));
-      const double2 a1 = __ldg(reinterpret_cast<const double2 *>(ar[r] + i + 2));
-      acc[r] = fma(a0.x, y0.x, acc[r]);
-      acc[r] = fma(a0.y, y0.y, acc[r]);
-      acc[r] = fma(a1.x, y1.x, acc[r]);
-      acc[r] = fma(a1.y, y1.y, acc[r]);
+    for (int u = 0; u < G / 2; ++u) {
+      yv[u] = __ldg(reinterpret_cast<const double2 *>(y + i) + u);
+#pragma unroll
+      for (int r = 0; r < NR; ++r) av[r][u] = __ldg(reinterpret_cast<const double2 *>(ar[r] + i) + u);
+    }
+  };
+  auto add = [&](const double2 *yv, const double2(*av)[G / 2], int left) {
+#pragma unroll
+    for (int u = 0; u < G / 2; ++u)
+      if (2 * u < left)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          acc[r] = fma(av[r][u].x, yv[u].x, acc[r]);
+          acc[r] = fma(av[r][u].y, yv[u].y, acc[r]);
+        }
+  };
+  load(2, cy, ca);
+  int i = 2;
+  for (; i + G <= m; i += G) {
+    double2 ny[G / 2], na[NR][G / 2];
+    load(i + G, ny, na);
+    add(cy, ca, G);
+#pragma unroll
+    for (int u = 0; u < G / 2; ++u) {
+      cy[u] = ny[u];
+#pragma unroll
+      for (int r = 0; r < NR; ++r) ca[r][u] = na[r][u];
     }
   }
+  add(cy, ca, m + 1 - i);
   if (lane >= T.fn) return;
   const YDesc yd = t.yd[f];
 #pragma unroll
@@ -1278,14 +1300,13 @@ __device__ __forceinline__ double ychain_run(double acc, const double *__restric
     }
   return acc;
 }
-// the chains' additions (Z: 16 points loaded ahead, W: 8); writes Z into Y,
-// W into W, each chain's K = 0 correction DIF and the function's asymptotic
-// value ZKLIM
+// the chains' additions (Z: 16 points loaded ahead, W: 8): blockIdx.y = 0
+// writes Z into Y, each chain's K = 0 correction DIF and the function's
+// asymptotic value ZKLIM, blockIdx.y = 1 writes W into W
 __global__ void k_ychain_sum(const YDesc *__restrict__ yd, int nf, const int *__restrict__ nfp,
-                             const double *__restrict__ TZ,
-                             const double *__restrict__ RZ, const double *__restrict__ RW, int np, QuadConst q,
-                             double *__restrict__ Y, double *__restrict__ W, double *__restrict__ dif_out,
-                             double *__restrict__ zk_out) {
+                             const double *__restrict__ TZ, const double *__restrict__ RZ,
+                             const double *__restrict__ RW, int np, QuadConst q, double *__restrict__ Y,
+                             double *__restrict__ W, double *__restrict__ dif_out, double *__restrict__ zk_out) {
   nf = nfuncs(nf, nfp);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int f = t >> 2, c = t & 3;
@@ -1293,9 +1314,17 @@ __global__ void k_ychain_sum(const YDesc *__restrict__ yd, int nf, const int *__
   const YDesc y = active ? yd[f] : yd[0];
   const int K = y.k, MTP = y.mtp, MTPP3 = MTP + 3, N = q.n;
   const size_t base = (size_t)(active ? f : 0) * np;
-  const double *T = TZ + base, *Rz = RZ + base, *Rw = RW + 3 * base;
-  double *Yf = Y + base, *Wf = W + base;
   const int s = c + 2;  // chain start: 2, 3, 4, 5
+  if (blockIdx.y == 1) {
+    // W from the top of this chain's points with i <= min(N, MTP) down to s
+    const int lim = min(N, MTP);
+    if (!active || lim < s) return;
+    const int cnt = (lim - s) / 4 + 1;  // the points s + 4 (cnt - 1), ..., s + 4, s
+    ychain_run<3, 8>(0.0, RW + 3 * base, W + base, s + 4 * (cnt - 1), -4, cnt);
+    return;
+  }
+  const double *T = TZ + base, *Rz = RZ + base;
+  double *Yf = Y + base;
   double z = 0.0;
   if (active) {
     if (s <= 4) {
@@ -1323,11 +1352,6 @@ __global__ void k_ychain_sum(const YDesc *__restrict__ yd, int nf, const int *__
   }
   dif_out[(size_t)f * 4 + c] = dif;
   if (c == 0) zk_out[f] = zklim;
-  // W from the top of this chain's points with i <= min(N, MTP) down to s
-  const int lim = min(N, MTP);
-  if (lim < s) return;
-  const int cnt = (lim - s) / 4 + 1;  // the points s + 4 (cnt - 1), ..., s + 4, s
-  ychain_run<3, 8>(0.0, Rw, Wf, s + 4 * (cnt - 1), -4, cnt);
 }
 
 __global__ void k_yassemble(const YDesc *__restrict__ yd, int nf, const int *__restrict__ nfp,
@@ -1398,7 +1422,7 @@ int build_y(gg_ctx *ctx, const YDesc *d_yd, int nf, double *dY, DBuf<double> &sc
     double *zk = dif + 4 * nf;
     k_yincr<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, nfp, TZ, TW, np, g.q, RZ, RW);
     // W goes where TW was: k_yincr was its last reader
-    k_ychain_sum<<<(nthr + 127) / 128, 128, 0, ctx->stream>>>(d_yd, nf, nfp, TZ, RZ, RW, np, g.q, dY, TW, dif, zk);
+    k_ychain_sum<<<dim3((nthr + 63) / 64, 2), 64, 0, ctx->stream>>>(d_yd, nf, nfp, TZ, RZ, RW, np, g.q, dY, TW, dif, zk);
     k_yassemble<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, nfp, g.dR.p, g.dPow.p, np, g.q, dif, zk, TW, dY);
     ::gg::note_launch();
     ::gg::note_launch();
@@ -1714,27 +1738,26 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
     ::gg::note_launch();
     GG_CUDA(cudaGetLastError());
   }
+  if (!tiles.empty()) {
+    // the items' number stays on the device: the blocks take it from there
+    const int wpb = 16;  // warps per block: an item each, their head terms by warp 0
+    const int blocks = (int)std::min<int64_t>((N + wpb - 1) / wpb, 4LL * ctx->sms);
+    k_quad_table<<<std::max(1, blocks), 32 * wpb, 0, ctx->stream>>>(C.dFb.p, C.dNfb.p, (int)N, tabs, g.q, rk.dVal.p);
+    ::gg::note_launch();
+    GG_CUDA(cudaGetLastError());
+  }
   int hfb[3] = {0, 0, 0};
   GG_CUDA(cudaMemcpyAsync(hfb, C.dNfb.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  GG_CUDA(cudaStreamSynchronize(ctx->stream));
+  double ms = 0;
+  GG_TRY(timer_stop(ctx, &ms));  // waits for all of it
+  ctx->stats[0] = ms;
   if (hfb[1]) return fail(GG_ERR_STATE, "genintrk: contraction produced a table position out of range");
   if (hfb[2] == 1)
     return fail(GG_ERR_TIMEOUT, "genintrk: a tensor-core tile timed out waiting for its copies or MMAs (drained; "
                                 "the table is not valid)");
   if (hfb[2] > 1)
     return fail(GG_ERR_TIMEOUT, "genintrk: a tensor-core tile timed out and its copies or MMAs did not drain");
-  const int nfb = hfb[0];
-  ctx->stats[20] = nfb;
-  if (nfb > 0) {
-    const int wpb = 16;  // warps per block: an item each, their head terms by warp 0
-    const int blocks = std::min((nfb + wpb - 1) / wpb, 4 * ctx->sms);
-    k_quad_table<<<blocks, 32 * wpb, 0, ctx->stream>>>(C.dFb.p, C.dNfb.p, nfb, tabs, g.q, rk.dVal.p);
-    ::gg::note_launch();
-    GG_CUDA(cudaGetLastError());
-  }
-  double ms = 0;
-  GG_TRY(timer_stop(ctx, &ms));
-  ctx->stats[0] = ms;
+  ctx->stats[20] = hfb[0];
   rk.valid = true;
   if (n_out) *n_out = N;
   if (j2max_out) *j2max_out = j2max;
