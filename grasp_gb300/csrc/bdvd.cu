@@ -11,8 +11,9 @@
 //   eig      one CTA per block: the k x k projected matrix S (k <= LIM) is
 //            reduced to tridiagonal form by Householder reflections in shared
 //            memory; its lowest eigenvalues by Sturm bisection and Newton
-//            steps; eigenvectors by inverse iteration (re-orthogonalised
-//            inside clusters), back-transformed by the reflectors
+//            steps; eigenvectors from twisted factorisations (inside
+//            clusters: inverse iteration, re-orthogonalised),
+//            back-transformed by the reflectors
 //   ritz     Ritz vectors X = V y, residuals R = W y - theta X, |R| per tile
 //   conv     per block: residual test (|r_j| <= CRITR), the targets that get a
 //            new vector, restart decision (basis full: collapse to REST Ritz
@@ -118,119 +119,229 @@ struct EigShape {
   int lmax, nvmax;
   __host__ __device__ int lda() const { return lmax | 1; }
   __host__ __device__ size_t bytes() const {
-    // A, seven vectors, Z, scalars, FP32 copies of d and e^2
-    return sizeof(double) * ((size_t)lmax * lda() + 7 * (size_t)lmax + (size_t)lmax * nvmax + 8) +
-           sizeof(float) * 2 * (size_t)lmax;
+    // A, seven vectors, the warps' partial products, Z, scalars, FP32 copies
+    // of d and e^2, the triangle's index pairs
+    return sizeof(double) * ((size_t)lmax * lda() + (7 + EIG_T / 32) * (size_t)lmax + (size_t)lmax * nvmax + 8) +
+           sizeof(float) * 2 * (size_t)lmax + sizeof(uchar2) * ((size_t)lmax * (lmax + 1) / 2);
   }
 };
 
+// 1/q and 1/sqrt(q) from an FP32 estimate and one third-order Newton step
+// (error 2^-22 cubed: a few ulps from rounding). The projected eigensolver is
+// a chain of dependent FP64 operations, and a division or square root is a
+// long subroutine of them. Arguments outside FP32's range take the exact
+// operation.
+__device__ __forceinline__ double rcp_nr(double q) {
+  const int t = (__double2hiint(q) >> 20) & 0x7ff;  // 2^-100 <= |q| < 2^101
+  if (t < 923 || t > 1123) return 1.0 / q;
+  const double y = (double)__fdividef(1.0f, (float)q);
+  const double e = fma(-q, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt_nr(double q) {
+  const int t = __double2hiint(q) >> 20;
+  if (t < 923 || t > 1123) return 1.0 / sqrt(q);
+  const double y = (double)rsqrtf((float)q);
+  const double e = fma(-q * y, y, 1.0);
+  return fma(y, e * fma(e, 0.375, 0.5), y);
+}
+
+// Eigenvector of the tridiagonal T for an isolated eigenvalue x, by one warp,
+// from the twisted factorisation of T - xI (Parlett & Dhillon, Linear Algebra
+// Appl. 267 (1997) 247): lane 0 forms the pivots from the top down (into z),
+// lane 1 those from the bottom up (into w) with the same instructions; the
+// vector solves (T - xI) z = gamma_r e_r with the smallest |gamma_r|, growing
+// from row r both ways. A row costs five FP64 instructions of the one warp,
+// where the pivoted factorisation and its two solves cost some twenty (m = 33:
+// 93,000 cycles -> 32,000). d, e2 and x are in units of a power of two above |T|
+// (e times sc is too); a pivot below 2^-90 is set to that.
+__device__ void twist_vec(int n, const double *d, const double *e, const double *e2, double sc, double x, double *z,
+                          double *w, int lane) {
+  auto mag = [](double v) { return __double_as_longlong(v) & 0x7fffffffffffffffll; };
+  if (lane < 2) {
+    double *q = lane ? w : z;
+    const int s = lane ? -1 : 1, se = lane ? 0 : -1;
+    double r = 0.0;
+    for (int k = 0, i = lane ? n - 1 : 0; k < n; ++k, i += s) {
+      double p = d[i] - x;
+      if (k) p = fma(-e2[i + se], r, p);
+      if ((__double2hiint(p) & 0x7fffffff) < (933 << 20)) p = __hiloint2double(933 << 20, 0);
+      q[i] = p;
+      r = rcp_nr(p);
+    }
+  }
+  __syncwarp();
+  long long best = 0x7fffffffffffffffll;  // min |gamma|
+  int row = 0;
+  for (int i = lane; i < n; i += 32) {
+    const long long g = mag(z[i] + (w[i] - (d[i] - x)));
+    if (g < best) {
+      best = g;
+      row = i;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const long long g = __shfl_xor_sync(0xffffffffu, best, o);
+    const int i = __shfl_xor_sync(0xffffffffu, row, o);
+    if (g < best || (g == best && i < row)) {
+      best = g;
+      row = i;
+    }
+  }
+  // z[i] = w[i] z[i +- 1], from row outwards
+  for (int i = lane; i < n; i += 32)
+    if (i != row) w[i] = -(e[i < row ? i : i - 1] * sc) * rcp_nr(i < row ? z[i] : w[i]);
+  __syncwarp();
+  if (lane < 2) {
+    const int s = lane ? 1 : -1, len = lane ? n - 1 - row : row;
+    double v = 1.0;
+    z[row] = 1.0;
+    for (int k = 1; k <= len; ++k) {
+      v *= w[row + s * k];
+      z[row + s * k] = v;
+    }
+  }
+  __syncwarp();
+  double nrm = 0.0;
+  for (int i = lane; i < n; i += 32) nrm = fma(z[i], z[i], nrm);
+  nrm = rsqrt_nr(warp_sum(nrm));
+  for (int i = lane; i < n; i += 32) z[i] *= nrm;
+  __syncwarp();
+}
+
 // LU of the tridiagonal T - lam I with partial pivoting, and inverse
 // iteration from a fixed pseudo-random start (Golub & Van Loan, 4th ed.,
-// sec. 8.2.2); x is re-orthogonalised against ncl earlier vectors of the same
-// cluster (columns cl[] of Z) at every step. The pivots are inverted once, so
-// the solves multiply instead of divide (GB300 issues FP64 slowly; a division
-// is a sequence of FP64 instructions).
+// sec. 8.2.2), for the vectors of a cluster; x is re-orthogonalised against
+// ncl earlier vectors of it (the columns c0.. of Z) at every step. One warp:
+// lane 0 runs the factorisation (one reciprocal per pivot serves the
+// elimination and both solves) and the solves, all lanes the sums and updates.
 __device__ void inv_iter_dev(int n, const double *d, const double *e, double lam, double tnorm, double *x,
-                             const double *Z, int ldz, const int *cl, int ncl, unsigned seed) {
+                             const double *Z, int ldz, int c0, int ncl, unsigned seed, int lane) {
   if (n == 1) {
-    x[0] = 1.0;
+    if (lane == 0) x[0] = 1.0;
+    __syncwarp();
     return;
   }
-  double l[MAXL], ru0[MAXL], u1[MAXL], u2[MAXL];
+  double l[MAXL], ru0[MAXL], u1[MAXL], u2[MAXL];  // lane 0's
   unsigned char piv[MAXL];
-  const double tiny = 2.220446049250313e-16 * fmax(tnorm, 1e-300);
-  double a0 = d[0] - lam, a1 = e[0];
-  for (int i = 0; i < n; ++i) {
-    double sub = 0, b0 = 0, b1 = 0;
-    if (i + 1 < n) {
-      sub = e[i];
-      b0 = d[i + 1] - lam;
-      b1 = (i + 2 < n) ? e[i + 1] : 0.0;
-    }
-    double u0;
-    if (i + 1 < n && fabs(sub) > fabs(a0)) {
-      piv[i] = 1;
-      const double m = a0 / sub;
+  if (lane == 0) {
+    const double tiny = 2.220446049250313e-16 * fmax(tnorm, 1e-300);
+    double a0 = d[0] - lam, a1 = e[0];
+    for (int i = 0; i < n; ++i) {
+      double sub = 0, b0 = 0, b1 = 0;
+      if (i + 1 < n) {
+        sub = e[i];
+        b0 = d[i + 1] - lam;
+        b1 = (i + 2 < n) ? e[i + 1] : 0.0;
+      }
+      // magnitudes compared as integers, off the FP64 pipe (|sub| above
+      // 2^-960: its reciprocal is finite)
+      const long long ms = __double_as_longlong(sub) & 0x7fffffffffffffffll;
+      const bool p = i + 1 < n && ms > (__double_as_longlong(a0) & 0x7fffffffffffffffll) && ms > (63ll << 52);
+      double u0 = p ? sub : a0;
+      if (!p && fabs(u0) < tiny) u0 = u0 < 0 ? -tiny : tiny;
+      const double r = rcp_nr(u0), m = (p ? a0 : sub) * r;
+      piv[i] = p;
       l[i] = m;
-      u0 = sub;
-      u1[i] = b0;
-      u2[i] = b1;
-      const double n0 = a1 - m * b0, n1 = -m * b1;
-      a0 = n0;
-      a1 = n1;
-    } else {
-      piv[i] = 0;
-      if (a0 == 0.0) a0 = tiny;
-      u0 = a0;
-      const double m = (i + 1 < n) ? sub / a0 : 0.0;
-      l[i] = m;
-      u1[i] = a1;
-      u2[i] = 0.0;
-      a0 = b0 - m * a1;
-      a1 = b1;
+      ru0[i] = (p && fabs(u0) < tiny) ? (u0 < 0 ? -1.0 / tiny : 1.0 / tiny) : r;
+      if (p) {
+        u1[i] = b0;
+        u2[i] = b1;
+        a0 = fma(-m, b0, a1);
+        a1 = -m * b1;
+      } else {
+        u1[i] = a1;
+        u2[i] = 0.0;
+        a0 = fma(-m, a1, b0);
+        a1 = b1;
+      }
     }
-    if (fabs(u0) < tiny) u0 = u0 < 0 ? -tiny : tiny;
-    ru0[i] = 1.0 / u0;
-  }
-  unsigned s = 2463534242u ^ (seed * 2654435761u);
-  for (int i = 0; i < n; ++i) {
-    s ^= s << 13;
-    s ^= s >> 17;
-    s ^= s << 5;
-    x[i] = (double)(s & 0xffff) / 65536.0 - 0.5 + 1e-3;
+    unsigned s = 2463534242u ^ (seed * 2654435761u);
+    for (int i = 0; i < n; ++i) {
+      s ^= s << 13;
+      s ^= s >> 17;
+      s ^= s << 5;
+      x[i] = (double)((float)(s & 0xffff) * (1.0f / 65536.0f) - 0.499f);
+    }
   }
   for (int it = 0; it < 2; ++it) {
-    for (int i = 0; i + 1 < n; ++i) {
-      if (piv[i]) {
-        const double t = x[i];
-        x[i] = x[i + 1];
-        x[i + 1] = t;
+    if (lane == 0) {
+      double c = x[0];  // x[i] as the rows above left it
+      for (int i = 0; i + 1 < n; ++i) {
+        const double nx = x[i + 1];
+        const double top = piv[i] ? nx : c, bot = piv[i] ? c : nx;
+        x[i] = top;
+        c = fma(-l[i], top, bot);
       }
-      x[i + 1] -= l[i] * x[i];
+      x[n - 1] = c;
+      double x1 = 0.0, x2 = 0.0;  // x[i + 1], x[i + 2]
+      for (int i = n - 1; i >= 0; --i) {
+        double v = x[i];
+        if (i + 2 < n) v = fma(-u2[i], x2, v);
+        if (i + 1 < n) v = fma(-u1[i], x1, v);
+        v = v * ru0[i];
+        x[i] = v;
+        x2 = x1;
+        x1 = v;
+      }
     }
-    for (int i = n - 1; i >= 0; --i) {
-      double v = x[i];
-      if (i + 1 < n) v -= u1[i] * x[i + 1];
-      if (i + 2 < n) v -= u2[i] * x[i + 2];
-      x[i] = v * ru0[i];
-    }
-    for (int c = 0; c < ncl; ++c) {
-      const double *q = Z + (size_t)cl[c] * ldz;
-      double dot = 0.0;
-      for (int i = 0; i < n; ++i) dot += q[i] * x[i];
-      for (int i = 0; i < n; ++i) x[i] -= dot * q[i];
+    __syncwarp();
+    for (int q = 0; q < ncl; ++q) {
+      const double *z = Z + (size_t)(c0 + q) * ldz;
+      double t = 0.0;
+      for (int i = lane; i < n; i += 32) t = fma(z[i], x[i], t);
+      t = warp_sum(t);
+      for (int i = lane; i < n; i += 32) x[i] = fma(-t, z[i], x[i]);
     }
     double nrm = 0.0;
-    for (int i = 0; i < n; ++i) nrm += x[i] * x[i];
-    nrm = sqrt(nrm);
-    if (nrm == 0.0) nrm = 1.0;
-    const double inv = 1.0 / nrm;
-    for (int i = 0; i < n; ++i) x[i] *= inv;
+    for (int i = lane; i < n; i += 32) nrm = fma(x[i], x[i], nrm);
+    nrm = warp_sum(nrm);
+    // a solve with a pivot at rounding level grows by up to 1 / (eps |T|)
+    const double inv = nrm > 0.0 ? rsqrt_nr(nrm) : 1.0;
+    for (int i = lane; i < n; i += 32) x[i] *= inv;
+    __syncwarp();
   }
 }
 
-// Sturm count of T - xI (number of eigenvalues below x) and, for Newton's
-// method, f'/f of det(T - xI) (Wilkinson, The Algebraic Eigenvalue Problem,
-// ch. 5, sec. 37-38: the LDL^T pivots q_i count the eigenvalues below x and
-// f'/f = sum q_i'/q_i).
-__device__ __forceinline__ int sturm64(int m, const double *dd, const double *e2, double x, double pivmin,
-                                       double *fpf) {
-  double q = dd[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  double inv = 1.0 / q, Sd = -inv, qp = -1.0;
-  int cnt = (q < 0.0);
-  for (int i = 1; i < m; ++i) {
-    const double ei2 = e2[i - 1];
-    double qi = fma(-ei2, inv, dd[i] - x);
-    qi = (fabs(qi) < pivmin) ? -pivmin : qi;
-    const double dq = fma(ei2 * qp, inv * inv, -1.0);
-    const double iv = 1.0 / qi;
-    cnt += (qi < 0.0);
-    Sd = fma(dq, iv, Sd);
-    qp = dq;
-    inv = iv;
+// Sturm count of T - xI (number of eigenvalues below x) and Newton's step
+// -f/f' on f = det(T - xI), from the leading principal minors p_i = (d_i - x)
+// p_{i-1} - e_{i-1}^2 p_{i-2} and their derivatives (Givens' Sturm sequence;
+// Wilkinson, The Algebraic Eigenvalue Problem, ch. 5, sec. 36-38): the count
+// is the number of sign changes, a minor that vanishes counts as one. The
+// chain per row is one FMA, where the pivots p_i / p_{i-1} need a reciprocal
+// (all eigenvalues at m = 33: 147,000 -> 85,000 cycles). d, e2 and x are in units of a power of
+// two above |T|, so four rows change a minor by less than 2^400 either way
+// (a minor below 2^-100 of the one before is set to that); every fourth row
+// the minors are rescaled by their exponent.
+__device__ __forceinline__ int sturm64(int m, const double *dd, const double *e2, double x, double *step) {
+  auto top = [](double v) { return __double2hiint(v) & 0x7fffffff; };
+  int cnt = 0;
+  double p1 = 1.0, p = dd[0] - x, g1 = 0.0, g = -1.0;
+  auto check = [&] {
+    if (top(p) < top(p1) - (100 << 20)) p = p1 * -0x1p-100;
+    cnt += (unsigned)(__double2hiint(p) ^ __double2hiint(p1)) >> 31;
+  };
+  check();
+  for (int i = 1; i < m; i += 4) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (i + u >= m) break;
+      const double dx = dd[i + u] - x, e = e2[i + u - 1];
+      const double pn = fma(dx, p, -e * p1), gn = fma(dx, g, fma(-e, g1, -p));
+      p1 = p;
+      p = pn;
+      g1 = g;
+      g = gn;
+      check();
+    }
+    const double sc = __hiloint2double((2046 << 20) - (max(top(p), top(p1)) & 0x7ff00000), 0);
+    p *= sc;
+    p1 *= sc;
+    g *= sc;
+    g1 *= sc;
   }
-  *fpf = Sd;
+  *step = g != 0.0 ? -p / g : 0.0;
   return cnt;
 }
 
@@ -265,10 +376,12 @@ __global__ void __launch_bounds__(EIG_T) k_b_eig(const BDesc *__restrict__ desc,
   double *pp = vv + sh.lmax;                 // p, then w
   double *ev = pp + sh.lmax;                 // eigenvalues
   double *e2 = ev + sh.lmax;                 // e^2
-  double *Z = e2 + sh.lmax;                  // eigenvectors [nv][m]
+  double *red = e2 + sh.lmax;                // the warps' partial sums of p
+  double *Z = red + (size_t)(EIG_T / 32) * sh.lmax;  // eigenvectors [nv][m]
   double *scal = Z + (size_t)sh.lmax * sh.nvmax;  // scalars
   float *d32 = reinterpret_cast<float *>(scal + 8);  // FP32 copies of d and e^2
   float *e232 = d32 + sh.lmax;
+  uchar2 *tri = reinterpret_cast<uchar2 *>(e232 + sh.lmax);  // (row, column) of the lower triangle
   // the eigenvectors needed: r, or REST when the basis may be collapsed
   const bool may_restart = (m + r > L) && (m > D.rest);
   const int nv = min(m, may_restart ? max(D.rest, r) : r);
@@ -278,85 +391,89 @@ __global__ void __launch_bounds__(EIG_T) k_b_eig(const BDesc *__restrict__ desc,
     const int i = idx % m, j = idx / m;
     if (i >= j) A[(size_t)j * lda + i] = Sb[(size_t)j * L + i];
   }
+  // the lower triangle's entries, last column first, so that the trailing
+  // block of every step is a prefix of the list
+  for (int t = tid; t < m * (m + 1) / 2; t += EIG_T) {
+    int u = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while (u * (u + 1) / 2 > t) --u;
+    while ((u + 1) * (u + 2) / 2 <= t) ++u;
+    const int c = m - 1 - u;
+    tri[t] = make_uchar2((unsigned char)(c + t - u * (u + 1) / 2), (unsigned char)c);
+  }
   __syncthreads();
-  // Householder tridiagonalisation (Golub & Van Loan, Alg. 8.3.1). GB300
-  // spends the same FP64 issue slots on a warp instruction whatever its
-  // active lanes, so the steps are laid out to keep lanes busy: one thread
-  // per row for p = A22 v, and the rank-2 update over the packed lower
-  // triangle only.
+  // Householder tridiagonalisation (Golub & Van Loan, Alg. 8.3.1, reflectors
+  // v with v(0) = 1 and the sign of v0 that does not cancel, so that beta =
+  // 1 + |x0| / |x| needs no division). A step is a chain of dependent FP64
+  // operations: warp 0 forms the reflector, the warps share the columns of
+  // p = A22 v, warp 0 reduces it to w, and all threads update the packed
+  // lower triangle - four barriers. A warp's FP64 instruction occupies its
+  // sub-partition for 64 cycles, so what counts is how many warp 0 issues.
+  // (m = 33: seven barriers, a thread per row of p and divisions 320,000
+  // cycles in all, now 175,000.)
   for (int k = 0; k + 2 < m; ++k) {
-    const int o = k + 1, mm = m - k - 1;
-    double *xk = A + (size_t)k * lda + o;
+    const int o = k + 1;
     if (warp == 0) {
+      double *xk = A + (size_t)k * lda;  // x = xk[o..m)
       double sig = 0.0;
-      for (int i = 1 + lane; i < mm; i += 32) sig = fma(xk[i], xk[i], sig);
+      for (int i = o + 1 + lane; i < m; i += 32) sig = fma(xk[i], xk[i], sig);
       sig = warp_sum(sig);
+      const double x0 = xk[o];
+      __syncwarp();
+      double beta = 0.0, rv = 0.0, off = x0;
+      if (sig != 0.0) {
+        const double s2 = fma(x0, x0, sig), y = rsqrt_nr(s2), mu = s2 * y;
+        beta = fma(fabs(x0), y, 1.0);
+        off = x0 < 0.0 ? mu : -mu;
+        rv = rcp_nr(x0 - off);
+      }
+      for (int i = o + lane; i < m; i += 32) {
+        const double v = (i == o) ? 1.0 : xk[i] * rv;
+        vv[i] = v;
+        if (i > o) xk[i] = v;  // kept for the back-transformation
+      }
       if (lane == 0) {
-        const double x0 = xk[0];
-        dd[k] = A[(size_t)k * lda + k];
-        if (sig == 0.0) {
-          ee[k] = x0;
-          bt[k] = 0.0;
-          scal[0] = 1.0;
-        } else {
-          const double mu = sqrt(x0 * x0 + sig);
-          const double v0 = (x0 <= 0.0) ? x0 - mu : -sig / (x0 + mu);
-          ee[k] = mu;
-          bt[k] = 2.0 * v0 * v0 / (sig + v0 * v0);
-          scal[0] = 1.0 / v0;
-        }
+        dd[k] = xk[k];
+        ee[k] = off;
+        bt[k] = beta;
       }
     }
     __syncthreads();
     const double beta = bt[k];
-    if (beta == 0.0) continue;
-    const double rv0 = scal[0];
-    for (int i = tid; i < mm; i += EIG_T) {
-      const double v = (i == 0) ? 1.0 : xk[i] * rv0;
-      vv[i] = v;
-      if (i > 0) xk[i] = v;  // kept for the back-transformation
-    }
-    __syncthreads();
-    // p = beta A22 v, one thread per row
-    for (int i = tid; i < mm; i += EIG_T) {
-      const double *row = A + (size_t)o * lda + (o + i);  // A(o+i, o+j), j <= i, at row[j * lda]
-      const double *col = A + (size_t)(o + i) * lda + o;  // A(o+j, o+i), j >= i, at col[j]
+    if (beta == 0.0) continue;  // uniform; the next write of bt is behind no reader
+    for (int i = o + lane; i < m; i += 32) {
       double s0 = 0.0, s1 = 0.0;
-      int j = 0;
-      for (; j + 1 < i; j += 2) {
-        s0 = fma(row[(size_t)j * lda], vv[j], s0);
-        s1 = fma(row[(size_t)(j + 1) * lda], vv[j + 1], s1);
+      const double *ai = A + (size_t)i * lda;
+      int j = o + warp;
+      for (; j + EIG_T / 32 < m; j += 2 * (EIG_T / 32)) {
+        const int j2 = j + EIG_T / 32;
+        s0 = fma(j <= i ? A[(size_t)j * lda + i] : ai[j], vv[j], s0);
+        s1 = fma(j2 <= i ? A[(size_t)j2 * lda + i] : ai[j2], vv[j2], s1);
       }
-      for (; j < i; ++j) s0 = fma(row[(size_t)j * lda], vv[j], s0);
-      for (j = i; j + 1 < mm; j += 2) {
-        s0 = fma(col[j], vv[j], s0);
-        s1 = fma(col[j + 1], vv[j + 1], s1);
-      }
-      for (; j < mm; ++j) s0 = fma(col[j], vv[j], s0);
-      pp[i] = beta * (s0 + s1);
+      if (j < m) s0 = fma(j <= i ? A[(size_t)j * lda + i] : ai[j], vv[j], s0);
+      red[(size_t)warp * sh.lmax + i] = s0 + s1;
     }
     __syncthreads();
     if (warp == 0) {
       double pv = 0.0;
-      for (int i = lane; i < mm; i += 32) pv = fma(pp[i], vv[i], pv);
+      for (int i = o + lane; i < m; i += 32) {
+        const double *r0 = red + i;
+        const size_t L0 = sh.lmax;
+        const double p = beta * (((r0[0] + r0[L0]) + (r0[2 * L0] + r0[3 * L0])) +
+                                 ((r0[4 * L0] + r0[5 * L0]) + (r0[6 * L0] + r0[7 * L0])));
+        pp[i] = p;
+        pv = fma(p, vv[i], pv);
+      }
       pv = warp_sum(pv);
-      if (lane == 0) scal[1] = 0.5 * beta * pv;
+      const double half = 0.5 * beta * pv;
+      for (int i = o + lane; i < m; i += 32) pp[i] = fma(-half, vv[i], pp[i]);
     }
     __syncthreads();
-    {
-      const double half = scal[1];
-      for (int i = tid; i < mm; i += EIG_T) pp[i] = fma(-half, vv[i], pp[i]);
-    }
-    __syncthreads();
-    // A22 -= v w^T + w v^T on the lower triangle, packed index t -> (i >= j)
-    const int ntri = mm * (mm + 1) / 2;
+    // A22 -= v w^T + w v^T on the lower triangle
+    const int mm = m - o, ntri = mm * (mm + 1) / 2;
     for (int t = tid; t < ntri; t += EIG_T) {
-      int i = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-      while (i * (i + 1) / 2 > t) --i;
-      while ((i + 1) * (i + 2) / 2 <= t) ++i;
-      const int j = t - i * (i + 1) / 2;
-      double &a = A[(size_t)(o + j) * lda + (o + i)];
-      a = fma(-vv[i], pp[j], fma(-pp[i], vv[j], a));
+      const uchar2 rc = tri[t];
+      double &a = A[(size_t)rc.y * lda + rc.x];
+      a = fma(-vv[rc.x], pp[rc.y], fma(-pp[rc.x], vv[rc.y], a));
     }
     __syncthreads();
   }
@@ -368,61 +485,71 @@ __global__ void __launch_bounds__(EIG_T) k_b_eig(const BDesc *__restrict__ desc,
     dd[m - 1] = A[(size_t)(m - 1) * lda + (m - 1)];
   }
   __syncthreads();
-  if (warp == 0) {  // norms and Gershgorin bounds; FP32 copies for the coarse search
-    double tn = 0.0, em = 0.0, glo = 1e308, ghi = -1e308;
+  if (warp == 0) {  // norm, Gershgorin bounds; T in units of a power of two above its norm, and an FP32 copy
+    double tn = 0.0, glo = 1e308, ghi = -1e308;
     for (int i = lane; i < m; i += 32) {
       const double el = (i > 0) ? fabs(ee[i - 1]) : 0.0, er = (i + 1 < m) ? fabs(ee[i]) : 0.0;
       glo = fmin(glo, dd[i] - el - er);
       ghi = fmax(ghi, dd[i] + el + er);
       tn = fmax(tn, fabs(dd[i]) + el + er);
-      if (i + 1 < m) {
-        e2[i] = ee[i] * ee[i];
-        em = fmax(em, e2[i]);
-        e232[i] = (float)e2[i];
-      }
-      d32[i] = (float)dd[i];
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       tn = fmax(tn, __shfl_xor_sync(0xffffffffu, tn, o));
-      em = fmax(em, __shfl_xor_sync(0xffffffffu, em, o));
       glo = fmin(glo, __shfl_xor_sync(0xffffffffu, glo, o));
       ghi = fmax(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
     }
+    const int be = __double2hiint(tn) >> 20;  // |T| = f 2^(be - 1023), 1 <= f < 2
+    const bool ok = be > 0 && be < 2045;
+    const double sc = ok ? __hiloint2double((2045 - be) << 20, 0) : 1.0;
+    for (int i = lane; i < m; i += 32) {
+      const double ei = i + 1 < m ? ee[i] * sc : 0.0;
+      pp[i] = dd[i] * sc;
+      e2[i] = ei * ei;
+      d32[i] = (float)pp[i];
+      e232[i] = (float)e2[i];
+    }
     if (lane == 0) {
       scal[2] = tn;
-      scal[3] = em;
-      scal[4] = glo;
-      scal[5] = ghi;
+      scal[3] = ok ? __hiloint2double((be + 1) << 20, 0) : 1.0;  // the unit, 1 / sc
+      scal[4] = glo * sc;
+      scal[5] = ghi * sc;
+      scal[6] = sc;
     }
   }
   __syncthreads();
-  // lowest ne eigenvalues, one lane per target (warps take 32 targets each).
-  // 1. FP32 bisection on Sturm counts of the FP32 copy of T, inside the
-  //    bracket from Cauchy interlacing: the leading mprev x mprev block of S
-  //    is the matrix of the previous pass (or, after a restart, diag(theta)),
-  //    whose eigenvalues are in theta, so with k = m - mprev new columns
-  //    theta_old[j - k] <= lambda_j <= theta_old[j].
+  // lowest ne eigenvalues: a warp per target while the warps suffice (a round
+  // of 32 points divides its interval by 33), else eight lanes (m = 33, four
+  // targets: 203,000 cycles with pivots by division and eight lanes, now 64,000).
+  // 1. FP32 multisection (a point per lane) on Sturm counts of the FP32
+  //    copy of T, inside the bracket from Cauchy interlacing: the leading
+  //    mprev x mprev block of S is the matrix of the previous pass (or, after
+  //    a restart, diag(theta)), whose eigenvalues are in theta, so with
+  //    k = m - mprev new columns theta_old[j - k] <= lambda_j <= theta_old[j].
   // 2. FP64: the bracket lambda32 +- delta (delta covers the FP32 copy's
-  //    perturbation) is checked by two FP64 counts, then bisection until
-  //    isolated and safeguarded Newton steps on det(T - xI).
+  //    perturbation) is checked by two FP64 counts while a third lane takes
+  //    the first Newton step from lambda32; then bisection until isolated and
+  //    safeguarded Newton steps on det(T - xI).
   {
     const double eps = 2.220446049250313e-16;
-    const double tnorm = scal[2];
-    const double pivmin = 2.2250738585072014e-308 * fmax(1.0, scal[3]) / eps;
+    const double sc = scal[6], tnorm = scal[2] * sc, *ds = pp;
+    const double pivmin = 1e-290;
     const double pad = 2.0 * eps * m * fmax(tnorm, 1e-300) + 2.0 * pivmin;
     const double atol = 4.0 * eps * fmax(tnorm, 1e-300);
     const double gl = scal[4] - pad, gu = scal[5] + pad;
     const int kadd = (S.mprev > 0 && m >= S.mprev) ? m - S.mprev : m;
     const int neold = (S.mprev > 0 && m >= S.mprev) ? S.neold : 0;
     const float eps32 = 5.9604645e-08f;
-    const float piv32 = 1e-30f * fmaxf(1.0f, (float)scal[3]);
-    for (int j = tid; j < ne; j += EIG_T) {
+    const float piv32 = 1e-30f;
+    const int G = ne <= EIG_T / 32 ? 32 : 8;  // lanes per target
+    const int g = lane & (G - 1), base = lane & (32 - G);
+    const unsigned gm = (G == 32 ? 0xffffffffu : 0xffu) << base;  // those of this one
+    for (int j = tid / G; j < ne; j += EIG_T / G) {
       // 1. coarse FP32 search
       double blo = gl, bhi = gu;
       {
-        const double bl = (j - kadd >= 0 && j - kadd < neold) ? S.theta[j - kadd] - 8.0 * pad : gl;
-        const double bh = (j < neold) ? S.theta[j] + 8.0 * pad : gu;
+        const double bl = (j - kadd >= 0 && j - kadd < neold) ? S.theta[j - kadd] * sc - 8.0 * pad : gl;
+        const double bh = (j < neold) ? S.theta[j] * sc + 8.0 * pad : gu;
         if (fmax(gl, bl) < fmin(gu, bh)) {
           blo = fmax(gl, bl);
           bhi = fmin(gu, bh);
@@ -430,45 +557,53 @@ __global__ void __launch_bounds__(EIG_T) k_b_eig(const BDesc *__restrict__ desc,
       }
       const float tol32 = 8.0f * eps32 * fmaxf((float)tnorm, 1e-30f);
       float lo = (float)blo, hi = (float)bhi;
-      if (sturm32(m, d32, e232, lo, piv32) > j) lo = (float)gl;  // hint did not hold
-      if (sturm32(m, d32, e232, hi, piv32) <= j) hi = (float)gu;
-      for (int it = 0; it < 80 && hi - lo > tol32; ++it) {
-        const float x = 0.5f * (lo + hi);
-        if (sturm32(m, d32, e232, x, piv32) <= j) lo = x;
-        else hi = x;
+      {
+        const int c = sturm32(m, d32, e232, g == 0 ? lo : hi, piv32);
+        if (__shfl_sync(gm, c, base) > j) lo = (float)gl;  // hint did not hold
+        if (__shfl_sync(gm, c, base + 1) <= j) hi = (float)gu;
+      }
+      for (int it = 0; it < 40 && hi - lo > tol32; ++it) {
+        const float h = (hi - lo) / (float)(G + 1);
+        const int c = sturm32(m, d32, e232, fmaf(h, (float)(g + 1), lo), piv32);
+        const int below = __popc(__ballot_sync(gm, c <= j));  // points at or below lambda_j
+        if (below < G) hi = fmaf(h, (float)(below + 1), lo);
+        if (below > 0) lo = fmaf(h, (float)below, lo);
       }
       // 2. FP64 refinement in lambda32 +- delta: verify both ends (a failed
       // end is replaced by the Gershgorin bound), then bisect until lambda_j
       // is isolated and take safeguarded Newton steps
       const double l32 = 0.5 * ((double)lo + (double)hi);
       const double delta = 64.0 * (double)eps32 * m * fmax(tnorm, 1e-300);
-      double dlo = fmax(gl, l32 - delta), dhi = fmin(gu, l32 + delta), fpf;
+      double dlo = fmax(gl, l32 - delta), dhi = fmin(gu, l32 + delta), step;
       int clo = 0, chi = m;
-      if (dlo > gl) {
-        const int c = sturm64(m, dd, e2, dlo, pivmin, &fpf);
-        if (c <= j) {
-          clo = c;
-        } else {  // lambda_j < dlo
-          dhi = dlo;
-          chi = c;
-          dlo = gl;
-        }
-      }
-      if (dhi < gu && chi == m) {
-        const int c = sturm64(m, dd, e2, dhi, pivmin, &fpf);
-        if (c > j) {
-          chi = c;
-        } else {  // lambda_j >= dhi
-          dlo = dhi;
-          clo = c;
-          dhi = gu;
+      int cnt = sturm64(m, ds, e2, g == 0 ? dlo : g == 1 ? dhi : l32, &step);
+      const int c0 = __shfl_sync(gm, cnt, base), c1 = __shfl_sync(gm, cnt, base + 1);
+      cnt = __shfl_sync(gm, cnt, base + 2);
+      step = __shfl_sync(gm, step, base + 2);
+      if (dlo > gl && c0 > j) {  // lambda_j < dlo
+        dhi = dlo;
+        chi = c0;
+        dlo = gl;
+      } else {
+        if (dlo > gl) clo = c0;
+        if (dhi < gu) {
+          if (c1 > j) {
+            chi = c1;
+          } else {  // lambda_j >= dhi
+            dlo = dhi;
+            clo = c1;
+            dhi = gu;
+          }
         }
       }
       bool newton = clo == j && chi == j + 1;  // already isolated: Newton from the FP32 estimate
-      double xj = (l32 > dlo && l32 < dhi) ? l32 : 0.5 * (dlo + dhi), w = 0.5 * (dlo + dhi);
+      bool have = l32 > dlo && l32 < dhi;      // the count and the step at l32 are known
+      double xj = have ? l32 : 0.5 * (dlo + dhi), w = 0.5 * (dlo + dhi);
+      double last = 0.0;  // the Newton step before, 0 if there was none
       for (int it = 0; it < 200; ++it) {
-        const double x = newton ? xj : 0.5 * (dlo + dhi);
-        const int cnt = sturm64(m, dd, e2, x, pivmin, &fpf);
+        const double x = newton || have ? xj : 0.5 * (dlo + dhi);
+        if (!have) cnt = sturm64(m, ds, e2, x, &step);
+        have = false;
         if (cnt <= j) {
           dlo = x;
           clo = cnt;
@@ -481,19 +616,19 @@ __global__ void __launch_bounds__(EIG_T) k_b_eig(const BDesc *__restrict__ desc,
           newton = true;  // isolated: Newton from the FP32 estimate
           xj = (l32 > dlo && l32 < dhi) ? l32 : 0.5 * (dlo + dhi);
         } else if (!done && newton) {
-          const double step = (fpf != 0.0) ? -1.0 / fpf : 0.0;
-          const double xn = x + step;
-          if (fabs(step) <= 2.0 * eps * fabs(x) + pivmin) {
-            done = true;
-            xj = (xn > dlo && xn < dhi) ? xn : x;
-          } else {
-            xj = (xn > dlo && xn < dhi) ? xn : 0.5 * (dlo + dhi);
-          }
+          // steps that shrink by a factor f shrink by f^2 next (quadratic
+          // convergence): the one after this is known to be below rounding
+          const double xn = x + step, as = fabs(step);
+          const bool in = xn > dlo && xn < dhi;
+          const float f = (float)as / (float)last;
+          done = as * (double)fminf(f * f, 1.0f) <= 2.0 * eps * fabs(x) + pivmin;
+          last = in ? as : 0.0;
+          xj = in ? xn : done ? x : 0.5 * (dlo + dhi);
         }
         w = newton ? xj : 0.5 * (dlo + dhi);
         if (done) break;
       }
-      ev[j] = w;
+      if (g == 0) ev[j] = w * scal[3];
     }
   }
   __syncthreads();
@@ -501,48 +636,61 @@ __global__ void __launch_bounds__(EIG_T) k_b_eig(const BDesc *__restrict__ desc,
     for (int j = 1; j < ne; ++j) ev[j] = fmax(ev[j], ev[j - 1]);
   __syncthreads();
   // eigenvectors of T: clusters (consecutive eigenvalues closer than
-  // 1e-3 |T|) are done by one thread in order, each vector orthogonalised
-  // against the earlier ones of its cluster
+  // 1e-3 |T|) go to the warps in turn; the vectors of one are done in order,
+  // each orthogonalised against the earlier ones
   {
     const double eps = 2.220446049250313e-16;
     const double tnorm = scal[2], ortol = 1e-3 * tnorm;
-    for (int j = tid; j < nv; j += EIG_T) {
+    int nc = -1;  // cluster of vector j
+    for (int j = 0; j < nv; ++j) {
       if (j > 0 && ev[j] - ev[j - 1] <= ortol) continue;  // not the first of its cluster
-      int cl[MAXL];
-      int ncl = 0;
+      if (++nc % (EIG_T / 32) != warp) continue;
+      if (j + 1 >= nv || ev[j + 1] - ev[j] > ortol) {
+        twist_vec(m, pp, ee, e2, scal[6], ev[j] * scal[6], Z + (size_t)j * m, red + (size_t)warp * sh.lmax, lane);
+        continue;
+      }
       double prev = 0.0;
       for (int jj = j; jj < nv; ++jj) {
         if (jj > j && ev[jj] - ev[jj - 1] > ortol) break;
         double lam = ev[jj];
         if (jj > j && lam - prev < 10.0 * eps * fabs(lam)) lam = prev + 10.0 * eps * fabs(lam);
-        inv_iter_dev(m, dd, ee, lam, tnorm, Z + (size_t)jj * m, Z, m, cl, ncl, (unsigned)jj + 1u);
-        cl[ncl++] = jj;
+        inv_iter_dev(m, dd, ee, lam, tnorm, Z + (size_t)jj * m, Z, m, j, jj - j, (unsigned)jj + 1u, lane);
         prev = lam;
       }
     }
   }
   __syncthreads();
-  // back-transformation y = H_0 H_1 ... H_{m-3} z: per reflector, one warp
-  // per vector for the dot products, then all threads for the update
-  for (int k = m - 3; k >= 0; --k) {
-    const double beta = bt[k];
-    if (beta == 0.0) continue;
-    const int o = k + 1, mm = m - k - 1;
-    const double *vk = A + (size_t)k * lda + o;  // vk[0] is implicitly 1
-    for (int c = warp; c < nv; c += EIG_T / 32) {
-      const double *zc = Z + (size_t)c * m + o;
-      double s0 = 0.0;
-      for (int i = lane; i < mm; i += 32) s0 = fma((i == 0) ? 1.0 : vk[i], zc[i], s0);
-      s0 = warp_sum(s0);
-      if (lane == 0) pp[c] = beta * s0;
+  // back-transformation y = H_0 H_1 ... H_{m-3} z, one warp per vector, which
+  // it holds in registers: no barriers
+  for (int c = warp; c < nv; c += EIG_T / 32) {
+    double *zc = Z + (size_t)c * m;
+    double z[MAXL / 32];
+#pragma unroll
+    for (int u = 0; u < MAXL / 32; ++u) z[u] = lane + 32 * u < m ? zc[lane + 32 * u] : 0.0;
+    for (int k = m - 3; k >= 0; --k) {
+      const double beta = bt[k];
+      if (beta == 0.0) continue;
+      const double *vk = A + (size_t)k * lda;  // v(k + 1) is implicitly 1
+      double v[MAXL / 32], s0 = 0.0;
+#pragma unroll
+      for (int u = 0; u < MAXL / 32; ++u) {
+        const int i = lane + 32 * u;
+        v[u] = 0.0;
+        if (32 * u < m) {
+          if (i > k && i < m) v[u] = i == k + 1 ? 1.0 : vk[i];
+          s0 = fma(v[u], z[u], s0);
+        }
+      }
+      s0 = beta * warp_sum(s0);
+#pragma unroll
+      for (int u = 0; u < MAXL / 32; ++u)
+        if (32 * u < m) z[u] = fma(-s0, v[u], z[u]);
     }
-    __syncthreads();
-    for (int idx = tid; idx < mm * nv; idx += EIG_T) {
-      const int i = idx % mm, c = idx / mm;
-      Z[(size_t)c * m + o + i] -= pp[c] * ((i == 0) ? 1.0 : vk[i]);
-    }
-    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < MAXL / 32; ++u)
+      if (lane + 32 * u < m) zc[lane + 32 * u] = z[u];
   }
+  __syncthreads();
   double *Yb = Ypool + D.soff;
   for (int idx = tid; idx < m * nv; idx += EIG_T) {
     const int i = idx % m, c = idx / m;
