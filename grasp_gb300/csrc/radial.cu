@@ -1432,6 +1432,209 @@ int build_y(gg_ctx *ctx, const YDesc *d_yd, int nf, double *dY, DBuf<double> &sc
   return GG_OK;
 }
 
+// The Y functions of a potential call, a block per function from densities to
+// Y with everything in between in shared memory: warp 0 runs the Z chains,
+// warp 1 the W chains, each lane a run of up to YF_P points with its four
+// chains' sums in registers; a scan over the lanes joins the runs. The sums
+// are regrouped (YZK adds along a chain point by point), so R^k, whose values
+// MANEIG's vectors follow to the last bit, keeps the passes above. Bound: the
+// FP64 pipe, 20 instructions per 32 points. (COFPOT of 34 subshells: the four
+// kernels above took 63 us per orbital, 15 us of it W's chain of 3 x 148
+// dependent additions; this one 26.)
+constexpr int YF_P = 20;       // points of a lane's run at most, a multiple of 4
+constexpr int YF_MAXN = 2560;  // longer grids don't fit 48 KB of shared memory
+__host__ __device__ __forceinline__ int yf_at(int i) { return i + (i >> 4); }  // spreads the lanes' runs over the banks
+constexpr int YF_SLACK = YF_P + 8;  // zeros above MTP that the windows read
+__global__ void __launch_bounds__(64) k_yfun(const YDesc *__restrict__ yd, int nf, const int *__restrict__ nfp,
+                                             const double *__restrict__ PF, const double *__restrict__ QF, int ld,
+                                             const double *__restrict__ R, const double *__restrict__ RP,
+                                             const double *__restrict__ pw, int np, QuadConst q,
+                                             double *__restrict__ Y) {
+  extern __shared__ double ysh[];
+  __shared__ double zfin[4];  // the Z chains' last values
+  double *TZ = ysh, *TW = ysh + yf_at(np + YF_SLACK);
+  const int tid = threadIdx.x, lane = tid & 31, N = q.n;
+  nf = nfuncs(nf, nfp);
+  for (int f = blockIdx.x; f < nf; f += gridDim.x) {
+    const YDesc y = yd[f];
+    const int K = y.k, MTP = y.mtp, top = MTP + 3;
+    {
+      const double *TK = K ? pw + (size_t)K * np : nullptr;
+      const double *TM = K ? pw + (size_t)(3 * (KLIMIT + 1) + K) * np : pw;
+      for (int i = tid; i < MTP + YF_SLACK; i += 64) {
+        double tz = 0.0, tw = 0.0;
+        if (i >= 2 && i <= MTP) {
+          const double rhop =
+              RP[i] * (pf(PF, ld, i, y.b) * pf(PF, ld, i, y.d) + pf(QF, ld, i, y.b) * pf(QF, ld, i, y.d));
+          tz = K ? TK[i] * rhop : rhop;
+          tw = rhop * TM[i];
+        }
+        TZ[yf_at(i)] = tz;
+        TW[yf_at(i)] = tw;
+      }
+    }
+    __syncthreads();
+    // runs of P points, 32 P to a pass; point i is on chain (i - 2) & 3, and a
+    // run starts on chain 0
+    const int P = min(YF_P, (top - 1 + 127) / 128 * 4), npass = (top - 1 + 32 * P - 1) / (32 * P);
+    double v[YF_P], acc[4], ex[4], h1 = 0.0, h2 = 0.0, h3 = 0.0, h4 = 0.0;  // h: the neighbouring pass's temps
+    double carry[4] = {0.0, 0.0, 0.0, 0.0};
+    if (tid < 32) {
+      // Z(2), Z(3), Z(4) from the five-point start formulas
+      double st = 0.0;
+      for (int kk = 2; kk <= 5; ++kk) st = fma(q.CNC5C[kk - 2][min(lane, 2)], TZ[yf_at(kk)], st);
+      const double st0 = __shfl_sync(0xffffffffu, st, 0), st1 = __shfl_sync(0xffffffffu, st, 1),
+                   st2 = __shfl_sync(0xffffffffu, st, 2);
+      for (int p = 0; p < npass; ++p) {
+        const int b = 2 + p * 32 * P, i0 = b + lane * P;
+        const bool in = i0 <= top;
+        double t1 = h1, t2 = h2, t3 = h3, t4 = h4;  // T(i - 1) ... T(i - 4)
+        if (lane && in) {
+          t1 = TZ[yf_at(i0 - 1)];
+          t2 = TZ[yf_at(i0 - 2)];
+          t3 = TZ[yf_at(i0 - 3)];
+          t4 = TZ[yf_at(i0 - 4)];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c] = lane ? 0.0 : carry[c];
+#pragma unroll
+        for (int j = 0; j < YF_P; ++j) {
+          if (j >= P) break;
+          const int i = i0 + j;
+          if (i <= top) {
+            const double t0 = TZ[yf_at(i)];
+            acc[j & 3] = fma(q.C3, t2, fma(q.C2, t3 + t1, fma(q.C1, t4 + t0, acc[j & 3])));
+            t4 = t3;
+            t3 = t2;
+            t2 = t1;
+            t1 = t0;
+          }
+          if (j < 3 && i < 5) acc[j] = j == 0 ? st0 : j == 1 ? st1 : st2;
+          v[j] = acc[j & 3];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          double s = acc[c];
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const double u = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += u;
+          }
+          ex[c] = __shfl_up_sync(0xffffffffu, s, 1);
+          if (lane == 0) ex[c] = 0.0;
+          carry[c] = __shfl_sync(0xffffffffu, s, 31);
+        }
+        const int e = b + 32 * P;  // the next pass's first point
+        if (e <= top) {
+          h1 = TZ[yf_at(e - 1)];
+          h2 = TZ[yf_at(e - 2)];
+          h3 = TZ[yf_at(e - 3)];
+          h4 = TZ[yf_at(e - 4)];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < YF_P; ++j) {
+          if (j >= P) break;
+          if (i0 + j <= top) TZ[yf_at(i0 + j)] = v[j] + ex[j & 3];
+        }
+        __syncwarp();
+      }
+      if (lane < 4) zfin[lane] = lane == 0 ? carry[0] : lane == 1 ? carry[1] : lane == 2 ? carry[2] : carry[3];
+    } else {
+      const int lim = min(N, MTP);
+      for (int p = npass - 1; p >= 0; --p) {
+        const int b = 2 + p * 32 * P, i0 = b + lane * P;
+        const bool in = i0 <= lim;
+        double t1 = h1, t2 = h2, t3 = h3, t4 = h4;  // TW(i + 1) ... TW(i + 4)
+        if (lane < 31 || p == npass - 1) {
+          t1 = in ? TW[yf_at(i0 + P)] : 0.0;
+          t2 = in ? TW[yf_at(i0 + P + 1)] : 0.0;
+          t3 = in ? TW[yf_at(i0 + P + 2)] : 0.0;
+          t4 = in ? TW[yf_at(i0 + P + 3)] : 0.0;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c] = lane < 31 ? 0.0 : carry[c];
+#pragma unroll
+        for (int j = YF_P - 1; j >= 0; --j) {
+          if (j >= P) continue;
+          const int i = i0 + j;
+          if (in) {
+            const double t0 = TW[yf_at(i)];
+            if (i <= lim) acc[j & 3] = fma(q.C3, t2, fma(q.C2, t1 + t3, fma(q.C1, t0 + t4, acc[j & 3])));
+            t4 = t3;
+            t3 = t2;
+            t2 = t1;
+            t1 = t0;
+          }
+          v[j] = acc[j & 3];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          double s = acc[c];
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const double u = __shfl_down_sync(0xffffffffu, s, o);
+            if (lane + o < 32) s += u;
+          }
+          ex[c] = __shfl_down_sync(0xffffffffu, s, 1);
+          if (lane == 31) ex[c] = 0.0;
+          carry[c] = __shfl_sync(0xffffffffu, s, 0);
+        }
+        h1 = TW[yf_at(b)];
+        h2 = TW[yf_at(b + 1)];
+        h3 = TW[yf_at(b + 2)];
+        h4 = TW[yf_at(b + 3)];
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < YF_P; ++j) {
+          if (j >= P) break;
+          if (i0 + j <= lim) TW[yf_at(i0 + j)] = v[j] + ex[j & 3];
+        }
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    // Y = Z r^-k + W r^(k+1); above MTP + 3 Z keeps its asymptotic value
+    // (yzk.f90:150-171), k = 0: the chains are shifted to end on it
+    const double *RTTKM = pw + (size_t)(1 * (KLIMIT + 1) + K) * np;
+    const double *RTTK1 = pw + (size_t)(2 * (KLIMIT + 1) + K) * np;
+    const double zklim = K ? zfin[(top - 2) & 3] : (y.b == y.d ? 1.0 : 0.0);
+    double dif = 0.0;  // this thread's points are all on one chain: 64 is a multiple of 4
+    if (K == 0) {
+      const double d0 = zfin[(tid - 2) & 3] - zklim;
+      if (fabs(d0) > q.accy) dif = d0;
+    }
+    double *Yf = Y + (size_t)f * np;
+    for (int i = tid; i < np; i += 64) {
+      double yv = 0.0;
+      if (i >= 2 && i <= N && i <= y.mtpb) {
+        if (K == 0) {
+          yv = i <= top ? TZ[yf_at(i)] - dif : zklim;
+          if (i <= MTP) yv = fma(TW[yf_at(i)], R[i], yv);
+        } else {
+          yv = (i <= top ? TZ[yf_at(i)] : zklim) * RTTKM[i];
+          if (i <= MTP) yv = fma(TW[yf_at(i)], RTTK1[i], yv);
+        }
+      }
+      Yf[i] = yv;
+    }
+    __syncthreads();
+  }
+}
+
+// The Y functions of a potential call: nfp (on the device) of them, at most nf
+int build_y_pot(gg_ctx *ctx, const YDesc *d_yd, int nf, double *dY, DBuf<double> &scratch, const int *nfp) {
+  Grid &g = ctx->grid;
+  Orbitals &o = ctx->orb;
+  if (g.q.n > YF_MAXN) return build_y(ctx, d_yd, nf, dY, scratch, nfp);
+  const size_t smem = 2 * sizeof(double) * yf_at(g.np + YF_SLACK);
+  k_yfun<<<std::min(nf, 32 * ctx->sms), 64, smem, ctx->stream>>>(d_yd, nf, nfp, o.dPF.p, o.dQF.p, o.ld, g.dR.p,
+                                                                 g.dRP.p, g.dPow.p, g.np, g.q, dY);
+  ::gg::note_launch();
+  GG_CUDA(cudaGetLastError());
+  return GG_OK;
+}
+
 template <class T> int upload(DBuf<T> &b, const std::vector<T> &h, cudaStream_t s) {
   GG_TRY(b.alloc(h.size()));
   if (!h.empty()) GG_CUDA(cudaMemcpyAsync(b.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
@@ -2013,7 +2216,7 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, double *
     nfb = std::max(1, cnt);
   }
   GG_TRY(W.Y.alloc((size_t)nfb * g.np));
-  if (T > 0) GG_TRY(build_y(ctx, W.yd.p, nfb, W.Y.p, W.scratch, W.info.p));
+  if (T > 0) GG_TRY(build_y_pot(ctx, W.yd.p, nfb, W.Y.p, W.scratch, W.info.p));
   // one launch for all chunks, one for every job's point values
   if (nch > 0) {
     k_pot_part<<<dim3((n + 63) / 64, (unsigned)nch), 256, 0, s>>>(reinterpret_cast<const PotChunk *>(W.up.p + ach),
