@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <map>
 #include <tuple>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -910,13 +911,16 @@ __global__ void k_quad_table(const QuadItem *__restrict__ items, const int *__re
 
 // YPOT / XPOT (rmcdhf90/ypot.f90:35-49, xpot.f90:31-54): sum_t COEFF TB (YPOT),
 // sum_t CTB QF and sum_t CTB PF with CTB = COEFF TB (XPOT), cut into chunks of
-// terms. A block takes 64 grid points of one chunk, its four rows of threads
-// every fourth term; the rows' sums meet in shared memory and the chunk's are
-// stored for k_pot_final, which adds them in list order. Bound: the FP64 pipe
-// (three operations per XPOT term and point; 34 subshells' lists of 6,600 terms
-// 24 us per orbital). One thread per point adding the terms in list order
-// left the pipe to one dependent addition per term: 233 us for the same list.
-constexpr int POT_CHUNK = 128;  // terms staged in shared memory at a time
+// terms. A block takes 64 grid points of one chunk, its four rows of threads a
+// quarter of the terms each; the rows' sums meet in shared memory and the
+// chunk's are stored for k_pot_final, which adds them in list order. An XPOT
+// chunk is ordered by the orbital the terms multiply, so that a run of terms
+// of one orbital sums COEFF TB and multiplies by QF and PF once. Bound: the
+// FP64 pipe, one operation per term and point and two per run (6,600 terms of
+// 34 subshells: 26 us per orbital, 34 with three operations per term; one
+// thread per point adding the terms in list order left the pipe to one
+// dependent addition per term: 233 us).
+constexpr int POT_CHUNK = 256;  // terms staged in shared memory at a time
 struct PotChunk {
   const int *key, *iorb;  // iorb null: YPOT
   const double *coef;
@@ -928,33 +932,58 @@ __global__ void __launch_bounds__(256) k_pot_part(const PotChunk *__restrict__ c
                                                   const double *__restrict__ PF, const double *__restrict__ QF,
                                                   int ld, int n, double *__restrict__ part) {
   __shared__ int sf[POT_CHUNK], so[POT_CHUNK];
+  __shared__ int4 sk[POT_CHUNK / 4];
   __shared__ double sc[POT_CHUNK], red[2][4][64];
   const PotChunk g = ch[blockIdx.y];
-  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+  const int tid = threadIdx.x, tx = tid & 63, ty = tid >> 6;
   const int i = 1 + blockIdx.x * 64 + tx;
   const bool x = g.iorb != nullptr, in = i <= n;
   double a0 = 0.0, a1 = 0.0;
   for (int t0 = 0; t0 < g.nt; t0 += POT_CHUNK) {
     const int nt = min(POT_CHUNK, g.nt - t0);
     __syncthreads();
-    if ((int)threadIdx.x < nt) {
-      sf[threadIdx.x] = max(tab[g.key[t0 + threadIdx.x]] - 1, 0);  // 0: a label the parser refused
-      so[threadIdx.x] = x ? g.iorb[t0 + threadIdx.x] : 1;
-      sc[threadIdx.x] = g.coef[t0 + threadIdx.x];
+    const int io = x && tid < nt ? g.iorb[t0 + tid] : 1, k = io * POT_CHUNK + tid;
+    int pos = tid;
+    if (x) {  // the term's place: how many have a lower orbital, or the same and stand before it
+      reinterpret_cast<int *>(sk)[tid] = tid < nt ? k : INT_MAX;
+      __syncthreads();
+      pos = 0;
+#pragma unroll 16
+      for (int u = 0; u < POT_CHUNK / 4; ++u) {
+        const int4 v = sk[u];
+        pos += (v.x < k) + (v.y < k) + (v.z < k) + (v.w < k);
+      }
+    }
+    if (tid < nt) {
+      sf[pos] = max(tab[g.key[t0 + tid]] - 1, 0);  // 0: a label the parser refused
+      so[pos] = io;
+      sc[pos] = g.coef[t0 + tid];
     }
     __syncthreads();
-    if (!in) continue;
-    if (x) {
-#pragma unroll 8
-      for (int t = ty; t < nt; t += 4) {
-        const double ctb = sc[t] * __ldg(Y + (size_t)sf[t] * np + i);
-        a0 = fma(ctb, pf(QF, ld, i, so[t]), a0);
-        a1 = fma(ctb, pf(PF, ld, i, so[t]), a1);
+    const int tb = nt * ty / 4, te = nt * (ty + 1) / 4;
+    if (!in || tb == te) continue;
+    int o = so[tb];
+    double run = 0.0, qv = x ? pf(QF, ld, i, o) : 1.0, pv = x ? pf(PF, ld, i, o) : 0.0;
+    for (int t = tb; t < te; t += 8) {
+      double yv[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) yv[u] = t + u < te ? __ldg(Y + (size_t)sf[t + u] * np + i) : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (t + u >= te) break;
+        if (so[t + u] != o) {  // the next run
+          a0 = fma(run, qv, a0);
+          a1 = fma(run, pv, a1);
+          run = 0.0;
+          o = so[t + u];
+          qv = pf(QF, ld, i, o);
+          pv = pf(PF, ld, i, o);
+        }
+        run = fma(sc[t + u], yv[u], run);
       }
-    } else {
-#pragma unroll 8
-      for (int t = ty; t < nt; t += 4) a0 = fma(sc[t], __ldg(Y + (size_t)sf[t] * np + i), a0);
     }
+    a0 = fma(run, qv, a0);
+    a1 = fma(run, pv, a1);
   }
   red[0][ty][tx] = a0;
   red[1][ty][tx] = a1;
