@@ -992,8 +992,8 @@ __global__ void __launch_bounds__(256) k_pot_part(const PotChunk *__restrict__ c
     part[g.out + (size_t)ty * n + i - 1] = (red[ty][0][tx] + red[ty][1][tx]) + (red[ty][2][tx] + red[ty][3][tx]);
 }
 
-// The lists' labels decoded on the device, one thread per term (mode 0:
-// YPOT labels, 1: XPOT labels): the term's (K, a, b) key into a dense table
+// The lists' labels decoded on the device, one thread per term (the
+// first ny YPOT labels, then XPOT labels): the term's (K, a, b) key into a dense table
 // over K <= KLIMIT and the orbital pairs; the orbital it multiplies (XPOT) and
 // COEFF (XPOT: XA/C, as the reference forms it). The first term of a key
 // takes the next function number (info[0]), writes its YZK descriptor and
@@ -1002,12 +1002,13 @@ __global__ void __launch_bounds__(256) k_pot_part(const PotChunk *__restrict__ c
 // key. (Marking the keys and numbering them by one block in table order took
 // 16 us of a 34-subshell COFPOT call.) A label outside the orbital set or
 // with K above KLIMIT sets info[1].
-__global__ void k_parse_terms(int mode, int64_t nt, const int32_t *__restrict__ lab, const double *__restrict__ co,
+__global__ void k_parse_terms(int64_t ny, int64_t nt, const int32_t *__restrict__ lab, const double *__restrict__ co,
                               int nw, double c, const int *__restrict__ MF, int n, int *__restrict__ tab,
                               YDesc *__restrict__ yd, int *__restrict__ key, int *__restrict__ iorb,
                               double *__restrict__ coef, int *__restrict__ info) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nt; e += (int64_t)gridDim.x * blockDim.x) {
     const int32_t l0 = lab[e];
+    const int mode = e < ny ? 0 : 1;
     int64_t l = l0;
     const int k = (int)(l % KEYORB);
     l /= KEYORB;
@@ -2128,7 +2129,7 @@ struct PotWork {
   void *stage = nullptr;
   size_t stage_bytes = 0;
   DBuf<char> up;  // the staged block on the device
-  DBuf<int> term, tab, info;
+  DBuf<int> term;
   DBuf<double> coef, Y, scratch, pot, part;
   DBuf<YDesc> yd;
   ~PotWork() { cudaFreeHost(stage); }
@@ -2171,7 +2172,7 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, double *
   const size_t alab = place(T * sizeof(int32_t)), aco = place(T * sizeof(double)), ach = place(nch * sizeof(PotChunk)),
                afin = place(jobs.size() * sizeof(PotFinal)), aint = place((nd + nl) * sizeof(int)),
                adbl = place((nd + nl) * sizeof(double));
-  const size_t ares = place(2 * sizeof(int) + (out ? (size_t)3 * n * jobs.size() * sizeof(double) : 0) + 16);
+  const size_t ares = place(((out ? (size_t)3 * n * jobs.size() : 0) + 1) * sizeof(double));
   if (need > W.stage_bytes) {
     cudaFreeHost(W.stage);
     W.stage = nullptr;
@@ -2186,10 +2187,11 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, double *
   GG_TRY(W.up.alloc(ares));
   GG_TRY(W.term.alloc(2 * T1));
   GG_TRY(W.coef.alloc(T1));
-  GG_TRY(W.tab.alloc(tsize));
-  GG_TRY(W.info.alloc(2));
   GG_TRY(W.yd.alloc(nfb));
-  GG_TRY(W.pot.alloc((size_t)3 * n * std::max<size_t>(1, jobs.size())));
+  // the potentials, the parser's two counts and its table: one read-back and one clearing
+  const size_t npot = (size_t)3 * n * jobs.size();
+  GG_TRY(W.pot.alloc(npot + 1 + (tsize + 1) / 2));
+  int *info = reinterpret_cast<int *>(W.pot.p + npot), *tab = info + 2;
   int *dkey = W.term.p, *diorb = dkey + T1;
   int32_t *hlab = reinterpret_cast<int32_t *>(stage + alab);
   double *hco = reinterpret_cast<double *>(stage + aco);
@@ -2226,30 +2228,27 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, double *
   }
   GG_TRY(W.part.alloc(std::max<size_t>(1, po)));
   if (ares > 0) GG_CUDA(cudaMemcpyAsync(W.up.p, stage, ares, cudaMemcpyHostToDevice, s));
-  GG_CUDA(cudaMemsetAsync(W.tab.p, 0, tsize * sizeof(int), s));
-  GG_CUDA(cudaMemsetAsync(W.info.p, 0, 2 * sizeof(int), s));
+  GG_CUDA(cudaMemsetAsync(info, 0, (2 + tsize) * sizeof(int), s));
   const int32_t *dlab = reinterpret_cast<const int32_t *>(W.up.p + alab);
   const double *dco = reinterpret_cast<const double *>(W.up.p + aco);
   const unsigned pgrid = (unsigned)std::max<size_t>(1, std::min<size_t>((T + 255) / 256, (size_t)8 * ctx->sms));
-  for (int m = 0; m < 2; ++m) {
-    const size_t a = m == 0 ? 0 : TY, cnt = m == 0 ? TY : T - TY;
-    if (cnt == 0) continue;
-    k_parse_terms<<<pgrid, 256, 0, s>>>(m, (int64_t)cnt, dlab + a, dco + a, nw, g.c, o.dMF.p, n, W.tab.p, W.yd.p,
-                                        dkey + a, diorb + a, W.coef.p + a, W.info.p);
+  if (T > 0) {
+    k_parse_terms<<<pgrid, 256, 0, s>>>((int64_t)TY, (int64_t)T, dlab, dco, nw, g.c, o.dMF.p, n, tab, W.yd.p, dkey,
+                                        diorb, W.coef.p, info);
     ::gg::note_launch();
   }
   if ((size_t)7 * nfb * g.np * sizeof(double) > POT_BOUND) {  // too much to reserve for a bound: wait for the number
     int cnt = 0;
-    GG_CUDA(cudaMemcpyAsync(&cnt, W.info.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    GG_CUDA(cudaMemcpyAsync(&cnt, info, sizeof(int), cudaMemcpyDeviceToHost, s));
     GG_CUDA(cudaStreamSynchronize(s));
     nfb = std::max(1, cnt);
   }
   GG_TRY(W.Y.alloc((size_t)nfb * g.np));
-  if (T > 0) GG_TRY(build_y_pot(ctx, W.yd.p, nfb, W.Y.p, W.scratch, W.info.p));
+  if (T > 0) GG_TRY(build_y_pot(ctx, W.yd.p, nfb, W.Y.p, W.scratch, info));
   // one launch for all chunks, one for every job's point values
   if (nch > 0) {
     k_pot_part<<<dim3((n + 63) / 64, (unsigned)nch), 256, 0, s>>>(reinterpret_cast<const PotChunk *>(W.up.p + ach),
-                                                                 W.tab.p, W.Y.p, g.np, o.dPF.p, o.dQF.p, o.ld, n,
+                                                                 tab, W.Y.p, g.np, o.dPF.p, o.dQF.p, o.ld, n,
                                                                  W.part.p);
     ::gg::note_launch();
   }
@@ -2260,14 +2259,14 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, double *
     ::gg::note_launch();
   }
   GG_CUDA(cudaGetLastError());
-  int *hinfo = reinterpret_cast<int *>(stage + ares);
-  double *hres = reinterpret_cast<double *>(stage + ares + 16);
-  GG_CUDA(cudaMemcpyAsync(hinfo, W.info.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-  const size_t nres = (size_t)3 * n * jobs.size();
-  if (out) GG_CUDA(cudaMemcpyAsync(hres, W.pot.p, nres * sizeof(double), cudaMemcpyDeviceToHost, s));
+  // with out: the potentials and the counts behind them
+  double *hres = reinterpret_cast<double *>(stage + ares);
+  const size_t skip = out ? 0 : npot;
+  int *hinfo = reinterpret_cast<int *>(hres + npot - skip);
+  GG_CUDA(cudaMemcpyAsync(hres, W.pot.p + skip, (npot - skip + 1) * sizeof(double), cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaStreamSynchronize(s));
   const bool bad = hinfo[1] != 0;
-  if (out && !bad) std::memcpy(out, hres, nres * sizeof(double));
+  if (out && !bad) std::memcpy(out, hres, npot * sizeof(double));
   auto bytes = [](const DBuf<double> &b) { return b.n * sizeof(double); };
   if (bytes(W.Y) + bytes(W.scratch) + bytes(W.part) + bytes(W.coef) * 2 + W.up.n > POT_KEEP) {
     W.Y.release();
