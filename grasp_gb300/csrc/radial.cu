@@ -437,19 +437,27 @@ constexpr int OZ_S = 10;
 // neighbours in K 128 B apart, in M/N 256 B apart), one block per 32 grid
 // points: 80 KB of Y slices, 30 KB of A slices.
 //
-// k_rk_tc, one CTA per tile, is warp-specialised. Warp 4 streams the blocks
-// into two shared-memory stages with cp.async.bulk (completion counted in
-// bytes on a per-stage "full" mbarrier) and issues, per K = 16 step, the 55
-// slice-pair MMAs tcgen05.mma.cta_group::1.kind::f16 into the FP32 tensor-
-// memory accumulator of their group q = s + t (OZ_S x TC_N columns); a
-// tcgen05.commit to the stage's "empty" mbarrier frees the stage. Every
-// TC_FLUSH stages (256 grid points, while every group sum is still an exact
-// integer below 2^24) warps 0-3 read their 32 lanes of each group
-// (tcgen05.ld) and fold group q, scaled by 2^(-7q), into double-float sums;
-// the next MMA of each group overwrites. The raw sum 2^(eA+eY-14) (h + l) is
-// stored at the entry's GENINTRK position; k_rk_finish_all adds the head
-// term. Every wait is bounded: on a timeout the CTA records it, waits
-// (bounded) for what it issued, frees its tensor memory and writes nothing.
+// k_rk_tc, one CTA per SM taking the tiles in turn, is warp-specialised. Warp
+// 4 streams the tiles' blocks into two shared-memory stages with
+// cp.async.bulk (completion counted in bytes on a per-stage "full" mbarrier)
+// and issues, per K = 16 step, the 55 slice-pair MMAs
+// tcgen05.mma.cta_group::1.kind::f16 into the FP32 tensor-memory accumulator
+// of their group q = s + t (OZ_S x TC_N columns); a tcgen05.commit to the
+// stage's "empty" mbarrier frees the stage. Every TC_FLUSH stages (256 grid
+// points, while every group sum is still an exact integer below 2^24) and at
+// a tile's end warps 0-3 read their 32 lanes of each group (tcgen05.ld) and
+// fold group q, scaled by 2^(-7q), into double-float sums; the next MMA of
+// each group overwrites. The raw sum 2^(eA+eY-14) (h + l) is stored at the
+// entry's GENINTRK position while the next tile runs; k_rk_finish_all adds
+// the head term. Every wait is bounded: on a timeout the CTA records it,
+// waits (bounded) for what it issued, frees its tensor memory and writes
+// nothing more.
+// Bound: an MMA takes 44 cycles whatever N is (16 to 48), the read of its 128
+// Y rows from shared memory, so a tile's 990 are 44,000 of its 75,000 cycles;
+// the rest are two flushes (7,000 each) and the waits for copies, 110 KB a
+// stage from L2 to every SM. 43 subshells, k <= 8 (194 tiles): 94 us; 175 us
+// with rolled MMA loops (descriptors formed by one thread, 80 cycles per
+// MMA), a CTA per tile and values scaled by scalbn one at a time after it.
 // ---------------------------------------------------------------------------
 constexpr int TC_M = 128, TC_N = 48, TC_KC = 32, TC_FLUSH = 8;
 constexpr int TC_YBLK = OZ_S * 2 * (TC_M / 8) * 2 * 64;  // fp16 elements per Y block (80 KB)
@@ -527,6 +535,13 @@ __device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity, int spin
   return done != 0;
 }
 
+// one lane of the converged warp, the same at every call
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}" : "=r"(p));
+  return p != 0;
+}
+
 // Slices of rows into their tile blocks: one CTA per row slot (slot = tile
 // block column g, row m < R); src_row[slot] < 0 pads with zeros. The row's
 // exponent goes to exps[src_row] (the same row always gets the same value).
@@ -579,7 +594,7 @@ __global__ void k_oz_tile(const double *__restrict__ M, int pitch, int K, int nc
   }
 }
 
-__global__ void __launch_bounds__(TC_THREADS, 1) k_rk_tc(const TcTile *__restrict__ tiles,
+__global__ void __launch_bounds__(TC_THREADS, 1) k_rk_tc(const TcTile *__restrict__ tiles, int ntiles,
                                                          const TcRow *__restrict__ rows,
                                                          const __half *__restrict__ Yt,
                                                          const __half *__restrict__ At, int nch,
@@ -594,9 +609,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_rk_tc(const TcTile *__restric
   uint32_t *tslot = reinterpret_cast<uint32_t *>(empty + 2);
   int *okflag = reinterpret_cast<int *>(tslot + 1);
   __shared__ TcRow trow[TC_N];
-  const TcTile T = tiles[blockIdx.x];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid < TC_N) trow[tid] = (tid < T.rn) ? rows[T.r0 + tid] : TcRow{-1, 0, 0, 0, 0, 0};
+  __shared__ int tex[TC_N];  // the rows' exponents
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
                  "r"(TC_TMEM_COLS));
@@ -613,141 +627,164 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_rk_tc(const TcTile *__restric
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = *tslot;
-  const int nloc = T.c1 - T.c0;  // chunks of this split
-  const int nflush = (nloc + TC_FLUSH - 1) / TC_FLUSH;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
   if (warp == 4) {
-    // copies and MMAs (lane 0 issues; the warp stays converged). A tile
-    // named by stall_tile (a test of the bounded waits) withholds its first
-    // copy and polls briefly: its first wait runs out with nothing in flight.
-    const bool stall = (int)blockIdx.x == stall_tile;
-    const int spin = stall ? (1 << 12) : TC_SPIN;
-    const uint32_t idesc = (1u << 4) | ((uint32_t)(TC_N >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
-    const char *ysrc = reinterpret_cast<const char *>(Yt + (size_t)T.fg * nch * TC_YBLK);
-    const char *asrc = reinterpret_cast<const char *>(At + (size_t)T.pg * nch * TC_ABLK);
+    // copies and MMAs (one elected lane issues; the warp stays converged).
+    // The chunks of the CTA's tiles form one stream, chunk j in stage j & 1.
+    // A tile named by stall_tile (a test of the bounded waits) withholds its
+    // first copy and polls briefly: its first wait runs out with nothing in
+    // flight.
     constexpr uint32_t YB = TC_YBLK * sizeof(__half), AB = TC_ABLK * sizeof(__half);
-    // local chunk j of the split is grid chunk T.c0 + j
-    auto copy = [&](int j) {
-      const int st = j & 1;
-      if (lane == 0) {
+    int ct = blockIdx.x, cc = 0, cn = 0;  // the copy stream: tile, next chunk of it, its chunks
+    const char *ysrc = nullptr, *asrc = nullptr;
+    auto open = [&] {
+      if (ct >= ntiles) return;
+      const TcTile C = tiles[ct];
+      cc = 0;
+      cn = C.c1 - C.c0;
+      ysrc = reinterpret_cast<const char *>(Yt) + ((size_t)C.fg * nch + C.c0) * YB;
+      asrc = reinterpret_cast<const char *>(At) + ((size_t)C.pg * nch + C.c0) * AB;
+    };
+    int issued = -1;  // last chunk whose MMAs were committed
+    int copied = -1;  // last chunk whose copy was issued
+    auto copy = [&] {
+      if (ct >= ntiles || ct == stall_tile) return;
+      const int st = (copied + 1) & 1;
+      if (elect_one()) {
         const uint32_t fb = smem_addr(&full[st]);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(YB + AB) : "memory");
         asm volatile(
             "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                 smem_addr(Ysm + st * TC_YBLK)),
-            "l"(ysrc + (size_t)(T.c0 + j) * YB), "r"(YB), "r"(fb)
+            "l"(ysrc + (size_t)cc * YB), "r"(YB), "r"(fb)
             : "memory");
         asm volatile(
             "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                 smem_addr(Asm + st * TC_ABLK)),
-            "l"(asrc + (size_t)(T.c0 + j) * AB), "r"(AB), "r"(fb)
+            "l"(asrc + (size_t)cc * AB), "r"(AB), "r"(fb)
             : "memory");
       }
       __syncwarp();
+      ++copied;
+      if (++cc == cn) {
+        ct += gridDim.x;
+        open();
+      }
     };
     bool ok = true;
-    uint32_t fresh = (1u << OZ_S) - 1;
-    int issued = -1;  // last chunk whose MMAs were committed
-    int copied = -1;  // last chunk whose copy was issued
-    if (!stall) {
-      copy(0);
-      copied = 0;
-    }
-    int fl = 0;
-    for (int j = 0; j < nloc; ++j) {
-      const int st = j & 1;
-      if (ok) ok = __all_sync(0xffffffffu, tc_wait(smem_addr(&full[st]), (j >> 1) & 1, spin));
-      if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        if (lane == 0) {
-          const uint32_t yb = smem_addr(Ysm + st * TC_YBLK), ab = smem_addr(Asm + st * TC_ABLK);
+    open();
+    copy();
+    int jg = 0;  // the stream's chunk
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+      const int nloc = __shfl_sync(0xffffffffu, tiles[tile].c1 - tiles[tile].c0, 0);
+      const int rn = __shfl_sync(0xffffffffu, tiles[tile].rn, 0);
+      const int spin = tile == stall_tile ? (1 << 12) : TC_SPIN;
+      // N: the tile's valid rows, rounded up to a multiple of 16
+      const uint32_t idesc = (1u << 4) | ((uint32_t)((rn + 15) / 16 * 2) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+      for (int j = 0; j < nloc; ++j, ++jg) {
+        const int st = jg & 1;
+        if (ok) ok = __all_sync(0xffffffffu, tc_wait(smem_addr(&full[st]), (jg >> 1) & 1, spin));
+        if (ok) {
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          if (elect_one()) {
+            const uint32_t yb = smem_addr(Ysm + st * TC_YBLK), ab = smem_addr(Asm + st * TC_ABLK);
+            // unrolled, so that a descriptor is one addition: with the loops
+            // rolled the issuing thread, not the tensor core, set the pace
 #pragma unroll 1
-          for (int ks = 0; ks < 2; ++ks)
-#pragma unroll 1
-            for (int sa = 0; sa < OZ_S; ++sa) {
-              const uint64_t bdesc = tc_desc(ab + (uint32_t)(sa * 2 + ks) * ((TC_N / 8) * 2 * 64 * 2));
-#pragma unroll 1
-              for (int t = 0; t < OZ_S - sa; ++t) {
-                const int qg = sa + t;
-                const uint64_t adesc = tc_desc(yb + (uint32_t)(t * 2 + ks) * ((TC_M / 8) * 2 * 64 * 2));
-                const uint32_t accum = ((fresh >> qg) & 1u) ? 0u : 1u;
-                fresh &= ~(1u << qg);
-                asm volatile(
-                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(
-                        tmem + (uint32_t)(qg * TC_N)),
-                    "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
-              }
+            for (int ks = 0; ks < 2; ++ks) {
+              // the first MMA of each group after a flush (slice 0 of A) overwrites
+              const uint32_t cont = (j % TC_FLUSH == 0 && ks == 0) ? 0u : 1u;
+              const uint64_t b0 = tc_desc(ab + (uint32_t)ks * ((TC_N / 8) * 2 * 64 * 2));
+              const uint64_t a0 = tc_desc(yb + (uint32_t)ks * ((TC_M / 8) * 2 * 64 * 2));
+#pragma unroll
+              for (int sa = 0; sa < OZ_S; ++sa)
+#pragma unroll
+                for (int t = 0; t < OZ_S - sa; ++t)
+                  asm volatile(
+                      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(
+                          tmem + (uint32_t)((sa + t) * TC_N)),
+                      "l"(a0 + (uint64_t)(t * 2 * (TC_M / 8) * 2 * 64 * 2 / 16)),
+                      "l"(b0 + (uint64_t)(sa * 2 * (TC_N / 8) * 2 * 64 * 2 / 16)), "r"(idesc), "r"(sa ? 1u : cont));
             }
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           smem_addr(&empty[st]))
-                       : "memory");
-        }
-        __syncwarp();
-        issued = j;
-        // refill the other stage with chunk j + 1 once chunk j - 1's MMAs are done
-        if (j + 1 < nloc) {
-          if (j >= 1)
-            ok = __all_sync(0xffffffffu, tc_wait(smem_addr(&empty[(j - 1) & 1]), ((j - 1) >> 1) & 1, spin));
-          if (ok) {
-            copy(j + 1);
-            copied = j + 1;
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_addr(&empty[st]))
+                         : "memory");
+          }
+          __syncwarp();
+          issued = jg;
+          // refill the other stage with the stream's next chunk once chunk jg - 1's MMAs are done
+          if (copied == jg) {
+            if (jg >= 1)
+              ok = __all_sync(0xffffffffu, tc_wait(smem_addr(&empty[(jg - 1) & 1]), ((jg - 1) >> 1) & 1, spin));
+            if (ok) copy();
           }
         }
-      }
-      if ((j + 1) % TC_FLUSH == 0 || j == nloc - 1) {
-        if (ok) ok = __all_sync(0xffffffffu, tc_wait(smem_addr(&empty[st]), (j >> 1) & 1, spin));  // MMAs done
-        if (!ok && lane == 0) *okflag = 0;
-        asm volatile("tcgen05.fence::before_thread_sync;");
-        __syncthreads();  // A: the accumulators are ready (or the flag says no)
-        __syncthreads();  // B: warps 0-3 have read them
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        fresh = (1u << OZ_S) - 1;
-        ++fl;
+        if ((j + 1) % TC_FLUSH == 0 || j == nloc - 1) {
+          if (ok) ok = __all_sync(0xffffffffu, tc_wait(smem_addr(&empty[st]), (jg >> 1) & 1, spin));  // MMAs done
+          if (!ok && lane == 0) *okflag = 0;
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          __syncthreads();  // A: the accumulators are ready (or the flag says no)
+          __syncthreads();  // B: warps 0-3 have read them
+          asm volatile("tcgen05.fence::after_thread_sync;");
+        }
       }
     }
-    for (; fl < nflush; ++fl) {  // a failed wait leaves the loop early: meet the remaining barriers
-      __syncthreads();
-      __syncthreads();
-    }
-    if (!ok && lane == 0) {
+    if (!ok) {
       // timed out: before the tensor memory is freed and the CTA leaves,
       // wait (bounded) for the last copy issued to land in shared memory and
       // for the last committed MMAs to finish; 2 records a failed drain
       bool drained = true;
       if (copied >= 0) drained = tc_wait(smem_addr(&full[copied & 1]), (copied >> 1) & 1);
       if (issued >= 0) drained = tc_wait(smem_addr(&empty[issued & 1]), (issued >> 1) & 1) && drained;
-      atomicMax(flags + 1, drained ? 1 : 2);
+      if (lane == 0) atomicMax(flags + 1, drained ? 1 : 2);
     }
   } else {
-    // warps 0-3: lane quadrant `warp` of each group accumulator
-    float ah[TC_N], al[TC_N];
+    // warps 0-3: lane quadrant `warp` of each group accumulator; a tile's
+    // values are stored while warp 4 works on the next tile
+    const int m = warp * 32 + lane;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+      const TcTile T = tiles[tile];
+      const int nflush = (T.c1 - T.c0 + TC_FLUSH - 1) / TC_FLUSH;
+      const bool valid = m < T.fn;
+      const int f = valid ? T.f0 + m : T.f0;
+      const YDesc y = yd[f];
+      const int ey = eY[f] - 14;
+      asm volatile("bar.sync 1, 128;" ::: "memory");  // the previous tile's rows are no longer read
+      if (tid < TC_N) {
+        trow[tid] = (tid < T.rn) ? rows[T.r0 + tid] : TcRow{-1, 0, 0, 0, 0, 0};
+        tex[tid] = (tid < T.rn) ? eA[trow[tid].p] : 0;
+      }
+      float ah[TC_N], al[TC_N];
 #pragma unroll
-    for (int n = 0; n < TC_N; ++n) ah[n] = al[n] = 0.f;
-    for (int fl = 0; fl < nflush; ++fl) {
-      __syncthreads();  // A
-      asm volatile("tcgen05.fence::after_thread_sync;");
-      if (*okflag) {
+      for (int n = 0; n < TC_N; ++n) ah[n] = al[n] = 0.f;
+      for (int fl = 0; fl < nflush; ++fl) {
+        __syncthreads();  // A
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        if (*okflag) {
 #pragma unroll 1
-        for (int qg = 0; qg < OZ_S; ++qg) {
-          const float scale = __int_as_float((127 - 7 * qg) << 23);  // 2^(-7 qg)
+          for (int qg = 0; qg < OZ_S; ++qg) {
+            const float scale = __int_as_float((127 - 7 * qg) << 23);  // 2^(-7 qg)
+            uint32_t r[TC_N];
 #pragma unroll
-          for (int h = 0; h < TC_N / 16; ++h) {
-            uint32_t r[16];
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(qg * TC_N + h * 16);
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-                "[%16];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15])
-                : "r"(taddr));
+            for (int h = 0; h < TC_N / 16; ++h) {
+              uint32_t *v = r + 16 * h;
+              const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(qg * TC_N + h * 16);
+              asm volatile(
+                  "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+                  "[%16];"
+                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                    "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                    "=r"(v[15])
+                  : "r"(taddr));
+            }
             asm volatile("tcgen05.wait::ld.sync.aligned;");
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
+            for (int n = 0; n < TC_N; ++n) asm volatile("" : "+r"(r[n]));  // read only after the wait
+#pragma unroll
+            for (int n = 0; n < TC_N; ++n) {
               // (ah, al) += v: TwoSum into the high part, the error into al
-              const int n = h * 16 + u;
-              const float v = __uint_as_float(r[u]) * scale;
+              const float v = __uint_as_float(r[n]) * scale;
               const float sv = ah[n] + v;
               const float bb = sv - ah[n];
               const float e = (ah[n] - (sv - bb)) + (v - bb);
@@ -756,28 +793,44 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_rk_tc(const TcTile *__restric
             }
           }
         }
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncthreads();  // B
       }
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      __syncthreads();  // B
-    }
-    const int m = warp * 32 + lane;
-    if (*okflag && m < T.fn) {
-      const int f = T.f0 + m;
-      const YDesc y = yd[f];
-      const int ey = eY[f];
+      if (!*okflag) continue;
+      // split s of the contraction: its partial sum (val + s nval), scaled in
+      // the exponent field where the result is a normal number
+      double *out = val + (long long)T.s * nval;
+      bool outside = false, scaled = true;
 #pragma unroll
       for (int n = 0; n < TC_N; ++n) {
         const TcRow rw = trow[n];
-        if (n >= T.rn || f < rw.cs_a) continue;  // padding, or b < a: not a GENINTRK entry
         const long long pos =
             rw.base + (long long)rw.ncA * (y.cs - rw.cs_a) + (long long)rw.ic * y.nd + (long long)(f - y.cs);
-        if (pos < 0 || pos >= nval) {
-          atomicExch(flags, 1);  // position outside the table
-          continue;
-        }
-        // split s of the contraction: its partial sum (val + s nval)
-        val[(long long)T.s * nval + pos] = scalbn((double)ah[n] + (double)al[n], eA[rw.p] + ey - 14);
+        const bool need = valid && n < T.rn && f >= rw.cs_a;  // not padding, nor b < a
+        const bool in = pos >= 0 && pos < nval;
+        const int e = tex[n] + ey;
+        const double v = (double)ah[n] + (double)al[n];
+        const int hi = __double2hiint(v), ex = (hi >> 20) & 0x7ff;
+        const bool zero = ((hi & 0x7fffffff) | __double2loint(v)) == 0;
+        const bool fast = (ex > 0 && ex + e > 0 && ex + e < 2047) || zero;
+        outside |= need && !in;
+        scaled &= !need || fast;
+        if (need && in) out[pos] = zero ? v : __hiloint2double(hi + (e << 20), __double2loint(v));
       }
+      if (!scaled) {
+#pragma unroll 1
+        for (int n = 0; n < T.rn; ++n) {
+          const TcRow rw = trow[n];
+          const long long pos =
+              rw.base + (long long)rw.ncA * (y.cs - rw.cs_a) + (long long)rw.ic * y.nd + (long long)(f - y.cs);
+          double v = 0.0;
+#pragma unroll
+          for (int u = 0; u < TC_N; ++u)
+            if (u == n) v = (double)ah[u] + (double)al[u];
+          if (f >= rw.cs_a && pos >= 0 && pos < nval) out[pos] = scalbn(v, tex[n] + ey);
+        }
+      }
+      if (outside) atomicExch(flags, 1);  // position outside the table
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -1948,8 +2001,8 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
         parts = C.dParts.p;
       }
       if (!C.tcs.empty()) {
-        k_rk_tc<<<(unsigned)C.tcs.size(), TC_THREADS, TC_SMEM, ctx->stream>>>(
-            C.dTcs.p, C.dTcr.p, C.dYt.p, C.dAt.p, nch, C.dEA.p, C.dEY.p, C.dYd.p, parts, (long long)N,
+        k_rk_tc<<<(unsigned)std::min<size_t>(C.tcs.size(), ctx->sms), TC_THREADS, TC_SMEM, ctx->stream>>>(
+            C.dTcs.p, (int)C.tcs.size(), C.dTcr.p, C.dYt.p, C.dAt.p, nch, C.dEA.p, C.dEY.p, C.dYd.p, parts, (long long)N,
             C.dNfb.p + 1, ctx->test_stall_tile);
         ctx->test_stall_tile = -1;  // one call only
         ::gg::note_launch();
