@@ -542,55 +542,113 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
-// Slices of rows into their tile blocks: one CTA per row slot (slot = tile
-// block column g, row m < R); src_row[slot] < 0 pads with zeros. The row's
-// exponent goes to exps[src_row] (the same row always gets the same value).
-template <int R>
-__global__ void k_oz_tile(const double *__restrict__ M, int pitch, int K, int nch, const int *__restrict__ src_row,
-                          int *__restrict__ exps, __half *__restrict__ dst) {
-  constexpr int BLK = OZ_S * 2 * (R / 8) * 2 * 64;
-  const int slot = blockIdx.x, g = slot / R, m = slot % R;
-  const int row = src_row[slot];
-  __shared__ double red[128];
-  double mx = 0.0;
-  if (row >= 0)
-    for (int i = threadIdx.x; i < K; i += blockDim.x) mx = fmax(mx, fabs(M[(size_t)row * pitch + i]));
-  red[threadIdx.x] = mx;
-  __syncthreads();
-  for (int st = 64; st > 0; st >>= 1) {
-    if ((int)threadIdx.x < st) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + st]);
-    __syncthreads();
+// x 2^(35-e) = X1 + d exactly with X1 = rint(x 2^(35-e)), |d| <= 1/2 (|x| <
+// 2^(e-1)), X2 = rint(d 2^35): x = (X1 + X2 2^-35) 2^(e-35) to 2^(e-71),
+// |X1|, |X2| <= 2^34. A normal x on its mantissa in integers (GB300 issues
+// FP64 slowly, and roundings to nearest even need none).
+__device__ __forceinline__ void oz_parts(double x, int e, long long &X1, long long &X2) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+  const int ex = (int)(bits >> 52) & 0x7ff;
+  X1 = X2 = 0;
+  if ((bits << 1) == 0) return;
+  if (ex == 0 || ex == 0x7ff) {
+    const double xs = scalbn(x, 35 - e), x1 = rint(xs);
+    X1 = (long long)x1;
+    X2 = (long long)rint((xs - x1) * 34359738368.0);  // 2^35
+    return;
   }
-  mx = red[0];
-  const int e = (mx > 0.0) ? ilogb(mx) + 2 : 0;  // mx < 2^(e-1)
-  if (threadIdx.x == 0 && row >= 0) exps[row] = e;
-  __half *base = dst + (size_t)g * nch * BLK;
-  const int KP = nch * TC_KC;
-  for (int i = threadIdx.x; i < KP; i += blockDim.x) {
-    // x 2^35 = X1 + d exactly with X1 = rint(x 2^35), |d| <= 1/2 (|x| < 1/2);
-    // X2 = rint(d 2^35); x = (X1 + X2 2^-35) 2^-35 to 2^-71, |X1|, |X2| <= 2^34.
-    // Each of X1 and X2 gives five balanced base-128 digits (|digit| <= 64)
-    // in integer arithmetic: only the two roundings use the FP64 pipe, which
-    // GB300 issues slowly.
-    const double xs = (row >= 0 && i < K) ? scalbn(M[(size_t)row * pitch + i], 35 - e) : 0.0;
-    const double x1 = rint(xs);
-    long long X[2] = {(long long)x1, (long long)rint((xs - x1) * 34359738368.0)};  // 2^35
-    int dg[OZ_S];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      long long v = X[h];
-#pragma unroll
-      for (int u = 4; u >= 1; --u) {
-        const int r = (int)(((v + 64) & 127) - 64);  // balanced remainder in [-64, 63]
-        dg[h * 5 + u] = r;
-        v = (v - r) >> 7;
+  const unsigned long long m = (bits & 0xfffffffffffffull) | (1ull << 52);
+  const int sh = 1040 + e - ex;  // |x| 2^(35 - e) = m 2^-sh < 2^34, so sh is 19 or more
+  // v / 2^s to nearest even, 0 < s <= 53 (v < 2^53: beyond that it rounds to 0)
+  auto div = [](unsigned long long v, int s) {
+    const unsigned long long q = v >> s, r = v & ((1ull << s) - 1), h = 1ull << (s - 1);
+    return q + (r > h || (r == h && (q & 1)));
+  };
+  const unsigned long long q = sh > 53 ? 0 : div(m, sh);
+  const long long d = sh > 53 ? (long long)m : (long long)(m - (q << sh));  // in units of 2^-sh
+  const unsigned long long a = d < 0 ? -d : d;
+  const long long t = sh <= 35 ? (long long)(a << (35 - sh)) : sh - 35 > 53 ? 0 : (long long)div(a, sh - 35);
+  const bool neg = (bits >> 63) != 0;
+  X1 = neg ? -(long long)q : (long long)q;
+  X2 = neg != (d < 0) ? -t : t;
+}
+
+// Slices of rows into their tile blocks: a CTA takes eight row slots (slot =
+// tile block column g, row m < R; src_row[slot] < 0 pads with zeros). A row's
+// exponent goes to exps[src_row] (the same row always gets the same value).
+// A thread takes eight points of a row, a 16-byte unit of the block per
+// slice; the eight rows' units make 128 bytes. Each of oz_parts' X1 and X2
+// gives five balanced base-128 digits (|digit| <= 64).
+// Bound: integer issue (43 subshells, k <= 8: 57 MB written, 35 us; a CTA per
+// row 46 us, and with the parts and the row's largest value in FP64 and 2-byte
+// stores 74 us).
+constexpr int OZ_T = 256;
+template <int R>
+__global__ void __launch_bounds__(OZ_T) k_oz_tile(const double *__restrict__ M, int pitch, int K, int nch,
+                                                  const int *__restrict__ src_row, int *__restrict__ exps,
+                                                  __half *__restrict__ dst) {
+  constexpr int BLK = OZ_S * 2 * (R / 8) * 2 * 64;
+  __shared__ int se[8];
+  const int s0 = blockIdx.x * 8, g = s0 / R, m8 = s0 % R / 8;
+  {
+    const int lane = threadIdx.x & 31, row = src_row[s0 + (threadIdx.x >> 5)];
+    const double *src = M + (size_t)max(row, 0) * pitch;
+    unsigned long long mx = 0;  // the largest |x| but NaN, as its bits
+    if (row >= 0)
+      for (int i = lane; i < K; i += 32) {
+        const unsigned long long v = (unsigned long long)__double_as_longlong(src[i]) & 0x7fffffffffffffffull;
+        if (v > mx && v <= 0x7ff0000000000000ull) mx = v;
       }
-      dg[h * 5] = (int)v;  // |v| <= 64
-    }
-    const int c = i / TC_KC, kk = i % TC_KC, j = kk / 16, k8 = (kk / 8) % 2, el = kk % 8;
-    __half *blk = base + (size_t)c * BLK + ((size_t)(m / 8) * 2 + k8) * 64 + (m % 8) * 8 + el;
 #pragma unroll
-    for (int q = 0; q < OZ_S; ++q) blk[(size_t)(q * 2 + j) * (R / 8) * 2 * 64] = __int2half_rn(dg[q]);
+    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) {
+      const int e = mx ? ilogb(__longlong_as_double((long long)mx)) + 2 : 0;  // mx < 2^(e-1)
+      se[threadIdx.x >> 5] = e;
+      if (row >= 0) exps[row] = e;
+    }
+  }
+  __syncthreads();
+  const int m = threadIdx.x & 7, row = src_row[s0 + m], e = se[m];
+  const double *src = M + (size_t)max(row, 0) * pitch;
+  __half *base = dst + (size_t)g * nch * BLK + (size_t)m8 * 2 * 64 + m * 8;
+  for (int u = threadIdx.x >> 3; u < nch * (TC_KC / 8); u += OZ_T / 8) {
+    const int i0 = 8 * u;
+    uint32_t out[OZ_S][4];  // the unit's digits + 1088 as fp16, two to a word
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        const int i = i0 + 2 * p + w;
+        long long X[2];
+        oz_parts(row >= 0 && i < K ? src[i] : 0.0, e, X[0], X[1]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          long long v = X[h];
+#pragma unroll
+          for (int q = 4; q >= 0; --q) {
+            const int r = q ? (int)(((v + 64) & 127) - 64) : (int)v;  // balanced remainder; at last |v| <= 64
+            const uint32_t c = (uint32_t)(0x6400 + 64 + r);           // fp16 of 1088 + r
+            out[h * 5 + q][p] = w ? out[h * 5 + q][p] | (c << 16) : c;
+            v = (v - r) >> 7;
+          }
+        }
+      }
+    }
+    const int c = u / (TC_KC / 8), j = (u / 2) % 2, k8 = u % 2;
+    __half *blk = base + (size_t)c * BLK + k8 * 64;
+    const __half2 off = __floats2half2_rn(1088.0f, 1088.0f);
+#pragma unroll
+    for (int q = 0; q < OZ_S; ++q) {
+      uint4 o;
+      uint32_t *ow = &o.x;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        __half2 h = *reinterpret_cast<__half2 *>(&out[q][p]);
+        h = __hsub2(h, off);
+        ow[p] = *reinterpret_cast<uint32_t *>(&h);
+      }
+      *reinterpret_cast<uint4 *>(blk + (size_t)(q * 2 + j) * (R / 8) * 2 * 64) = o;
+    }
   }
 }
 
@@ -1958,12 +2016,12 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
       GG_TRY(C.dYt.alloc(std::max<size_t>(1, C.yslot.size() / TC_M * nch * TC_YBLK)));
       GG_TRY(C.dAt.alloc(std::max<size_t>(1, C.aslot.size() / TC_N * nch * TC_ABLK)));
       if (!C.yslot.empty()) {
-        k_oz_tile<TC_M><<<(unsigned)C.yslot.size(), 128, 0, ctx->stream>>>(C.dY.p, np, KC, nch, C.dYslot.p, C.dEY.p,
+        k_oz_tile<TC_M><<<(unsigned)C.yslot.size() / 8, OZ_T, 0, ctx->stream>>>(C.dY.p, np, KC, nch, C.dYslot.p, C.dEY.p,
                                                                           C.dYt.p);
         ::gg::note_launch();
       }
       if (!C.aslot.empty()) {
-        k_oz_tile<TC_N><<<(unsigned)C.aslot.size(), 128, 0, ctx->stream>>>(C.dA.p, KC, KC, nch, C.dAslot.p, C.dEA.p,
+        k_oz_tile<TC_N><<<(unsigned)C.aslot.size() / 8, OZ_T, 0, ctx->stream>>>(C.dA.p, KC, KC, nch, C.dAslot.p, C.dEA.p,
                                                                           C.dAt.p);
         ::gg::note_launch();
       }
