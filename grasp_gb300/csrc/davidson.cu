@@ -597,24 +597,6 @@ __global__ void __launch_bounds__(TPB) k_multbc(const double *__restrict__ X, in
   }
 }
 
-// t = AB_j - lambda_j B_j, partial sums of t^2 for the final residual norms
-__global__ void k_final_res_part(const double *__restrict__ B, const double *__restrict__ AB, int64_t ld, int j,
-                                 double lam, int n, double *__restrict__ part) {
-  __shared__ double s[TPB];
-  double acc = 0.0;
-  for (int i = blockIdx.x * TPB + threadIdx.x; i < n; i += gridDim.x * TPB) {
-    const double t = AB[(size_t)j * ld + i] + (-lam) * B[(size_t)j * ld + i];
-    acc = fma(t, t, acc);
-  }
-  s[threadIdx.x] = acc;
-  __syncthreads();
-  for (int st = TPB / 2; st > 0; st >>= 1) {
-    if ((int)threadIdx.x < st) s[threadIdx.x] += s[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = s[0];
-}
-
 // ---------------------------------------------------------------------------
 // Block Gram-Schmidt for the block pass (MBLOCK > 1). The m new columns
 // kpass .. kpass+m-1 (kpass = pv[0].c on the device) are orthogonalised
@@ -1751,37 +1733,19 @@ struct Dvd {
       note_launches(3);
     }
     GG_CUDA(cudaGetLastError());
-    if (split) {
-      // all m columns in one sweep over the matrix (dropped columns are zero)
-      const int *dcol0 = reinterpret_cast<const int *>(reinterpret_cast<const char *>(dpv.p) + offsetof(IterParams, c));
-      if (in_capture) {
-        GG_CUDA(cudaEventRecordWithFlags(bev[0], s, cudaEventRecordExternal));
-      } else {
-        GG_CUDA(cudaEventRecord(bev[0], s));
-      }
+    // all m columns in one launch between two events (read after the pass):
+    // SPLIT in one sweep over the matrix (dropped columns are zero), FP64 a
+    // grid row per column (dropped columns skipped)
+    const int *dcol0 = reinterpret_cast<const int *>(reinterpret_cast<const char *>(dpv.p) + offsetof(IterParams, c));
+    auto record = [&](cudaEvent_t e) {
+      return in_capture ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s);
+    };
+    GG_CUDA(record(bev[0]));
+    if (split)
       GG_TRY(spmm_block(h, m, bxs.p, B.p, AB.p, ld, dcol0, s));
-      if (in_capture) {
-        GG_CUDA(cudaEventRecordWithFlags(bev[1], s, cudaEventRecordExternal));
-      } else {
-        GG_CUDA(cudaEventRecord(bev[1], s));
-      }
-    }
-    for (int v = 0; v < m && !split; ++v) {
-      const int *dcol = reinterpret_cast<const int *>(reinterpret_cast<const char *>(dpv.p + v) +
-                                                      offsetof(IterParams, c));
-      // each matvec between two events (read after the pass)
-      if (in_capture) {
-        GG_CUDA(cudaEventRecordWithFlags(bev[2 * v], s, cudaEventRecordExternal));
-      } else {
-        GG_CUDA(cudaEventRecord(bev[2 * v], s));
-      }
-      GG_TRY(spmv_col(h, precision, B.p, AB.p, ld, dcol, bskip.p + v, s));
-      if (in_capture) {
-        GG_CUDA(cudaEventRecordWithFlags(bev[2 * v + 1], s, cudaEventRecordExternal));
-      } else {
-        GG_CUDA(cudaEventRecord(bev[2 * v + 1], s));
-      }
-    }
+    else
+      GG_TRY(spmv64_cols(h, m, B.p, AB.p, ld, dcol0, sizeof(IterParams) / sizeof(int), bskip.p, s));
+    GG_CUDA(record(bev[1]));
     if (split) {
       GG_CUDA(launch_pdl(k_bdx_dots<2>, gdx, BD_T, 0, s, B.p, AB.p, Bx.p, ABx.p, ld, dpv.p, m, bst.p, n, bd_cpc, bpx,
                          bd_ps, -1, wx.p));
@@ -1804,7 +1768,7 @@ struct Dvd {
     if (m <= 0) return GG_OK;
     if (m > MT_MAX) return fail(GG_ERR_ARG, "block pass: more new vectors than supported");
     if (bev.empty()) {
-      bev.resize(2 * MT_MAX, nullptr);
+      bev.resize(2, nullptr);
       for (auto &e : bev) GG_CUDA(cudaEventCreate(&e));
     }
     if (!dpv.p) {
@@ -1892,14 +1856,12 @@ struct Dvd {
     if (nk < 0 || nk > m) return fail(GG_ERR_STATE, "block pass: kept column count out of range");
     if (use_x()) cgs_once += hout_bst()[2];
     std::memcpy(S.data() + o0, hout_scol(), (o1 - o0) * sizeof(double));
-    for (int v = 0; v < (use_x() ? 1 : m); ++v) {
-      float ms = 0.f;
-      GG_CUDA(cudaEventElapsedTime(&ms, bev[2 * v], bev[2 * v + 1]));
-      mv_ms += ms;
-      if (use_x() && m == full_m) {
-        spmm_full_ms += ms;
-        ++spmm_full_n;
-      }
+    float ms = 0.f;
+    GG_CUDA(cudaEventElapsedTime(&ms, bev[0], bev[1]));
+    mv_ms += ms;
+    if (use_x() && m == full_m) {
+      spmm_full_ms += ms;
+      ++spmm_full_n;
     }
     nmv += nk;
     mv_count += nk;
@@ -2182,7 +2144,7 @@ struct Dvd {
     GG_CUDA(cudaMemcpyAsync(X.p, T.p, (size_t)m * ld * sizeof(double), cudaMemcpyDeviceToDevice, s));
     return GG_OK;
   }
-  // BASIS and AB both times C (OVFLOW's restart, the final eigenvectors)
+  // BASIS and AB both times C (OVFLOW's restart)
   int multbc2(int k, int m, const double *hC) {
     GG_TRY(multbc(B, Bx, k, m, hC));
     GG_TRY(multbc(AB, ABx, k, m, hC));
@@ -2209,16 +2171,6 @@ struct Dvd {
     GG_CUDA(cudaGetLastError());
     return GG_OK;
   }
-  double host_sum_sqrt(int np) {
-    std::vector<double> hp(np);
-    cudaMemcpyAsync(hp.data(), part.p, np * sizeof(double), cudaMemcpyDeviceToHost, s);
-    const auto t0 = std::chrono::steady_clock::now();
-    cudaStreamSynchronize(s);
-    t_wait += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-    double a = 0.0;
-    for (int i = 0; i < np; ++i) a += hp[i];
-    return std::sqrt(a);
-  }
 };
 
 struct DvdParams {
@@ -2230,8 +2182,7 @@ struct DvdParams {
 // DVDSON for ILOW = 1, IHIGH = NUME; BASIS columns 0..niv-1 hold the initial
 // estimates on entry. On exit BASIS[:, 0:nume) are the eigenvectors and
 // eigval[0:nume] the eigenvalues.
-int dvdson(Dvd &D, const DvdParams &P, std::vector<double> &eigval_out, std::vector<double> &resid_out, int *nloops_out,
-           int *ierr_out) {
+int dvdson(Dvd &D, const DvdParams &P, std::vector<double> &eigval_out, int *nloops_out, int *ierr_out) {
   const int n = D.n, LIM = P.lim, NUME = P.nume, MBLOCK = P.mblock, MAXITER = P.maxiter;
   int NIV = P.niv;
   int IERR = 0;
@@ -2545,14 +2496,9 @@ int dvdson(Dvd &D, const DvdParams &P, std::vector<double> &eigval_out, std::vec
   }
   // label 30 (dvdson.f90:821-836)
   for (int i = 0; i < NUME; ++i) OLDVAL[i] = std::fabs(OLDVAL[i] - EIGVAL[i]);
-  GG_TRY(D.multbc2(KPASS, NUME, SVEC.data()));
-  resid_out.assign(NUME, 0.0);
-  for (int i = 0; i < NUME; ++i) {
-    const int nb = std::min((n + TPB - 1) / TPB, 1024);
-    k_final_res_part<<<nb, TPB, 0, D.s>>>(D.B.p, D.AB.p, D.ld, i, EIGVAL[i], n, D.part.p); ::gg::note_launch();
-    GG_CUDA(cudaGetLastError());
-    resid_out[i] = D.host_sum_sqrt(nb);
-  }
+  // (the eigenvectors; DVDSON's AB and residual norms at this point have no reader)
+  GG_TRY(D.multbc(D.B, D.Bx, KPASS, NUME, SVEC.data()));
+  D.bx_cols = 0;
   eigval_out.assign(EIGVAL.begin(), EIGVAL.begin() + NUME);
   *nloops_out = NLOOPS;
   *ierr_out = IERR;
@@ -2669,7 +2615,7 @@ extern "C" int gg_maneig(gg_ctx *ctx, gg_hmat *h, int nvec, const gg_dvd_params 
   using hclock = std::chrono::steady_clock;
   const auto th0 = hclock::now();
   GG_TRY(refresh_sym_values(h));
-  std::vector<double> ev, res;
+  std::vector<double> ev;
   double mv_ms = 0;
   int mv_count = 0, nmv_total = 0, nl_total = 0;
   // Stage 1 (INIEST2, lib9290/iniest2.f90:49-95): lowest eigenvectors of the
@@ -2770,7 +2716,7 @@ extern "C" int gg_maneig(gg_ctx *ctx, gg_hmat *h, int nvec, const gg_dvd_params 
       GG_TRY(unit_start(D1, blk, P1.niv));
     }
     int nl = 0, ie = 0;
-    GG_TRY(dvdson(D1, P1, ev, res, &nl, &ie));
+    GG_TRY(dvdson(D1, P1, ev, &nl, &ie));
     mv_ms += D1.mv_ms;
     mv_count += D1.mv_count;
     nmv_total += D1.nmv;
@@ -2800,7 +2746,7 @@ extern "C" int gg_maneig(gg_ctx *ctx, gg_hmat *h, int nvec, const gg_dvd_params 
                                 ctx->stream));
     }
     int nl = 0, ie = 0;
-    GG_TRY(dvdson(D2, P2, ev, res, &nl, &ie));
+    GG_TRY(dvdson(D2, P2, ev, &nl, &ie));
     mv_ms += D2.mv_ms;
     mv_count += D2.mv_count;
     nmv_total += D2.nmv;

@@ -294,6 +294,8 @@ int spmv(gg_hmat *h, int precision, const double *dx, double *dy, int m, cudaStr
 // xs: the split (hi + lo FP32) copy of x to read; null = the matrix's dXs
 int spmv_col(gg_hmat *h, int precision, const double *Bbase, double *ABbase, int64_t ld, const int *dcol,
              const double *skip, cudaStream_t s, const float2 *xs = nullptr);
+int spmv64_cols(gg_hmat *h, int m, const double *Bbase, double *ABbase, int64_t ld, const int *dcol, int dstride,
+                const double *skip, cudaStream_t s);
 // Row pitch (in float2) of the interleaved split copies of m vectors that the
 // block matvec reads: m rounded up to a power of two (at least 2), so that a
 // row is whole 16-byte pieces and never straddles a 128-byte line.

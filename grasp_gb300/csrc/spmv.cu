@@ -281,15 +281,18 @@ __global__ void __launch_bounds__(256) k_spmv_split(const int64_t *__restrict__ 
 // Column-indexed forms for the Davidson iteration graph: x = Bbase + c ld,
 // y = ABbase + c ld with c read from device memory at run time; nothing is
 // done when skip points to a non-zero flag. The split form reads x from its
-// hi+lo copy, which the caller prepared.
+// hi+lo copy, which the caller prepared. k_spmv64_col: grid row v takes the
+// v-th c (pcs ints apart) and flag, so the columns of a block pass share a
+// launch (361 CSFs, three columns: 6 us; a launch per column between its own
+// events 3 x 5 us, and the events).
 __global__ void __launch_bounds__(256) k_spmv64_col(const int64_t *__restrict__ ptr, const int32_t *__restrict__ col,
                                                     const double *__restrict__ val, const double *__restrict__ Bbase,
                                                     double *__restrict__ ABbase, int64_t ld,
-                                                    const int *__restrict__ pc, const double *skip, int n) {
-  if (skip && *skip != 0.0) return;
+                                                    const int *__restrict__ pc, int pcs, const double *skip, int n) {
+  if (skip && skip[blockIdx.y] != 0.0) return;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (row >= n) return;
-  const size_t off = (size_t)(*pc) * ld;
+  const size_t off = (size_t)pc[blockIdx.y * pcs] * ld;
   const double *x = Bbase + off;
   const int64_t lo = ptr[row], hi = ptr[row + 1];
   double acc = 0.0;
@@ -625,21 +628,26 @@ int check_precision(const gg_hmat *h, int precision) {
 // GG_SPLIT reads x from h->dXs (the caller's split copy of the same column)
 int spmv_col(gg_hmat *h, int precision, const double *Bbase, double *ABbase, int64_t ld, const int *dcol,
              const double *skip, cudaStream_t s, const float2 *xs) {
+  if (precision != GG_SPLIT) return spmv64_cols(h, 1, Bbase, ABbase, ld, dcol, 0, skip, s);
   GG_TRY(check_precision(h, precision));
+  if (!xs) {
+    if (h->dXs.n < (size_t)h->ncf) return fail(GG_ERR_STATE, "spmv_col: split copy of x not allocated");
+    xs = h->dXs.p;
+  }
+  int v = 0;
+  GG_TRY(tune_variant(h, 1, 1, s, &v));
+  return launch_spmv(h, v, xs, nullptr, nullptr, Bbase, ABbase, ld, dcol, skip, true, s);
+}
+
+// the FP64 form for m columns: the v-th reads c from dcol[v dstride], its flag from skip[v]
+int spmv64_cols(gg_hmat *h, int m, const double *Bbase, double *ABbase, int64_t ld, const int *dcol, int dstride,
+                const double *skip, cudaStream_t s) {
+  GG_TRY(check_precision(h, GG_FP64));
   const int n = h->ncf;
   const unsigned blocks = (unsigned)(((int64_t)n * 32 + 255) / 256);
-  if (precision == GG_SPLIT) {
-    if (!xs) {
-      if (h->dXs.n < (size_t)n) return fail(GG_ERR_STATE, "spmv_col: split copy of x not allocated");
-      xs = h->dXs.p;
-    }
-    int v = 0;
-    GG_TRY(tune_variant(h, 1, 1, s, &v));
-    return launch_spmv(h, v, xs, nullptr, nullptr, Bbase, ABbase, ld, dcol, skip, true, s);
-  } else {
-    k_spmv64_col<<<blocks, 256, 0, s>>>(h->dSymPtr.p, h->dSymCol.p, h->dSymVal.p, Bbase, ABbase, ld, dcol, skip, n);
-    ::gg::note_launch();
-  }
+  k_spmv64_col<<<dim3(blocks, m), 256, 0, s>>>(h->dSymPtr.p, h->dSymCol.p, h->dSymVal.p, Bbase, ABbase, ld, dcol,
+                                               dstride, skip, n);
+  ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
   return GG_OK;
 }
