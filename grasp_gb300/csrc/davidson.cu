@@ -618,11 +618,12 @@ constexpr int BD_PAIRS = (BD_AC * MT_MAX + BD_T - 1) / BD_T;
 template <int MODE>
 __global__ void __launch_bounds__(BD_T) k_bd_dots(const double *__restrict__ B, const double *__restrict__ AB,
                                                   int64_t ld, const IterParams *__restrict__ pv, int m,
-                                                  const int *__restrict__ bst, int n, int cpc,
+                                                  const int *__restrict__ bst, int n, int cpc, int acw,
                                                   double *__restrict__ part, int ps) {
   pdl_wait();
   __shared__ double Bs[BD_R * MT_MAX];       // [i][q]
   __shared__ double As[BD_R * (BD_AC + 1)];  // [i][a]
+  __shared__ double odd[BD_T / 2];
   const int kpass = pv[0].c;
   const int nb = (MODE == 0) ? m : bst[0];
   if (nb <= 0) return;
@@ -632,22 +633,40 @@ __global__ void __launch_bounds__(BD_T) k_bd_dots(const double *__restrict__ B, 
   const double *Xb = B + (size_t)a0 * ld;
   double *out = part + (size_t)blockIdx.x * ps;
   const int rbeg = blockIdx.x * cpc * BD_R, rend = min(n, rbeg + cpc * BD_R);
-  for (int ac = blockIdx.y * BD_AC; ac < na; ac += gridDim.y * BD_AC) {
-    const int nac = min(BD_AC, na - ac), np = nac * nb;
+  for (int ac = blockIdx.y * acw; ac < na; ac += gridDim.y * acw) {
+    const int nac = min(acw, na - ac), np = nac * nb;
+    // the two sums of a pair are chains of 32 dependent FMAs per chunk: with
+    // few pairs a warp takes the even rows' sums of 32 pairs and the next
+    // warp, on another sub-partition, the odd rows'
+    const bool halves = np <= BD_T / 2;
+    const int hp = (threadIdx.x >> 6) * 32 + (threadIdx.x & 31), par = (threadIdx.x >> 5) & 1;
     double acc[BD_PAIRS];
 #pragma unroll
     for (int k = 0; k < BD_PAIRS; ++k) acc[k] = 0.0;
     for (int r0 = rbeg; r0 < rend; r0 += BD_R) {
       const int nr = min(BD_R, rend - r0);
-      for (int idx = threadIdx.x; idx < nr * nb; idx += BD_T) {
-        const int i = idx % nr, q = idx / nr;
-        Bs[i * MT_MAX + q] = Wb[(size_t)q * ld + r0 + i];
+      for (int idx = threadIdx.x; idx < BD_R * nb; idx += BD_T) {
+        const int i = idx % BD_R, q = idx / BD_R;
+        if (i < nr) Bs[i * MT_MAX + q] = Wb[(size_t)q * ld + r0 + i];
       }
-      for (int idx = threadIdx.x; idx < nr * nac; idx += BD_T) {
-        const int i = idx % nr, a = idx / nr;
-        As[i * (BD_AC + 1) + a] = Xb[(size_t)(ac + a) * ld + r0 + i];
+      for (int idx = threadIdx.x; idx < BD_R * nac; idx += BD_T) {
+        const int i = idx % BD_R, a = idx / BD_R;
+        if (i < nr) As[i * (BD_AC + 1) + a] = Xb[(size_t)(ac + a) * ld + r0 + i];
       }
       __syncthreads();
+      if (halves) {
+        double sum = 0.0;
+        if (hp < np) {
+          const int a = hp % nac, q = hp / nac;
+#pragma unroll 8
+          for (int i = par; i < nr; i += 2) sum = fma(As[i * (BD_AC + 1) + a], Bs[i * MT_MAX + q], sum);
+          if (par) odd[hp] = sum;
+        }
+        __syncthreads();
+        if (!par && hp < np) acc[0] += sum + odd[hp];
+        __syncthreads();
+        continue;
+      }
 #pragma unroll
       for (int k = 0; k < BD_PAIRS; ++k) {
         const int pr = threadIdx.x + k * BD_T;
@@ -667,7 +686,7 @@ __global__ void __launch_bounds__(BD_T) k_bd_dots(const double *__restrict__ B, 
     }
 #pragma unroll
     for (int k = 0; k < BD_PAIRS; ++k) {
-      const int pr = threadIdx.x + k * BD_T;
+      const int pr = halves ? (k || par ? np : hp) : (int)threadIdx.x + k * BD_T;
       if (pr < np) out[(ac + pr % nac) * nb + pr / nac] = acc[k];
     }
   }
@@ -901,7 +920,11 @@ __global__ void __launch_bounds__(BD_RED) k_bd_chol(int m, int *__restrict__ bst
 
 
 // new columns minus their projections: B(:, kpass+q) -= B(:, 0:kpass) C(:, q)
+// A row's sum is a chain over the columns, whose loads go out BD_PF columns
+// ahead of their FMAs (361 CSFs, 60 columns: 5.3 us; 6.7 us when each group
+// of four waited for its own loads).
 constexpr int BD_CCH = 64;  // rows of C staged per step
+constexpr int BD_PF = 8;
 // (columns q0 = blockIdx.y M .. q0 + M of the m; C row a at a m)
 template <int M>
 __global__ void __launch_bounds__(RT) k_bd_sub(double *__restrict__ B, int64_t ld, const IterParams *__restrict__ pv,
@@ -919,11 +942,22 @@ __global__ void __launch_bounds__(RT) k_bd_sub(double *__restrict__ B, int64_t l
     for (int idx = threadIdx.x; idx < na * M; idx += RT) Cs[idx] = C[(size_t)(a0 + idx / M) * m + q0 + idx % M];
     __syncthreads();
     if (i < n) {
-#pragma unroll 4
-      for (int a = 0; a < na; ++a) {
-        const double v = B[(size_t)(a0 + a) * ld + i];
+      const double *b = B + (size_t)a0 * ld + i;
+      double v[BD_PF], w[BD_PF];  // the columns at hand, those loaded ahead
 #pragma unroll
-        for (int q = 0; q < M; ++q) acc[q] = fma(v, Cs[a * M + q], acc[q]);
+      for (int u = 0; u < BD_PF; ++u) w[u] = u < na ? b[(size_t)u * ld] : 0.0;
+      for (int a = 0; a < na; a += BD_PF) {
+#pragma unroll
+        for (int u = 0; u < BD_PF; ++u) {
+          v[u] = w[u];
+          w[u] = a + BD_PF + u < na ? b[(size_t)(a + BD_PF + u) * ld] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < BD_PF; ++u) {
+          if (a + u >= na) break;
+#pragma unroll
+          for (int q = 0; q < M; ++q) acc[q] = fma(v[u], Cs[(a + u) * M + q], acc[q]);
+        }
       }
     }
   }
@@ -1674,7 +1708,12 @@ struct Dvd {
     const bool sub_split = (int64_t)nrow * 2 < ctx->sms;  // small blocks: one column per grid row
     // the split kernels' CTA partials are double-float pairs in the same buffer
     float2 *bpx = reinterpret_cast<float2 *>(bpart.p);
-    const dim3 gd(bd_G, bd_Y);
+    // columns per grid row: where SMs are idle as few as make 64 pairs, one
+    // chain per sub-partition (361 CSFs, three columns: 6.3 us; 7.8 with
+    // BD_AC columns and both chains of a pair in one thread)
+    int acw = std::max(1, 64 / m);
+    if (acw > BD_AC || (int64_t)bd_G * ((lim + acw - 1) / acw) > ctx->sms) acw = BD_AC;
+    const dim3 gd(bd_G, acw == BD_AC ? bd_Y : (lim + acw - 1) / acw);
     // split dots: chunks of max(1, BD_T / m) columns (one pair per thread)
     const dim3 gdx(bd_G, (lim + std::min(BD_AC, std::max(1, BD_T / m)) - 1) / std::min(BD_AC, std::max(1, BD_T / m)));
     for (int round = 0; round < 2; ++round) {
@@ -1686,7 +1725,7 @@ struct Dvd {
         GG_CUDA(launch_pdl(k_bd_reduce<0, float2>, nred, BD_T, 0, s, dpv.p, m, bst.p, bpx, bd_ps, bd_G, bC.p, dS.p,
                            round == 0, round));
       } else {
-        GG_CUDA(launch_pdl(k_bd_dots<0>, gd, BD_T, 0, s, B.p, AB.p, ld, dpv.p, m, bst.p, n, bd_cpc, bpart.p, bd_ps));
+        GG_CUDA(launch_pdl(k_bd_dots<0>, gd, BD_T, 0, s, B.p, AB.p, ld, dpv.p, m, bst.p, n, bd_cpc, acw, bpart.p, bd_ps));
         GG_CUDA(launch_pdl(k_bd_reduce<0, double>, nred, BD_T, 0, s, dpv.p, m, bst.p, bpart.p, bd_ps, bd_G, bC.p, dS.p,
                            round == 0, -1));
       }
@@ -1726,7 +1765,7 @@ struct Dvd {
         GG_CUDA(launch_pdl(k_bdx_apply, nrow, RT, 0, s, B.p, ld, dpv.p, bst.p, bC.p, n, round == 1 ? bxs.p : nullptr,
                                         spmm_pitch(m), Bx.p, wx.p));
       } else {
-        GG_CUDA(launch_pdl(k_bd_dots<1>, dim3(bd_G, 1), BD_T, 0, s, B.p, AB.p, ld, dpv.p, m, bst.p, n, bd_cpc, bpart.p, bd_ps));
+        GG_CUDA(launch_pdl(k_bd_dots<1>, dim3(bd_G, 1), BD_T, 0, s, B.p, AB.p, ld, dpv.p, m, bst.p, n, bd_cpc, BD_AC, bpart.p, bd_ps));
         GG_CUDA(launch_pdl(k_bd_chol<double>, 1, BD_RED, 0, s, m, bst.p, bpart.p, bd_ps, bd_G, bC.p, bskip.p, round));
         GG_CUDA(launch_pdl(k_bd_apply, nrow, RT, 0, s, B.p, ld, dpv.p, bst.p, bC.p, n, nullptr, spmm_pitch(m), Bx.p));
       }
@@ -1752,7 +1791,7 @@ struct Dvd {
       GG_CUDA(launch_pdl(k_bd_reduce<2, float2>, nred, BD_T, 0, s, dpv.p, m, bst.p, bpx, bd_ps, bd_G, bC.p,
                          dout_scol(), 0, -1));
     } else {
-      GG_CUDA(launch_pdl(k_bd_dots<2>, gd, BD_T, 0, s, B.p, AB.p, ld, dpv.p, m, bst.p, n, bd_cpc, bpart.p, bd_ps));
+      GG_CUDA(launch_pdl(k_bd_dots<2>, gd, BD_T, 0, s, B.p, AB.p, ld, dpv.p, m, bst.p, n, bd_cpc, acw, bpart.p, bd_ps));
       GG_CUDA(launch_pdl(k_bd_reduce<2, double>, nred, BD_T, 0, s, dpv.p, m, bst.p, bpart.p, bd_ps, bd_G, bC.p,
                          dout_scol(), 0, -1));
     }
