@@ -2208,7 +2208,7 @@ static int run_rinti(gg_ctx *ctx, const std::vector<int2> &jk, int mode, double 
 }
 
 // YPOT / XPOT on the device: the list's distinct Y^k_ab (every grid point,
-// YZK's TB), then k_potential. A list as the caller passed it: YPOT labels
+// YZK's TB), then k_pot_part and k_pot_final. A list as the caller passed it: YPOT labels
 // NYA = (IOY2 KEY + IOY1) KEY + K, XPOT labels NXA = ((IORB KEY + IOY2) KEY +
 // IOY1) KEY + K, and their coefficients.
 struct RawList {
