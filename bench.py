@@ -634,7 +634,10 @@ def setcof_leg(ctx, H, w, vec, cpu=True):
         ref = o.setcof(blk, True, 5, 2.0)
         dt = time.perf_counter() - t0
         same = all(np.array_equal(got[4][k], ref[k]) for k in ref)
-        out["cpu_oracle"] = {"one_orbital_s": dt, "all_orbitals_s_1core": dt * nw, "identical_lists": bool(same)}
+        out["cpu_oracle"] = {"one_orbital_s": dt, "all_orbitals_s_1core": dt * nw, "identical_lists": bool(same),
+                             "max_rel_diff": max([float(np.abs(got[4][k] - ref[k]).max() / np.abs(ref[k]).max())
+                                                  for k in ("ya", "xa", "da") if len(ref[k])
+                                                  and len(ref[k]) == len(got[4][k])], default=None)}
         t0 = time.perf_counter()
         yp0, xp0, xq0 = o.cofpot(5, ucf[4], got[4])
         out["cpu_oracle"]["cofpot_one_orbital_s"] = time.perf_counter() - t0

@@ -107,8 +107,8 @@ int gg_rkintc(gg_ctx *ctx, int ia, int ib, int ic, int id, int k, double *tegral
 int gg_slater(gg_ctx *ctx, int ia, int ib, int ic, int id, int k, double *out);
 /* ---- SCF potentials from the Y^k functions (rmcdhf) ------------------------
  * The Y^k_ab functions of YZK (lib9290/yzk.f90:3: TB(1:N), every grid point),
- * built on the device for a coefficient list of SETCOF and combined in the
- * list's order, each grid point's operations those of the reference loop.
+ * built on the device for a coefficient list of SETCOF and combined in sums
+ * of a fixed order (the reference's values to rounding).
  * gg_ypot: YPOT(J) (rmcdhf90/ypot.f90:35-49), the direct potential
  *   yp[i-1] = ZZ(i) - sum_t ya[t] Y^K_{IOY1 IOY2}(r_i), i = 1..N;
  *   nya[t] = (IOY2 * 215 + IOY1) * 215 + K (rmcdhf's NYA, KEY = KEYORB).
@@ -161,8 +161,8 @@ typedef struct {
  * stay with the context until the next call.
  * gg_setcof: SETCOF(EOL, J)'s lists for orbital j with UCF(J) = ucfj, from
  * the prepared sums: YPOT's (*ny, nya, ya), XPOT's (*nx, nxa, xa) and
- * DACON's (*nd, nda, da), entry for entry the reference's (its order and
- * its merging of repeated labels across blocks). Each output array holds
+ * DACON's (*nd, nda, da), the reference's entries in its order, repeated
+ * labels merged across blocks as it does, the sums to rounding. Each output array holds
  * cap entries; GG_ERR_RANGE (with the counts set) when a list is longer.   */
 int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *nev, const double *const *evec,
                       const double *const *wt, int eol);
@@ -181,7 +181,9 @@ int gg_setlag(gg_ctx *ctx, int nec, const int32_t *iecc, const double *ucf, cons
  * |E(a) - E(b)| / C (bessel.f90:88) from the orbital energies e[nw] (orb_C's
  * E) and WFACT (bess_C; 1 is rci's default, 0 the zero-frequency limit);
  * accy: ACCY (<= 0: H^6). *nb_out = NB, *j2max_out = J2MAX. The table stays
- * with the context (one per type).
+ * with the context (one per type), on the device until it is read. Its
+ * integrals are sums of the reference's terms regrouped by pairs of orbitals
+ * (1e-13 of the largest value); gg_brintf keeps the reference's order.
  * BRINTF is evaluated from its arguments alone: where the reference skips a
  * BESSEL call for two equal orbitals and reads its slot's earlier content
  * (brintf.f90:47-48), the zero-frequency function (zero) is used.
@@ -401,8 +403,8 @@ int gg_maneig_batched(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *nv
  * 30 block passes of the last split gg_maneig whose second Gram-Schmidt
  * pass was skipped (the first kept at least half of every new column's
  * squared norm), 31 device and host ms of the last gg_genintbreit, 32 / 33
- * its host ms enumerating the integrals and their terms / its device ms of
- * the Bessel, term and combination kernels.                                                            */
+ * its host ms from the table's planning to its last launch (one wait for the
+ * kernels in it) / its device ms of the Bessel and table kernels.                                                            */
 double gg_stage_stat(gg_ctx *ctx, int which);
 
 /* gg_projected_eig: DVDSON's projected eigenproblem, CALL DSPEVX('Vectors
