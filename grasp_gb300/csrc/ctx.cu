@@ -26,6 +26,10 @@ int timer_start(gg_ctx *ctx) {
 }
 int timer_stop(gg_ctx *ctx, double *ms) {
   GG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
+  return timer_read(ctx, ms);
+}
+// the time to an ev1 recorded before, whose work the caller has waited for or waits for here
+int timer_read(gg_ctx *ctx, double *ms) {
   GG_CUDA(cudaEventSynchronize(ctx->ev1));
   float f = 0.f;
   GG_CUDA(cudaEventElapsedTime(&f, ctx->ev0, ctx->ev1));
@@ -290,21 +294,25 @@ int gg_set_orbitals(gg_ctx *ctx, int nw, int ld, const int *nak, const int *mf, 
   }
   // device copies with ld rounded up so that each orbital starts 64-byte aligned
   const int ldd = (n + GPAD + 7) / 8 * 8;
-  std::vector<double> hp((size_t)nw * ldd, 0.0), hq((size_t)nw * ldd, 0.0);
-  for (int j = 0; j < nw; ++j)
-    for (int i = 0; i < n; ++i) {
-      hp[(size_t)j * ldd + i] = pf[(size_t)j * ld + i];
-      hq[(size_t)j * ldd + i] = qf[(size_t)j * ld + i];
-    }
+  // (PF, QF, MF and NAK lie in dPF's buffer: one copy)
+  const size_t half = (size_t)nw * ldd;
+  std::vector<double> h(2 * half + nw + 1, 0.0);
+  for (int j = 0; j < nw; ++j) {
+    std::memcpy(&h[(size_t)j * ldd], pf + (size_t)j * ld, n * sizeof(double));
+    std::memcpy(&h[half + (size_t)j * ldd], qf + (size_t)j * ld, n * sizeof(double));
+  }
+  std::memcpy(&h[2 * half], o.mf.data(), (nw + 1) * sizeof(int));
+  std::memcpy(reinterpret_cast<int *>(&h[2 * half]) + nw + 1, o.nak.data(), (nw + 1) * sizeof(int));
   o.ld = ldd;
-  GG_TRY(o.dPF.alloc(hp.size()));
-  GG_TRY(o.dQF.alloc(hq.size()));
-  GG_CUDA(cudaMemcpy(o.dPF.p, hp.data(), hp.size() * 8, cudaMemcpyHostToDevice));
-  GG_CUDA(cudaMemcpy(o.dQF.p, hq.data(), hq.size() * 8, cudaMemcpyHostToDevice));
-  GG_TRY(o.dMF.alloc(nw + 1));
-  GG_TRY(o.dNAK.alloc(nw + 1));
-  GG_CUDA(cudaMemcpy(o.dMF.p, o.mf.data(), (nw + 1) * sizeof(int), cudaMemcpyHostToDevice));
-  GG_CUDA(cudaMemcpy(o.dNAK.p, o.nak.data(), (nw + 1) * sizeof(int), cudaMemcpyHostToDevice));
+  if (const int st = o.dPF.alloc(h.size())) {
+    o.nw = 0;  // no orbitals: the others' pointers lay in the buffer that is gone
+    return st;
+  }
+  o.dQF.p = o.dPF.p + half;
+  o.dMF.p = reinterpret_cast<int *>(o.dPF.p + 2 * half);
+  o.dNAK.p = o.dMF.p + nw + 1;
+  o.dQF.own = o.dMF.own = o.dNAK.own = false;
+  GG_CUDA(cudaMemcpy(o.dPF.p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
   ctx->rk.valid = false;
   ctx->iab_valid = false;
   return GG_OK;

@@ -136,7 +136,7 @@ struct Orbitals {
   int nw = 0, ld = 0;
   std::vector<int> nak, mf, nkl, nkj;   // 1-based host copies
   DBuf<double> dPF, dQF;                // [nw][ld]
-  DBuf<int> dMF, dNAK;                  // 1-based
+  DBuf<int> dMF, dNAK;                  // 1-based; these and dQF lie in dPF's buffer
 };
 
 // GENINTBREIT1/2's tables (breit.cu): type 1 and type 2
@@ -282,6 +282,7 @@ int ensure_orbitals(gg_ctx *ctx);
 // timing helpers (ctx.cu)
 int timer_start(gg_ctx *ctx);
 int timer_stop(gg_ctx *ctx, double *ms);
+int timer_read(gg_ctx *ctx, double *ms);
 // spmv.cu
 int build_sym(gg_hmat *h);
 // setham.cu: CLRX (lib9290/clrx.f90) on the host

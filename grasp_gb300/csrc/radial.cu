@@ -1304,11 +1304,11 @@ __global__ void k_setlag_final(int np_, const int4 *__restrict__ pj, const doubl
   }
 }
 
-// RINTI (lib9290/rinti.f90:53-100) for a list of (J, K) pairs: one block of
+// RINTI (lib9290/rinti.f90:53-100) for a list of (J, K, place) entries: one block of
 // four warps each, the four integrands formed by all threads, one QUAD per warp.
 constexpr int RINTI_WARPS = 4;
 __host__ __device__ constexpr size_t rinti_smem(int np) { return (size_t)RINTI_WARPS * (np + np / 4 + 4); }  // doubles
-__global__ void __launch_bounds__(32 * RINTI_WARPS) k_rinti(const int2 *__restrict__ jk, int npairs, int mode,
+__global__ void __launch_bounds__(32 * RINTI_WARPS) k_rinti(const int4 *__restrict__ jk, int npairs, int mode,
                                                            const double *__restrict__ PF,
                                                            const double *__restrict__ QF, int ld,
                                                            const int *__restrict__ MF, const int *__restrict__ NAK,
@@ -1316,7 +1316,7 @@ __global__ void __launch_bounds__(32 * RINTI_WARPS) k_rinti(const int2 *__restri
                                                            const double *__restrict__ RP,
                                                            const double *__restrict__ RPOR,
                                                            const double *__restrict__ ZZ, int np, QuadConst q,
-                                                           double *__restrict__ out, const int *__restrict__ outidx) {
+                                                           double *__restrict__ out) {
   extern __shared__ double sm[];
   __shared__ double piece[RINTI_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1352,7 +1352,7 @@ __global__ void __launch_bounds__(32 * RINTI_WARPS) k_rinti(const int2 *__restri
       piece[warp] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) out[outidx ? outidx[it] : it] = piece[0] + piece[1] + piece[2] + piece[3];
+    if (threadIdx.x == 0) out[jk[it].z] = piece[0] + piece[1] + piece[2] + piece[3];
   }
 }
 
@@ -2091,9 +2091,11 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
     GG_CUDA(cudaGetLastError());
   }
   int hfb[3] = {0, 0, 0};
+  GG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
   GG_CUDA(cudaMemcpyAsync(hfb, C.dNfb.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  GG_CUDA(cudaStreamSynchronize(ctx->stream));
   double ms = 0;
-  GG_TRY(timer_stop(ctx, &ms));  // waits for all of it
+  GG_TRY(timer_read(ctx, &ms));
   ctx->stats[0] = ms;
   if (hfb[1]) return fail(GG_ERR_STATE, "genintrk: contraction produced a table position out of range");
   if (hfb[2] == 1)
@@ -2657,17 +2659,16 @@ extern "C" {
 static int run_rinti(gg_ctx *ctx, const std::vector<int2> &jk, int mode, double *dOut, const std::vector<int> *outidx) {
   Orbitals &o = ctx->orb;
   Grid &g = ctx->grid;
-  DBuf<int2> djk;
-  DBuf<int> didx;
-  GG_TRY(upload(djk, jk, ctx->stream));
-  if (outidx) GG_TRY(upload(didx, *outidx, ctx->stream));
+  std::vector<int4> h(jk.size());
+  for (size_t i = 0; i < jk.size(); ++i) h[i] = make_int4(jk[i].x, jk[i].y, outidx ? (*outidx)[i] : (int)i, 0);
+  DBuf<int4> djk;  // freed in stream order
+  GG_TRY(upload(djk, h, ctx->stream));
   const size_t smem = rinti_smem(g.np) * sizeof(double);
   const int blocks = std::max(1, std::min((int)jk.size(), 2048));
   k_rinti<<<blocks, 32 * RINTI_WARPS, smem, ctx->stream>>>(djk.p, (int)jk.size(), mode, o.dPF.p, o.dQF.p, o.ld, o.dMF.p,
-                                                   o.dNAK.p, g.dR.p, g.dRP.p, g.dRPOR.p, g.dZZ.p, g.np, g.q, dOut,
-                                                   outidx ? didx.p : nullptr); ::gg::note_launch();
+                                                   o.dNAK.p, g.dR.p, g.dRP.p, g.dRPOR.p, g.dZZ.p, g.np, g.q, dOut);
+  ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
-  GG_CUDA(cudaStreamSynchronize(ctx->stream));
   return GG_OK;
 }
 
@@ -2702,11 +2703,14 @@ int gg_iabint_table(gg_ctx *ctx, double *iab) {
         idx.push_back((a - 1) * nw + (b - 1));
       }
   if (!jk.empty()) GG_TRY(run_rinti(ctx, jk, 0, ctx->dIab.p, &idx));
+  GG_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
+  if (iab)
+    GG_CUDA(cudaMemcpyAsync(iab, ctx->dIab.p, (size_t)nw * nw * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  GG_CUDA(cudaStreamSynchronize(ctx->stream));
   double ms = 0;
-  GG_TRY(timer_stop(ctx, &ms));
+  GG_TRY(timer_read(ctx, &ms));
   ctx->stats[1] = ms;
   ctx->iab_valid = true;
-  if (iab) GG_CUDA(cudaMemcpy(iab, ctx->dIab.p, (size_t)nw * nw * sizeof(double), cudaMemcpyDeviceToHost));
   return GG_OK;
 }
 
