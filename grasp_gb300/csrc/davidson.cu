@@ -925,12 +925,20 @@ __global__ void __launch_bounds__(BD_RED) k_bd_chol(int m, int *__restrict__ bst
 // of four waited for its own loads).
 constexpr int BD_CCH = 64;  // rows of C staged per step
 constexpr int BD_PF = 8;
+// With at most BD_FEW CTA partials per coefficient (and one column per grid
+// row) each CTA adds them itself, as k_bd_reduce would (its warps then hold
+// one partial each, added in warp order), and the launch of that kernel is
+// saved: 361 CSFs, 57 us of kernels less in a ten-pass solve.
+constexpr int BD_FEW = BD_T / 32;
 // (columns q0 = blockIdx.y M .. q0 + M of the m; C row a at a m)
 template <int M>
 __global__ void __launch_bounds__(RT) k_bd_sub(double *__restrict__ B, int64_t ld, const IterParams *__restrict__ pv,
-                                               const double *__restrict__ C, int m, int n) {
+                                               const double *__restrict__ C, int m, int n,
+                                               const double *__restrict__ part, int ps, int ntiles,
+                                               int *__restrict__ bst) {
   pdl_wait();
   __shared__ double Cs[BD_CCH * M];
+  if (bst && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) bst[0] = bst[1] = m;
   const int ka = pv[0].c, q0 = blockIdx.y * M;
   const int i = blockIdx.x * RT + threadIdx.x;
   double acc[M];
@@ -939,7 +947,18 @@ __global__ void __launch_bounds__(RT) k_bd_sub(double *__restrict__ B, int64_t l
   for (int a0 = 0; a0 < ka; a0 += BD_CCH) {
     const int na = min(BD_CCH, ka - a0);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < na * M; idx += RT) Cs[idx] = C[(size_t)(a0 + idx / M) * m + q0 + idx % M];
+    for (int idx = threadIdx.x; idx < na * M; idx += RT) {
+      const size_t o = (size_t)(a0 + idx / M) * m + q0 + idx % M;
+      if (part) {
+        double sum = 0.0;
+#pragma unroll
+        for (int t = 0; t < BD_FEW; ++t)
+          if (t < ntiles) sum += part[(size_t)t * ps + o];
+        Cs[idx] = sum;
+      } else {
+        Cs[idx] = C[o];
+      }
+    }
     __syncthreads();
     if (i < n) {
       const double *b = B + (size_t)a0 * ld + i;
@@ -1706,6 +1725,7 @@ struct Dvd {
     const bool split = (precision == GG_SPLIT);
     const int nred = std::max(1, (lim * m + 31) / 32);
     const bool sub_split = (int64_t)nrow * 2 < ctx->sms;  // small blocks: one column per grid row
+    const bool few = !split && sub_split && bd_G <= BD_FEW;  // k_bd_sub adds the dots' partials itself
     // the split kernels' CTA partials are double-float pairs in the same buffer
     float2 *bpx = reinterpret_cast<float2 *>(bpart.p);
     // columns per grid row: where SMs are idle as few as make 64 pairs, one
@@ -1726,15 +1746,17 @@ struct Dvd {
                            round == 0, round));
       } else {
         GG_CUDA(launch_pdl(k_bd_dots<0>, gd, BD_T, 0, s, B.p, AB.p, ld, dpv.p, m, bst.p, n, bd_cpc, acw, bpart.p, bd_ps));
-        GG_CUDA(launch_pdl(k_bd_reduce<0, double>, nred, BD_T, 0, s, dpv.p, m, bst.p, bpart.p, bd_ps, bd_G, bC.p, dS.p,
-                           round == 0, -1));
+        if (!few)
+          GG_CUDA(launch_pdl(k_bd_reduce<0, double>, nred, BD_T, 0, s, dpv.p, m, bst.p, bpart.p, bd_ps, bd_G, bC.p,
+                             dS.p, round == 0, -1));
       }
       if (sub_split) {
         if (split)
           GG_CUDA(launch_pdl(k_bdx_sub<1, SP>, dim3(nrow4, m), RT, 0, s, B.p, Bx.p, ld, dpv.p, bC.p, m, n, bst.p, round,
                              wx.p));
         else
-          GG_CUDA(launch_pdl(k_bd_sub<1>, dim3(nrow, m), RT, 0, s, B.p, ld, dpv.p, bC.p, m, n));
+          GG_CUDA(launch_pdl(k_bd_sub<1>, dim3(nrow, m), RT, 0, s, B.p, ld, dpv.p, bC.p, m, n, few ? bpart.p : nullptr,
+                             bd_ps, bd_G, few && round == 0 ? bst.p : nullptr));
       } else {
         // an even m as m / 2 grid rows of two columns (more warps in flight;
         // each grid row reads the basis, from L2; all m columns with two
@@ -1747,7 +1769,8 @@ struct Dvd {
       GG_CUDA(launch_pdl(k_bdx_sub<K, 1>, dim3(nrow, half), RT, 0, s, B.p, Bx.p, ld, dpv.p, bC.p, m, n, bst.p,   \
                          round, wx.p));                                                     \
     else                                                                                    \
-      GG_CUDA(launch_pdl(k_bd_sub<K>, dim3(nrow, half), RT, 0, s, B.p, ld, dpv.p, bC.p, m, n));              \
+      GG_CUDA(launch_pdl(k_bd_sub<K>, dim3(nrow, half), RT, 0, s, B.p, ld, dpv.p, bC.p, m, n, nullptr, 0, 0, \
+                         nullptr));                                                                          \
     break;
         BD_SUB(1) BD_SUB(2) BD_SUB(3) BD_SUB(4) BD_SUB(5) BD_SUB(6) BD_SUB(7) BD_SUB(8)
         BD_SUB(9) BD_SUB(10) BD_SUB(11) BD_SUB(12) BD_SUB(13) BD_SUB(14) BD_SUB(15) BD_SUB(16)
@@ -1755,7 +1778,7 @@ struct Dvd {
           default: return fail(GG_ERR_ARG, "block pass: more new vectors than supported");
         }
       }
-      note_launches(3);
+      note_launches(few ? 2 : 3);
     }
     for (int round = 0; round < 2; ++round) {
       if (split) {
