@@ -1042,6 +1042,7 @@ __global__ void __launch_bounds__(256) k_pot_part(const PotChunk *__restrict__ c
                                                   const double *__restrict__ Y, int np,
                                                   const double *__restrict__ PF, const double *__restrict__ QF,
                                                   int ld, int n, double *__restrict__ part) {
+  pdl_wait();
   __shared__ int sf[POT_CHUNK], so[POT_CHUNK];
   __shared__ int4 sk[POT_CHUNK / 4];
   __shared__ double sc[POT_CHUNK], red[2][4][64];
@@ -1203,6 +1204,7 @@ __global__ void __launch_bounds__(32 * PF_ROWS) k_pot_final(const PotFinal *__re
                                                             const double *__restrict__ ZZ,
                                                             const double *__restrict__ PF,
                                                             const double *__restrict__ QF, int ld, QuadConst q) {
+  pdl_wait();
   __shared__ double red[3][PF_ROWS][32];
   const PotFinal g = jobs[blockIdx.y];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -1591,6 +1593,7 @@ __global__ void __launch_bounds__(64) k_yfun(const YDesc *__restrict__ yd, int n
                                              const double *__restrict__ R, const double *__restrict__ RP,
                                              const double *__restrict__ pw, int np, QuadConst q,
                                              double *__restrict__ Y) {
+  pdl_wait();
   extern __shared__ double ysh[];
   __shared__ double zfin[4];  // the Z chains' last values
   double *TZ = ysh, *TW = ysh + yf_at(np + YF_SLACK);
@@ -1769,10 +1772,9 @@ int build_y_pot(gg_ctx *ctx, const YDesc *d_yd, int nf, double *dY, DBuf<double>
   Orbitals &o = ctx->orb;
   if (g.q.n > YF_MAXN) return build_y(ctx, d_yd, nf, dY, scratch, nfp);
   const size_t smem = 2 * sizeof(double) * yf_at(g.np + YF_SLACK);
-  k_yfun<<<std::min(nf, 32 * ctx->sms), 64, smem, ctx->stream>>>(d_yd, nf, nfp, o.dPF.p, o.dQF.p, o.ld, g.dR.p,
-                                                                 g.dRP.p, g.dPow.p, g.np, g.q, dY);
+  GG_CUDA(launch_pdl(k_yfun, std::min(nf, 32 * ctx->sms), 64, smem, ctx->stream, d_yd, nf, nfp, o.dPF.p, o.dQF.p, o.ld,
+                     g.dR.p, g.dRP.p, g.dPow.p, g.np, g.q, dY));
   ::gg::note_launch();
-  GG_CUDA(cudaGetLastError());
   return GG_OK;
 }
 
@@ -2360,15 +2362,15 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, double *
   if (T > 0) GG_TRY(build_y_pot(ctx, W.yd.p, nfb, W.Y.p, W.scratch, info));
   // one launch for all chunks, one for every job's point values
   if (nch > 0) {
-    k_pot_part<<<dim3((n + 63) / 64, (unsigned)nch), 256, 0, s>>>(reinterpret_cast<const PotChunk *>(W.up.p + ach),
-                                                                 tab, W.Y.p, g.np, o.dPF.p, o.dQF.p, o.ld, n,
-                                                                 W.part.p);
+    GG_CUDA(launch_pdl(k_pot_part, dim3((n + 63) / 64, (unsigned)nch), 256, 0, s,
+                       reinterpret_cast<const PotChunk *>(W.up.p + ach), tab, W.Y.p, g.np, o.dPF.p, o.dQF.p, o.ld, n,
+                       W.part.p));
     ::gg::note_launch();
   }
   if (!jobs.empty()) {
-    k_pot_final<<<dim3((n + 31) / 32, (unsigned)jobs.size()), 32 * PF_ROWS, 0, s>>>(
-        reinterpret_cast<const PotFinal *>(W.up.p + afin), W.part.p, n, o.dNAK.p, o.dMF.p, g.dR.p, g.dRPOR.p,
-        g.dZZ.p, o.dPF.p, o.dQF.p, o.ld, g.q);
+    GG_CUDA(launch_pdl(k_pot_final, dim3((n + 31) / 32, (unsigned)jobs.size()), 32 * PF_ROWS, 0, s,
+                       reinterpret_cast<const PotFinal *>(W.up.p + afin), W.part.p, n, o.dNAK.p, o.dMF.p, g.dR.p,
+                       g.dRPOR.p, g.dZZ.p, o.dPF.p, o.dQF.p, o.ld, g.q));
     ::gg::note_launch();
   }
   GG_CUDA(cudaGetLastError());
