@@ -253,6 +253,7 @@ __global__ void k_apairs(const int2 *__restrict__ pairs, int npairs, const doubl
                          const double *__restrict__ QF, int ld, const int *__restrict__ MF,
                          const double *__restrict__ RPOR, int KC, QuadConst q, double *__restrict__ A,
                          double *__restrict__ D) {
+  pdl_wait();
   const int p = blockIdx.y;
   if (p >= npairs) return;
   const int a = pairs[p].x, c = pairs[p].y;
@@ -337,6 +338,7 @@ __global__ void __launch_bounds__(128) k_rk_dot(const RkTile *__restrict__ tiles
                                                 const TcRow *__restrict__ rows, const double *__restrict__ A,
                                                 RkTabs t, QuadConst q, double *__restrict__ val, long long nval,
                                                 QuadItem *__restrict__ fb, int *__restrict__ nfb) {
+  pdl_wait();
   const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (w >= ntiles) return;
   const RkTile T = tiles[w];
@@ -587,6 +589,7 @@ template <int R>
 __global__ void __launch_bounds__(OZ_T) k_oz_tile(const double *__restrict__ M, int pitch, int K, int nch,
                                                   const int *__restrict__ src_row, int *__restrict__ exps,
                                                   __half *__restrict__ dst) {
+  pdl_wait();
   constexpr int BLK = OZ_S * 2 * (R / 8) * 2 * 64;
   __shared__ int se[8];
   const int s0 = blockIdx.x * 8, g = s0 / R, m8 = s0 % R / 8;
@@ -659,6 +662,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_rk_tc(const TcTile *__restric
                                                          const int *__restrict__ eA, const int *__restrict__ eY,
                                                          const YDesc *__restrict__ yd, double *__restrict__ val,
                                                          long long nval, int *__restrict__ flags, int stall_tile) {
+  pdl_wait();
   extern __shared__ __align__(1024) unsigned char tsm[];
   __half *Ysm = reinterpret_cast<__half *>(tsm);
   __half *Asm = Ysm + 2 * TC_YBLK;
@@ -905,6 +909,7 @@ __global__ void k_rk_finish_all(const int32_t *__restrict__ ind, long long n, co
                                 int kloop, int KEY, const int *__restrict__ fidx, const int *__restrict__ pidx,
                                 RkTabs tb, QuadConst q, double *__restrict__ val, QuadItem *__restrict__ fb,
                                 int *__restrict__ nfb, const double *__restrict__ parts, int nsplit) {
+  pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     int p = ind[i];
     const int d = p % KEY;
@@ -960,6 +965,7 @@ __global__ void k_quad_items(const QuadItem *__restrict__ items, const int *__re
 // items took 103 us, so 55 us.
 __global__ void k_quad_table(const QuadItem *__restrict__ items, const int *__restrict__ nitems_p, int nitems_max,
                              RkTabs tb, QuadConst q, double *__restrict__ out) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   const int nitems = min(*nitems_p, nitems_max);
@@ -1384,6 +1390,7 @@ bool triangrk(int la, int k, int lb) {  // rci90/triangrk.f90:27-37
 __global__ void k_yincr(const YDesc *__restrict__ yd, int nf, const int *__restrict__ nfp,
                         const double *__restrict__ TZ, const double *__restrict__ TW, int np, QuadConst q,
                         double *__restrict__ RZ, double *__restrict__ RW) {
+  pdl_wait();
   nf = nfuncs(nf, nfp);
   for (int f = blockIdx.y; f < nf; f += gridDim.y) {
     const int MTP = yd[f].mtp;
@@ -1450,6 +1457,7 @@ __global__ void k_ychain_sum(const YDesc *__restrict__ yd, int nf, const int *__
                              const double *__restrict__ TZ, const double *__restrict__ RZ,
                              const double *__restrict__ RW, int np, QuadConst q, double *__restrict__ Y,
                              double *__restrict__ W, double *__restrict__ dif_out, double *__restrict__ zk_out) {
+  pdl_wait();
   nf = nfuncs(nf, nfp);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int f = t >> 2, c = t & 3;
@@ -1501,6 +1509,7 @@ __global__ void k_yassemble(const YDesc *__restrict__ yd, int nf, const int *__r
                             const double *__restrict__ R, const double *__restrict__ pw, int np, QuadConst q,
                             const double *__restrict__ dif, const double *__restrict__ zk,
                             const double *__restrict__ W, double *__restrict__ Y) {
+  pdl_wait();
   nf = nfuncs(nf, nfp);
   for (int f = blockIdx.y; f < nf; f += gridDim.y) {
     const YDesc y = yd[f];
@@ -1563,10 +1572,12 @@ int build_y(gg_ctx *ctx, const YDesc *d_yd, int nf, double *dY, DBuf<double> &sc
     // RZ: one term per point; RW: three terms per point; DIF per chain; ZKLIM
     double *RZ = TW + (size_t)nf * np, *RW = RZ + (size_t)nf * np, *dif = RW + (size_t)3 * nf * np;
     double *zk = dif + 4 * nf;
-    k_yincr<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, nfp, TZ, TW, np, g.q, RZ, RW);
+    GG_CUDA(launch_pdl(k_yincr, grid1, 128, 0, ctx->stream, d_yd, nf, nfp, TZ, TW, np, g.q, RZ, RW));
     // W goes where TW was: k_yincr was its last reader
-    k_ychain_sum<<<dim3((nthr + 63) / 64, 2), 64, 0, ctx->stream>>>(d_yd, nf, nfp, TZ, RZ, RW, np, g.q, dY, TW, dif, zk);
-    k_yassemble<<<grid1, 128, 0, ctx->stream>>>(d_yd, nf, nfp, g.dR.p, g.dPow.p, np, g.q, dif, zk, TW, dY);
+    GG_CUDA(launch_pdl(k_ychain_sum, dim3((nthr + 63) / 64, 2), 64, 0, ctx->stream, d_yd, nf, nfp, TZ, RZ, RW, np, g.q,
+                       dY, TW, dif, zk));
+    GG_CUDA(launch_pdl(k_yassemble, grid1, 128, 0, ctx->stream, d_yd, nf, nfp, g.dR.p, g.dPow.p, np, g.q, dif, zk, TW,
+                       dY));
     ::gg::note_launch();
     ::gg::note_launch();
     ::gg::note_launch();
@@ -1997,8 +2008,8 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
   GG_TRY(C.dD.alloc((size_t)std::max(npairs, 1) * KC + KC_TILE));
   if (npairs > 0) {
     dim3 gr((KC + 127) / 128, npairs);
-    k_apairs<<<gr, 128, 0, ctx->stream>>>(C.dPairs.p, npairs, o.dPF.p, o.dQF.p, o.ld, o.dMF.p, g.dRPOR.p, KC, g.q,
-                                          C.dA.p, C.dD.p);
+    GG_CUDA(launch_pdl(k_apairs, gr, 128, 0, ctx->stream, C.dPairs.p, npairs, o.dPF.p, o.dQF.p, o.ld, o.dMF.p,
+                       g.dRPOR.p, KC, g.q, C.dA.p, C.dD.p));
     ::gg::note_launch();
     GG_CUDA(cudaGetLastError());
   }
@@ -2018,13 +2029,13 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
       GG_TRY(C.dYt.alloc(std::max<size_t>(1, C.yslot.size() / TC_M * nch * TC_YBLK)));
       GG_TRY(C.dAt.alloc(std::max<size_t>(1, C.aslot.size() / TC_N * nch * TC_ABLK)));
       if (!C.yslot.empty()) {
-        k_oz_tile<TC_M><<<(unsigned)C.yslot.size() / 8, OZ_T, 0, ctx->stream>>>(C.dY.p, np, KC, nch, C.dYslot.p, C.dEY.p,
-                                                                          C.dYt.p);
+        GG_CUDA(launch_pdl(k_oz_tile<TC_M>, (unsigned)C.yslot.size() / 8, OZ_T, 0, ctx->stream, C.dY.p, np, KC, nch,
+                           C.dYslot.p, C.dEY.p, C.dYt.p));
         ::gg::note_launch();
       }
       if (!C.aslot.empty()) {
-        k_oz_tile<TC_N><<<(unsigned)C.aslot.size() / 8, OZ_T, 0, ctx->stream>>>(C.dA.p, KC, KC, nch, C.dAslot.p, C.dEA.p,
-                                                                          C.dAt.p);
+        GG_CUDA(launch_pdl(k_oz_tile<TC_N>, (unsigned)C.aslot.size() / 8, OZ_T, 0, ctx->stream, C.dA.p, KC, KC, nch,
+                           C.dAslot.p, C.dEA.p, C.dAt.p));
         ::gg::note_launch();
       }
       static bool attr = false;
@@ -2061,26 +2072,25 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
         parts = C.dParts.p;
       }
       if (!C.tcs.empty()) {
-        k_rk_tc<<<(unsigned)std::min<size_t>(C.tcs.size(), ctx->sms), TC_THREADS, TC_SMEM, ctx->stream>>>(
-            C.dTcs.p, (int)C.tcs.size(), C.dTcr.p, C.dYt.p, C.dAt.p, nch, C.dEA.p, C.dEY.p, C.dYd.p, parts, (long long)N,
-            C.dNfb.p + 1, ctx->test_stall_tile);
+        GG_CUDA(launch_pdl(k_rk_tc, (unsigned)std::min<size_t>(C.tcs.size(), ctx->sms), TC_THREADS, TC_SMEM,
+                           ctx->stream, C.dTcs.p, (int)C.tcs.size(), C.dTcr.p, C.dYt.p, C.dAt.p, nch, C.dEA.p,
+                           C.dEY.p, C.dYd.p, parts, (long long)N, C.dNfb.p + 1, ctx->test_stall_tile));
         ctx->test_stall_tile = -1;  // one call only
         ::gg::note_launch();
       }
       ctx->stats[25] = nsplit;
       GG_CUDA(cudaGetLastError());
       const unsigned fb_blocks = (unsigned)std::min<long long>((N + 255) / 256, 8LL * ctx->sms);
-      k_rk_finish_all<<<std::max(1u, fb_blocks), 256, 0, ctx->stream>>>(
-          rk.dInd.p, (long long)N, C.dKst.p, kloop, KEY, C.dFidx.p, C.dPidx.p, tabs, g.q, rk.dVal.p, C.dFb.p, C.dNfb.p,
-          parts, nsplit);
+      GG_CUDA(launch_pdl(k_rk_finish_all, std::max(1u, fb_blocks), 256, 0, ctx->stream, rk.dInd.p, (long long)N,
+                         C.dKst.p, kloop, KEY, C.dFidx.p, C.dPidx.p, tabs, g.q, rk.dVal.p, C.dFb.p, C.dNfb.p, parts,
+                         nsplit));
       ::gg::note_launch();
     }
     GG_CUDA(cudaGetLastError());
   } else if (!tiles.empty()) {
     auto dot = C.nr == 8 ? k_rk_dot<8> : C.nr == 4 ? k_rk_dot<4> : C.nr == 2 ? k_rk_dot<2> : k_rk_dot<1>;
-    dot<<<(unsigned)((tiles.size() + 3) / 4), 128, 0, ctx->stream>>>(C.dTiles.p, (int)tiles.size(), C.dTcr.p, C.dA.p,
-                                                                    tabs, g.q, rk.dVal.p, (long long)N, C.dFb.p,
-                                                                    C.dNfb.p);
+    GG_CUDA(launch_pdl(dot, (unsigned)((tiles.size() + 3) / 4), 128, 0, ctx->stream, C.dTiles.p, (int)tiles.size(),
+                       C.dTcr.p, C.dA.p, tabs, g.q, rk.dVal.p, (long long)N, C.dFb.p, C.dNfb.p));
     ::gg::note_launch();
     GG_CUDA(cudaGetLastError());
   }
@@ -2088,7 +2098,8 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
     // the items' number stays on the device: the blocks take it from there
     const int wpb = 16;  // warps per block: an item each, their head terms by warp 0
     const int blocks = (int)std::min<int64_t>((N + wpb - 1) / wpb, 4LL * ctx->sms);
-    k_quad_table<<<std::max(1, blocks), 32 * wpb, 0, ctx->stream>>>(C.dFb.p, C.dNfb.p, (int)N, tabs, g.q, rk.dVal.p);
+    GG_CUDA(launch_pdl(k_quad_table, std::max(1, blocks), 32 * wpb, 0, ctx->stream, C.dFb.p, C.dNfb.p, (int)N, tabs,
+                       g.q, rk.dVal.p));
     ::gg::note_launch();
     GG_CUDA(cudaGetLastError());
   }
