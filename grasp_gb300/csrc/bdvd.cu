@@ -360,6 +360,7 @@ __device__ __forceinline__ int sturm32(int m, const float *d, const float *e2, f
 __global__ void __launch_bounds__(EIG_T) k_b_eig(const BDesc *__restrict__ desc, BState *__restrict__ st,
                                                  const double *__restrict__ Spool, double *__restrict__ Ypool,
                                                  EigShape sh) {
+  pdl_wait();
   extern __shared__ double smem[];
   const int b = blockIdx.x;
   BState &S = st[b];
@@ -760,6 +761,7 @@ __global__ void __launch_bounds__(RT) k_b_ritz(const BTile *__restrict__ tiles, 
                                                const double *__restrict__ W, const double *__restrict__ Ypool,
                                                double *__restrict__ X, double *__restrict__ R,
                                                double *__restrict__ part, int ps) {
+  pdl_wait();
   const BTile T = tiles[blockIdx.x];
   const BState &S = st[T.b];
   if (!S.active) return;
@@ -792,6 +794,7 @@ __global__ void __launch_bounds__(RT) k_b_ritz(const BTile *__restrict__ tiles, 
 // (m = n) is converged: its Ritz pairs are exact up to rounding.
 __global__ void k_b_conv(const BDesc *__restrict__ desc, BState *__restrict__ st, const double *__restrict__ part,
                          int ps, int nb, double critr, int *__restrict__ nactive) {
+  pdl_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
   BState &S = st[b];
@@ -836,6 +839,7 @@ __global__ void k_b_conv(const BDesc *__restrict__ desc, BState *__restrict__ st
 __global__ void __launch_bounds__(BT) k_b_restart(const BTile *__restrict__ tiles, const BDesc *__restrict__ desc,
                                                   const BState *__restrict__ st, double *__restrict__ V,
                                                   double *__restrict__ W, const double *__restrict__ Ypool) {
+  pdl_wait();
   extern __shared__ double sm[];
   const BTile T = tiles[blockIdx.x];
   const BState &S = st[T.b];
@@ -877,6 +881,7 @@ __global__ void __launch_bounds__(BT) k_b_restart(const BTile *__restrict__ tile
 
 // after the collapse: S = diag(theta_1..REST), m = REST
 __global__ void k_b_restart_fin(const BDesc *__restrict__ desc, BState *__restrict__ st, double *__restrict__ Spool) {
+  pdl_wait();
   const int b = blockIdx.x;
   BState &S = st[b];
   if (!S.active || !S.restart) return;
@@ -900,6 +905,7 @@ __global__ void k_b_restart_fin(const BDesc *__restrict__ desc, BState *__restri
 __global__ void __launch_bounds__(RT) k_b_precond(const BTile *__restrict__ tiles, const BDesc *__restrict__ desc,
                                                   const BState *__restrict__ st, double *__restrict__ V,
                                                   const double *__restrict__ R) {
+  pdl_wait();
   const BTile T = tiles[blockIdx.x];
   const BState &S = st[T.b];
   if (!S.active || threadIdx.x >= T.nr) return;
@@ -924,6 +930,7 @@ template <int MODE>
 __global__ void __launch_bounds__(BT) k_b_dots(const BTile *__restrict__ tiles, const BDesc *__restrict__ desc,
                                                const BState *__restrict__ st, const double *__restrict__ V,
                                                const double *__restrict__ W, double *__restrict__ part, int ps) {
+  pdl_wait();
   extern __shared__ double sm[];
   const BTile T = tiles[blockIdx.x];
   const BState &S = st[T.b];
@@ -989,6 +996,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256) k_b_colsum(const BDesc *__restrict__ desc, BState *__restrict__ st,
                                                   const double *__restrict__ part, int ps, double *__restrict__ Spool,
                                                   double *__restrict__ Cpool, int first) {
+  pdl_wait();
   __shared__ double buf[(MAXL + 1) * MAXR];
   const int b = blockIdx.x;
   BState &S = st[b];
@@ -1093,6 +1101,7 @@ __device__ __forceinline__ void sub_row(double *Vi, int m, int n, const double *
 __global__ void __launch_bounds__(RT) k_b_sub(const BTile *__restrict__ tiles, const BDesc *__restrict__ desc,
                                               const BState *__restrict__ st, double *__restrict__ V,
                                               const double *__restrict__ Cpool) {
+  pdl_wait();
   __shared__ double Cs[MAXL * MAXR];
   const BTile T = tiles[blockIdx.x];
   const BState &S = st[T.b];
@@ -1123,6 +1132,7 @@ __global__ void __launch_bounds__(RT) k_b_sub(const BTile *__restrict__ tiles, c
 __global__ void __launch_bounds__(RT) k_b_apply(const BTile *__restrict__ tiles, const BDesc *__restrict__ desc,
                                                 const BState *__restrict__ st, double *__restrict__ V,
                                                 const double *__restrict__ Cpool) {
+  pdl_wait();
   __shared__ double Cs[MAXR * MAXR];
   const BTile T = tiles[blockIdx.x];
   const BState &S = st[T.b];
@@ -1156,6 +1166,7 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(RT) k_b_gatherx(const BTile *__restrict__ tiles, const BDesc *__restrict__ desc,
                                                   const BState *__restrict__ st, const double *__restrict__ V,
                                                   double *__restrict__ XD, float2 *__restrict__ XS) {
+  pdl_wait();
   const BTile T = tiles[blockIdx.x];
   const BState &S = st[T.b];
   if (!S.active || threadIdx.x >= T.nr) return;
@@ -1292,6 +1303,7 @@ __global__ void __launch_bounds__(256) k_b_spmm(const BTile *__restrict__ tiles,
                                                 const BState *__restrict__ st, const double *__restrict__ V,
                                                 double *__restrict__ W, const double *__restrict__ XD,
                                                 const float2 *__restrict__ XS, int sx_rows) {
+  pdl_wait();
   extern __shared__ X32 smx[];
   const BTile T = tiles[blockIdx.x];
   const BState &S = st[T.b];
@@ -1435,16 +1447,17 @@ struct BatchRun {
   // and S update
   int gidx(const Group &g) const { return &g == &all ? 0 : (&g == &grp[0] ? 1 : 2); }
   // W = H V for the new columns of the group's blocks with matvec variant v
-  void launch_spmm(cudaStream_t s, const Group &g, int v) {
+  int launch_spmm(cudaStream_t s, const Group &g, int v) {
     const int ts = v / 2, gi = gidx(g), nt = sp_nt[ts][gi];
-    if (nt == 0) return;
+    if (nt == 0) return GG_OK;
     const BTile *tl = dSpTiles[ts].p + sp_t0[ts][gi];
     const int thr = SPMM_T[v % 2];
     const size_t sx = (size_t)sx_rows * sizeof(X32);
     if (precision == GG_SPLIT)
-      k_b_spmm<true><<<nt, thr, sx, s>>>(tl, dDesc.p, dSt.p, V.p, W.p, XD.p, XS.p, sx_rows);
+      GG_CUDA(launch_pdl(k_b_spmm<true>, nt, thr, sx, s, tl, dDesc.p, dSt.p, V.p, W.p, XD.p, XS.p, sx_rows));
     else
-      k_b_spmm<false><<<nt, thr, sx, s>>>(tl, dDesc.p, dSt.p, V.p, W.p, XD.p, XS.p, sx_rows);
+      GG_CUDA(launch_pdl(k_b_spmm<false>, nt, thr, sx, s, tl, dDesc.p, dSt.p, V.p, W.p, XD.p, XS.p, sx_rows));
+    return GG_OK;
   }
   int enqueue_expand(cudaStream_t s, const Group &g, int *count, const cudaEvent_t *tune_ev = nullptr,
                      double *tune_ms = nullptr) {
@@ -1454,16 +1467,16 @@ struct BatchRun {
     BState *sb = dSt.p + g.b0;
     double *pt = part.p + (size_t)g.t0 * ps;
     if (precision == GG_SPLIT)
-      k_b_gatherx<true><<<g.nt, RT, 0, s>>>(tl, dDesc.p, dSt.p, V.p, XD.p, XS.p);
+      GG_CUDA(launch_pdl(k_b_gatherx<true>, g.nt, RT, 0, s, tl, dDesc.p, dSt.p, V.p, XD.p, XS.p));
     else
-      k_b_gatherx<false><<<g.nt, RT, 0, s>>>(tl, dDesc.p, dSt.p, V.p, XD.p, XS.p);
+      GG_CUDA(launch_pdl(k_b_gatherx<false>, g.nt, RT, 0, s, tl, dDesc.p, dSt.p, V.p, XD.p, XS.p));
     if (tune_ev) {
       // the autotuner: every variant computes the same W (each row is one
       // warp's whatever the tiles, and W is overwritten), so all run here,
       // each between events
       for (int v = 0; v < SPMM_NVAR; ++v) {
         GG_CUDA(cudaEventRecord(tune_ev[2 * v], s));
-        launch_spmm(s, g, v);
+        GG_TRY(launch_spmm(s, g, v));
         GG_CUDA(cudaEventRecord(tune_ev[2 * v + 1], s));
       }
       GG_CUDA(cudaEventSynchronize(tune_ev[2 * SPMM_NVAR - 1]));
@@ -1479,10 +1492,10 @@ struct BatchRun {
       }
       *count += SPMM_NVAR - 1;
     } else {
-      launch_spmm(s, g, sp_var);
+      GG_TRY(launch_spmm(s, g, sp_var));
     }
-    k_b_dots<2><<<g.nt, BT, dots_smem, s>>>(tl, dDesc.p, dSt.p, V.p, W.p, pt, ps);
-    k_b_colsum<2><<<g.nb, 256, 0, s>>>(de, sb, part.p, ps, Sp.p, Cp.p, 0);
+    GG_CUDA(launch_pdl(k_b_dots<2>, g.nt, BT, dots_smem, s, tl, dDesc.p, dSt.p, V.p, W.p, pt, ps));
+    GG_CUDA(launch_pdl(k_b_colsum<2>, g.nb, 256, 0, s, de, sb, part.p, ps, Sp.p, Cp.p, 0));
     *count += 4;
     GG_CUDA(cudaGetLastError());
     return GG_OK;
@@ -1496,23 +1509,23 @@ struct BatchRun {
     const BDesc *de = dDesc.p + g.b0;
     BState *sb = dSt.p + g.b0;
     double *pt = part.p + (size_t)g.t0 * ps;
-    k_b_eig<<<g.nb, EIG_T, eig.bytes(), s>>>(de, sb, Sp.p, Yp.p, eig);
-    k_b_ritz<<<g.nt, RT, 0, s>>>(tl, dDesc.p, dSt.p, V.p, W.p, Yp.p, X.p, R.p, pt, ps);
-    k_b_conv<<<(g.nb + 127) / 128, 128, 0, s>>>(de, sb, part.p, ps, g.nb, critr, dNact.p);
-    k_b_restart<<<g.nt, BT, restart_smem, s>>>(tl, dDesc.p, dSt.p, V.p, W.p, Yp.p);
-    k_b_restart_fin<<<g.nb, 256, 0, s>>>(de, sb, Sp.p);
-    k_b_precond<<<g.nt, RT, 0, s>>>(tl, dDesc.p, dSt.p, V.p, R.p);
+    GG_CUDA(launch_pdl(k_b_eig, g.nb, EIG_T, eig.bytes(), s, de, sb, Sp.p, Yp.p, eig));
+    GG_CUDA(launch_pdl(k_b_ritz, g.nt, RT, 0, s, tl, dDesc.p, dSt.p, V.p, W.p, Yp.p, X.p, R.p, pt, ps));
+    GG_CUDA(launch_pdl(k_b_conv, (g.nb + 127) / 128, 128, 0, s, de, sb, part.p, ps, g.nb, critr, dNact.p));
+    GG_CUDA(launch_pdl(k_b_restart, g.nt, BT, restart_smem, s, tl, dDesc.p, dSt.p, V.p, W.p, Yp.p));
+    GG_CUDA(launch_pdl(k_b_restart_fin, g.nb, 256, 0, s, de, sb, Sp.p));
+    GG_CUDA(launch_pdl(k_b_precond, g.nt, RT, 0, s, tl, dDesc.p, dSt.p, V.p, R.p));
     *count += 6;
     for (int pass = 0; pass < 2; ++pass) {
-      k_b_dots<0><<<g.nt, BT, dots_smem, s>>>(tl, dDesc.p, dSt.p, V.p, W.p, pt, ps);
-      k_b_colsum<0><<<g.nb, 256, 0, s>>>(de, sb, part.p, ps, Sp.p, Cp.p, pass == 0);
-      k_b_sub<<<g.nt, RT, 0, s>>>(tl, dDesc.p, dSt.p, V.p, Cp.p);
+      GG_CUDA(launch_pdl(k_b_dots<0>, g.nt, BT, dots_smem, s, tl, dDesc.p, dSt.p, V.p, W.p, pt, ps));
+      GG_CUDA(launch_pdl(k_b_colsum<0>, g.nb, 256, 0, s, de, sb, part.p, ps, Sp.p, Cp.p, pass == 0));
+      GG_CUDA(launch_pdl(k_b_sub, g.nt, RT, 0, s, tl, dDesc.p, dSt.p, V.p, Cp.p));
       *count += 3;
     }
     for (int pass = 0; pass < 2; ++pass) {
-      k_b_dots<1><<<g.nt, BT, dots_smem, s>>>(tl, dDesc.p, dSt.p, V.p, W.p, pt, ps);
-      k_b_colsum<1><<<g.nb, 256, 0, s>>>(de, sb, part.p, ps, Sp.p, Cp.p, pass == 0);
-      k_b_apply<<<g.nt, RT, 0, s>>>(tl, dDesc.p, dSt.p, V.p, Cp.p);
+      GG_CUDA(launch_pdl(k_b_dots<1>, g.nt, BT, dots_smem, s, tl, dDesc.p, dSt.p, V.p, W.p, pt, ps));
+      GG_CUDA(launch_pdl(k_b_colsum<1>, g.nb, 256, 0, s, de, sb, part.p, ps, Sp.p, Cp.p, pass == 0));
+      GG_CUDA(launch_pdl(k_b_apply, g.nt, RT, 0, s, tl, dDesc.p, dSt.p, V.p, Cp.p));
       *count += 3;
     }
     GG_CUDA(cudaGetLastError());
