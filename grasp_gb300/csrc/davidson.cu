@@ -239,6 +239,7 @@ template <bool PRE>
 __global__ void __launch_bounds__(CD_T) k_cdots(const double *X, int64_t ld, PSrc ps, int kofs, double *W, double *AB,
                                                 double *diag, const double *scal, const double *skip, int n,
                                                 int rows, int pitch, double *__restrict__ part) {
+  pdl_wait();
   if (skip && *skip != 0.0) return;
   const IterParams P = ps.get();
   const int c = P.c, k = c + kofs;
@@ -299,6 +300,7 @@ __global__ void __launch_bounds__(CD_T) k_cdots(const double *X, int64_t ld, PSr
 __global__ void __launch_bounds__(CS_T) k_colsum(const double *__restrict__ part, int pitch, int nb, PSrc ps, int kofs,
                                                  const double *skip, const double *__restrict__ scal, int fslot,
                                                  double *__restrict__ out, int packed) {
+  pdl_wait();
   if (skip && *skip != 0.0) return;
   const IterParams P = ps.get();
   const int j = blockIdx.x;
@@ -319,6 +321,7 @@ __global__ void __launch_bounds__(RTH) k_csub(double *X, int64_t ld, PSrc ps, co
                                               const double *skip, int fin, int fout, int n,
                                               double *__restrict__ part, unsigned *__restrict__ counter,
                                               double *scal) {
+  pdl_wait();
   if (skip && *skip != 0.0) return;
   const IterParams P = ps.get();
   const int k = P.c;
@@ -555,6 +558,7 @@ __global__ void k_newvec_precond(const NvIn *__restrict__ in, const double *__re
 // column c <- scal[fslot] * column c; with xs, also its hi+lo split for the matvec
 __global__ void k_cscale(double *X, int64_t ld, PSrc ps, const double *skip, const double *__restrict__ scal,
                          int fslot, int n, float2 *__restrict__ xs) {
+  pdl_wait();
   if (skip && *skip != 0.0) return;
   const IterParams P = ps.get();
   const double f = scal[fslot];
@@ -1638,22 +1642,19 @@ struct Dvd {
   void launch_dots(bool pre, const PSrc &ps, int kofs, double *W, const double *skip, int fslot,
                    double *out = nullptr, int packed = 0) {
     if (!out) out = dots.p;
-    if (pre)
-      k_cdots<true><<<cd_blocks, CD_T, 0, s>>>(B.p, ld, ps, kofs, W, AB.p, diag.p, scal(), skip, n, cd_rows,
-                                               cd_blocks, part.p);
-    else
-      k_cdots<false><<<cd_blocks, CD_T, 0, s>>>(B.p, ld, ps, kofs, W, AB.p, diag.p, scal(), skip, n, cd_rows,
-                                                cd_blocks, part.p);
-    k_colsum<<<lim + 1, CS_T, 0, s>>>(part.p, cd_blocks, cd_blocks, ps, kofs, skip, scal(), fslot, out, packed);
+    // (a failed launch is found by the cudaGetLastError that ends the pass)
+    launch_pdl(pre ? k_cdots<true> : k_cdots<false>, cd_blocks, CD_T, 0, s, B.p, ld, ps, kofs, W, AB.p, diag.p, scal(),
+               skip, n, cd_rows, cd_blocks, part.p);
+    launch_pdl(k_colsum, lim + 1, CS_T, 0, s, part.p, cd_blocks, cd_blocks, ps, kofs, skip, scal(), fslot, out, packed);
     note_launch();
     note_launch();
   }
   void launch_csub(const PSrc &ps, const double *skip, int fin, int fout) {
-    k_csub<<<nrr, RTH, 0, s>>>(B.p, ld, ps, dots.p, skip, fin, fout, n, part.p, counters.p + 2, scal());
+    launch_pdl(k_csub, nrr, RTH, 0, s, B.p, ld, ps, dots.p, skip, fin, fout, n, part.p, counters.p + 2, scal());
     note_launch();
   }
   void launch_cscale(const PSrc &ps, const double *skip, int fslot, float2 *xs) {
-    k_cscale<<<std::min((n + TPB - 1) / TPB, 4 * 152), TPB, 0, s>>>(B.p, ld, ps, skip, scal(), fslot, n, xs);
+    launch_pdl(k_cscale, std::min((n + TPB - 1) / TPB, 4 * 152), TPB, 0, s, B.p, ld, ps, skip, scal(), fslot, n, xs);
     note_launch();
   }
   // two-pass classical Gram-Schmidt of column ps.c against columns
@@ -1690,6 +1691,7 @@ struct Dvd {
       GG_CUDA(cudaEventRecord(gev1, s));
     }
     launch_dots(false, ps, 1, AB.p, skip, -1);
+    GG_CUDA(cudaGetLastError());
     GG_CUDA(cudaMemcpyAsync(hdown, dots.p, (size_t)(lim + 8 + SC_N) * sizeof(double), cudaMemcpyDeviceToHost, s));
     return GG_OK;
   }
