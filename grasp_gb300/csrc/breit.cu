@@ -1125,7 +1125,12 @@ __global__ void k_br_table(const BrRow *__restrict__ rows, const int *__restrict
 }
 
 // an entry of the table term by term: one thread per (entry, term), then the
-// combination
+// combination. A launch takes up to BR_REDO entries of the list: enough threads
+// for many waves, 4 n and a thread's index stay ints whatever the table's size
+// (up to 2^31 - 1 integrals), and the terms' values take 17 MB instead of 32
+// bytes for every entry of the list.
+constexpr int BR_REDO = 1 << 19;
+static_assert(4LL * BR_REDO + 128 <= INT32_MAX, "k_br_redo's thread index is an int");
 __global__ void __launch_bounds__(128) k_br_redo(int type, const BrRedo *__restrict__ redo, int n,
                                                  const BrRow *__restrict__ rows, PlanTabs T, TermTabs tt, QuadConst q,
                                                  double *__restrict__ v, BrInt *__restrict__ ints) {
@@ -1512,18 +1517,23 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
     // k_bessel ran to the longest orbital, which covers every term
     DBuf<double> dv, dout;
     DBuf<BrInt> dints;
-    GG_TRY(dv.alloc((size_t)4 * nredo));
-    GG_TRY(dout.alloc(nredo));
-    GG_TRY(dints.alloc(nredo));
+    const int piece = std::min(nredo, BR_REDO);
+    GG_TRY(dv.alloc((size_t)4 * piece));
+    GG_TRY(dout.alloc(piece));
+    GG_TRY(dints.alloc(piece));
     const TermTabs tt{o.dPF.p, o.dQF.p, o.ld, o.dMF.p, g.dR.p, g.dRP.p, g.dRPOR.p, g.dPow.p, np, dBJ.p, dBN.p};
-    k_br_redo<<<(unsigned)((4LL * nredo + 127) / 128), 128, 0, s>>>(type, dredo.p, nredo, drows.p, P.tabs(), tt, g.q,
-                                                                   dv.p, dints.p);
-    ::gg::note_launch();
-    k_breit_combine<<<(nredo + 255) / 256, 256, 0, s>>>(dints.p, nredo, dv.p, dout.p);
-    ::gg::note_launch();
-    k_br_redo_store<<<(nredo + 255) / 256, 256, 0, s>>>(dredo.p, nredo, dout.p, T.dVal.p);
-    ::gg::note_launch();
-    GG_CUDA(cudaGetLastError());
+    for (int done = 0; done < nredo;) {
+      const int n = std::min(piece, nredo - done);
+      const BrRedo *part = dredo.p + done;
+      k_br_redo<<<(4 * n + 127) / 128, 128, 0, s>>>(type, part, n, drows.p, P.tabs(), tt, g.q, dv.p, dints.p);
+      ::gg::note_launch();
+      k_breit_combine<<<(n + 255) / 256, 256, 0, s>>>(dints.p, n, dv.p, dout.p);
+      ::gg::note_launch();
+      k_br_redo_store<<<(n + 255) / 256, 256, 0, s>>>(part, n, dout.p, T.dVal.p);
+      ::gg::note_launch();
+      GG_CUDA(cudaGetLastError());
+      done += n;
+    }
   }
   ctx->stats[34] = nredo;
   GG_CUDA(cudaEventRecord(e1, s));
