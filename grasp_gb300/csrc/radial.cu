@@ -85,12 +85,18 @@ __device__ double quad_seq(double *TA, int mtp, const double *R, const double *R
   return 0.0;
 }
 
+// dynamic shared memory of any launch without opting in: 48 KB less the 1 KB
+// that a kernel with a static array takes
+constexpr size_t SMEM_PLAIN = 47 * 1024;
+__host__ __device__ constexpr int quad_panels(int np) { return np / 4 + 4; }
+
 // quad_seq by the lanes of a warp, the same value to the bit: the head index
-// by ballot, the four-point panels (quad.f90:94-99) one per lane into `panel`,
-// then lane 0 adds them in order, the only serial part. TA is zero beyond
-// MTP; the result is lane 0's. (Sequential QUADs on one lane of each warp were
-// most of RINTI: four of 148 panels of seven operations each, 168 us per I(ab)
-// table whatever its size; this form RNT us.)
+// by ballot, the four-point panels (quad.f90:94-99) one per lane into `panel`
+// (quad_panels(np) doubles), then lane 0 adds them in order, the only serial
+// part. TA is zero beyond MTP; the result is lane 0's. (Sequential QUADs on
+// one lane of each warp were most of RINTI: four of 148 panels of seven
+// operations each, 168 us per I(ab) table whatever its size; this form 22 us
+// for 16 subshells, 36 us for 43.)
 __device__ double quad_warp(const double *TA, double *panel, int mtp, const double *R, const double *RP,
                             const QuadConst &q, int lane) {
   int h = 0;
@@ -1261,6 +1267,9 @@ __global__ void __launch_bounds__(32 * PF_ROWS) k_pot_final(const PotFinal *__re
 // {J, M, case, MTP}: TA(I), I = 2..MTP, from the two orbitals' potentials
 // (pot + 3 n slot: YP, XP, XQ, 0-based), then QUAD by one warp. case 0: M
 // fixed; 1: J fixed; 2: occupations more than 10 % apart; 3: otherwise.
+// QUAD's panels lie in shared memory while they fit what every launch
+// has (SH; N <= 24,024), else behind the pair's TA.
+template <bool SH>
 __global__ void k_setlag_quad(const int4 *__restrict__ pj, const int2 *__restrict__ slots,
                               const double *__restrict__ pot, int n, const double *__restrict__ PF,
                               const double *__restrict__ QF, int ld, const double *__restrict__ R,
@@ -1271,7 +1280,8 @@ __global__ void k_setlag_quad(const int4 *__restrict__ pj, const int2 *__restric
   const int J = w.x, M = w.y, cs = w.z, mtp = w.w;
   const double *ypj = pot + (size_t)3 * n * slots[blockIdx.x].x, *xpj = ypj + n, *xqj = xpj + n;
   const double *ypm = pot + (size_t)3 * n * slots[blockIdx.x].y, *xpm = ypm + n, *xqm = xpm + n;
-  double *TA = TAall + (size_t)blockIdx.x * np;
+  const size_t rec = SH ? (size_t)np : (size_t)np + quad_panels(np);
+  double *TA = TAall + (size_t)blockIdx.x * rec, *panel = SH ? sm : TA + np;
   const double C = q.c;
   for (int i = threadIdx.x; i < np; i += blockDim.x) {
     double v = 0.0;
@@ -1292,7 +1302,7 @@ __global__ void k_setlag_quad(const int4 *__restrict__ pj, const int2 *__restric
   }
   __syncthreads();
   if (threadIdx.x < 32) {
-    const double v = quad_warp(TA, sm, mtp, R, RP, q, threadIdx.x);
+    const double v = quad_warp(TA, panel, mtp, R, RP, q, threadIdx.x);
     if (threadIdx.x == 0) result[blockIdx.x] = v;
   }
 }
@@ -1314,8 +1324,13 @@ __global__ void k_setlag_final(int np_, const int4 *__restrict__ pj, const doubl
 
 // RINTI (lib9290/rinti.f90:53-100) for a list of (J, K, place) entries: one block of
 // four warps each, the four integrands formed by all threads, one QUAD per warp.
+// The integrands and panels lie in shared memory while they fit what
+// every launch has (SH; N <= 1,174: GRASP's 590 points take 25 KB), else in
+// `work`, rinti_work(np) doubles per block: the same operations
+// and bits (I(ab) of 8 subshells: 53 us at 1,174 points, 54 us at 1,175).
 constexpr int RINTI_WARPS = 4;
-__host__ __device__ constexpr size_t rinti_smem(int np) { return (size_t)RINTI_WARPS * (np + np / 4 + 4); }  // doubles
+__host__ __device__ constexpr size_t rinti_work(int np) { return (size_t)RINTI_WARPS * (np + quad_panels(np)); }
+template <bool SH>
 __global__ void __launch_bounds__(32 * RINTI_WARPS) k_rinti(const int4 *__restrict__ jk, int npairs, int mode,
                                                            const double *__restrict__ PF,
                                                            const double *__restrict__ QF, int ld,
@@ -1324,11 +1339,12 @@ __global__ void __launch_bounds__(32 * RINTI_WARPS) k_rinti(const int4 *__restri
                                                            const double *__restrict__ RP,
                                                            const double *__restrict__ RPOR,
                                                            const double *__restrict__ ZZ, int np, QuadConst q,
-                                                           double *__restrict__ out) {
+                                                           double *work, double *__restrict__ out) {
   extern __shared__ double sm[];
   __shared__ double piece[RINTI_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double *TA = sm, *panel = sm + (size_t)RINTI_WARPS * np + (size_t)warp * (np / 4 + 4);
+  double *TA = SH ? sm : work + blockIdx.x * rinti_work(np);
+  double *panel = TA + (size_t)RINTI_WARPS * np + (size_t)warp * quad_panels(np);
   for (int it = blockIdx.x; it < npairs; it += gridDim.x) {
     const int J = jk[it].x, K = jk[it].y;
     const int mtp = max(MF[J], MF[K]);
@@ -2546,13 +2562,15 @@ int gg_setlag(gg_ctx *ctx, int nec, const int32_t *iecc, const double *ucf, cons
   GG_TRY(upload(dpj, pj, s));
   GG_TRY(upload(dps, ps, s));
   GG_TRY(upload(duc, uc, s));
-  GG_TRY(dTA.alloc((size_t)nec * g.np));
+  const size_t psm = quad_panels(g.np) * sizeof(double);
+  const bool sh = psm <= SMEM_PLAIN;
+  GG_TRY(dTA.alloc((size_t)nec * (g.np + (sh ? 0 : quad_panels(g.np)))));
   GG_TRY(dres.alloc(nec));
   GG_TRY(drij.alloc(nec));
   GG_TRY(decv.alloc(nec));
   GG_CUDA(cudaMemsetAsync(drij.p, 0, nec * sizeof(double), s));
-  k_setlag_quad<<<nec, 128, (g.np / 4 + 4) * sizeof(double), s>>>(dpj.p, dps.p, pot.p, g.n, o.dPF.p, o.dQF.p, o.ld, g.dR.p, g.dRP.p, g.dRPOR.p,
-                                    g.q, g.np, dTA.p, dres.p);
+  (sh ? k_setlag_quad<true> : k_setlag_quad<false>)<<<nec, 128, sh ? psm : 0, s>>>(
+      dpj.p, dps.p, pot.p, g.n, o.dPF.p, o.dQF.p, o.ld, g.dR.p, g.dRP.p, g.dRPOR.p, g.q, g.np, dTA.p, dres.p);
   ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
   if (!rjk.empty()) GG_TRY(run_rinti(ctx, rjk, 1, drij.p, &ridx));
@@ -2676,10 +2694,15 @@ static int run_rinti(gg_ctx *ctx, const std::vector<int2> &jk, int mode, double 
   for (size_t i = 0; i < jk.size(); ++i) h[i] = make_int4(jk[i].x, jk[i].y, outidx ? (*outidx)[i] : (int)i, 0);
   DBuf<int4> djk;  // freed in stream order
   GG_TRY(upload(djk, h, ctx->stream));
-  const size_t smem = rinti_smem(g.np) * sizeof(double);
-  const int blocks = std::max(1, std::min((int)jk.size(), 2048));
-  k_rinti<<<blocks, 32 * RINTI_WARPS, smem, ctx->stream>>>(djk.p, (int)jk.size(), mode, o.dPF.p, o.dQF.p, o.ld, o.dMF.p,
-                                                   o.dNAK.p, g.dR.p, g.dRP.p, g.dRPOR.p, g.dZZ.p, g.np, g.q, dOut);
+  const size_t smem = rinti_work(g.np) * sizeof(double);
+  const bool sh = smem <= SMEM_PLAIN;
+  // with its arrays in global memory a block per SM is enough, and 0.6 GB at N = 100,000
+  const int blocks = std::max(1, std::min((int)jk.size(), sh ? 2048 : ctx->sms));
+  DBuf<double> work;
+  if (!sh) GG_TRY(work.alloc(blocks * rinti_work(g.np)));
+  (sh ? k_rinti<true> : k_rinti<false>)<<<blocks, 32 * RINTI_WARPS, sh ? smem : 0, ctx->stream>>>(
+      djk.p, (int)jk.size(), mode, o.dPF.p, o.dQF.p, o.ld, o.dMF.p, o.dNAK.p, g.dR.p, g.dRP.p, g.dRPOR.p, g.dZZ.p,
+      g.np, g.q, work.p, dOut);
   ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
   return GG_OK;
