@@ -1,4 +1,5 @@
 // ctx.cu - context, grid (RADGRD/SETQIC) and orbital state of libgraspgpu.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -10,6 +11,10 @@ namespace gg {
 static thread_local std::string g_last_error;
 static std::atomic<long long> g_launches{0};
 static std::atomic<long long> g_allocs{0};
+
+// the live contexts, for gg_release_memory
+static std::mutex g_ctx_mu;
+static std::vector<gg_ctx *> g_ctxs;
 
 void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void note_launches(long long m) { g_launches.fetch_add(m, std::memory_order_relaxed); }
@@ -84,12 +89,20 @@ int gg_ctx_create(int device, gg_ctx **out) {
     delete c;
     return fail(GG_ERR_CUDA, std::string("gg_ctx_create: ") + cudaGetErrorString(e));
   }
+  {
+    std::lock_guard<std::mutex> lock(g_ctx_mu);
+    g_ctxs.push_back(c);
+  }
   *out = c;
   return GG_OK;
 }
 
 int gg_ctx_destroy(gg_ctx *ctx) {
   if (!ctx) return GG_OK;
+  {
+    std::lock_guard<std::mutex> lock(g_ctx_mu);
+    g_ctxs.erase(std::remove(g_ctxs.begin(), g_ctxs.end(), ctx), g_ctxs.end());
+  }
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   for (cudaEvent_t &e : ctx->marks)
@@ -113,6 +126,14 @@ int gg_release_memory(int device) {
   GG_CUDA(cudaGetDeviceCount(&ndev));
   if (device < 0 || device >= ndev) return fail(GG_ERR_ARG, "gg_release_memory: no such device");
   GG_CUDA(cudaSetDevice(device));
+  {
+    std::lock_guard<std::mutex> lock(g_ctx_mu);
+    for (gg_ctx *c : g_ctxs)
+      if (c->device == device) {
+        std::lock_guard<std::mutex> use(c->pot_mu);  // a call in another thread ends first
+        c->pot_work.reset();
+      }
+  }
   GG_CUDA(cudaDeviceSynchronize());
   cudaMemPool_t pool = nullptr;
   GG_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <memory>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -213,7 +214,10 @@ struct gg_ctx {
   cudaEvent_t aux_done = nullptr;
   gg::BreitTable breit[2];      // GENINTBREIT1, GENINTBREIT2
   std::shared_ptr<void> setcof; // setcof.cu: the sums of the last gg_setcof_prepare
-  std::shared_ptr<void> pot_work;  // radial.cu: the potentials' staging and device buffers
+  // radial.cu: the potentials' staging and device buffers, kept between calls;
+  // a call holds pot_mu for as long as it uses them, gg_release_memory takes them
+  std::shared_ptr<void> pot_work;
+  std::mutex pot_mu;
 };
 
 struct gg_hmat {

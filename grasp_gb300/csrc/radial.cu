@@ -2264,9 +2264,10 @@ struct PotJob {
   std::vector<double> lag_wa;  // and their weights ECV WB
 };
 
-// What run_potentials keeps on the context between calls: a pinned staging
-// buffer and the device buffers, as far as a call's fit in POT_KEEP bytes (a
-// COFPOT call for each orbital of an SCF cycle then allocates nothing)
+// What a potential call keeps on the context for the next: a pinned staging
+// buffer and the device buffers (a COFPOT call for each orbital of an SCF cycle
+// then allocates nothing), until gg_release_memory or a call whose buffers pass
+// POT_KEEP bytes.
 struct PotWork {
   void *stage = nullptr;
   size_t stage_bytes = 0;
@@ -2275,8 +2276,26 @@ struct PotWork {
   DBuf<double> coef, Y, scratch, pot, part;
   DBuf<YDesc> yd;
   ~PotWork() { cudaFreeHost(stage); }
+  size_t bytes() const {
+    return stage_bytes + up.n + term.n * sizeof(int) + yd.n * sizeof(YDesc) +
+           (coef.n + Y.n + scratch.n + pot.n + part.n) * sizeof(double);
+  }
 };
 constexpr size_t POT_KEEP = (size_t)512 << 20, POT_BOUND = (size_t)256 << 20;
+
+// a call's use of the context's PotWork: no other call nor gg_release_memory
+// touches it meanwhile
+struct PotUse {
+  gg_ctx *ctx;
+  std::lock_guard<std::mutex> lock;
+  explicit PotUse(gg_ctx *c) : ctx(c), lock(c->pot_mu) {
+    if (!ctx->pot_work) ctx->pot_work = std::make_shared<PotWork>();
+  }
+  ~PotUse() {
+    if (work().bytes() > POT_KEEP) ctx->pot_work.reset();
+  }
+  PotWork &work() const { return *std::static_pointer_cast<PotWork>(ctx->pot_work); }
+};
 
 // the jobs' YPOT, XPOT, then LAGCON and DACON, into W.pot (3 n per job): all
 // Y functions of all lists built once. Everything the host prepares (lists,
@@ -2284,13 +2303,11 @@ constexpr size_t POT_KEEP = (size_t)512 << 20, POT_BOUND = (size_t)256 << 20;
 // end; the launches over functions are sized by a bound and read the number
 // of functions on the device. out (may be null): where the potentials go on
 // the host.
-static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, double *out = nullptr) {
+static int run_potentials(gg_ctx *ctx, PotWork &W, const std::vector<PotJob> &jobs, double *out = nullptr) {
   Orbitals &o = ctx->orb;
   Grid &g = ctx->grid;
   cudaStream_t s = ctx->stream;
   const int n = g.n, nw = o.nw;
-  if (!ctx->pot_work) ctx->pot_work = std::make_shared<PotWork>();
-  PotWork &W = *std::static_pointer_cast<PotWork>(ctx->pot_work);
   // every job's YPOT list, then every job's XPOT list, as the caller passed
   // them; the chunks of every list; the DACON and LAGCON lists; the job records
   std::vector<size_t> oy(jobs.size()), ox(jobs.size());
@@ -2409,15 +2426,6 @@ static int run_potentials(gg_ctx *ctx, const std::vector<PotJob> &jobs, double *
   GG_CUDA(cudaStreamSynchronize(s));
   const bool bad = hinfo[1] != 0;
   if (out && !bad) std::memcpy(out, hres, npot * sizeof(double));
-  auto bytes = [](const DBuf<double> &b) { return b.n * sizeof(double); };
-  if (bytes(W.Y) + bytes(W.scratch) + bytes(W.part) + bytes(W.coef) * 2 + W.up.n > POT_KEEP) {
-    W.Y.release();
-    W.scratch.release();
-    W.part.release();
-    W.coef.release();
-    W.term.release();
-    W.up.release();
-  }
   if (bad) return fail(GG_ERR_ARG, "potential: label outside the orbital set or K above 20");
   return GG_OK;
 }
@@ -2431,7 +2439,8 @@ static int potential(gg_ctx *ctx, int mode, int ncof, const int32_t *lab, const 
   GG_TRY(raw_list(ncof, lab, co, mode == 0 ? jobs[0].y : jobs[0].x));
   const int n = ctx->grid.n;
   std::vector<double> h((size_t)3 * n);
-  GG_TRY(run_potentials(ctx, jobs, h.data()));
+  PotUse use(ctx);
+  GG_TRY(run_potentials(ctx, use.work(), jobs, h.data()));
   if (mode == 0) {
     std::copy(h.begin(), h.begin() + n, out0);
   } else {
@@ -2498,7 +2507,8 @@ int gg_cofpot(gg_ctx *ctx, int j, double ucfj, const gg_cof *cof, int nec, const
   }
   const int n = ctx->grid.n;
   std::vector<double> h((size_t)3 * n);  // one read-back of YP, XP, XQ
-  GG_TRY(run_potentials(ctx, jobs, h.data()));
+  PotUse use(ctx);
+  GG_TRY(run_potentials(ctx, use.work(), jobs, h.data()));
   std::copy(h.begin(), h.begin() + n, yp);
   std::copy(h.begin() + n, h.begin() + 2 * n, xp);
   std::copy(h.begin() + 2 * n, h.end(), xq);
@@ -2552,8 +2562,9 @@ int gg_setlag(gg_ctx *ctx, int nec, const int32_t *iecc, const double *ucf, cons
   }
   std::vector<PotJob> jobs(orbs.size());
   for (size_t i = 0; i < orbs.size(); ++i) GG_TRY(cof_job(ctx, &cof[orbs[i] - 1], jobs[i]));
-  GG_TRY(run_potentials(ctx, jobs));
-  const DBuf<double> &pot = std::static_pointer_cast<PotWork>(ctx->pot_work)->pot;
+  PotUse use(ctx);
+  GG_TRY(run_potentials(ctx, use.work(), jobs));
+  const DBuf<double> &pot = use.work().pot;
   cudaStream_t s = ctx->stream;
   DBuf<int4> dpj;
   DBuf<int2> dps;

@@ -64,8 +64,10 @@ int gg_ctx_create(int device, gg_ctx **out);
 int gg_ctx_destroy(gg_ctx *ctx);
 /* Blocks until all work on the context's stream has finished. */
 int gg_ctx_synchronize(gg_ctx *ctx);
-/* Waits for the device, then returns the memory the library's freed
- * buffers left in the device's default memory pool to the driver. */
+/* Frees the work buffers that the device's contexts keep between potential
+ * calls (at most 512 MB each, their staging included), waits for the device, then returns the memory
+ * the library's freed buffers left in the device's default memory pool to the
+ * driver. */
 int gg_release_memory(int device);
 
 /* ---- grid (grid_C, npot_C, def_C) ---------------------------------------
