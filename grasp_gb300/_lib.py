@@ -91,6 +91,7 @@ GPU_SYMBOLS = {
     "gg_launch_count": (C.c_longlong, []),
     "gg_alloc_count": (C.c_longlong, []),
     "gg_test_stall_rk_tile": (C.c_int, [C.c_void_p, C.c_int]),
+    "gg_test_setcof_positions": (C.c_int, [C.c_void_p, C.c_int64]),
     "gg_host_register": (C.c_int, [C.c_void_p, C.c_size_t]),
     "gg_host_unregister": (C.c_int, [C.c_void_p]),
     "gg_event_record": (C.c_int, [C.c_void_p, C.c_int]),

@@ -363,6 +363,12 @@ int gg_test_stall_rk_tile(gg_ctx *ctx, int tile) {
   return GG_OK;
 }
 
+int gg_test_setcof_positions(gg_ctx *ctx, int64_t positions) {
+  if (!ctx) return fail(GG_ERR_ARG, "gg_test_setcof_positions: no context");
+  ctx->test_setcof_pos = positions > 0 ? positions : 0;
+  return GG_OK;
+}
+
 int gg_projected_eig(int n, const double *ap, int m, int mvec, double *w, double *z) {
   if (n < 1 || !ap || m < 1 || m > n || mvec < 0 || mvec > m || !w || (mvec > 0 && !z))
     return fail(GG_ERR_ARG, "gg_projected_eig: bad arguments");

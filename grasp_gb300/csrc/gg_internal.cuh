@@ -208,6 +208,7 @@ struct gg_ctx {
   cudaEvent_t ev_mid = nullptr;  // a point inside a timed call (gg_maneig: after its structures)
   cudaEvent_t marks[8] = {};  // gg_event_record slots
   int test_stall_tile = -1;     // gg_test_stall_rk_tile: one tensor-core tile withholds a copy, once
+  int64_t test_setcof_pos = 0;  // gg_test_setcof_positions: the next gg_setcof_prepare's pieces
   int btune_var = -1;           // the last gg_maneig_batched's matvec variant and the
   double btune_ms[6] = {};      // tuner's times of its variants (ms)
   cudaStream_t aux = nullptr;   // second blocking stream: uploads that overlap work on `stream`

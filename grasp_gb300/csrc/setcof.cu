@@ -20,6 +20,7 @@
 #include <cstring>
 #include <memory>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "gg_internal.cuh"
@@ -88,18 +89,27 @@ __global__ void k_by_csf(const double *__restrict__ evec, int ncf, int nev, doub
 // value also goes to diag. Bound: the FP64 pipe, one FMA per position and
 // level. (Formed per contribution, three operations per level and about 2.4
 // contributions per position, the label sums took 9.2 ms for 20,011 CSFs and
-// 10 levels; now 98 us, and 100 us for the sums.)
+// 10 levels; now 97 us, and 118 us for the sums.)
+// The positions [c0, c1) go to d (PART), or all of them.
 constexpr int LS_WARPS = 4;
+template <bool PART>
 __global__ void __launch_bounds__(LS_WARPS * 32) k_dsubrs_pos(const int64_t *__restrict__ iendc,
-                                                              const int32_t *__restrict__ irow, int ncf, int eol,
-                                                              int nev, const double *__restrict__ ev,
+                                                              const int32_t *__restrict__ irow, int64_t c0,
+                                                              int64_t c1, int ncf, int eol, int nev,
+                                                              const double *__restrict__ ev,
                                                               const double *__restrict__ wt, double *__restrict__ d,
                                                               double *__restrict__ diag) {
   __shared__ double sb[LS_WARPS][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = blockIdx.x * LS_WARPS + w;
   if (r >= ncf) return;
-  const int64_t p0 = iendc[r], p1 = iendc[r + 1];
+  int64_t p0 = iendc[r], p1 = iendc[r + 1];
+  if (PART) {
+    p0 = max(p0, c0);
+    p1 = min(p1, c1);
+    if (p0 >= p1) return;
+    d -= c0;
+  }
   for (int k0 = 0; k0 < (eol ? nev : 1); k0 += 32) {
     const int nk = min(32, nev - k0);
     if (eol) {
@@ -128,17 +138,27 @@ __global__ void __launch_bounds__(LS_WARPS * 32) k_dsubrs_pos(const int64_t *__r
 // :302-311 for the V lists), one block per label: its threads take every
 // 256th contribution, eight gathers in flight, and a fixed tree adds them. Lists
 // are uneven (a few labels hold tens of thousands of contributions), so the
-// longest label sets the time: 193 us with 128 threads and four gathers.
+// longest label sets the time: 193 us with 128 threads and four gathers. PART:
+// only the contributions of the positions [c0, c1), added to out unless c0 = 0.
 constexpr int LAB_THREADS = 256;
+template <bool PART>
 __global__ void __launch_bounds__(LAB_THREADS) k_label_sums(const int64_t *__restrict__ start,
                                                             const int32_t *__restrict__ loc,
                                                             const double *__restrict__ coeff,
-                                                            const double *__restrict__ d, double *__restrict__ out) {
+                                                            const double *__restrict__ d, int64_t c0, int64_t c1,
+                                                            double *__restrict__ out) {
   __shared__ double ws[LAB_THREADS / 32];
   const int64_t l = blockIdx.x, i0 = start[l], i1 = start[l + 1];
   double sum = 0.0;
 #pragma unroll 8
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += LAB_THREADS) sum = fma(__ldg(d + loc[i] - 1), coeff[i], sum);
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += LAB_THREADS) {
+    if (!PART) {
+      sum = fma(__ldg(d + loc[i] - 1), coeff[i], sum);
+    } else {
+      const int64_t p = loc[i] - 1 - c0;
+      if (p >= 0 && p < c1 - c0) sum = fma(__ldg(d + p), coeff[i], sum);
+    }
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
@@ -146,7 +166,7 @@ __global__ void __launch_bounds__(LAB_THREADS) k_label_sums(const int64_t *__res
   if (threadIdx.x == 0) {
     double v = ws[0];
     for (int w = 1; w < LAB_THREADS / 32; ++w) v += ws[w];
-    out[l] = v;
+    out[l] = PART && c0 ? out[l] + v : v;
   }
 }
 
@@ -164,7 +184,7 @@ struct DiagBlock {
 // forms them all: a < b, sum d qa qb over all CSFs and over those where a or b
 // is full; a = b, sum d qa (qa - 1) / 2 and sum d qa^2 over those where a is
 // full. (One warp per (J, IB, K), adding 32 terms at a time on one lane, took
-// 5.0 ms for 34 subshells and 20,011 CSFs; now 117 us.)
+// 5.0 ms for 34 subshells and 20,011 CSFs; now 139 us.)
 constexpr int DIAG_THREADS = 256;
 __global__ void __launch_bounds__(DIAG_THREADS) k_diag_pairs(const int *__restrict__ full,
                                                              const DiagBlock *__restrict__ blocks, int nblocks,
@@ -202,6 +222,9 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_diag_pairs(const int *__restri
   }
 }
 
+// positions of a block whose DSUBRS are held at a time; the fewest it is tried with
+constexpr int64_t SETCOF_POS = 1 << 27, SETCOF_POS_MIN = 1 << 16;
+
 template <class T> int upv(DBuf<T> &b, const std::vector<T> &h, cudaStream_t s) {
   GG_TRY(b.alloc(std::max<size_t>(1, h.size())));
   if (!h.empty()) GG_CUDA(cudaMemcpyAsync(b.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
@@ -224,6 +247,7 @@ int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *ne
   const Orbitals &o = ctx->orb;
   const int nw = o.nw;
   cudaStream_t s = ctx->stream;
+  const int64_t test_pos = std::exchange(ctx->test_setcof_pos, 0);
   auto st = std::make_shared<SetcofState>();
   st->nw = nw;
   std::vector<std::vector<int32_t>> labs;  // per block: the labels of all its lists
@@ -254,17 +278,29 @@ int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *ne
       GG_TRY(dwt[b].alloc(ncf));
       GG_CUDA(cudaMemcpyAsync(dwt[b].p, wt[b], ncf * sizeof(double), cudaMemcpyHostToDevice, s));
     }
-    // DSUBRS by position, then every label's sum
+    // DSUBRS by position, then every label's sum, SETCOF_POS positions (1 GB)
+    // at a time, fewer where the device has no room for them: beside the lists
+    // of a block that fills it, 8 bytes for every position need not fit. A
+    // piece costs one more reading of LOC.
     DBuf<double> dpos, dsum;
-    GG_TRY(dpos.alloc(std::max<int64_t>(1, m->nnz)));
+    int64_t len = std::max<int64_t>(1, std::min<int64_t>(m->nnz, test_pos > 0 ? test_pos : SETCOF_POS));
+    while (const int st_pos = dpos.alloc(len)) {
+      if (st_pos != GG_ERR_NOMEM || len <= SETCOF_POS_MIN) return st_pos;
+      len = (len + 1) / 2;
+    }
     GG_TRY(ddiag[b].alloc(ncf));
-    k_dsubrs_pos<<<(ncf + LS_WARPS - 1) / LS_WARPS, LS_WARPS * 32, 0, s>>>(m->dIendc.p, m->dIrow.p, ncf, eol ? 1 : 0, ne,
-                                                                          devec[b].p, dwt[b].p, dpos.p, ddiag[b].p);
-    ::gg::note_launch();
-    GG_TRY(dsum.alloc(std::max<int64_t>(1, L.nlab)));
-    if (L.nlab > 0) {
-      k_label_sums<<<(unsigned)L.nlab, LAB_THREADS, 0, s>>>(L.dStart.p, L.dLoc.p, L.dCoeff.p, dpos.p, dsum.p);
+    const bool part = len < m->nnz;
+    for (int64_t c0 = 0; c0 < m->nnz; c0 += len) {
+      const int64_t c1 = std::min(m->nnz, c0 + len);
+      (part ? k_dsubrs_pos<true> : k_dsubrs_pos<false>)<<<(ncf + LS_WARPS - 1) / LS_WARPS, LS_WARPS * 32, 0, s>>>(
+          m->dIendc.p, m->dIrow.p, c0, c1, ncf, eol ? 1 : 0, ne, devec[b].p, dwt[b].p, dpos.p, ddiag[b].p);
       ::gg::note_launch();
+      GG_TRY(dsum.alloc(std::max<int64_t>(1, L.nlab)));
+      if (L.nlab > 0) {
+        (part ? k_label_sums<true> : k_label_sums<false>)<<<(unsigned)L.nlab, LAB_THREADS, 0, s>>>(
+            L.dStart.p, L.dLoc.p, L.dCoeff.p, dpos.p, c0, c1, dsum.p);
+        ::gg::note_launch();
+      }
     }
     GG_CUDA(cudaGetLastError());
     labs.emplace_back(L.nlab);

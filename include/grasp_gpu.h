@@ -469,6 +469,11 @@ long long gg_launch_count(void);
  * with nothing in flight. The call then returns GG_ERR_TIMEOUT and leaves
  * no valid table; the context stays usable. tile < 0 cancels.             */
 int gg_test_stall_rk_tile(gg_ctx *ctx, int tile);
+/* Test hook of gg_setcof_prepare's bounded workspace: the next call on ctx
+ * works through each block `positions` element positions at a time, as it
+ * does with 2^27 for a block larger than that, or with fewer on a device
+ * that is nearly full. positions <= 0 cancels.                            */
+int gg_test_setcof_positions(gg_ctx *ctx, int64_t positions);
 long long gg_alloc_count(void);
 /* Page-locks (pins) caller memory so that uploads from it run at full link
  * rate; unregister before freeing it. */
