@@ -2054,11 +2054,8 @@ int gg_genintrk(gg_ctx *ctx, int kmax, int precision, int64_t *n_out, int *j2max
                            C.dAslot.p, C.dEA.p, C.dAt.p));
         ::gg::note_launch();
       }
-      static bool attr = false;
-      if (!attr) {
-        GG_CUDA(cudaFuncSetAttribute(k_rk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-        attr = true;
-      }
+      // (on every call: the attribute is the current device's)
+      GG_CUDA(cudaFuncSetAttribute(k_rk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
       // split-K: one CTA per SM holds a tile (shared memory), so with
       // fewer tiles than SMs each tile's grid chunks are cut into nsplit
       // ranges of at least TC_FLUSH chunks, whose partial sums
