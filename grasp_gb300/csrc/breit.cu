@@ -1337,7 +1337,6 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   }
   if (ni > INT32_MAX || nj > INT32_MAX) return fail(GG_ERR_RANGE, "gg_genintbreit: table too large");
   T.n = ni;
-  T.hInd.clear();
   const int R = (int)rows.size();
   if (ni == 0) return GG_OK;
   // the contraction takes orbitals that reach past the chains' start and end
@@ -1576,6 +1575,7 @@ int gg_genintbreit(gg_ctx *ctx, int type, double wfact, const double *e, double 
   if (j2max + 1 > KLIM) return fail(GG_ERR_ARG, "gg_genintbreit: 2j above 19");
   BreitTable &T = ctx->breit[type - 1];
   T.valid = false;
+  T.on_host = false;
   T.j2max = j2max;
   cudaStream_t s = ctx->stream;
   // TRIANGBREIT1 (rci90/triangbreit1.f90:27-46) and TRIANGBREIT2
@@ -1637,14 +1637,19 @@ int gg_brint(gg_ctx *ctx, int type, int ia, int ib, int ic, int id, int k, doubl
   const int nw = ctx->orb.nw, KEY = nw + 1;
   if (k < 0 || k > T.j2max || ia < 1 || ib < 1 || ic < 1 || id < 1 || ia > nw || ib > nw || ic > nw || id > nw)
     return fail(GG_ERR_NOTFOUND, "gg_brint: integral not in the table");
-  GG_CUDA(cudaSetDevice(ctx->device));
-  if (T.hInd.empty() && T.n) {
-    std::vector<int32_t> ind(T.n);
-    T.hVal.resize(T.n);
-    GG_CUDA(cudaMemcpyAsync(ind.data(), T.dInd.p, T.n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    GG_CUDA(cudaMemcpyAsync(T.hVal.data(), T.dVal.p, T.n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    GG_CUDA(cudaStreamSynchronize(ctx->stream));
-    T.hInd.swap(ind);
+  if (!T.on_host.load(std::memory_order_acquire)) {
+    std::lock_guard<std::mutex> lock(T.host_mu);
+    if (!T.on_host.load(std::memory_order_relaxed)) {
+      GG_CUDA(cudaSetDevice(ctx->device));
+      T.hInd.resize(T.n);
+      T.hVal.resize(T.n);
+      if (T.n) {
+        GG_CUDA(cudaMemcpyAsync(T.hInd.data(), T.dInd.p, T.n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+        GG_CUDA(cudaMemcpyAsync(T.hVal.data(), T.dVal.p, T.n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        GG_CUDA(cudaStreamSynchronize(ctx->stream));
+      }
+      T.on_host.store(true, std::memory_order_release);
+    }
   }
   const int32_t index = ((ia * KEY + ib) * KEY + ic) * KEY + id;
   const int32_t *b = T.hInd.data() + (T.kstart[k] - 1), *e = T.hInd.data() + (T.kstart[k + 1] - 1);

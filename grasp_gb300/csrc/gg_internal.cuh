@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -148,8 +149,12 @@ struct BreitTable {
   std::vector<int32_t> kstart;          // KSTARTBREIT(0:j2max+1), 1-based positions
   DBuf<int32_t> dInd;                   // INDTP
   DBuf<double> dVal;                    // VALTP
-  std::vector<int32_t> hInd;            // both on the host, from the first gg_brint on the table
+  // both on the host, from the first gg_brint on the table (several threads may
+  // look up one table: host_mu makes the copy, on_host publishes it)
+  std::vector<int32_t> hInd;
   std::vector<double> hVal;
+  std::mutex host_mu;
+  std::atomic<bool> on_host{false};
 };
 
 struct RkCache;  // radial.cu: GENINTRK's orbital-set structure, reused between calls
