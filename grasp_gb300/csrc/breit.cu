@@ -1273,6 +1273,7 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   const int nw = o.nw, KEY = nw + 1, np = g.np;
   const size_t msz = (size_t)(nw + 1) * (nw + 1);
   const auto th0 = std::chrono::steady_clock::now();
+  *plan_ms = *kernel_ms = 0.0;
   // rows: the admitted pairs of each k in (a, b) order, padded to whole warps
   std::vector<BrRow> rows;
   std::vector<int> lo(j2max + 2, 0), cnt(j2max + 1, 0);
@@ -1344,7 +1345,7 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   const bool plain = m0 >= BR_MIN_MF && maxm <= g.n;
 
   // the operators, forward vectors and class sums need no buckets: they run
-  // while the host waits for the heads and builds them
+  // while the host builds these from the heads
   const int nch = type == 1 ? 1 : 3, nset = type == 1 ? 1 : 2;
   const size_t plane = plain ? (size_t)(maxm + 1) * R : 0;
   const int j0 = 5 + 4 * ((m0 - 9) / 4);
@@ -1396,13 +1397,12 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   GG_CUDA(cudaEventCreate(&e0));
   GG_CUDA(cudaEventCreate(&e1));
   struct Ev {
-    cudaEvent_t a, b, c;
+    cudaEvent_t a, b;
     ~Ev() {
       cudaEventDestroy(a);
       cudaEventDestroy(b);
-      if (c) cudaEventDestroy(c);
     }
-  } ev{e0, e1, nullptr};
+  } ev{e0, e1};
   GG_CUDA(cudaEventRecord(e0, s));
   GG_CUDA(cudaMemsetAsync(dnredo.p, 0, sizeof(int), s));
   k_br_rho<<<dim3(nw, nw), 128, 0, s>>>(nw, o.dPF.p, o.dQF.p, o.ld, o.dMF.p, np, drho.p);
@@ -1412,10 +1412,7 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   ::gg::note_launch();
   std::vector<unsigned char> heads((size_t)3 * R);
   GG_CUDA(cudaMemcpyAsync(heads.data(), dheads.p, heads.size(), cudaMemcpyDeviceToHost, s));
-  cudaEvent_t eh = nullptr;
-  GG_CUDA(cudaEventCreateWithFlags(&eh, cudaEventDisableTiming));
-  ev.c = eh;
-  GG_CUDA(cudaEventRecord(eh, s));
+  GG_CUDA(cudaStreamSynchronize(s));  // the densities and heads, a few us of kernels
   if (nb > 0) {
     k_bessel<<<nb, 128, 0, s>>>(dbd.p, g.dR.p, std::min(maxm, g.n), np, P.epsi, dBJ.p, dBN.p);
     ::gg::note_launch();
@@ -1436,7 +1433,6 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
     }
     k_br_base<<<dim3(R / 32, (j0 + 31) / 32, nset), dim3(32, 8), 0, s>>>(drows.p, A, g.q, fold);
     ::gg::note_launch();
-    GG_CUDA(cudaEventSynchronize(eh));
 
     // buckets: the columns of each (set, k) by (MTP, head as a source)
     bool moving = false;
@@ -1508,9 +1504,9 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
                                T.dVal.p, dredo.p, dnredo.p);
   ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
+  *plan_ms = 1e3 * std::chrono::duration<double>(std::chrono::steady_clock::now() - th0).count();
   int nredo = 0;
   GG_CUDA(cudaMemcpyAsync(&nredo, dnredo.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  *plan_ms = 1e3 * std::chrono::duration<double>(std::chrono::steady_clock::now() - th0).count();
   GG_CUDA(cudaStreamSynchronize(s));
   if (nredo > 0) {
     // k_bessel ran to the longest orbital, which covers every term
@@ -1534,7 +1530,6 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
       done += n;
     }
   }
-  ctx->stats[34] = nredo;
   GG_CUDA(cudaEventRecord(e1, s));
   GG_CUDA(cudaStreamSynchronize(s));
   float ms = 0.f;

@@ -405,8 +405,9 @@ int gg_maneig_batched(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *nv
  * 30 block passes of the last split gg_maneig whose second Gram-Schmidt
  * pass was skipped (the first kept at least half of every new column's
  * squared norm), 31 device and host ms of the last gg_genintbreit, 32 / 33
- * its host ms from the table's planning to its last launch (one wait for the
- * kernels in it) / its device ms of the Bessel and table kernels.                                                            */
+ * its host ms from the table's planning to its last launch (with one wait,
+ * for the pairs' head indexes) / its device ms of the Bessel and table
+ * kernels.                                                                  */
 double gg_stage_stat(gg_ctx *ctx, int which);
 
 /* gg_projected_eig: DVDSON's projected eigenproblem, CALL DSPEVX('Vectors
