@@ -264,8 +264,8 @@ __global__ void k_apairs(const int2 *__restrict__ pairs, int npairs, const doubl
   if (p >= npairs) return;
   const int a = pairs[p].x, c = pairs[p].y;
   const int m = min(MF[a], MF[c]);
-  // the last row is followed by zeros: k_rk_dot reads up to three points past
-  // a row's last one
+  // the last row is followed by KC_TILE zeros: k_rk_dot reads up to G - 1
+  // points past a row's last one
   const int end = p + 1 < npairs ? KC : KC + KC_TILE;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
     double v = 0.0, rho = 0.0;
@@ -366,6 +366,8 @@ __global__ void __launch_bounds__(128) k_rk_dot(const RkTile *__restrict__ tiles
   // A(m + 1) is zero (the row's end or point 0 of the next row); the last
   // group's loads reach up to G - 1 points past m, its sums stop at m
   constexpr int G = NR >= 8 ? 4 : NR == 4 ? 8 : 16;
+  static_assert(G - 1 <= KC_TILE, "the loads past the last pair's points stay in k_apairs's zeros");
+  static_assert(G - 1 <= GPAD, "the loads past the last function's points stay in its row");
   double2 cy[G / 2], ca[NR][G / 2];
   auto load = [&](int i, double2 *yv, double2(*av)[G / 2]) {
 #pragma unroll
