@@ -40,12 +40,9 @@ void note_alloc();
 // scheduled while the kernel before it on the stream is still running, so
 // that its launch overlaps that kernel's last wave; it must call pdl_wait()
 // before it touches memory (griddepcontrol.wait returns once every
-// prerequisite grid has completed and its writes are visible). pdl_trigger()
-// lets the next such kernel be scheduled (it only starts waiting: the
-// ordering is kept by its own pdl_wait). In a stream capture the launches
-// become programmatic graph edges.
+// prerequisite grid has completed and its writes are visible). In a stream
+// capture the launches become programmatic graph edges.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                               Args &&...args) {

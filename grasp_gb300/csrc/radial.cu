@@ -432,8 +432,6 @@ __global__ void __launch_bounds__(128) k_rk_dot(const RkTile *__restrict__ tiles
 // ---------------------------------------------------------------------------
 constexpr int OZ_S = 10;
 
-// General per-integral QUAD: TA(i) = ((P_a P_c + Q_a Q_c) RPOR) Y_f(i),
-// one warp per integral, sequential reference-order sum on lane 0.
 // ---------------------------------------------------------------------------
 // The Ozaki contraction on GB300's fifth-generation tensor cores (tcgen05).
 //
@@ -938,7 +936,9 @@ __global__ void k_rk_finish_all(const int32_t *__restrict__ ind, long long n, co
   }
 }
 
-__global__ void k_quad_items(const QuadItem *__restrict__ items, const int *__restrict__ nitems_p, int nitems_max,
+// General per-integral QUAD (SLATER): TA(i) = ((P_a P_c + Q_a Q_c) RPOR) Y_f(i),
+// one warp per integral, sequential reference-order sum on lane 0.
+__global__ void k_quad_items(const QuadItem *__restrict__ items, int nitems,
                              const double *__restrict__ Y, int np, const double *__restrict__ PF,
                              const double *__restrict__ QF, int ld, const double *__restrict__ R,
                              const double *__restrict__ RP, const double *__restrict__ RPOR, QuadConst q,
@@ -947,7 +947,6 @@ __global__ void k_quad_items(const QuadItem *__restrict__ items, const int *__re
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   double *TA = sm + (size_t)warp * np;
-  const int nitems = nitems_p ? min(*nitems_p, nitems_max) : nitems_max;
   for (int it = blockIdx.x * wpb + warp; it < nitems; it += gridDim.x * wpb) {
     const QuadItem w = items[it];
     const double *Yf = Y + (size_t)w.f * np;
@@ -2222,7 +2221,7 @@ int gg_slater(gg_ctx *ctx, int ia, int ib, int ic, int id, int k, double *out) {
   GG_TRY(dY.alloc(g.np));
   GG_TRY(dout.alloc(1));
   GG_TRY(build_y(ctx, dy.p, 1, dY.p, scratch));
-  k_quad_items<<<1, 32, g.np * sizeof(double), ctx->stream>>>(di.p, nullptr, 1, dY.p, g.np, o.dPF.p, o.dQF.p, o.ld,
+  k_quad_items<<<1, 32, g.np * sizeof(double), ctx->stream>>>(di.p, 1, dY.p, g.np, o.dPF.p, o.dQF.p, o.ld,
                                                              g.dR.p, g.dRP.p, g.dRPOR.p, g.q, dout.p); ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
   GG_CUDA(cudaMemcpyAsync(out, dout.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2686,7 +2685,7 @@ extern "C" int gg_slater_noalloc(gg_ctx *ctx, int ia, int ib, int ic, int id, in
   GG_CUDA(cudaMemsetAsync(Y, 0, (size_t)np * sizeof(double), ctx->stream));
   k_ychain<<<1, 128, 0, ctx->stream>>>(dyd, 1, nullptr, TZ, TW, g.dR.p, g.dPow.p, np, g.q, Y);
   ::gg::note_launch();
-  k_quad_items<<<1, 32, np * sizeof(double), ctx->stream>>>(ditem, nullptr, 1, Y, np, o.dPF.p, o.dQF.p, o.ld, g.dR.p,
+  k_quad_items<<<1, 32, np * sizeof(double), ctx->stream>>>(ditem, 1, Y, np, o.dPF.p, o.dQF.p, o.ld, g.dR.p,
                                                             g.dRP.p, g.dRPOR.p, g.q, dout);
   ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
