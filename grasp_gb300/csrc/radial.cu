@@ -937,16 +937,17 @@ __global__ void k_rk_finish_all(const int32_t *__restrict__ ind, long long n, co
 }
 
 // General per-integral QUAD (SLATER): TA(i) = ((P_a P_c + Q_a Q_c) RPOR) Y_f(i),
-// one warp per integral, sequential reference-order sum on lane 0.
+// one warp per integral, sequential reference-order sum on lane 0. TA lies in
+// shared memory, or in `work` (np doubles per warp) on a grid too long for it.
 __global__ void k_quad_items(const QuadItem *__restrict__ items, int nitems,
                              const double *__restrict__ Y, int np, const double *__restrict__ PF,
                              const double *__restrict__ QF, int ld, const double *__restrict__ R,
                              const double *__restrict__ RP, const double *__restrict__ RPOR, QuadConst q,
-                             double *__restrict__ out) {
+                             double *work, double *__restrict__ out) {
   extern __shared__ double sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
-  double *TA = sm + (size_t)warp * np;
+  double *TA = work ? work + ((size_t)blockIdx.x * wpb + warp) * np : sm + (size_t)warp * np;
   for (int it = blockIdx.x * wpb + warp; it < nitems; it += gridDim.x * wpb) {
     const QuadItem w = items[it];
     const double *Yf = Y + (size_t)w.f * np;
@@ -2221,8 +2222,12 @@ int gg_slater(gg_ctx *ctx, int ia, int ib, int ic, int id, int k, double *out) {
   GG_TRY(dY.alloc(g.np));
   GG_TRY(dout.alloc(1));
   GG_TRY(build_y(ctx, dy.p, 1, dY.p, scratch));
-  k_quad_items<<<1, 32, g.np * sizeof(double), ctx->stream>>>(di.p, 1, dY.p, g.np, o.dPF.p, o.dQF.p, o.ld,
-                                                             g.dR.p, g.dRP.p, g.dRPOR.p, g.q, dout.p); ::gg::note_launch();
+  // (the long grid's TA goes where build_y had its TEMP arrays)
+  const size_t smem = g.np * sizeof(double);
+  const bool sh = smem <= SMEM_PLAIN;
+  k_quad_items<<<1, 32, sh ? smem : 0, ctx->stream>>>(di.p, 1, dY.p, g.np, o.dPF.p, o.dQF.p, o.ld, g.dR.p, g.dRP.p,
+                                                      g.dRPOR.p, g.q, sh ? nullptr : scratch.p, dout.p);
+  ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
   GG_CUDA(cudaMemcpyAsync(out, dout.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   GG_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -2686,7 +2691,7 @@ extern "C" int gg_slater_noalloc(gg_ctx *ctx, int ia, int ib, int ic, int id, in
   k_ychain<<<1, 128, 0, ctx->stream>>>(dyd, 1, nullptr, TZ, TW, g.dR.p, g.dPow.p, np, g.q, Y);
   ::gg::note_launch();
   k_quad_items<<<1, 32, np * sizeof(double), ctx->stream>>>(ditem, 1, Y, np, o.dPF.p, o.dQF.p, o.ld, g.dR.p,
-                                                            g.dRP.p, g.dRPOR.p, g.q, dout);
+                                                            g.dRP.p, g.dRPOR.p, g.q, nullptr, dout);
   ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
   GG_CUDA(cudaMemcpyAsync(out, dout, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));

@@ -1,10 +1,11 @@
-"""RINTI, the I(ab) table and SETLAG on grids around the lengths where their
-working arrays leave shared memory (k_rinti above 1,174 points, k_setlag_quad
-above 24,024), against the oracle.
+"""RINTI, the I(ab) table, SETLAG and SLATER on grids around the lengths where
+their working arrays leave shared memory (k_rinti above 1,174 points,
+k_setlag_quad above 24,024, k_quad_items above 5,990), against the oracle.
 
 Bars: a RINTI runs the oracle's operations in their order up to QUAD's log, so
 1e-12 of the table's largest value holds with room for the cancellation of its
-four integrals; the multipliers' bar is test_setlag_matches_oracle's."""
+four integrals; the multipliers' bar is test_setlag_matches_oracle's; a SLATER
+runs the oracle's operations in their order up to QUAD's log: 1e-14."""
 import numpy as np
 import pytest
 
@@ -34,3 +35,11 @@ def test_one_electron_integrals_and_multipliers(gpu_ready, oracle_mod, n):
         lfix[[1, 2]] = fixed
         ecv, ecv0 = ctx.setlag(iecc, ucf, lfix, cofs), o.setlag(iecc, ucf, lfix, cofs)
         assert np.abs(ecv - ecv0).max() <= 1e-12 * max(1.0, np.abs(ecv0).max())
+
+
+@pytest.mark.parametrize("n", [590, 5990, 5991, 24537])
+def test_slater(gpu_ready, oracle_mod, n):
+    o, ctx, _ = _setup(n, 23.6 / n)
+    for a, b, c, d, k in [(1, 2, 1, 2, 0), (3, 8, 8, 3, 0), (2, 4, 7, 5, 1), (6, 6, 6, 6, 2), (8, 7, 8, 7, 0)]:
+        v, v0 = ctx.slater(a, b, c, d, k), o.slater(a, b, c, d, k)
+        assert abs(v - v0) <= 1e-14 * abs(v0), (a, b, c, d, k)
