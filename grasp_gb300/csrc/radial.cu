@@ -85,8 +85,9 @@ __device__ double quad_seq(double *TA, int mtp, const double *R, const double *R
   return 0.0;
 }
 
-// dynamic shared memory of any launch without opting in: 48 KB less the 1 KB
-// that a kernel with a static array takes
+// dynamic shared memory of a launch without opting in: 48 KB less the 1 KB that
+// a static array takes before it (the dynamic arrays of this file start on
+// k_rk_tc's 1,024-byte alignment)
 constexpr size_t SMEM_PLAIN = 47 * 1024;
 __host__ __device__ constexpr int quad_panels(int np) { return np / 4 + 4; }
 
@@ -2399,7 +2400,10 @@ static int run_potentials(gg_ctx *ctx, PotWork &W, const std::vector<PotJob> &jo
                                         diorb, W.coef.p, info);
     ::gg::note_launch();
   }
-  if ((size_t)7 * nfb * g.np * sizeof(double) > POT_BOUND) {  // too much to reserve for a bound: wait for the number
+  if ((size_t)7 * nfb * g.np * sizeof(double) > POT_BOUND) {
+    // too much to reserve for a bound: wait for the number. (7 arrays: Y and
+    // the six of the long grids' build; k_yfun's grids need Y only and could
+    // reserve seven times as many functions.)
     int cnt = 0;
     GG_CUDA(cudaMemcpyAsync(&cnt, info, sizeof(int), cudaMemcpyDeviceToHost, s));
     GG_CUDA(cudaStreamSynchronize(s));

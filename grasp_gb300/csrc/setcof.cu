@@ -10,12 +10,13 @@
 // through the final 1/UCF(J), so here one pass computes them for every label
 // of every block, together with the diagonal FCO/GCO sums of every pair of
 // orbitals. DSUBRS depends on the position only, so it is formed once per EMT
-// position (k_dsubrs_pos) and a contribution costs one FMA. The same pass
-// decodes every label once on the host and leaves each orbital's lists up to
-// the division by UCF(J), in the reference's order (FCO, GCO, the T list by
-// block, the V^k lists by k and block), so they are the reference's entry for
-// entry and a call for orbital J only divides. (Decoding the labels per
-// orbital took 3.4 of a 3.85 ms SETCOF over 34 subshells.)
+// position (k_dsubrs_pos) and a contribution costs one FMA. The labels are
+// decoded and their sums listed by orbital at the same time, so that a call
+// for orbital J reads its own labels only; it forms the lists in the
+// reference's order (FCO, GCO, the T list by block, the V^k lists by k and
+// block), so they are the reference's entry for entry. (Forming every
+// orbital's lists beforehand cost a caller who wants one of them the merging of
+// all: 17.9 ms for five blocks over 23 subshells, now 2.7 and 0.44 a call.)
 #include <algorithm>
 #include <cstring>
 #include <memory>
@@ -27,16 +28,11 @@
 
 namespace gg {
 
-// One list of one orbital: its labels, and the values added to them in order,
-// each before the division by UCF(J). A value's entry is `at`; the first value
-// of an entry sets it (the labels of a later block that repeat one join it).
+// One list of one orbital: its labels and values. The labels of a later block
+// (merge) that repeat one join its first entry.
 struct SetcofList {
-  struct Add {
-    int at;
-    double v;
-  };
   std::vector<int32_t> lab;
-  std::vector<Add> add;
+  std::vector<double> val;
   std::unordered_map<int32_t, int> first;  // first entry of each label, filled when merging
   size_t merged = 0;                       // labels entered into `first` so far
   void put(int32_t l, double v, bool merge) {
@@ -44,30 +40,36 @@ struct SetcofList {
       for (; merged < lab.size(); ++merged) first.emplace(lab[merged], (int)merged);
       const auto f = first.find(l);
       if (f != first.end()) {
-        add.push_back(Add{f->second, v});
+        val[f->second] = val[f->second] + v;
         return;
       }
     }
-    add.push_back(Add{(int)lab.size(), v});
     lab.push_back(l);
-  }
-  void write(double ucf, int32_t *label, double *val) const {
-    std::copy(lab.begin(), lab.end(), label);
-    int n = 0;
-    for (const Add &a : add) {
-      const double v = a.v / ucf;
-      if (a.at == n)
-        val[n++] = v;
-      else
-        val[a.at] = val[a.at] + v;
-    }
+    val.push_back(v);
   }
 };
 
-// the lists of the last gg_setcof_prepare, [orbital] YPOT, XPOT, DACON
+// A label: half its sum, and its orbitals, a byte each (KEYORB = 215): a, b, c,
+// d of R^k(ab;cd); a T label stays as it is
+struct SetcofLabel {
+  double v;
+  uint32_t ix;
+  uint8_t k;
+  uint8_t places;  // bit f: the f-th orbital stands in no earlier place
+  bool merge;      // not of the first block
+};
+
+// the sums of the last gg_setcof_prepare
 struct SetcofState {
   int nw = 0;
-  std::vector<SetcofList> y, x, d;
+  std::vector<int> nak, nkj;        // of the orbital set, 1-based
+  std::vector<double> diag;         // k_diag_pairs' sums
+  std::vector<SetcofLabel> labels;  // in SETCOF's order: the T lists by block, the V^k lists by k and block
+  size_t nt = 0;                    // of them T labels
+  // [ref0[j], ref0[j + 1]): the labels that name orbital j, in order, as 4 l +
+  // the place that names it first (T: 0 or 1)
+  std::vector<uint32_t> refs;
+  std::vector<size_t> ref0;
 };
 
 namespace {
@@ -324,99 +326,75 @@ int gg_setcof_prepare(gg_ctx *ctx, int nblocks, gg_hmat *const *h, const int *ne
   k_diag_pairs<<<dim3(nw, nw), DIAG_THREADS, 0, s>>>(dfull.p, dblocks.p, nblocks, nw, dout.p);
   ::gg::note_launch();
   GG_CUDA(cudaGetLastError());
-  std::vector<double> hv((size_t)2 * nw * nw);
-  GG_CUDA(cudaMemcpyAsync(hv.data(), dout.p, hv.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+  st->diag.resize((size_t)2 * nw * nw);
+  GG_CUDA(cudaMemcpyAsync(st->diag.data(), dout.p, st->diag.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaStreamSynchronize(s));
-  st->y.resize(nw + 1);
-  st->x.resize(nw + 1);
-  st->d.resize(nw + 1);
-  const int KEY = KEYORB;
-  for (int j = 1; j <= nw; ++j)
-    for (int ib = 1; ib <= nw; ++ib) {
-      const double *v = &hv[2 * ((size_t)(std::min(j, ib) - 1) * nw + (std::max(j, ib) - 1))];
-      // Y from FCO (setcof.f90:73-105): NYA = K + IB KEY (KEY + 1)
-      const int64_t ly = (int64_t)ib * KEY * (KEY + 1);
-      if (ib == j) {
-        st->y[j].put((int32_t)ly, 2.0 * v[0], false);
-        for (int k = 2; k <= o.nkj[j] - 1; k += 2) {
-          const double c = clrx_host(o.nak[j], k, o.nak[j]);
-          st->y[j].put((int32_t)(k + ly), -(c * c * v[1]), false);
-        }
-        continue;
-      }
-      st->y[j].put((int32_t)ly, v[0], false);
-      // X from GCO (:107-147): NXA = K + KEY J + IB KEY^2 (KEY + 1)
-      const int64_t lx = (int64_t)KEY * j + (int64_t)ib * KEY * KEY * (KEY + 1);
-      const int kmin = (o.nak[j] * o.nak[ib] > 0) ? std::abs((o.nkj[j] - o.nkj[ib]) / 2)
-                                                   : std::abs((o.nkj[j] - o.nkj[ib]) / 2) + 1;
-      for (int k = kmin; k <= (o.nkj[j] + o.nkj[ib]) / 2; k += 2) {
-        const double c = clrx_host(o.nak[j], k, o.nak[ib]);
-        st->x[j].put((int32_t)(k + lx), -(c * c * v[1]), false);
-      }
-    }
-  // DA from the T lists, block by block (:188-285)
+  st->nak = o.nak;
+  st->nkj = o.nkj;
+  // the labels in order, and how many name each orbital
+  int64_t total = 0;
   int kmaxf = -1;
   for (int b = 0; b < nblocks; ++b) {
+    total += h[b]->lists->nlab;
+    kmaxf = std::max(kmaxf, h[b]->lists->kmaxf);
+  }
+  if (total > UINT32_MAX / 4) return fail(GG_ERR_RANGE, "gg_setcof_prepare: more than 2^30 - 1 labels");
+  const int KEY = KEYORB;
+  std::vector<SetcofLabel> &labels = st->labels;
+  labels.reserve(total);
+  std::vector<size_t> &ref0 = st->ref0;
+  ref0.assign(258, 0);  // by byte; those that are no orbital of the set are not read
+  auto named = [&](int a) { return a >= 1 && a <= nw; };
+  // T labels (setcof.f90:188-285): DA of orbital a at b, of b at a
+  for (int b = 0; b < nblocks; ++b) {
     const Lists &L = *h[b]->lists;
-    kmaxf = std::max(kmaxf, L.kmaxf);
     for (int64_t l = L.list_lab0[0]; l < L.list_lab0[1]; ++l) {
       const int32_t lab = labs[b][l];
-      const int ia = lab % KEY, ib = lab / KEY;
-      const double v = 0.5 * sums[b][l];
-      if (ia >= 1 && ia <= nw) st->d[ia].put(ib, v, b > 0);
-      if (ib != ia && ib >= 1 && ib <= nw) st->d[ib].put(ia, v, b > 0);
+      const int x = lab % KEY, y = lab / KEY;
+      const int places = (named(x) ? 1 : 0) | (y != x && named(y) ? 2 : 0);
+      labels.push_back(SetcofLabel{0.5 * sums[b][l], (uint32_t)lab, 0, (uint8_t)places, b > 0});
+      if (places & 1) ++ref0[x + 1];
+      if (places & 2) ++ref0[y + 1];
     }
   }
-  // the V^k lists, k by k and block by block (:287-515): INDEXS = (a, b, c, d)
-  // of R^k(ab;cd), each orbital named in it
+  st->nt = labels.size();
+  // V^k labels (:287-515)
   for (int k = 0; k <= kmaxf; ++k)
     for (int b = 0; b < nblocks; ++b) {
       const Lists &L = *h[b]->lists;
       if (k > L.kmaxf) continue;
-      const bool merge = b > 0;
       for (int64_t l = L.list_lab0[k + 1]; l < L.list_lab0[k + 2]; ++l) {
         if (labs[b][l] < 0) continue;
         uint32_t lab = (uint32_t)labs[b][l];  // unsigned: the divisions by KEY are multiplications
-        int ix[4];
+        uint32_t ix[4];
         ix[3] = lab % KEYORB;
         lab /= KEYORB;
         ix[1] = lab % KEYORB;
         lab /= KEYORB;
         ix[2] = lab % KEYORB;
-        ix[0] = lab / KEYORB;
-        const double v = 0.5 * sums[b][l];
-        for (int f = 0; f < 4; ++f) {
-          const int j = ix[f];
-          if (j < 1 || j > nw) continue;
-          int irank = 0, second = f, other = j;
-          bool seen = false;
-          for (int u = 0; u < 4; ++u) {
-            if (ix[u] != j) {
-              other = ix[u];
-              continue;
-            }
-            seen = seen || u < f;
-            if (++irank == 2) second = u;
-          }
-          if (seen) continue;  // done at its first place
-          const int o1 = ix[(f + 1) & 3], o2 = ix[(f + 2) & 3], o3 = ix[(f + 3) & 3];
-          const int32_t lx = ((o2 * KEY + o3) * KEY + o1) * KEY + k;
-          if (irank == 1) {
-            st->x[j].put(lx, v, merge);
-          } else if (irank == 2) {
-            if (second - f == 2)
-              st->y[j].put((o3 * KEY + o1) * KEY + k, v + v, merge);
-            else
-              st->x[j].put(lx, v + v, merge);
-          } else if (irank == 3) {
-            st->y[j].put((other * KEY + j) * KEY + k, v + v, merge);
-            st->x[j].put(((other * KEY + j) * KEY + j) * KEY + k, v, merge);
-          } else {
-            st->y[j].put((j * KEY + j) * KEY + k, 4.0 * v, merge);
-          }
-        }
+        ix[0] = lab / KEYORB;  // at most 216: 2^31 / KEYORB^3
+        const int places = 1 | (ix[1] != ix[0]) << 1 | (ix[2] != ix[0] && ix[2] != ix[1]) << 2 |
+                           (ix[3] != ix[0] && ix[3] != ix[1] && ix[3] != ix[2]) << 3;
+        labels.push_back(SetcofLabel{0.5 * sums[b][l], ix[0] | ix[1] << 8 | ix[2] << 16 | ix[3] << 24, (uint8_t)k,
+                                     (uint8_t)places, b > 0});
+        for (int f = 0; f < 4; ++f) ref0[ix[f] + 1] += places >> f & 1;
       }
     }
+  for (int a = 1; a <= 257; ++a) ref0[a] += ref0[a - 1];
+  std::vector<uint32_t> &refs = st->refs;
+  refs.resize(ref0[257]);
+  std::vector<size_t> at(ref0);
+  for (size_t l = 0; l < labels.size(); ++l) {
+    const SetcofLabel &L = labels[l];
+    if (l < st->nt) {
+      const int32_t lab = (int32_t)L.ix;
+      if (L.places & 1) refs[at[lab % KEY]++] = (uint32_t)(4 * l);
+      if (L.places & 2) refs[at[lab / KEY]++] = (uint32_t)(4 * l + 1);
+      continue;
+    }
+    for (int f = 0; f < 4; ++f)
+      if (L.places >> f & 1) refs[at[L.ix >> 8 * f & 255]++] = (uint32_t)(4 * l + f);
+  }
   ctx->setcof = st;
   return GG_OK;
 }
@@ -428,15 +406,77 @@ int gg_setcof(gg_ctx *ctx, int j, double ucfj, int cap, int *ny, int32_t *nya, d
   const auto st = std::static_pointer_cast<SetcofState>(ctx->setcof);
   if (!st) return fail(GG_ERR_STATE, "gg_setcof: call gg_setcof_prepare first");
   if (j < 1 || j > st->nw || ctx->orb.nw != st->nw) return fail(GG_ERR_ARG, "gg_setcof: orbital outside the orbital set");
-  const SetcofList &ly = st->y[j], &lx = st->x[j], &ld = st->d[j];
+  const int nw = st->nw, KEY = KEYORB;
+  const std::vector<int> &nak = st->nak, &nkj = st->nkj;
+  SetcofList ly, lx, ld;
+  const uint32_t *ref = st->refs.data() + st->ref0[j], *end = st->refs.data() + st->ref0[j + 1];
+  for (SetcofList *l : {&ly, &lx}) {
+    l->lab.reserve(end - ref + 16 * nw);
+    l->val.reserve(end - ref + 16 * nw);
+  }
+  for (int ib = 1; ib <= nw; ++ib) {
+    const double *v = &st->diag[2 * ((size_t)(std::min(j, ib) - 1) * nw + (std::max(j, ib) - 1))];
+    // Y from FCO (setcof.f90:73-105): NYA = K + IB KEY (KEY + 1)
+    const int64_t l0 = (int64_t)ib * KEY * (KEY + 1);
+    if (ib == j) {
+      ly.put((int32_t)l0, 2.0 * v[0] / ucfj, false);
+      for (int k = 2; k <= nkj[j] - 1; k += 2) {
+        const double c = clrx_host(nak[j], k, nak[j]);
+        ly.put((int32_t)(k + l0), -(c * c * v[1]) / ucfj, false);
+      }
+      continue;
+    }
+    ly.put((int32_t)l0, v[0] / ucfj, false);
+    // X from GCO (:107-147): NXA = K + KEY J + IB KEY^2 (KEY + 1)
+    const int64_t x0 = (int64_t)KEY * j + (int64_t)ib * KEY * KEY * (KEY + 1);
+    const int kmin = (nak[j] * nak[ib] > 0) ? std::abs((nkj[j] - nkj[ib]) / 2) : std::abs((nkj[j] - nkj[ib]) / 2) + 1;
+    for (int k = kmin; k <= (nkj[j] + nkj[ib]) / 2; k += 2) {
+      const double c = clrx_host(nak[j], k, nak[ib]);
+      lx.put((int32_t)(k + x0), -(c * c * v[1]) / ucfj, false);
+    }
+  }
+  for (; ref != end; ++ref) {
+    const size_t l = *ref >> 2;
+    const int f = *ref & 3;
+    const SetcofLabel &L = st->labels[l];
+    const bool merge = L.merge;
+    const double v = L.v;
+    if (l < st->nt) {
+      ld.put(f ? (int32_t)L.ix % KEY : (int32_t)L.ix / KEY, v / ucfj, merge);
+      continue;
+    }
+    // the orbitals after J's first place, wrapped round: those that are J again
+    // stand in later places
+    const uint32_t r = f == 3 ? L.ix : L.ix >> 8 * (f + 1) | L.ix << 8 * (3 - f);
+    const int o1 = r & 255, o2 = r >> 8 & 255, o3 = r >> 16 & 255, k = L.k;
+    const int again = (o1 == j) + (o2 == j) + (o3 == j);
+    if (again == 0) {
+      lx.put(((o2 * KEY + o3) * KEY + o1) * KEY + k, v / ucfj, merge);
+    } else if (again == 1) {
+      if (o2 == j)
+        ly.put((o3 * KEY + o1) * KEY + k, (v + v) / ucfj, merge);
+      else
+        lx.put(((o2 * KEY + o3) * KEY + o1) * KEY + k, (v + v) / ucfj, merge);
+    } else if (again == 2) {
+      const int other = o1 != j ? o1 : o2 != j ? o2 : o3;
+      ly.put((other * KEY + j) * KEY + k, (v + v) / ucfj, merge);
+      lx.put(((other * KEY + j) * KEY + j) * KEY + k, v / ucfj, merge);
+    } else {
+      ly.put((j * KEY + j) * KEY + k, 4.0 * v / ucfj, merge);
+    }
+  }
   *ny = (int)ly.lab.size();
   *nx = (int)lx.lab.size();
   *nd = (int)ld.lab.size();
   if (*ny > cap || *nx > cap || *nd > cap)
     return fail(GG_ERR_RANGE, "gg_setcof: a list is longer than cap (the counts are set)");
-  ly.write(ucfj, nya, ya);
-  lx.write(ucfj, nxa, xa);
-  ld.write(ucfj, nda, da);
+  auto give = [](const SetcofList &l, int32_t *lab, double *val) {
+    std::copy(l.lab.begin(), l.lab.end(), lab);
+    std::copy(l.val.begin(), l.val.end(), val);
+  };
+  give(ly, nya, ya);
+  give(lx, nxa, xa);
+  give(ld, nda, da);
   return GG_OK;
 }
 
