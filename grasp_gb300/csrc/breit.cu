@@ -1124,25 +1124,27 @@ __global__ void k_br_table(const BrRow *__restrict__ rows, const int *__restrict
   }
 }
 
-// an entry of the table term by term: one thread per (entry, term), then the
+// an entry of the table term by term: one thread per (entry, term), 2^tsh terms
+// to an entry (4, or 2 in a type 2 table without a frequency, whose warps would
+// be half empty: 15.4 ms for 120,818 entries, 8.4 so), then the
 // combination. A launch takes up to BR_REDO entries of the list: enough threads
 // for many waves, 4 n and a thread's index stay ints whatever the table's size
 // (up to 2^31 - 1 integrals), and the terms' values take 17 MB instead of 32
 // bytes for every entry of the list.
 constexpr int BR_REDO = 1 << 19;
 static_assert(4LL * BR_REDO + 128 <= INT32_MAX, "k_br_redo's thread index is an int");
-__global__ void __launch_bounds__(128) k_br_redo(int type, const BrRedo *__restrict__ redo, int n,
+__global__ void __launch_bounds__(128) k_br_redo(int type, int tsh, const BrRedo *__restrict__ redo, int n,
                                                  const BrRow *__restrict__ rows, PlanTabs T, TermTabs tt, QuadConst q,
                                                  double *__restrict__ v, BrInt *__restrict__ ints) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 4 * n) return;
-  const BrRedo e = redo[t >> 2];
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> tsh, u = t & ((1 << tsh) - 1);
+  if (i >= n) return;
+  const BrRedo e = redo[i];
   const BrRow a = rows[e.row], c = rows[e.col];
   BrJob jb[4];
   BrInt bi;
-  const int k = plan_one(type, a.a, a.b, c.a, c.b, a.K, T, (t >> 2) * 4, &bi, jb);
-  if ((t & 3) == 0) ints[t >> 2] = bi;
-  if ((t & 3) < k) v[t] = breit_term(jb[t & 3], tt, q);
+  const int k = plan_one(type, a.a, a.b, c.a, c.b, a.K, T, i << tsh, &bi, jb);
+  if (u == 0) ints[i] = bi;
+  if (u < k) v[t] = breit_term(jb[u], tt, q);
 }
 
 __global__ void k_br_redo_store(const BrRedo *__restrict__ redo, int n, const double *__restrict__ v,
@@ -1343,6 +1345,8 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
   // the contraction takes orbitals that reach past the chains' start and end
   // on the grid; any other set is evaluated term by term
   const bool plain = m0 >= BR_MIN_MF && maxm <= g.n;
+  bool moving = false;  // some pair is at a frequency
+  for (const BrRow &r : rows) moving |= r.a && std::fabs(r.w) >= 1.0e-10;
 
   // the operators, forward vectors and class sums need no buckets: they run
   // while the host builds these from the heads
@@ -1435,8 +1439,6 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
     ::gg::note_launch();
 
     // buckets: the columns of each (set, k) by (MTP, head as a source)
-    bool moving = false;
-    for (const BrRow &r : rows) moving |= r.a && std::fabs(r.w) >= 1.0e-10;
     std::vector<BrBucket> bk;
     std::vector<BrEnt> ents;
     std::vector<int> cols;
@@ -1512,7 +1514,7 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
     // k_bessel ran to the longest orbital, which covers every term
     DBuf<double> dv, dout;
     DBuf<BrInt> dints;
-    const int piece = std::min(nredo, BR_REDO);
+    const int piece = std::min(nredo, BR_REDO), tsh = type == 1 || moving ? 2 : 1;
     GG_TRY(dv.alloc((size_t)4 * piece));
     GG_TRY(dout.alloc(piece));
     GG_TRY(dints.alloc(piece));
@@ -1520,7 +1522,7 @@ int run_table(gg_ctx *ctx, int type, const Plan &P, int j2max, const std::vector
     for (int done = 0; done < nredo;) {
       const int n = std::min(piece, nredo - done);
       const BrRedo *part = dredo.p + done;
-      k_br_redo<<<(4 * n + 127) / 128, 128, 0, s>>>(type, part, n, drows.p, P.tabs(), tt, g.q, dv.p, dints.p);
+      k_br_redo<<<((n << tsh) + 127) / 128, 128, 0, s>>>(type, tsh, part, n, drows.p, P.tabs(), tt, g.q, dv.p, dints.p);
       ::gg::note_launch();
       k_breit_combine<<<(n + 255) / 256, 256, 0, s>>>(dints.p, n, dv.p, dout.p);
       ::gg::note_launch();
