@@ -91,6 +91,17 @@ __device__ double quad_seq(double *TA, int mtp, const double *R, const double *R
 constexpr size_t SMEM_PLAIN = 47 * 1024;
 __host__ __device__ constexpr int quad_panels(int np) { return np / 4 + 4; }
 
+// QUAD's test of a head index (quad.f90:58-63), TA(i) != 0 and not TA(i+1)/TA(i)
+// <= 0, without the division: ordinary numbers whose ratio does not underflow
+// pass when their signs are equal. A ratio that is not a number passes, as in
+// quad_seq.
+__device__ __forceinline__ bool quad_head(double tai, double taip1) {
+  const int h0 = __double2hiint(tai), h1 = __double2hiint(taip1);
+  const int e0 = h0 >> 20 & 0x7ff, e1 = h1 >> 20 & 0x7ff;
+  if (e0 > 0 && e0 < 0x7ff && e1 > 0 && e1 < 0x7ff && e1 - e0 > -1000) return (h0 ^ h1) >= 0;
+  return !(fabs(tai) <= 0.0) && !(taip1 / tai <= 0.0);
+}
+
 // quad_seq by the lanes of a warp, the same value to the bit: the head index
 // by ballot, the four-point panels (quad.f90:94-99) one per lane into `panel`
 // (quad_panels(np) doubles), then lane 0 adds them in order, the only serial
@@ -965,8 +976,8 @@ __global__ void k_quad_items(const QuadItem *__restrict__ items, int nitems,
 }
 
 // The same QUAD for the table's items, one warp per integral with the work
-// spread over the lanes: the head index (first i in [2, MTP-1] with
-// TA(i) != 0 and TA(i+1)/TA(i) > 0) by ballot, the 4-point panel sums
+// spread over the lanes: the head index (first i in [2, MTP-1] that passes
+// quad_head) by ballot, the 4-point panel sums
 // (quad.f90:94-99) split over the lanes and combined by a fixed butterfly,
 // so the result is deterministic. Only the order of the panel sum differs
 // from quad_seq (a few ulps of the sum of |terms|). TA(i) = D(i) Y(i) from the
@@ -996,8 +1007,7 @@ __global__ void k_quad_table(const QuadItem *__restrict__ items, const int *__re
         const int i = i0 + lane;
         bool hit = false;
         if (i <= w.mtp - 1) {
-          const double t0 = D[i] * Y[i], t1 = D[i + 1] * Y[i + 1];
-          hit = (t0 > 0.0 && t1 > 0.0) || (t0 < 0.0 && t1 < 0.0);
+          hit = quad_head(D[i] * Y[i], D[i + 1] * Y[i + 1]);
         }
         const unsigned bal = __ballot_sync(0xffffffffu, hit);
         if (bal) head = i0 + __ffs(bal) - 1;
